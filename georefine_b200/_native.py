@@ -22,7 +22,7 @@ VOIDP = ctypes.c_void_p
 
 EXPORTS = (
     "bcx_encode", "bcx_frequencies", "bcx_decode", "bcx_decode_compact", "bcx_free", "bcx_pack6", "bcx_unpack6",
-    "bcx_checkpoint", "grb_bctx_build_lookup", "grb_bctx_decode_words", "bxr_build", "bxr_free", "bxr_decode_host",
+    "bcx_checkpoint", "grb_bctx_build_lookup", "grb_bctx_decode_words", "grb_bctx_pack_tables", "grb_bctx_decode_packed", "bxr_build", "bxr_free", "bxr_decode_host",
     "bxr_validate", "bxr_layout_version", "grb_bxr_workspace_bytes", "grb_bxr_decode", "grb_bxr_gemm", "grb_bxr_gemv", "grb_bxr_gemm_next", "grb_kernel_attributes",
     "grb_static_scratch_bytes", "grb_bxr_gemv_static", "grb_dense_gemv_bf16", "grb_peer_control_bytes", "grb_peer_enable", "grb_peer_allreduce_bf16",
     "grb_peer_alloc", "grb_peer_free", "grb_peer_open", "grb_peer_close",
@@ -57,6 +57,10 @@ class BctxTensor(ctypes.Structure):
                 ("main_bucket_shift", ctypes.c_uint32), ("residual_bucket_shift", ctypes.c_uint32)]
 
 
+class BctxPacked(ctypes.Structure):
+    _fields_ = [("tables", VOIDP), ("shape", ctypes.c_uint32 * 5)]
+
+
 class AttnStep(ctypes.Structure):
     _fields_ = [("qkv", VOIDP), ("ldq", ctypes.c_int64), ("cos_table", VOIDP), ("sin_table", VOIDP), ("row_seq", VOIDP),
                 ("row_pos", VOIDP), ("page_table", VOIDP), ("max_pages", ctypes.c_uint32), ("k_pages", VOIDP), ("v_pages", VOIDP),
@@ -78,6 +82,8 @@ def _declare(lib):
     lib.bcx_checkpoint.argtypes = [U8P, sz, u64, u32, u32, U8P, U8P, u32, u32, u32, U16P, U32P, u32, U32P, U32P, U16P]
     lib.grb_bctx_build_lookup.argtypes = [U32P, u32, u32, U32P, U16P]
     lib.grb_bctx_decode_words.argtypes = [ctypes.POINTER(BctxTensor), VOIDP, u64, VOIDP, VOIDP, VOIDP]
+    lib.grb_bctx_pack_tables.argtypes = [U32P, u32, U32P, u32, ctypes.POINTER(u32 * 5), U8P]
+    lib.grb_bctx_decode_packed.argtypes = [ctypes.POINTER(BctxTensor), ctypes.POINTER(BctxPacked), VOIDP, u64, VOIDP, VOIDP, VOIDP, VOIDP]
     lib.bxr_build.argtypes = [U16P, u32, u32, u32, u32, u32, U8P, ctypes.POINTER(U8P), ctypes.POINTER(u64)]
     lib.bxr_free.argtypes = [VOIDP]
     lib.bxr_free.restype = None

@@ -6,7 +6,9 @@
 //   main     = exponent(8) << 2 | mantissa[6:5]      10 bits, vocabulary 1024
 //   residual = sign << 5 | mantissa[4:0]              6 bits, vocabulary 64
 #pragma once
+#include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 namespace grb {
@@ -71,6 +73,108 @@ class Model {
   std::vector<uint32_t> cum_;
   std::vector<uint16_t> bucket_;
   std::vector<uint8_t> live_;
+};
+
+// The models of a frame packed for shared memory (csrc/bctx_packed.cuh).  A context has few live symbols (60 to 80 of 1024
+// on Gaussian weights), so its model is: u8 rank[65536 >> shift], the rank among the live symbols of the one that owns each
+// bucket's first slot; and entries of 8 bytes in rank order, {first slot u16 | frequency - 1 u16, what the symbol means
+// u32}.  An entry that matches any slot follows the last one where there is room and the last one matches everything up to
+// the table's end, so that a forward scan always ends.
+// Layout: the main contexts at multiples of ctx_bytes; from resid_at on the residual contexts (coded residuals only) of the
+// main symbols that occur anywhere, each as long as its live symbols need.  The meaning of a main entry is
+// symbol << 5 | (offset of its residual context from resid_at) / 8 << 16, that of a residual entry its bits of the word.
+struct PackedShape {
+  uint32_t shift, ctx_bytes, resid_shift, resid_at, bytes;
+};
+
+class PackedTables {
+ public:
+  // resid_freq == nullptr: raw residuals.  False when the frequencies are invalid.
+  bool load(const uint32_t* main_freq, uint32_t nctx, const uint32_t* resid_freq) {
+    main_ = main_freq;
+    resid_ = resid_freq;
+    nctx_ = nctx;
+    ranks_ = 1;
+    occurs_.assign(1024, 0);
+    for (uint32_t cx = 0; cx < nctx; ++cx) {
+      uint32_t live = 0;
+      if (!count(main_freq + size_t(cx) * 1024, 1024, live)) return false;
+      for (uint32_t s = 0; s < 1024; ++s) occurs_[s] |= main_freq[size_t(cx) * 1024 + s] != 0;
+      ranks_ = std::max(ranks_, live);
+    }
+    resid_live_.assign(1024, 0);
+    resid_entries_ = resid_contexts_ = 0;
+    for (uint32_t s = 0; resid_ && s < 1024; ++s) {
+      if (!count(resid_ + size_t(s) * 64, 64, resid_live_[s])) return false;
+      if (!occurs_[s]) continue;
+      if (!resid_live_[s]) return false;      // a main symbol that occurs has a residual
+      ++resid_contexts_;
+      resid_entries_ += resid_live_[s];
+    }
+    return true;
+  }
+  // The bucket widths with the fewest scan steps whose tables fit `limit` bytes; false when none do.
+  bool shape(uint32_t limit, PackedShape& out) const {
+    if (ranks_ > 255) return false;
+    uint64_t best = ~uint64_t(0);
+    for (uint32_t ms = 4; ms <= 8; ++ms)
+      for (uint32_t rs = resid_ ? 4 : 9; rs <= 9; ++rs) {
+        const uint64_t ctx = ((65536u >> ms) + ranks_ * 8 + 15) & ~15u, resid_at = ctx * nctx_;
+        const uint64_t resid = resid_ ? uint64_t(resid_contexts_) * (65536u >> rs) + uint64_t(resid_entries_) * 8 : 0;
+        const uint64_t bytes = (resid_at + resid + 15) & ~uint64_t(15), cost = (uint64_t(ranks_) << ms) + (resid_ ? uint64_t(64) << rs : 0);
+        if (bytes > limit || resid > 65535u * 8 || cost >= best) continue;
+        best = cost;
+        out = PackedShape{ms, uint32_t(ctx), rs, uint32_t(resid_at), uint32_t(bytes)};
+      }
+    return best != ~uint64_t(0);
+  }
+  void write(const PackedShape& p, uint8_t* image) const {
+    std::memset(image, 0, p.bytes);
+    std::vector<uint32_t> resid_of(1024, 0);
+    uint32_t at = 0;
+    for (uint32_t s = 0; resid_ && s < 1024; ++s) {
+      if (!occurs_[s]) continue;
+      resid_of[s] = at;
+      context(resid_ + size_t(s) * 64, 64, p.resid_shift, resid_live_[s], image + p.resid_at + at,
+              [](uint32_t r) { return (r & 31u) | (r & 32u) << 10; });
+      at += (65536u >> p.resid_shift) + resid_live_[s] * 8;
+    }
+    for (uint32_t cx = 0; cx < nctx_; ++cx)
+      context(main_ + size_t(cx) * 1024, 1024, p.shift, ranks_, image + size_t(cx) * p.ctx_bytes,
+              [&](uint32_t s) { return s << 5 | (resid_of[s] >> 3) << 16; });
+  }
+
+ private:
+  static bool count(const uint32_t* freq, uint32_t vocab, uint32_t& live) {
+    uint64_t sum = 0;
+    live = 0;
+    for (uint32_t s = 0; s < vocab; ++s) { sum += freq[s]; live += freq[s] != 0; }
+    return sum == 0 || sum == 65536u;
+  }
+  template <class Meaning>
+  static void context(const uint32_t* freq, uint32_t vocab, uint32_t shift, uint32_t ranks, uint8_t* at, Meaning meaning) {
+    uint8_t* entry = at + (65536u >> shift);
+    uint32_t r = 0, run = 0;
+    auto put = [&](uint32_t lo, uint32_t last, uint32_t what) {
+      const uint32_t words[2] = {lo | last << 16, what};
+      std::memcpy(entry + size_t(r++) * 8, words, 8);
+    };
+    const uint32_t round = (1u << shift) - 1;
+    for (uint32_t s = 0; s < vocab; ++s) {
+      const uint32_t f = freq[s];
+      if (!f) continue;
+      const uint32_t first = (run + round) >> shift, end = (run + f + round) >> shift;   // buckets whose first slot is the symbol's
+      std::memset(at + first, int(r), end - first);
+      put(run, f - 1, meaning(s));
+      run += f;
+    }
+    while (r < ranks) put(0, 65535, 0);
+  }
+
+  const uint32_t *main_ = nullptr, *resid_ = nullptr;
+  uint32_t nctx_ = 0, ranks_ = 0, resid_entries_ = 0, resid_contexts_ = 0;
+  std::vector<uint8_t> occurs_;
+  std::vector<uint32_t> resid_live_;
 };
 
 }  // namespace grb

@@ -9,6 +9,7 @@
 
 #include "../../include/georefine_b200.h"
 #include "bctx_decode.cuh"
+#include "bctx_packed.cuh"
 #include "bxr_kernels.cuh"
 #include "bxw_kernels.cuh"
 #include "bxq_kernels.cuh"
@@ -233,6 +234,30 @@ int device_sm_count(int dev) {
   return sms[dev];
 }
 
+template <bool ALIGNED, int RESIDUAL>
+int packed_launch(BctxPackedArgs a, int sms, int dev, cudaStream_t stream) {
+  static std::once_flag once[64];
+  static int prepared[64];
+  if (dev < 0 || dev >= 64) return GRB_ERR_UNSUPPORTED;
+  std::call_once(once[dev], [&] {
+    prepared[dev] = cuda_status(cudaFuncSetAttribute(bctx_packed_kernel<ALIGNED, RESIDUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPackedSmemMax)));
+  });
+  if (prepared[dev]) return prepared[dev];
+  constexpr uint32_t kLane = kPackedLaneBytes<RESIDUAL>;
+  const uint64_t fixed = kPackedTablesAt + uint64_t(a.table_bytes) + packed_class_bytes(a.cols);
+  if (fixed + 32 * kLane > kPackedSmemMax) return GRB_ERR_UNSUPPORTED;
+  // A CTA has to bring the tables in before it starts: no more CTAs than give each four warps of lanes, then equal shares,
+  // in as few and as equal rounds as shared memory allows.
+  const uint64_t ctas = std::min<uint64_t>(uint64_t(sms), (a.count + 127) / 128);
+  a.per_cta = uint32_t(((a.count + ctas - 1) / ctas + 31) & ~uint64_t(31));
+  const uint32_t most = std::min(kPackedThreads<RESIDUAL>, uint32_t((kPackedSmemMax - fixed) / kLane) & ~31u);
+  const uint32_t rounds = (a.per_cta + most - 1) / most;
+  const uint32_t threads = ((a.per_cta + rounds - 1) / rounds + 31) & ~31u;
+  const uint32_t grid = uint32_t((a.count + a.per_cta - 1) / a.per_cta);
+  bctx_packed_kernel<ALIGNED, RESIDUAL><<<grid, threads, uint32_t(fixed) + threads * kLane, stream>>>(a);
+  return cuda_status(cudaGetLastError());
+}
+
 template <int G>
 int attn_part_launch(const AttnArgs& a, cudaStream_t stream) {
   static std::once_flag once[64];
@@ -291,6 +316,72 @@ int grb_bctx_decode_words(const grb_bctx_tensor* t, const int64_t* block_ids, ui
   const unsigned grid = unsigned((count + 63) / 64);
   bctx_decode_kernel<<<grid, 64, 0, stream>>>(a);
   return cuda_status(cudaGetLastError());
+}
+
+int grb_bctx_decode_packed(const grb_bctx_tensor* t, const grb_bctx_packed* p, const int64_t* row_ids, uint64_t count,
+                           uint16_t* out, uint32_t* status, uint32_t* host_flags, void* cuda_stream) {
+  if (!t || !p || !out || !status || !t->row_class || !t->col_class || !t->main_stream || !t->main_states || !t->main_offsets ||
+      !t->residual_stream || !t->rows || !t->cols || !t->stride || t->n != uint64_t(t->rows) * t->cols || !p->tables)
+    return GRB_ERR_ARGUMENT;
+  const bool coded = t->mode == 128;
+  if ((t->mode != 0 && !coded) || (coded && (!t->residual_states || !t->residual_offsets))) return GRB_ERR_ARGUMENT;
+  const uint32_t contexts = t->nr * t->nc, shift = p->shape[0], ctx_bytes = p->shape[1], bytes = p->shape[4];
+  if (shift < 4 || shift > 8 || !contexts || (ctx_bytes & 15) || (bytes & 15) || ctx_bytes < (65536u >> shift) + 8 ||
+      p->shape[3] != uint64_t(contexts) * ctx_bytes || p->shape[3] > bytes || p->shape[2] < 4 || p->shape[2] > 9)
+    return GRB_ERR_ARGUMENT;
+  if ((t->stride & 15) || t->cols < 16 || t->cols > kPackedColsMax || t->main_bytes >= 0xFFFFFF00ull ||
+      (coded && t->residual_bytes >= 0xFFFFFF00ull) || t->n > 0xFFFFFFFFull)
+    return GRB_ERR_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(p->tables) | (coded ? 0 : reinterpret_cast<uintptr_t>(t->residual_stream)) | reinterpret_cast<uintptr_t>(out)) & 15)
+    return GRB_ERR_ARGUMENT;
+  if (count == 0) return GRB_OK;
+  // rows that start on block boundaries touch cols / stride blocks; others up to one more at either end
+  const uint32_t per_row = t->cols % t->stride == 0 ? t->cols / t->stride : (t->cols - 1) / t->stride + 2;
+  if (row_ids) {
+    if (count > (uint64_t(1) << 31) / per_row) return GRB_ERR_ARGUMENT;
+    count *= per_row;
+  } else if (count > (t->n + t->stride - 1) / t->stride) {
+    return GRB_ERR_ARGUMENT;
+  }
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return cuda_status(e);
+  const int sms = device_sm_count(dev);
+  if (sms <= 0) return GRB_ERR_CUDA;
+  BctxPackedArgs a{};
+  a.tables = p->tables;
+  a.table_bytes = bytes;
+  a.shift = shift;
+  a.ctx_bytes = ctx_bytes;
+  a.resid_shift = p->shape[2];
+  a.resid_at = p->shape[3];
+  a.bytes = t->main_stream;
+  a.size = uint32_t(t->main_bytes);
+  a.states = t->main_states;
+  a.offsets = t->main_offsets;
+  a.raw = t->residual_stream;
+  a.raw_size = t->residual_bytes;
+  a.raw_states = t->residual_states;
+  a.raw_offsets = t->residual_offsets;
+  a.row_class = t->row_class;
+  a.col_class = t->col_class;
+  a.n = t->n;
+  a.rows = t->rows;
+  a.cols = t->cols;
+  a.nr = t->nr;
+  a.nc = t->nc;
+  a.stride = t->stride;
+  a.ids = reinterpret_cast<const long long*>(row_ids);
+  a.per_row = per_row;
+  a.count = count;
+  a.out = out;
+  a.status = status;
+  a.host_flags = host_flags;
+  const auto stream = static_cast<cudaStream_t>(cuda_stream);
+  const bool wide = (t->stride & 63) == 0, aligned = (t->cols & 15) == 0;
+  if (coded) return aligned ? packed_launch<true, kCoded>(a, sms, dev, stream) : packed_launch<false, kCoded>(a, sms, dev, stream);
+  if (wide) return aligned ? packed_launch<true, kRaw64>(a, sms, dev, stream) : packed_launch<false, kRaw64>(a, sms, dev, stream);
+  return aligned ? packed_launch<true, kRaw16>(a, sms, dev, stream) : packed_launch<false, kRaw16>(a, sms, dev, stream);
 }
 
 int grb_bxr_decode(const void* image, const bxr_header* h, uint16_t* out, uint32_t* status, void* cuda_stream) {

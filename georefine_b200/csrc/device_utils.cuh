@@ -140,6 +140,14 @@ __device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
 }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// 16-byte asynchronous copy global -> shared of the calling thread; the last 16 - src_bytes bytes are zero-filled.
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 // ---- shared memory by address -----------------------------------------------------------------------
 __device__ __forceinline__ uint32_t lds32(uint32_t a) {
   uint32_t v;

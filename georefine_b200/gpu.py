@@ -112,6 +112,33 @@ def _lookup_tables(freq):
     return cum, np.ascontiguousarray(bucket[:, ::1 << (shift - 4)]), shift
 
 
+def _packed_tables(indexed, stride):
+    """A frame's models packed for the shared memory of one SM and their descriptor, or None when the frame is one the packed
+    kernel does not take (see ``grb_bctx_decode_packed``)."""
+    cols = indexed["shape"][1]
+    if stride % 16 or not 16 <= cols <= 24576:
+        return None
+    # what shared memory leaves beside the column classes and the stream rings of half a 4096 x 4096 frame's lanes (448 of
+    # them with two streams, 896 with one)
+    limit = 232448 - 128 - 448 * 128 - (cols + cols // 8 + 64)
+    main = np.ascontiguousarray(indexed["main_freq"], dtype="<u4")
+    residual = _native.U32P()
+    if "residual_freq" in indexed:
+        residual_freq = np.ascontiguousarray(indexed["residual_freq"], dtype="<u4")
+        residual = _p(residual_freq, ctypes.c_uint32)
+    packed, pack = _native.BctxPacked(), _native.lib().grb_bctx_pack_tables
+    args = (_p(main, ctypes.c_uint32), main.shape[0], residual, limit, ctypes.byref(packed.shape))
+    status = pack(*args, None)
+    if status == 4:
+        return None
+    if not status:
+        image = np.empty(packed.shape[4], dtype=np.uint8)
+        status = pack(*args, _p(image, ctypes.c_uint8))
+    if status:
+        raise base.CodecError(f"invalid frequency tables ({status})")
+    return image, packed
+
+
 class CudaContextTensor:
     """A BCTX frame resident on one GPU: the unchanged streams with their restart index (for ``decode`` and
     ``gather_rows``) and, for rank-2 weights, the resident image the fused linear streams.
@@ -150,14 +177,23 @@ class CudaContextTensor:
         # every array of the index goes to the device under its own name; coded streams get their lookup tables
         self.buffers = {name: torch.from_numpy(array).to(self.device) for name, array in indexed.items() if isinstance(array, np.ndarray)}
         self._bucket_shift = {}
+        self._packed = None
+        if self.mode != 1 and (packed := _packed_tables(indexed, walk_stride)) is not None:
+            self.buffers["packed"] = torch.from_numpy(packed[0]).to(self.device)
+            self._packed = packed[1]
+            self._packed.tables = self.buffers["packed"].data_ptr()
         for kind in ("main", "residual"):
             table = indexed.get(kind + "_freq")
-            if table is not None:
+            if table is not None and self._packed is None:
                 cum, bucket, shift = _lookup_tables(table)
                 self.buffers[kind + "_cum"] = torch.from_numpy(cum).to(self.device)
                 self.buffers[kind + "_bucket"] = torch.from_numpy(bucket).to(self.device)
                 self._bucket_shift[kind] = shift
         self.error = torch.zeros((), device=self.device, dtype=torch.int32)
+        self._error_clear = True
+        # outcome of a checked decode, written by the kernel into host memory: {status bits, an index was out of range}
+        self._flags = torch.zeros(2, dtype=torch.int32).pin_memory()
+        self._flag_words = self._flags.numpy()
         self.resident = None
         if fused and words is not None:
             self.resident = ResidentWeight.from_words(words, device=self.device, source_sha256=bytes.fromhex(self.source_sha256),
@@ -175,14 +211,50 @@ class CudaContextTensor:
         t.row_class, t.col_class = b["rows"].data_ptr(), b["columns"].data_ptr()
         t.main_stream, t.main_bytes = b["main_stream"].data_ptr(), b["main_stream"].numel()
         t.main_states, t.main_offsets = b["main_states"].data_ptr(), b["main_offsets"].data_ptr()
-        t.main_cum, t.main_bucket = b["main_cum"].data_ptr(), b["main_bucket"].data_ptr()
-        t.main_bucket_shift = self._bucket_shift["main"]
+        if self._packed is None:
+            t.main_cum, t.main_bucket = b["main_cum"].data_ptr(), b["main_bucket"].data_ptr()
+            t.main_bucket_shift = self._bucket_shift["main"]
         t.residual_stream, t.residual_bytes = b["residual_stream"].data_ptr(), b["residual_stream"].numel()
         if self.mode == 128:
             t.residual_states, t.residual_offsets = b["residual_states"].data_ptr(), b["residual_offsets"].data_ptr()
-            t.residual_cum, t.residual_bucket = b["residual_cum"].data_ptr(), b["residual_bucket"].data_ptr()
-            t.residual_bucket_shift = self._bucket_shift["residual"]
+            if self._packed is None:
+                t.residual_cum, t.residual_bucket = b["residual_cum"].data_ptr(), b["residual_bucket"].data_ptr()
+                t.residual_bucket_shift = self._bucket_shift["residual"]
         return t
+
+    def _decode_packed(self, ids=None, *, check):
+        """All blocks, or the rows ``ids``, through the packed tables.  The host waits when ``check`` asks for the outcome or
+        ``ids`` have to be known to be rows of the tensor."""
+        import torch
+
+        if ids is None:
+            count = -(-self.n // self.walk_stride)
+            result = torch.empty(count * self.walk_stride, device=self.device, dtype=torch.bfloat16)
+        else:
+            count = ids.numel()
+            result = torch.empty((*ids.shape, self.shape[1]), device=self.device, dtype=torch.bfloat16)
+        if not self._error_clear:
+            self.error.zero_()
+        wait = check or ids is not None
+        flags = self._flag_words
+        if wait:
+            flags[:] = 0
+        self._error_clear = wait        # unknown until somebody waits for the launch
+        with torch.cuda.device(self.device):
+            stream = torch.cuda.current_stream()
+            status = _native.lib().grb_bctx_decode_packed(
+                ctypes.byref(self._descriptor), ctypes.byref(self._packed), None if ids is None else ids.data_ptr(), count,
+                result.data_ptr(), self.error.data_ptr(), self._flags.data_ptr() if wait else None, stream.cuda_stream)
+        _native.check(status, "grb_bctx_decode_packed")
+        if wait:
+            stream.synchronize()
+            if flags[0] or flags[1]:
+                self._error_clear = False
+                if flags[1]:
+                    raise IndexError("embedding row outside tensor")
+                if check:
+                    raise base.CodecError("CUDA decoder checkpoint mismatch")
+        return result
 
     def _decode_blocks(self, blocks=None, *, check=True):
         import torch
@@ -195,6 +267,7 @@ class CudaContextTensor:
             count, ids = blocks.numel(), blocks.data_ptr()
         result = torch.empty(count * walk, device=self.device, dtype=torch.uint16)
         self.error.zero_()
+        self._error_clear = False
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream().cuda_stream
             status = _native.lib().grb_bctx_decode_words(ctypes.byref(self._descriptor), ids, count, result.data_ptr(),
@@ -210,18 +283,22 @@ class CudaContextTensor:
 
         if self.mode == 1:
             return self.buffers["raw"].view(torch.bfloat16).reshape(self.shape)
+        if self._packed is not None:
+            return self._decode_packed(check=check)[:self.n].reshape(self.shape)
         return self._decode_blocks(check=check)[:self.n].reshape(self.shape)
 
     def gather_rows(self, ids, *, check=True):
-        """Rows ``ids`` (any shape) as BF16 [..., cols].  When a row is a whole number of restart blocks only the blocks of
-        the requested rows are decoded; otherwise (raw frames, strides that do not divide the row) the tensor is decoded
-        once and indexed."""
+        """Rows ``ids`` (any shape) as BF16 [..., cols].  Only the blocks of the requested rows are decoded when the frame has
+        packed tables or a row is a whole number of restart blocks; otherwise (raw frames, strides that do not divide the
+        row) the tensor is decoded once and indexed."""
         import torch
 
         rows, cols = self.shape
         ids = ids.to(device=self.device, dtype=torch.int64)
         if ids.numel() == 0:
             return torch.empty((*ids.shape, cols), device=self.device, dtype=torch.bfloat16)
+        if self._packed is not None:
+            return self._decode_packed(ids.contiguous(), check=check)
         lowest, highest = torch.aminmax(ids)
         if int(lowest) < 0 or int(highest) >= rows:
             raise IndexError("embedding row outside tensor")

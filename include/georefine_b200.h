@@ -126,6 +126,28 @@ typedef struct grb_bctx_tensor {
 int grb_bctx_decode_words(const grb_bctx_tensor* tensor, const int64_t* block_ids, uint64_t count, uint16_t* out,
                           uint32_t* status, void* cuda_stream);
 
+/* A frame's models packed for the shared memory of one SM (csrc/bcx_model.h, PackedShape): shape = {log2 slots per main
+ * bucket, bytes per main context, log2 slots per residual bucket, offset of the residual contexts, bytes}.  residual_freq:
+ * the tables of a mode 128 frame, NULL for raw residuals.  image == NULL computes the shape only.  0 ok, 1 arguments,
+ * 2 invalid tables, 4 they do not fit `limit` bytes: use grb_bctx_decode_words.  The kernel keeps them in the 227 KB of an
+ * SM's shared memory next to 64 bytes per lane and stream and 9/8 bytes per column. */
+int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t limit, uint32_t shape[5],
+                         uint8_t* image);
+
+typedef struct grb_bctx_packed {
+  const uint8_t* tables;      /* device, 16-byte aligned: the image grb_bctx_pack_tables wrote */
+  uint32_t shape[5];
+} grb_bctx_packed;
+
+/* grb_bctx_decode_words for frames with packed tables, strides that are multiples of 16 and 16 to 24576 columns
+ * (GRB_ERR_UNSUPPORTED otherwise); the *_cum and *_bucket tables are not read.  row_ids == NULL decodes blocks 0..count-1
+ * and out receives count * stride words; else out receives `count` rows of the tensor, [count][cols], and a row number
+ * outside it is reported instead of followed.  host_flags (optional): two words of host memory the device can write; [0]
+ * receives the status bits of a failed block, [1] is set for a row out of range, and both stay as they are otherwise, so
+ * that a caller who has synchronised anyway reads the outcome there. */
+int grb_bctx_decode_packed(const grb_bctx_tensor* tensor, const grb_bctx_packed* packed, const int64_t* row_ids, uint64_t count,
+                           uint16_t* out, uint32_t* status, uint32_t* host_flags, void* cuda_stream);
+
 /* ---------------------------------------------------------------------------------------------------
  * 3. Resident layout (bxr_format.h) and the fused kernels.
  * ------------------------------------------------------------------------------------------------- */

@@ -1,0 +1,38 @@
+"""The shared-memory kernel for indexed decoding (csrc/bctx_packed.cuh) at the edges of its range, bit for bit (needs a B200)."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+CASES = [((16, 16), 128), ((3, 129), 16), ((257, 272), 64), ((300, 1000), 128), ((97, 4111), 1024), ((64, 4096), 48), ((7, 24576), 128),
+         ((5, 24577), 128), ((4, 15), 128)]     # the last two: one column too many, one too few for the kernel
+
+
+@pytest.mark.parametrize("shape,stride", CASES)
+@pytest.mark.parametrize("coarse", [False, True])     # True: three mantissa bits are zero, so that coded residuals (mode 128) win
+@pytest.mark.parametrize("classes", [(16, 4), (1, 1), (64, 16)])
+def test_packed_decode_and_row_gather_are_exact(orc, shape, stride, classes, coarse):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from georefine_b200 import codec
+    from georefine_b200.gpu import CudaContextTensor
+
+    words = orc.synthetic_weight_words(*shape, 3)
+    words[0, :5] = (0, 0x8000, 0x7F80, 1, 0xFFFF)             # far-off symbols: rare entries at the ends of the tables
+    if coarse:
+        words &= 0xFFF8
+    t = CudaContextTensor(codec.encode(words, row_classes=classes[0], col_classes=classes[1]), stride=stride, walk_stride=stride,
+                          device="cuda:0", fused=False)
+    assert not coarse or words.size < 20000 or t.mode == 128
+    if t.mode != 1:
+        assert (t._packed is not None) == (stride % 16 == 0 and 16 <= shape[1] <= 24576 and classes != (64, 16))
+    for check in (True, False):
+        assert np.array_equal(t.decode(check=check).view(torch.uint16).cpu().numpy(), words)
+    ids = torch.tensor([[shape[0] - 1, 0], [shape[0] // 2, 0]])
+    assert np.array_equal(t.gather_rows(ids).view(torch.uint16).cpu().numpy(), words[ids.numpy()])
+    assert int(t.error.item()) == 0
+    for wrong in (-1, shape[0]):
+        with pytest.raises(IndexError):
+            t.gather_rows(torch.tensor([0, wrong]))
+    assert np.array_equal(t.gather_rows(ids).view(torch.uint16).cpu().numpy(), words[ids.numpy()])
