@@ -58,7 +58,7 @@ class BctxTensor(ctypes.Structure):
 
 
 class BctxPacked(ctypes.Structure):
-    _fields_ = [("tables", VOIDP), ("shape", ctypes.c_uint32 * 5)]
+    _fields_ = [("tables", VOIDP), ("shape", ctypes.c_uint32 * 5), ("parts", ctypes.c_uint32), ("share", ctypes.c_uint32), ("rows_by_class", VOIDP), ("part_of", VOIDP)]
 
 
 class AttnStep(ctypes.Structure):
@@ -82,7 +82,7 @@ def _declare(lib):
     lib.bcx_checkpoint.argtypes = [U8P, sz, u64, u32, u32, U8P, U8P, u32, u32, u32, U16P, U32P, u32, U32P, U32P, U16P]
     lib.grb_bctx_build_lookup.argtypes = [U32P, u32, u32, U32P, U16P]
     lib.grb_bctx_decode_words.argtypes = [ctypes.POINTER(BctxTensor), VOIDP, u64, VOIDP, VOIDP, VOIDP]
-    lib.grb_bctx_pack_tables.argtypes = [U32P, u32, U32P, u32, ctypes.POINTER(u32 * 5), U8P]
+    lib.grb_bctx_pack_tables.argtypes = [U32P, u32, U32P, u32, u32, ctypes.POINTER(u32 * 5), U8P]
     lib.grb_bctx_decode_packed.argtypes = [ctypes.POINTER(BctxTensor), ctypes.POINTER(BctxPacked), VOIDP, u64, VOIDP, VOIDP, VOIDP, VOIDP]
     lib.bxr_build.argtypes = [U16P, u32, u32, u32, u32, u32, U8P, ctypes.POINTER(U8P), ctypes.POINTER(u64)]
     lib.bxr_free.argtypes = [VOIDP]

@@ -7,10 +7,14 @@
 // the lanes of a warp renew their windows at different steps, a warp waits for a register whichever of its lanes has a load
 // outstanding on it, and so nearly every step waits for an L2 round trip that another lane has just begun.  Here stream bytes
 // come to shared memory by asynchronous copies, which no register waits for, and everything a symbol needs is there: its
-// bucket's rank byte, the 8-byte entry (first slot, frequency, symbol), every second symbol a word of the stream.  The
-// window moves by selects, not by a branch.  A main symbol and the residual of the one before it are looked up together:
-// their chains are independent.  Raw residuals come as three 16-byte loads per 64 symbols, column classes as one 16-byte
-// load per 16.  One CTA per SM, so that the tables (150 to 170 KB at 64 contexts) come in once per SM, by one bulk copy.
+// bucket, its 8-byte entry (first slot, frequency, symbol), every second symbol a word of the stream.  The window moves by
+// selects, not by a branch; a bucket tells its two symbols apart, so that the forward scan is left to rare symbols (with one
+// rank per bucket some lane of a warp scanned at nearly every symbol).  A main symbol and the residual of the one before it
+// are looked up together: their chains are independent.  What is left is 100 instructions per warp and pair of symbols at
+// 68 % of the issue slots, the integer pipe 71 % and shared memory 70 % busy.
+// 4096 x 4096 words with coded residuals, 128 per lane: 305 us before (tables in global memory, one CTA of 64 lanes after
+// another), 118 us with the tables of all 64 contexts in shared memory (room for 14 warps), 86 us with one row class per CTA
+// (28 warps).  128 rows of 5120 words with raw residuals: 160 us before, 25 us.
 #pragma once
 #include "bctx_decode.cuh"
 
@@ -18,7 +22,7 @@ namespace grb {
 
 struct BctxPackedArgs {
   const uint8_t* tables;
-  uint32_t table_bytes, shift, ctx_bytes;    // main context c: rank bytes at c * ctx_bytes, entries behind them
+  uint32_t table_bytes, shift, ctx_bytes;    // main context c: buckets at c * ctx_bytes, entries behind them
   uint32_t resid_shift, resid_at;            // residual contexts: from resid_at on, found through the main entries
   const uint8_t* bytes;                      // main stream
   uint32_t size;
@@ -32,10 +36,12 @@ struct BctxPackedArgs {
   const uint8_t* col_class;
   uint64_t n;
   uint32_t rows, cols, nr, nc, stride;
-  const long long* ids;        // nullptr: blocks 0..count-1; else rows: lane i takes the (i % per_row)-th block that row
+  const long long* ids;        // nullptr: all blocks; else rows: lane i takes the (i % per_row)-th block that row
   uint32_t per_row;            // ids[i / per_row] touches, and writes what of it lies in the row
   uint64_t count;              // lanes' blocks
   uint32_t per_cta;
+  const uint32_t* rows_by_class;   // kByClass
+  const uint4* part_of;            // kByClass, all blocks: {row class, place of its first row, first block, end block} per CTA
   uint16_t* out;
   uint32_t* status;
   uint32_t* host_flags;        // optional, host memory: [0] = status bits, [1] = an id was out of range
@@ -48,8 +54,12 @@ constexpr uint32_t kPackedSmemMax = 232448;       // the 227 KB of shared memory
 struct Yes { static constexpr bool value = true; };
 struct No { static constexpr bool value = false; };
 enum PackedResidual { kRaw16, kRaw64, kCoded };   // raw: loaded per 16 symbols, or per 64 (strides that are multiples of 64)
-template <int RESIDUAL>
-constexpr uint32_t kPackedThreads = RESIDUAL == kCoded ? 512 : 1024;
+// kByClass: rows are whole blocks, and a CTA decodes rows of one row class - a share of them (part_of), or one row of `ids` -
+// with the tables of that class alone, so that buckets are fine and 28 warps' rings fit beside them.  Otherwise a block
+// may run from one row into the next, and a CTA keeps the tables of all classes: rows that are a multiple of 16 columns (a
+// run of 16 symbols stays in its row and its classes are one 16-byte load), or any rows.
+enum PackedRows { kByClass, kRows16, kAnyRows };
+constexpr uint32_t kPackedThreads = 1024;
 template <int RESIDUAL>
 constexpr uint32_t kPackedLaneBytes = RESIDUAL == kCoded ? 2 * kPackedRing : kPackedRing;
 
@@ -67,29 +77,24 @@ __device__ __forceinline__ void packed_report(const BctxPackedArgs& a, uint32_t 
 // of three words: w0 w1 hold the eight bytes from word `word` on, most significant first, w2 the four after them; `bit` is
 // how far the window has been used up.  Symbols are taken in pairs, at most 32 bits each pair.
 struct PackedStream {
-  const uint8_t* ring;
-  const uint8_t* pieces;   // the stream's address rounded down to 16 bytes
-  uint32_t end;            // bytes from `pieces` to the end of the stream
+  uint32_t ring;           // shared address
   uint32_t x, w0, w1, w2, ahead, bit, word, next_piece, first_take;
 
-  __device__ __forceinline__ void request() {   // the next piece; what lies beyond the stream reads as zero
-    const uint32_t from = next_piece << 4;
+  // The next piece; what lies beyond the stream reads as zero.  Pieces count from the stream's address rounded down to 16.
+  __device__ __forceinline__ void request(const uint8_t* bytes, uint32_t size) {
+    const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(bytes) & 15u), end = size + skew, from = next_piece << 4;
     const bool in = from < end;
-    cp_async_16(smem_u32(ring) + ((next_piece & 3u) << 4), pieces + (in ? from : 0u), in ? min(16u, end - from) : 0u);
+    cp_async_16(ring + ((next_piece & 3u) << 4), bytes - skew + (in ? from : 0u), in ? min(16u, end - from) : 0u);
     ++next_piece;
   }
-  __device__ __forceinline__ uint32_t ring_word(uint32_t i) const {
-    return __byte_perm(*reinterpret_cast<const uint32_t*>(ring + ((i & 15u) << 2)), 0, 0x0123);
-  }
+  __device__ __forceinline__ uint32_t ring_word(uint32_t i) const { return __byte_perm(lds32(ring + ((i & 15u) << 2)), 0, 0x0123); }
   __device__ __forceinline__ void ask(const uint8_t* bytes, uint32_t size, uint32_t offset) {
     const uint32_t skew = uint32_t(reinterpret_cast<uintptr_t>(bytes) & 15u);
-    pieces = bytes - skew;
-    end = size + skew;
     word = (offset + skew) >> 2;
     bit = ((offset + skew) & 3u) * 8;
     next_piece = word >> 2;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) request();
+    for (int k = 0; k < 4; ++k) request(bytes, size);
   }
   __device__ __forceinline__ void open() {
     w0 = ring_word(word);
@@ -100,8 +105,8 @@ struct PackedStream {
   // asked for when one has been used up, and the one asked for eight symbols ago has arrived.  64 bytes are then requested
   // from the start of the current piece on and 48 are there, so at least 33 from the read position on, of which the eight
   // symbols and the window touch at most 28.
-  __device__ __forceinline__ void refill() {
-    if (next_piece - (word >> 2) < 4) request();
+  __device__ __forceinline__ void refill(const uint8_t* bytes, uint32_t size) {
+    if (next_piece - (word >> 2) < 4) request(bytes, size);
   }
   __device__ __forceinline__ void begin_pair() {
     const bool roll = bit >= 32;
@@ -117,7 +122,7 @@ struct PackedStream {
   __device__ __forceinline__ void advance(uint32_t frequency_minus_1, uint32_t above_first, bool second) {
     const uint32_t hi = x >> 16;
     x = frequency_minus_1 * hi + (hi + above_first);
-    const uint32_t take = x < (1u << 15) ? 16u : x < (1u << 23) ? 8u : 0u;
+    const uint32_t take = (uint32_t(__clz(int(x))) - 1u) & 24u;   // 0 from 2^23 on, 8 from 2^15 on, else 16 bits
     x = __funnelshift_l(ahead, x, take);
     if (second) bit += first_take + take;
     else first_take = take;
@@ -129,41 +134,72 @@ struct PackedStream {
   }
 };
 
-// ALIGNED: rows are a multiple of 16 columns, so a run of 16 symbols stays in its row and its classes are one 16-byte load.
-template <bool ALIGNED, int RESIDUAL>
-__global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kernel(const BctxPackedArgs a) {
-  constexpr bool CODED = RESIDUAL == kCoded;
+template <int ROWS, int RESIDUAL>
+__global__ void __launch_bounds__(kPackedThreads, 1) bctx_packed_kernel(const BctxPackedArgs a) {
+  constexpr bool CODED = RESIDUAL == kCoded, ALIGNED = ROWS != kAnyRows, BY_CLASS = ROWS == kByClass;
   extern __shared__ __align__(128) uint8_t packed_smem[];
-  const uint8_t* const tables = packed_smem + kPackedTablesAt;
-  uint8_t* const rings = packed_smem + kPackedTablesAt + a.table_bytes;
-  uint8_t* const classes = rings + blockDim.x * kPackedLaneBytes<RESIDUAL>;
-  const uint32_t bar = smem_u32(packed_smem);
+  const uint32_t main_bytes = BY_CLASS ? a.nc * a.ctx_bytes : a.resid_at, resid_bytes = a.table_bytes - a.resid_at;
+  const uint32_t bar = smem_u32(packed_smem), tables = bar + kPackedTablesAt, rtables = tables + main_bytes, rings = rtables + resid_bytes;
+  const uint32_t classes = rings + blockDim.x * kPackedLaneBytes<RESIDUAL>;
+  uint4 part = {0, 0, 0, 0};
+  uint64_t lane_begin = uint64_t(blockIdx.x) * a.per_cta, lane_end = min(a.count, lane_begin + a.per_cta);
+  if (BY_CLASS) {
+    if (a.ids) {
+      const long long id = a.ids[blockIdx.x];
+      if (id < 0 || id >= (long long)(a.rows)) {
+        if (threadIdx.x == 0) packed_report(a, kStatusBadArgument, true);
+        return;
+      }
+      part.x = __ldg(a.row_class + id);
+    } else {
+      part = __ldg(a.part_of + blockIdx.x);
+      lane_begin = part.z;
+      lane_end = part.w;
+    }
+    if (part.x >= a.nr) {
+      if (threadIdx.x == 0) packed_report(a, kStatusBadSymbol, false);
+      part.x = 0;
+    }
+  }
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     mbar_fence_init();
     fence_proxy_async_smem();
-    mbar_arrive_expect_tx(bar, a.table_bytes);
-    bulk_g2s(bar + kPackedTablesAt, a.tables, a.table_bytes, bar);
+    mbar_arrive_expect_tx(bar, main_bytes + resid_bytes);
+    bulk_g2s(tables, a.tables + size_t(part.x) * main_bytes, main_bytes, bar);
+    if (resid_bytes) bulk_g2s(rtables, a.tables + a.resid_at, resid_bytes, bar);
   }
-  // labels outside the model are flagged here, once, and read as class 0
-  for (uint32_t c = threadIdx.x; c < a.cols + 16; c += blockDim.x) {
-    const uint32_t cls = __ldg(a.col_class + (c < a.cols ? c : (c - a.cols) % a.cols));
-    if (cls >= a.nc) packed_report(a, kStatusBadSymbol, false);
-    classes[packed_class_at(c)] = uint8_t(cls < a.nc ? cls : 0);
+  // Labels outside the model are flagged here, once, and read as the last class.
+  const bool wide_classes = (a.cols & 15u) == 0 && (reinterpret_cast<uintptr_t>(a.col_class) & 15u) == 0;
+  const uint32_t nc4 = a.nc * 0x01010101u;
+  for (uint32_t c = threadIdx.x * (wide_classes ? 16 : 1); c < a.cols + 16; c += blockDim.x * (wide_classes ? 16 : 1)) {
+    const uint8_t* const src = a.col_class + (c < a.cols ? c : (c - a.cols) % a.cols);
+    if (wide_classes) {
+      uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+      if (__vcmpgeu4(v.x, nc4) | __vcmpgeu4(v.y, nc4) | __vcmpgeu4(v.z, nc4) | __vcmpgeu4(v.w, nc4)) {
+        packed_report(a, kStatusBadSymbol, false);
+        const uint32_t last = nc4 - 0x01010101u;
+        v = make_uint4(__vminu4(v.x, last), __vminu4(v.y, last), __vminu4(v.z, last), __vminu4(v.w, last));
+      }
+      sts128(classes + packed_class_at(c), v);
+    } else {
+      const uint32_t cls = __ldg(src);
+      if (cls >= a.nc) packed_report(a, kStatusBadSymbol, false);
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(classes + packed_class_at(c)), "r"(min(cls, a.nc - 1)) : "memory");
+    }
   }
   __syncthreads();
-  if (!mbar_wait(bar, 0)) {
-    if (threadIdx.x == 0) packed_report(a, kStatusTimeout, false);
-    return;
-  }
-  const uint32_t shift = a.shift, rank_bytes = 65536u >> shift, rshift = a.resid_shift, rrank_bytes = 65536u >> rshift;
-  const uint8_t* const rtables = tables + a.resid_at;
+  const uint32_t shift = a.shift, bucket_bytes = 131072u >> shift, place = (1u << shift) - 1;
+  const uint32_t rshift = a.resid_shift, rbucket_bytes = 131072u >> rshift, rplace = (1u << rshift) - 1;
   const uint64_t blocks_total = (a.n + a.stride - 1) / a.stride;
-  const uint64_t lane_end = min(a.count, (uint64_t(blockIdx.x) + 1) * a.per_cta);
-  for (uint64_t i = uint64_t(blockIdx.x) * a.per_cta + threadIdx.x; i < lane_end; i += blockDim.x) {
+  for (uint64_t i = lane_begin + threadIdx.x; i < lane_end; i += blockDim.x) {
     uint64_t block = i;
-    uint16_t* out = a.out + i * a.stride;         // where the block's word 0 goes
-    uint32_t keep_from = 0, keep_to = a.stride;   // words of the block that are wanted
+    uint32_t keep_from = 0, keep_to = a.stride;   // words of the block that are wanted (kByClass: all)
+    if (BY_CLASS && !a.ids) {
+      const uint32_t q = uint32_t(i) / a.per_row;
+      block = uint64_t(__ldg(a.rows_by_class + part.y + q)) * a.per_row + (uint32_t(i) - q * a.per_row);
+    }
+    uint16_t* out = a.out + block * a.stride;     // where the block's word 0 goes
     if (a.ids) {
       const uint64_t q = i / a.per_row;
       const long long id = a.ids[q];
@@ -175,14 +211,14 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
       block = begin / a.stride + (i - q * a.per_row);
       const uint64_t first = block * a.stride;
       if (first >= begin + a.cols) continue;
-      keep_from = first < begin ? uint32_t(begin - first) : 0u;
-      keep_to = uint32_t(min(uint64_t(a.stride), begin + a.cols - first));
+      if (!BY_CLASS) keep_from = first < begin ? uint32_t(begin - first) : 0u;
+      if (!BY_CLASS) keep_to = uint32_t(min(uint64_t(a.stride), begin + a.cols - first));
       out = a.out + (q * a.cols + (first - begin));
     }
     const bool has_next = block + 1 < blocks_total;
     PackedStream s, t;
-    s.ring = rings + threadIdx.x * kPackedLaneBytes<RESIDUAL>;
-    t.ring = s.ring + kPackedRing;
+    s.ring = rings + threadIdx.x * kPackedRing;                // each kind of ring together: lanes 64 bytes apart share banks
+    t.ring = s.ring + blockDim.x * kPackedRing;                // less than lanes 128 bytes apart
     s.x = a.states[block];
     s.ask(a.bytes, a.size, a.offsets[block]);
     if (CODED) {
@@ -195,44 +231,46 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
     const uint32_t steps = uint32_t(min(uint64_t(a.stride), a.n - start));
     const bool wide_out = (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
     uint32_t bad = 0;
-    auto row_tables = [&](uint32_t r) {   // offset of the tables of row r's class, column class 0
+    auto row_tables = [&](uint32_t r) {   // the tables of row r's class, column class 0
+      if (BY_CLASS) return tables;
       const uint32_t cls = __ldg(a.row_class + r);
       if (cls >= a.nr) bad |= kStatusBadSymbol;
-      return (cls < a.nr ? cls : 0u) * a.nc * a.ctx_bytes;
+      return tables + min(cls, a.nr - 1) * a.nc * a.ctx_bytes;
     };
     uint32_t here = row_tables(row);
     cp_async_wait<0>();
+    if (!mbar_wait(bar, 0)) {   // the tables, on their way since the start
+      packed_report(a, kStatusTimeout, false);
+      break;
+    }
     s.open();
     if (CODED) t.open();
     auto refill = [&]() {
-      s.refill();
-      if (CODED) t.refill();
+      s.refill(a.bytes, a.size);
+      if (CODED) t.refill(a.raw, uint32_t(a.raw_size));
       cp_async_commit();
       cp_async_wait<1>();
     };
-    // Looks a main symbol up in the tables at offset `ctx` (MAIN) and / or a residual in those the entry `resid_of` names.
+    // Looks a main symbol up in the tables at `ctx` (MAIN) and / or a residual in those the entry `resid_of` names.
     // Returns their second entry words: symbol << 5 | residual tables / 8 << 16, and the residual's bits of the word.
     auto look_up = [&](auto main_too, auto resid_too, bool main_second, bool resid_second, uint32_t ctx, uint32_t resid_of, uint32_t& main_word,
                        uint32_t& resid_word) {
       constexpr bool MAIN = decltype(main_too)::value, RESID = decltype(resid_too)::value;
-      uint32_t ms = 0, rs = 0;
-      const uint8_t *me = nullptr, *re = nullptr;
+      uint32_t me = 0, re = 0, md = 0, rd = 0;
       uint2 m = {0, 0}, r = {0, 0};
-      uint32_t md = 0, rd = 0;
-      if (MAIN) {
-        ms = s.x & 0xFFFFu;
-        me = tables + ctx + rank_bytes + 8u * tables[ctx + (ms >> shift)];
+      if (MAIN) {   // (bucket + place in it) >> 8 = the rank
+        const uint32_t v = lds_u16(ctx + ((s.x >> (shift - 1)) & (bucket_bytes - 2)));
+        me = ctx + bucket_bytes + (((v + (s.x & place)) >> 5) & ~7u);
       }
       if (RESID) {
-        const uint8_t* const base = rtables + ((resid_of >> 16) << 3);
-        rs = t.x & 0xFFFFu;
-        re = base + rrank_bytes + 8u * base[rs >> rshift];
+        const uint32_t base = rtables + ((resid_of >> 16) << 3), v = lds_u16(base + ((t.x >> (rshift - 1)) & (rbucket_bytes - 2)));
+        re = base + rbucket_bytes + (((v + (t.x & rplace)) >> 5) & ~7u);
       }
-      if (MAIN) { m = *reinterpret_cast<const uint2*>(me); md = ms - (m.x & 0xFFFFu); }
-      if (RESID) { r = *reinterpret_cast<const uint2*>(re); rd = rs - (r.x & 0xFFFFu); }
-      while ((MAIN && md > (m.x >> 16)) || (RESID && rd > (r.x >> 16))) {   // forward scan inside a bucket
-        if (MAIN && md > (m.x >> 16)) { me += 8; m = *reinterpret_cast<const uint2*>(me); md = ms - (m.x & 0xFFFFu); }
-        if (RESID && rd > (r.x >> 16)) { re += 8; r = *reinterpret_cast<const uint2*>(re); rd = rs - (r.x & 0xFFFFu); }
+      if (MAIN) { m = lds64(me); md = (s.x - m.x) & 0xFFFFu; }   // slot - first slot of the symbol
+      if (RESID) { r = lds64(re); rd = (t.x - r.x) & 0xFFFFu; }
+      while ((MAIN && md > (m.x >> 16)) || (RESID && rd > (r.x >> 16))) {   // rare: a bucket of several symbols
+        if (MAIN && md > (m.x >> 16)) { me += 8; m = lds64(me); md = (s.x - m.x) & 0xFFFFu; }
+        if (RESID && rd > (r.x >> 16)) { re += 8; r = lds64(re); rd = (t.x - r.x) & 0xFFFFu; }
       }
       if (MAIN) { s.advance(m.x >> 16, md, main_second); main_word = m.y; }
       if (RESID) { t.advance(r.x >> 16, rd, resid_second); resid_word = r.y; }
@@ -264,11 +302,11 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
       uint4 cls = {0, 0, 0, 0};
       uint32_t below = here;
       if (ALIGNED) {
-        if (col >= a.cols) {
+        if (!BY_CLASS && col >= a.cols) {
           col -= a.cols;
           here = row_tables(++row);
         }
-        cls = *reinterpret_cast<const uint4*>(classes + packed_class_at(col));
+        cls = lds128(classes + packed_class_at(col));
       } else if (col + 16 >= a.cols) {   // a run of 16 reaches at most one row end (cols >= 16)
         if (row + 1 < a.rows) below = row_tables(row + 1);
       }
@@ -293,7 +331,7 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
             ctx = here + __byte_perm(j < 4 ? c_lo : c_hi, 0, 0x4440 + (j & 3)) * a.ctx_bytes;
           } else {
             const uint32_t c = col + half * 8 + j;
-            ctx = (c >= a.cols ? below : here) + classes[packed_class_at(c)] * a.ctx_bytes;
+            ctx = (c >= a.cols ? below : here) + lds_u8(classes + packed_class_at(c)) * a.ctx_bytes;
           }
           if (j & 1) s.mid_pair();
           else s.begin_pair();
@@ -321,7 +359,7 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
           keep(7, (before & 0xFFFFu) | resid_word);
         }
         const uint32_t k = 16 * g + 8 * half;
-        if (wide_out && k >= keep_from && k + 8 <= keep_to) {
+        if (BY_CLASS || (wide_out && k >= keep_from && k + 8 <= keep_to)) {
           *reinterpret_cast<uint4*>(out + k) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         } else {
 #pragma unroll
@@ -335,7 +373,7 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
         ++row;
       }
     }
-    if (ALIGNED && col >= a.cols) {
+    if (ROWS == kRows16 && col >= a.cols) {
       col -= a.cols;
       if (++row < a.rows) here = row_tables(row);
     }
@@ -343,7 +381,7 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
       if ((step & 7u) == 0) refill();
       uint32_t main_word = 0, word = 0, unused = 0;
       s.begin_pair();
-      look_up(Yes{}, No{}, false, false, here + classes[packed_class_at(col)] * a.ctx_bytes, 0, main_word, unused);
+      look_up(Yes{}, No{}, false, false, here + lds_u8(classes + packed_class_at(col)) * a.ctx_bytes, 0, main_word, unused);
       s.end_odd();
       if (CODED) {
         t.begin_pair();
@@ -371,6 +409,7 @@ __global__ void __launch_bounds__(kPackedThreads<RESIDUAL>, 1) bctx_packed_kerne
     if (CODED) check(t, a.raw, uint32_t(a.raw_size), a.raw_states, a.raw_offsets);
     if (bad) packed_report(a, bad, false);
   }
+  if (threadIdx.x == 0) mbar_wait(bar, 0);   // no copy may be under way when the CTA ends
 }
 
 }  // namespace grb

@@ -329,16 +329,16 @@ int grb_bctx_build_lookup(const uint32_t* freq, uint32_t nctx, uint32_t vocab, u
 
 // The models packed for shared memory (PackedShape in bcx_model.h): shape = {log2 slots per main bucket, bytes per main
 // context, log2 slots per residual bucket, offset of the residual contexts, bytes}.  residual_freq == NULL: raw residuals.
-// With image == NULL only the shape is computed.  Returns 0, 1 on bad arguments, 2 for invalid tables, 4 when they do not
-// fit `limit` bytes.
-int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t limit, uint32_t shape[5],
-                         uint8_t* image) {
+// With image == NULL only the shape is computed.  Returns 0, 1 on bad arguments, 2 for invalid tables, 4 when `resident` main
+// contexts and the residual contexts do not fit `limit` bytes.
+int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t resident, uint32_t limit,
+                         uint32_t shape[5], uint8_t* image) {
   try {
-    if (!main_freq || !nctx || !shape) return 1;
+    if (!main_freq || !nctx || !resident || resident > nctx || !shape) return 1;
     PackedTables tables;
     if (!tables.load(main_freq, nctx, residual_freq)) return 2;
     PackedShape p;
-    if (!tables.shape(limit, p)) return 4;
+    if (!tables.shape(resident, limit, p)) return 4;
     const uint32_t values[5] = {p.shift, p.ctx_bytes, p.resid_shift, p.resid_at, p.bytes};
     std::copy(values, values + 5, shape);
     if (image) tables.write(p, image);

@@ -76,16 +76,21 @@ class Model {
 };
 
 // The models of a frame packed for shared memory (csrc/bctx_packed.cuh).  A context has few live symbols (60 to 80 of 1024
-// on Gaussian weights), so its model is: u8 rank[65536 >> shift], the rank among the live symbols of the one that owns each
-// bucket's first slot; and entries of 8 bytes in rank order, {first slot u16 | frequency - 1 u16, what the symbol means
-// u32}.  An entry that matches any slot follows the last one where there is room and the last one matches everything up to
-// the table's end, so that a forward scan always ends.
-// Layout: the main contexts at multiples of ctx_bytes; from resid_at on the residual contexts (coded residuals only) of the
+// on Gaussian weights), so its model is: u16 bucket[65536 >> shift] = rank << 8 | 255 - last, where rank is the rank among the
+// live symbols of the one that owns the bucket's first slot and `last` (0..255) the last place in the bucket that symbol owns
+// (255 when it owns all of it), so that (bucket + place) >> 8 is the rank at any place up to the bucket's second boundary;
+// and entries of 8 bytes in rank order, {first slot u16 | frequency - 1 u16, what the symbol means u32}.  Buckets with more
+// boundaries, where rare symbols lie, end in a forward scan of the entries, which always ends: the last live entry reaches up
+// to slot 65535, and entries past it match any slot.
+// Layout: the main contexts at multiples of ctx_bytes (those of one row class, one per column class, side by side: a kernel
+// may keep one row class only, `resident` contexts); from resid_at on the residual contexts (coded residuals only) of the
 // main symbols that occur anywhere, each as long as its live symbols need.  The meaning of a main entry is
 // symbol << 5 | (offset of its residual context from resid_at) / 8 << 16, that of a residual entry its bits of the word.
 struct PackedShape {
   uint32_t shift, ctx_bytes, resid_shift, resid_at, bytes;
 };
+
+constexpr uint64_t kPackedImageMax = 4u << 20;   // what the prefix sums of a 64 x 16 frame take, too
 
 class PackedTables {
  public:
@@ -113,16 +118,17 @@ class PackedTables {
     }
     return true;
   }
-  // The bucket widths with the fewest scan steps whose tables fit `limit` bytes; false when none do.
-  bool shape(uint32_t limit, PackedShape& out) const {
+  // The bucket widths with the fewest scan steps (rare symbols, which share buckets, are mostly main symbols) whose tables, `resident` main contexts of them, fit `limit` bytes; false
+  // when none do.
+  bool shape(uint32_t resident, uint32_t limit, PackedShape& out) const {
     if (ranks_ > 255) return false;
     uint64_t best = ~uint64_t(0);
-    for (uint32_t ms = 4; ms <= 8; ++ms)
-      for (uint32_t rs = resid_ ? 4 : 9; rs <= 9; ++rs) {
-        const uint64_t ctx = ((65536u >> ms) + ranks_ * 8 + 15) & ~15u, resid_at = ctx * nctx_;
-        const uint64_t resid = resid_ ? uint64_t(resid_contexts_) * (65536u >> rs) + uint64_t(resid_entries_) * 8 : 0;
-        const uint64_t bytes = (resid_at + resid + 15) & ~uint64_t(15), cost = (uint64_t(ranks_) << ms) + (resid_ ? uint64_t(64) << rs : 0);
-        if (bytes > limit || resid > 65535u * 8 || cost >= best) continue;
+    for (uint32_t ms = 3; ms <= 8; ++ms)
+      for (uint32_t rs = resid_ ? 4 : 8; rs <= 8; ++rs) {
+        const uint64_t ctx = ((131072u >> ms) + ranks_ * 8 + 15) & ~15u, resid_at = ctx * nctx_;
+        const uint64_t resid = resid_ ? uint64_t(resid_contexts_) * (131072u >> rs) + uint64_t(resid_entries_) * 8 : 0;
+        const uint64_t bytes = (resid_at + resid + 15) & ~uint64_t(15), kept = bytes - resid_at + ctx * resident, cost = (uint64_t(ranks_) << ms) + (resid_ ? uint64_t(16) << rs : 0);
+        if (kept > limit || bytes > kPackedImageMax || resid > 65535u * 8 || cost >= best) continue;
         best = cost;
         out = PackedShape{ms, uint32_t(ctx), rs, uint32_t(resid_at), uint32_t(bytes)};
       }
@@ -137,7 +143,7 @@ class PackedTables {
       resid_of[s] = at;
       context(resid_ + size_t(s) * 64, 64, p.resid_shift, resid_live_[s], image + p.resid_at + at,
               [](uint32_t r) { return (r & 31u) | (r & 32u) << 10; });
-      at += (65536u >> p.resid_shift) + resid_live_[s] * 8;
+      at += (131072u >> p.resid_shift) + resid_live_[s] * 8;
     }
     for (uint32_t cx = 0; cx < nctx_; ++cx)
       context(main_ + size_t(cx) * 1024, 1024, p.shift, ranks_, image + size_t(cx) * p.ctx_bytes,
@@ -153,7 +159,7 @@ class PackedTables {
   }
   template <class Meaning>
   static void context(const uint32_t* freq, uint32_t vocab, uint32_t shift, uint32_t ranks, uint8_t* at, Meaning meaning) {
-    uint8_t* entry = at + (65536u >> shift);
+    uint8_t* entry = at + (131072u >> shift);
     uint32_t r = 0, run = 0;
     auto put = [&](uint32_t lo, uint32_t last, uint32_t what) {
       const uint32_t words[2] = {lo | last << 16, what};
@@ -164,7 +170,11 @@ class PackedTables {
       const uint32_t f = freq[s];
       if (!f) continue;
       const uint32_t first = (run + round) >> shift, end = (run + f + round) >> shift;   // buckets whose first slot is the symbol's
-      std::memset(at + first, int(r), end - first);
+      for (uint32_t b = first; b < end; ++b) {
+        const uint32_t last = std::min(run + f - 1 - (b << shift), 255u);
+        const uint16_t v = uint16_t(r << 8 | (255u - last));
+        std::memcpy(at + 2 * size_t(b), &v, 2);
+      }
       put(run, f - 1, meaning(s));
       run += f;
     }

@@ -234,28 +234,42 @@ int device_sm_count(int dev) {
   return sms[dev];
 }
 
-template <bool ALIGNED, int RESIDUAL>
-int packed_launch(BctxPackedArgs a, int sms, int dev, cudaStream_t stream) {
+template <int ROWS, int RESIDUAL>
+int packed_launch(BctxPackedArgs a, uint32_t parts, uint32_t share, int sms, int dev, cudaStream_t stream) {
   static std::once_flag once[64];
   static int prepared[64];
   if (dev < 0 || dev >= 64) return GRB_ERR_UNSUPPORTED;
   std::call_once(once[dev], [&] {
-    prepared[dev] = cuda_status(cudaFuncSetAttribute(bctx_packed_kernel<ALIGNED, RESIDUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPackedSmemMax)));
+    prepared[dev] = cuda_status(cudaFuncSetAttribute(bctx_packed_kernel<ROWS, RESIDUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPackedSmemMax)));
   });
   if (prepared[dev]) return prepared[dev];
   constexpr uint32_t kLane = kPackedLaneBytes<RESIDUAL>;
-  const uint64_t fixed = kPackedTablesAt + uint64_t(a.table_bytes) + packed_class_bytes(a.cols);
+  const uint64_t fixed = kPackedTablesAt + uint64_t(ROWS == kByClass ? a.nc * a.ctx_bytes + (a.table_bytes - a.resid_at) : a.table_bytes) + packed_class_bytes(a.cols);
   if (fixed + 32 * kLane > kPackedSmemMax) return GRB_ERR_UNSUPPORTED;
-  // A CTA has to bring the tables in before it starts: no more CTAs than give each four warps of lanes, then equal shares,
-  // in as few and as equal rounds as shared memory allows.
-  const uint64_t ctas = std::min<uint64_t>(uint64_t(sms), (a.count + 127) / 128);
-  a.per_cta = uint32_t(((a.count + ctas - 1) / ctas + 31) & ~uint64_t(31));
-  const uint32_t most = std::min(kPackedThreads<RESIDUAL>, uint32_t((kPackedSmemMax - fixed) / kLane) & ~31u);
+  uint32_t grid;
+  if (ROWS == kByClass) {   // the share of a CTA is laid down (part_of), or it is a row
+    grid = a.ids ? uint32_t(a.count / a.per_row) : parts;
+    a.per_cta = a.ids ? a.per_row : share;
+  } else {
+    // A CTA has to bring the tables in before it starts: no more CTAs than give each four warps of lanes, then equal shares.
+    const uint64_t ctas = std::min<uint64_t>(uint64_t(sms), (a.count + 127) / 128);
+    a.per_cta = uint32_t(((a.count + ctas - 1) / ctas + 31) & ~uint64_t(31));
+    grid = uint32_t((a.count + a.per_cta - 1) / a.per_cta);
+  }
+  // as few and as equal rounds as shared memory allows
+  const uint32_t most = std::min(kPackedThreads, uint32_t((kPackedSmemMax - fixed) / kLane) & ~31u);
   const uint32_t rounds = (a.per_cta + most - 1) / most;
   const uint32_t threads = ((a.per_cta + rounds - 1) / rounds + 31) & ~31u;
-  const uint32_t grid = uint32_t((a.count + a.per_cta - 1) / a.per_cta);
-  bctx_packed_kernel<ALIGNED, RESIDUAL><<<grid, threads, uint32_t(fixed) + threads * kLane, stream>>>(a);
+  bctx_packed_kernel<ROWS, RESIDUAL><<<grid, threads, uint32_t(fixed) + threads * kLane, stream>>>(a);
   return cuda_status(cudaGetLastError());
+}
+template <int RESIDUAL>
+int packed_launch_rows(int rows, const BctxPackedArgs& a, uint32_t parts, uint32_t share, int sms, int dev, cudaStream_t stream) {
+  switch (rows) {
+    case kByClass: return packed_launch<kByClass, RESIDUAL>(a, parts, share, sms, dev, stream);
+    case kRows16: return packed_launch<kRows16, RESIDUAL>(a, parts, share, sms, dev, stream);
+    default: return packed_launch<kAnyRows, RESIDUAL>(a, parts, share, sms, dev, stream);
+  }
 }
 
 template <int G>
@@ -326,8 +340,8 @@ int grb_bctx_decode_packed(const grb_bctx_tensor* t, const grb_bctx_packed* p, c
   const bool coded = t->mode == 128;
   if ((t->mode != 0 && !coded) || (coded && (!t->residual_states || !t->residual_offsets))) return GRB_ERR_ARGUMENT;
   const uint32_t contexts = t->nr * t->nc, shift = p->shape[0], ctx_bytes = p->shape[1], bytes = p->shape[4];
-  if (shift < 4 || shift > 8 || !contexts || (ctx_bytes & 15) || (bytes & 15) || ctx_bytes < (65536u >> shift) + 8 ||
-      p->shape[3] != uint64_t(contexts) * ctx_bytes || p->shape[3] > bytes || p->shape[2] < 4 || p->shape[2] > 9)
+  if (shift < 3 || shift > 8 || !contexts || (ctx_bytes & 15) || (bytes & 15) || ctx_bytes < (131072u >> shift) + 8 ||
+      p->shape[3] != uint64_t(contexts) * ctx_bytes || p->shape[3] > bytes || p->shape[2] < 4 || p->shape[2] > 8)
     return GRB_ERR_ARGUMENT;
   if ((t->stride & 15) || t->cols < 16 || t->cols > kPackedColsMax || t->main_bytes >= 0xFFFFFF00ull ||
       (coded && t->residual_bytes >= 0xFFFFFF00ull) || t->n > 0xFFFFFFFFull)
@@ -340,9 +354,10 @@ int grb_bctx_decode_packed(const grb_bctx_tensor* t, const grb_bctx_packed* p, c
   if (row_ids) {
     if (count > (uint64_t(1) << 31) / per_row) return GRB_ERR_ARGUMENT;
     count *= per_row;
-  } else if (count > (t->n + t->stride - 1) / t->stride) {
+  } else if (count != (t->n + t->stride - 1) / t->stride) {
     return GRB_ERR_ARGUMENT;
   }
+  if (p->parts && (t->cols % t->stride || !p->share || !p->rows_by_class || !p->part_of || (reinterpret_cast<uintptr_t>(p->part_of) & 15))) return GRB_ERR_ARGUMENT;
   int dev = 0;
   const cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return cuda_status(e);
@@ -373,15 +388,19 @@ int grb_bctx_decode_packed(const grb_bctx_tensor* t, const grb_bctx_packed* p, c
   a.stride = t->stride;
   a.ids = reinterpret_cast<const long long*>(row_ids);
   a.per_row = per_row;
+  a.rows_by_class = p->rows_by_class;
+  a.part_of = reinterpret_cast<const uint4*>(p->part_of);
   a.count = count;
   a.out = out;
   a.status = status;
   a.host_flags = host_flags;
   const auto stream = static_cast<cudaStream_t>(cuda_stream);
-  const bool wide = (t->stride & 63) == 0, aligned = (t->cols & 15) == 0;
-  if (coded) return aligned ? packed_launch<true, kCoded>(a, sms, dev, stream) : packed_launch<false, kCoded>(a, sms, dev, stream);
-  if (wide) return aligned ? packed_launch<true, kRaw64>(a, sms, dev, stream) : packed_launch<false, kRaw64>(a, sms, dev, stream);
-  return aligned ? packed_launch<true, kRaw16>(a, sms, dev, stream) : packed_launch<false, kRaw16>(a, sms, dev, stream);
+  const int rows = p->parts ? kByClass : (t->cols & 15) == 0 ? kRows16 : kAnyRows;
+  switch (coded ? kCoded : (t->stride & 63) == 0 ? kRaw64 : kRaw16) {
+    case kCoded: return packed_launch_rows<kCoded>(rows, a, p->parts, p->share, sms, dev, stream);
+    case kRaw64: return packed_launch_rows<kRaw64>(rows, a, p->parts, p->share, sms, dev, stream);
+    default: return packed_launch_rows<kRaw16>(rows, a, p->parts, p->share, sms, dev, stream);
+  }
 }
 
 int grb_bxr_decode(const void* image, const bxr_header* h, uint16_t* out, uint32_t* status, void* cuda_stream) {

@@ -16,7 +16,7 @@ import numpy as np
 
 from . import _native
 from . import codec as base
-from .resident import ResidentWeight
+from .resident import ResidentWeight, sm_count
 
 
 def _p(a, t):
@@ -112,23 +112,45 @@ def _lookup_tables(freq):
     return cum, np.ascontiguousarray(bucket[:, ::1 << (shift - 4)]), shift
 
 
+def _class_shares(row_class, per_row, ctas):
+    """Rows sorted by class and the share of the tensor each CTA decodes (``grb_bctx_packed.part_of``): every class gets CTAs in
+    proportion to its rows, and its blocks are split evenly over them, in whole warps."""
+    rows_by_class = np.argsort(row_class, kind="stable").astype(np.uint32)
+    counts = np.bincount(row_class)
+    used = np.flatnonzero(counts)
+    blocks = counts[used].astype(np.int64) * per_row
+    given = np.ones(len(used), dtype=np.int64)
+    most = max(1, int(-(-blocks.sum() // 128)))        # a CTA brings its tables in first: four warps of lanes at least
+    for _ in range(min(ctas, most) - len(used)):
+        given[np.argmax(blocks / given)] += 1
+    parts, first_row = [], np.concatenate([[0], np.cumsum(counts)])
+    for cls, n, g in zip(used, blocks, given):
+        share = (-(-int(n) // int(g)) + 31) // 32 * 32
+        parts += [(cls, first_row[cls], lo, min(int(n), lo + share)) for lo in range(0, int(n), share)]
+    return rows_by_class, np.array(parts, dtype=np.uint32)
+
+
 def _packed_tables(indexed, stride):
-    """A frame's models packed for the shared memory of one SM and their descriptor, or None when the frame is one the packed
-    kernel does not take (see ``grb_bctx_decode_packed``)."""
-    cols = indexed["shape"][1]
+    """A frame's models packed for the shared memory of one SM: (descriptor, image, whether CTAs keep one row class's tables),
+    or None when the frame is one the packed kernel does not take (see ``grb_bctx_decode_packed``)."""
+    cols, nc = indexed["shape"][1], indexed["nc"]
     if stride % 16 or not 16 <= cols <= 24576:
         return None
-    # what shared memory leaves beside the column classes and the stream rings of half a 4096 x 4096 frame's lanes (448 of
-    # them with two streams, 896 with one)
-    limit = 232448 - 128 - 448 * 128 - (cols + cols // 8 + 64)
     main = np.ascontiguousarray(indexed["main_freq"], dtype="<u4")
-    residual = _native.U32P()
-    if "residual_freq" in indexed:
+    residual, coded = _native.U32P(), "residual_freq" in indexed
+    if coded:
         residual_freq = np.ascontiguousarray(indexed["residual_freq"], dtype="<u4")
         residual = _p(residual_freq, ctypes.c_uint32)
     packed, pack = _native.BctxPacked(), _native.lib().grb_bctx_pack_tables
-    args = (_p(main, ctypes.c_uint32), main.shape[0], residual, limit, ctypes.byref(packed.shape))
-    status = pack(*args, None)
+    by_class = cols % stride == 0
+    # What shared memory leaves beside the column classes and the stream rings: those of 928 lanes (a 4096 x 4096 frame on all
+    # SMs in one round), else, for tables that take more, of half of them.
+    for lanes in (928, 464):
+        limit = 232448 - 128 - lanes * (128 if coded else 64) - (cols + cols // 8 + 64)
+        args = (_p(main, ctypes.c_uint32), main.shape[0], residual, nc if by_class else main.shape[0], limit, ctypes.byref(packed.shape))
+        status = pack(*args, None)
+        if status != 4:
+            break
     if status == 4:
         return None
     if not status:
@@ -136,7 +158,7 @@ def _packed_tables(indexed, stride):
         status = pack(*args, _p(image, ctypes.c_uint8))
     if status:
         raise base.CodecError(f"invalid frequency tables ({status})")
-    return image, packed
+    return packed, image, by_class
 
 
 class CudaContextTensor:
@@ -160,6 +182,8 @@ class CudaContextTensor:
         if not torch.cuda.is_available():
             raise RuntimeError("CUDA is required")
         self.device = torch.device(device)
+        if self.device.index is None:
+            self.device = torch.device(self.device.type, torch.cuda.current_device())
         self.stride = stride
         if not isinstance(stride, int) or not 1 <= stride <= 65536:
             raise base.CodecError("invalid checkpoint stride")
@@ -179,9 +203,15 @@ class CudaContextTensor:
         self._bucket_shift = {}
         self._packed = None
         if self.mode != 1 and (packed := _packed_tables(indexed, walk_stride)) is not None:
-            self.buffers["packed"] = torch.from_numpy(packed[0]).to(self.device)
-            self._packed = packed[1]
+            self._packed, image, by_class = packed
+            self.buffers["packed"] = torch.from_numpy(image).to(self.device)
             self._packed.tables = self.buffers["packed"].data_ptr()
+            if by_class:
+                rows_by_class, parts = _class_shares(indexed["rows"], self.shape[1] // walk_stride, sm_count(self.device))
+                self.buffers["rows_by_class"] = torch.from_numpy(rows_by_class.view(np.int32)).to(self.device)
+                self.buffers["part_of"] = torch.from_numpy(parts.view(np.int32)).to(self.device)
+                self._packed.parts, self._packed.share = len(parts), int((parts[:, 3] - parts[:, 2]).max())
+                self._packed.rows_by_class, self._packed.part_of = self.buffers["rows_by_class"].data_ptr(), self.buffers["part_of"].data_ptr()
         for kind in ("main", "residual"):
             table = indexed.get(kind + "_freq")
             if table is not None and self._packed is None:
@@ -193,7 +223,8 @@ class CudaContextTensor:
         self._error_clear = True
         # outcome of a checked decode, written by the kernel into host memory: {status bits, an index was out of range}
         self._flags = torch.zeros(2, dtype=torch.int32).pin_memory()
-        self._flag_words = self._flags.numpy()
+        self._flags_at = self._flags.data_ptr()
+        self._flag_words = (ctypes.c_uint32 * 2).from_address(self._flags_at)
         self.resident = None
         if fused and words is not None:
             self.resident = ResidentWeight.from_words(words, device=self.device, source_sha256=bytes.fromhex(self.source_sha256),
@@ -202,6 +233,8 @@ class CudaContextTensor:
         if self.resident is not None:
             self.resident_bytes += self.resident.resident_bytes
         self._descriptor = None if self.mode == 1 else self._make_descriptor()
+        if self._packed is not None:
+            self._packed_args = ctypes.byref(self._descriptor), ctypes.byref(self._packed)
 
     def _make_descriptor(self):
         b = self.buffers
@@ -238,14 +271,18 @@ class CudaContextTensor:
         wait = check or ids is not None
         flags = self._flag_words
         if wait:
-            flags[:] = 0
+            flags[0] = flags[1] = 0
         self._error_clear = wait        # unknown until somebody waits for the launch
-        with torch.cuda.device(self.device):
-            stream = torch.cuda.current_stream()
-            status = _native.lib().grb_bctx_decode_packed(
-                ctypes.byref(self._descriptor), ctypes.byref(self._packed), None if ids is None else ids.data_ptr(), count,
-                result.data_ptr(), self.error.data_ptr(), self._flags.data_ptr() if wait else None, stream.cuda_stream)
-        _native.check(status, "grb_bctx_decode_packed")
+        stream = torch.cuda.current_stream(self.device)
+        args = (*self._packed_args, None if ids is None else ids.data_ptr(), count, result.data_ptr(), self.error.data_ptr(),
+                self._flags_at if wait else None, stream.cuda_stream)
+        if torch.cuda.current_device() == self.device.index:
+            status = _native.lib().grb_bctx_decode_packed(*args)
+        else:
+            with torch.cuda.device(self.device):
+                status = _native.lib().grb_bctx_decode_packed(*args)
+        if status:
+            _native.check(status, "grb_bctx_decode_packed")
         if wait:
             stream.synchronize()
             if flags[0] or flags[1]:

@@ -129,19 +129,27 @@ int grb_bctx_decode_words(const grb_bctx_tensor* tensor, const int64_t* block_id
 /* A frame's models packed for the shared memory of one SM (csrc/bcx_model.h, PackedShape): shape = {log2 slots per main
  * bucket, bytes per main context, log2 slots per residual bucket, offset of the residual contexts, bytes}.  residual_freq:
  * the tables of a mode 128 frame, NULL for raw residuals.  image == NULL computes the shape only.  0 ok, 1 arguments,
- * 2 invalid tables, 4 they do not fit `limit` bytes: use grb_bctx_decode_words.  The kernel keeps them in the 227 KB of an
- * SM's shared memory next to 64 bytes per lane and stream and 9/8 bytes per column. */
-int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t limit, uint32_t shape[5],
-                         uint8_t* image);
+ * 2 invalid tables, 4 `resident` main contexts and the residual contexts do not fit `limit` bytes: use
+ * grb_bctx_decode_words.  The kernel keeps them in the 227 KB of an SM's shared memory next to 64 bytes per lane and stream
+ * and 9/8 bytes per column. */
+int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t resident, uint32_t limit,
+                         uint32_t shape[5], uint8_t* image);
 
+/* parts > 0 (needs cols % stride == 0): the rows are decoded class by class, every CTA with the tables of one row class only
+ * (resident = nc).  rows_by_class u32[rows]: the rows, sorted by class; part_of u32[parts][4]: what CTA p decodes = {row class,
+ * place of the class's first row in rows_by_class, first block, end block}, blocks counted within the class's rows.
+ * parts == 0: every CTA keeps the tables of all contexts (resident = nctx). */
 typedef struct grb_bctx_packed {
   const uint8_t* tables;      /* device, 16-byte aligned: the image grb_bctx_pack_tables wrote */
   uint32_t shape[5];
+  uint32_t parts, share;      /* share: the most blocks a CTA decodes */
+  const uint32_t* rows_by_class;
+  const uint32_t* part_of;
 } grb_bctx_packed;
 
 /* grb_bctx_decode_words for frames with packed tables, strides that are multiples of 16 and 16 to 24576 columns
- * (GRB_ERR_UNSUPPORTED otherwise); the *_cum and *_bucket tables are not read.  row_ids == NULL decodes blocks 0..count-1
- * and out receives count * stride words; else out receives `count` rows of the tensor, [count][cols], and a row number
+ * (GRB_ERR_UNSUPPORTED otherwise); the *_cum and *_bucket tables are not read.  row_ids == NULL decodes the whole tensor
+ * (count = its blocks; out receives count * stride words); else out receives `count` rows of the tensor, [count][cols], and a row number
  * outside it is reported instead of followed.  host_flags (optional): two words of host memory the device can write; [0]
  * receives the status bits of a failed block, [1] is set for a row out of range, and both stay as they are otherwise, so
  * that a caller who has synchronised anyway reads the outcome there. */
