@@ -22,7 +22,8 @@ VOIDP = ctypes.c_void_p
 
 EXPORTS = (
     "bcx_encode", "bcx_frequencies", "bcx_decode", "bcx_decode_compact", "bcx_free", "bcx_pack6", "bcx_unpack6",
-    "bcx_checkpoint", "grb_bctx_build_lookup", "grb_bctx_decode_words", "grb_bctx_pack_tables", "grb_bctx_decode_packed", "bxr_build", "bxr_free", "bxr_decode_host",
+    "bcx_checkpoint", "grb_bctx_build_lookup", "grb_bctx_decode_words", "grb_bctx_magnitudes", "grb_bctx_frequencies", "grb_bctx_encode_stream",
+    "grb_bctx_frame_words", "grb_bctx_pack_tables", "grb_bctx_decode_packed", "bxr_build", "bxr_free", "bxr_decode_host",
     "bxr_validate", "bxr_layout_version", "grb_bxr_workspace_bytes", "grb_bxr_decode", "grb_bxr_gemm", "grb_bxr_gemv", "grb_bxr_gemm_next", "grb_kernel_attributes",
     "grb_static_scratch_bytes", "grb_bxr_gemv_static", "grb_dense_gemv_bf16", "grb_peer_control_bytes", "grb_peer_enable", "grb_peer_allreduce_bf16",
     "grb_peer_alloc", "grb_peer_free", "grb_peer_open", "grb_peer_close",
@@ -82,6 +83,11 @@ def _declare(lib):
     lib.bcx_checkpoint.argtypes = [U8P, sz, u64, u32, u32, U8P, U8P, u32, u32, u32, U16P, U32P, u32, U32P, U32P, U16P]
     lib.grb_bctx_build_lookup.argtypes = [U32P, u32, u32, U32P, U16P]
     lib.grb_bctx_decode_words.argtypes = [ctypes.POINTER(BctxTensor), VOIDP, u64, VOIDP, VOIDP, VOIDP]
+    lib.grb_bctx_magnitudes.argtypes = [VOIDP, u32, u32, VOIDP, VOIDP]
+    lib.grb_bctx_frequencies.argtypes = [VOIDP, u32, u32, VOIDP, VOIDP, u32, u32, VOIDP, VOIDP, ctypes.POINTER(u64)]
+    lib.grb_bctx_encode_stream.argtypes = [VOIDP, u32, u32, VOIDP, VOIDP, u32, u32, u32, VOIDP, ctypes.POINTER(U8P), ctypes.POINTER(sz)]
+    lib.grb_bctx_frame_words.argtypes = [VOIDP, sz, VOIDP, sz, u32, u32, VOIDP, VOIDP, u32, u32, VOIDP, VOIDP, u32, VOIDP, VOIDP, VOIDP, VOIDP,
+                                         VOIDP, VOIDP]
     lib.grb_bctx_pack_tables.argtypes = [U32P, u32, U32P, u32, u32, ctypes.POINTER(u32 * 5), U8P]
     lib.grb_bctx_decode_packed.argtypes = [ctypes.POINTER(BctxTensor), ctypes.POINTER(BctxPacked), VOIDP, u64, VOIDP, VOIDP, VOIDP, VOIDP]
     lib.bxr_build.argtypes = [U16P, u32, u32, u32, u32, u32, U8P, ctypes.POINTER(U8P), ctypes.POINTER(u64)]

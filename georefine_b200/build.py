@@ -15,7 +15,7 @@ from pathlib import Path
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT = PKG / "_build" / "libgeorefine_b200.so"
-SOURCES = [CSRC / "capi.cu", CSRC / "bcx_host.cpp", CSRC / "bxr_build.cpp"]
+SOURCES = [CSRC / "capi.cu", CSRC / "bcx_host.cpp", CSRC / "bcx_frame.cpp", CSRC / "bxr_build.cpp"]
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
          "-Xcompiler", "-pthread", "-shared"]
 

@@ -25,6 +25,8 @@ import ctypes
 import hashlib
 import os
 import struct
+import threading
+import time
 import zlib
 from dataclasses import dataclass
 
@@ -110,12 +112,47 @@ class _Head:
         return cls(mode, nr, nc, rows, cols, (ml, tl, sl, dl), digest)
 
 
-def _sealed(body: bytes) -> bytes:
-    return body + hashlib.sha256(body).digest()
+def _sealed(*pieces) -> bytes:
+    seal = hashlib.sha256()
+    for piece in pieces:
+        seal.update(piece)
+    return b"".join((*pieces, seal.digest()))
 
 
 def _seal_is_intact(frame: bytes) -> bool:
-    return len(frame) >= HEADER.size + _TRAILER and hashlib.sha256(frame[:-_TRAILER]).digest() == frame[-_TRAILER:]
+    return len(frame) >= HEADER.size + _TRAILER and hashlib.sha256(memoryview(frame)[:-_TRAILER]).digest() == frame[-_TRAILER:]
+
+
+_BESIDE_WORDS = 1 << 16      # smaller tensors are done before another thread has started
+
+
+class _Beside:
+    """``fn()`` on another thread while this one goes on (hashing, compression and the library's calls release the
+    interpreter lock); at once when ``worth`` is false.  ``result()`` waits and returns or raises."""
+
+    def __init__(self, fn, worth=True):
+        self._value, self._error, self._thread = None, None, None
+        if worth:
+            self._thread = threading.Thread(target=self._run, args=(fn,), daemon=True)
+            self._thread.start()
+        else:
+            self._run(fn)
+
+    def _run(self, fn):
+        try:
+            self._value = fn()
+        except BaseException as exc:      # handed to whoever asks for the result
+            self._error = exc
+
+    def done(self) -> bool:
+        return self._thread is None or not self._thread.is_alive()
+
+    def result(self):
+        if self._thread is not None:
+            self._thread.join()
+        if self._error is not None:
+            raise self._error
+        return self._value
 
 
 def _inflate_exact(data, expected):
@@ -159,16 +196,12 @@ def _quantile_classes(weight, k):
 
 
 def _labels(a, nr, nc):
-    """Row and column classes by total magnitude (sum of word & 0x7FFF), accumulated over row slabs so that a very
-    large tensor never needs a second array of its own size."""
+    """Row and column classes by total magnitude (sum of word & 0x7FFF)."""
     rows, cols = a.shape
-    row_sum = np.zeros(rows, dtype=np.uint64)
-    col_sum = np.zeros(cols, dtype=np.uint64)
-    step = max(1, min(rows, (1 << 20) // cols))
-    for lo in range(0, rows, step):
-        magnitude = a[lo:lo + step] & np.uint16(0x7FFF)
-        row_sum[lo:lo + step] = magnitude.sum(axis=1, dtype=np.uint64)
-        col_sum += magnitude.sum(axis=0, dtype=np.uint64)
+    row_sum, col_sum = np.empty(rows, dtype=np.uint64), np.empty(cols, dtype=np.uint64)
+    status = _lib().grb_bctx_magnitudes(a.ctypes.data, rows, cols, row_sum.ctypes.data, col_sum.ctypes.data)
+    if status:
+        raise CodecError(f"class labelling failed ({status})")
     return _quantile_classes(row_sum, nr), _quantile_classes(col_sum, nc)
 
 
@@ -195,6 +228,29 @@ def _encode_kind(lib, a, rc, cc, nr, nc, kind):
     return freq.tobytes(), stream
 
 
+def _both_frequencies(lib, a, rc, cc, nr, nc):
+    """Tables of the main stream and of the conditional residual stream, and the fewest bytes the latter can take."""
+    main, residual = np.zeros(nr * nc * _MAIN_VOCAB, dtype="<u4"), np.zeros(_MAIN_VOCAB * _RESIDUAL_VOCAB, dtype="<u4")
+    floor = ctypes.c_uint64()
+    status = lib.grb_bctx_frequencies(a.ctypes.data, *a.shape, rc.ctypes.data, cc.ctypes.data, nr, nc, main.ctypes.data, residual.ctypes.data,
+                                      ctypes.byref(floor))
+    if status:
+        raise CodecError(f"rANS encode failed ({status})")
+    return main, residual, floor.value
+
+
+def _encode_under(lib, a, rc, cc, nr, nc, kind, freq):
+    ptr, length = _native.U8P(), ctypes.c_size_t()
+    status = lib.grb_bctx_encode_stream(a.ctypes.data, *a.shape, rc.ctypes.data, cc.ctypes.data, nr, nc, kind, freq.ctypes.data,
+                                        ctypes.byref(ptr), ctypes.byref(length))
+    if status:
+        raise CodecError(f"rANS encode failed ({status})")
+    try:
+        return ctypes.string_at(ptr, length.value)
+    finally:
+        lib.bcx_free(ptr)
+
+
 def _frequencies_kind(lib, a, rc, cc, nr, nc, kind):
     vocab, nctx = _dims(kind, nr, nc)
     freq = np.zeros(nctx * vocab, dtype="<u4")
@@ -206,10 +262,15 @@ def _frequencies_kind(lib, a, rc, cc, nr, nc, kind):
     return freq.tobytes()
 
 
-def _decode_kind(lib, stream, freq, rc, cc, rows, cols, nr, nc, kind, main=None):
+def _decoder_choice():
     choice = os.environ.get("GEOREFINE_CONTEXT_COMPACT_RANS")
     if choice not in (None, "0", "1"):
         raise CodecError("GEOREFINE_CONTEXT_COMPACT_RANS must be 0 or 1")
+    return choice
+
+
+def _decode_kind(lib, stream, freq, rc, cc, rows, cols, nr, nc, kind, main=None):
+    choice = _decoder_choice()
     decoder = lib.bcx_decode_compact if choice == "1" else lib.bcx_decode
     vocab, nctx = _dims(kind, nr, nc)
     if len(freq) != nctx * vocab * 4:
@@ -252,6 +313,51 @@ def join_words(main, residual):
     return (((m >> 2) << 7) | ((m & 3) << 5) | (q & 31) | ((q >> 5) << 15)).astype("<u2")
 
 
+def _address(data) -> int:
+    """Address of a bytes object's (or array's) first byte."""
+    return np.frombuffer(data, dtype=np.uint8).ctypes.data if len(data) else 0
+
+
+def frame_words(f, stride=0):
+    """The words of a parsed frame in one pass of the library, their digest taken as rows get finished, and with ``stride`` the
+    restart points: (words [rows, cols], {"main_states": ..., ...}).  None when the pass meets anything it does not take; raises
+    when the digest is wrong."""
+    rows, cols = f["shape"]
+    n, coded = rows * cols, f["mode"] == MODE_CONDITIONAL
+    if not len(f["main_stream"]) or not len(f["residual_stream"]):
+        return None
+    words, progress, marks = np.empty((rows, cols), dtype="<u2"), ctypes.c_uint64(), {}
+    if stride:
+        for name in ("main_states", "main_offsets") + (("residual_states", "residual_offsets") if coded else ()):
+            marks[name] = np.empty(-(-n // stride), dtype=np.uint32)
+    at = lambda name: marks[name].ctypes.data if name in marks else None
+    lib = _lib()
+
+    def walk():
+        return lib.grb_bctx_frame_words(
+            _address(f["main_stream"]), len(f["main_stream"]), _address(f["residual_stream"]), len(f["residual_stream"]), rows, cols,
+            f["rows"].ctypes.data, f["columns"].ctypes.data, f["nr"], f["nc"], _address(f["main_table"]),
+            _address(f["residual_table"]) if coded else None, stride, at("main_states"), at("main_offsets"), at("residual_states"),
+            at("residual_offsets"), words.ctypes.data, ctypes.addressof(progress))
+
+    walking, digest, hashed = _Beside(walk, n >= _BESIDE_WORDS), hashlib.sha256(), 0
+    while True:
+        over = walking.done()
+        ready = progress.value
+        if ready > hashed:
+            digest.update(words[hashed:ready])
+            hashed = ready
+        elif over:
+            break
+        else:
+            time.sleep(5e-5)
+    if walking.result():
+        return None
+    if digest.digest() != f["digest"]:
+        raise CodecError("decoded checksum mismatch")
+    return words, marks
+
+
 # ---------------------------------------------------------------------------------------------- public API
 def encode(words, *, row_classes=16, col_classes=4):
     """Encode a 2-D array of BF16 bit patterns into a self-contained frame: the smaller of the two coded forms (6-bit
@@ -260,34 +366,46 @@ def encode(words, *, row_classes=16, col_classes=4):
     if row_classes not in ROWS or col_classes not in COLS:
         raise CodecError("unsupported class count")
     rows, cols = a.shape
-    source = a.tobytes()
-    digest = hashlib.sha256(source).digest()
-
-    def frame(mode, labels=b"", tables=b"", main=b"", residual=b"", raw=b""):
-        head = _Head(mode, row_classes, col_classes, rows, cols, (len(labels), len(tables), len(main), len(residual)), digest)
-        return _sealed(head.pack() + labels + tables + main + residual + raw)
-
-    lib = _lib()
-    rc, cc = _labels(a, row_classes, col_classes)
+    nr, nc, lib, beside = row_classes, col_classes, _lib(), a.size >= _BESIDE_WORDS
+    digest = _Beside(lambda: hashlib.sha256(a).digest(), beside)
+    rc, cc = _labels(a, nr, nc)
+    main_table, cond_table, cond_floor = _both_frequencies(lib, a, rc, cc, nr, nc)
+    main_stream = _Beside(lambda: _encode_under(lib, a, rc, cc, nr, nc, 0, main_table), beside)
+    packed = _Beside(lambda: _pack6(lib, a), beside)
+    raw6_tables = _Beside(lambda: zlib.compress(main_table, 6), beside)
     labels = zlib.compress(rc.tobytes() + cc.tobytes(), 6)
-    main_table, main_stream = _encode_kind(lib, a, rc, cc, row_classes, col_classes, 0)
-    cond_table, cond_stream = _encode_kind(lib, a, rc, cc, row_classes, col_classes, 1)
-    candidates = [   # in order of preference at equal size
-        frame(MODE_RAW6, labels, zlib.compress(main_table, 6), main_stream, _pack6(lib, a)),
-        frame(MODE_CONDITIONAL, labels, zlib.compress(main_table + cond_table, 6), main_stream, cond_stream),
-    ]
-    best = min(candidates, key=len)
-    plain = frame(MODE_WORDS, raw=source)
-    return best if len(best) < len(plain) else plain
+    cond_tables = zlib.compress(main_table.tobytes() + cond_table.tobytes(), 6)
+    raw6_tables, packed = raw6_tables.result(), packed.result()
+    # the coded residuals are produced only where they may turn out smaller
+    mode, tables, residual = MODE_RAW6, raw6_tables, packed
+    if len(cond_tables) + cond_floor < len(raw6_tables) + len(packed):
+        cond_stream = _encode_under(lib, a, rc, cc, nr, nc, 1, cond_table)
+        if len(cond_tables) + len(cond_stream) < len(raw6_tables) + len(packed):
+            mode, tables, residual = MODE_CONDITIONAL, cond_tables, cond_stream
+    main_stream = main_stream.result()
+    lengths = (len(labels), len(tables), len(main_stream), len(residual))
+    head = lambda mode, lengths: _Head(mode, nr, nc, rows, cols, lengths, digest.result()).pack()
+    if sum(lengths) < 2 * a.size:
+        return _sealed(head(mode, lengths), labels, tables, main_stream, residual)
+    return _sealed(head(MODE_WORDS, (0, 0, 0, 0)), a.tobytes())
+
+
+def _frame_bytes(frame) -> bytes:
+    if not isinstance(frame, (bytes, bytearray, memoryview)) or len(frame) < HEADER.size + _TRAILER:
+        raise CodecError("short frame")
+    return bytes(frame)
 
 
 def parse(frame):
     """Validated sections of a frame: header fields, labels, tables, stream slices (no entropy decoding)."""
-    if not isinstance(frame, (bytes, bytearray, memoryview)) or len(frame) < HEADER.size + _TRAILER:
-        raise CodecError("short frame")
-    frame = bytes(frame)
+    frame = _frame_bytes(frame)
     if not _seal_is_intact(frame):
         raise CodecError("frame checksum mismatch")
+    return parse_sealed(frame)
+
+
+def parse_sealed(frame: bytes):
+    """``parse`` of a frame whose trailing checksum the caller looks after."""
     head = _Head.read(frame)
     out = {"mode": head.mode, "nr": head.nr, "nc": head.nc, "shape": (head.rows, head.cols), "digest": head.digest}
     if head.mode == MODE_WORDS:
@@ -316,10 +434,30 @@ def parse(frame):
 
 def decode(frame):
     """Decode a complete frame on the host and verify the source checksum; trailing data rejects."""
-    f = parse(frame)
+    frame = _frame_bytes(frame)
+    # The checksum over the frame is taken beside the decoding of what it covers, and has the first word about it.
+    intact = _Beside(lambda: _seal_is_intact(frame), len(frame) >= _BESIDE_WORDS)
+    try:
+        words = _decode_sealed(frame)
+    except CodecError:
+        if not intact.result():
+            raise CodecError("frame checksum mismatch") from None
+        raise
+    if not intact.result():
+        raise CodecError("frame checksum mismatch")
+    return words
+
+
+def _decode_sealed(frame):
+    f = parse_sealed(frame)
     rows, cols = f["shape"]
     if f["mode"] == MODE_WORDS:
         return f["raw"].reshape(rows, cols)
+    _decoder_choice()
+    quick = frame_words(f)
+    if quick is not None:
+        return quick[0]
+    # something is wrong with a stream or its tables, or they are unusual: one stream after the other, with its own verdict
     lib = _lib()
     common = (f["rows"], f["columns"], rows, cols, f["nr"], f["nc"])
     main = _decode_kind(lib, f["main_stream"], f["main_table"], *common, 0)

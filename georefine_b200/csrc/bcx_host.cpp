@@ -23,6 +23,35 @@
 
 namespace grb {
 
+// Counts -> integer frequencies with sum 2^16.  Every symbol that occurs keeps at least one slot; the
+// rounding surplus or deficit goes to the symbols with the largest (smallest) division remainders,
+// ties resolved by symbol index, cycling if one pass is not enough.
+void quantise_counts(const uint64_t* counts, uint32_t vocab, uint32_t* freq) {
+  const uint64_t total = std::accumulate(counts, counts + vocab, uint64_t(0));
+  if (total == 0) return;  // an unused context keeps an all-zero row
+  std::vector<uint32_t> seen;
+  std::vector<uint64_t> rem(vocab, 0);
+  int64_t sum = 0;
+  for (uint32_t s = 0; s < vocab; ++s) {
+    if (counts[s] == 0) { freq[s] = 0; continue; }
+    const uint64_t scaled = counts[s] << 16;
+    freq[s] = std::max<uint32_t>(1u, uint32_t(scaled / total));
+    rem[s] = scaled % total;
+    sum += freq[s];
+    seen.push_back(s);
+  }
+  if (sum < int64_t(65536u)) {
+    std::sort(seen.begin(), seen.end(), [&](uint32_t a, uint32_t b) { return rem[a] != rem[b] ? rem[a] > rem[b] : a < b; });
+    uint32_t lack = 65536u - uint32_t(sum);
+    for (size_t j = 0; lack; j = (j + 1) % seen.size(), --lack) ++freq[seen[j]];
+  } else if (sum > int64_t(65536u)) {
+    std::sort(seen.begin(), seen.end(), [&](uint32_t a, uint32_t b) { return rem[a] != rem[b] ? rem[a] < rem[b] : a > b; });
+    uint32_t extra = uint32_t(sum) - 65536u;
+    for (size_t j = 0; extra; j = (j + 1) % seen.size())
+      if (freq[seen[j]] > 1) { --freq[seen[j]]; --extra; }
+  }
+}
+
 namespace {
 
 constexpr uint32_t kProbBits = 16;
@@ -47,35 +76,6 @@ inline uint32_t context_of(const Geometry& g, const Cursor& c) {
   return uint32_t(g.row_class[c.row]) * g.nc + g.col_class[c.col];
 }
 
-// Counts -> integer frequencies with sum 2^16.  Every symbol that occurs keeps at least one slot; the
-// rounding surplus or deficit goes to the symbols with the largest (smallest) division remainders,
-// ties resolved by symbol index, cycling if one pass is not enough.
-void quantise_counts(const uint64_t* counts, uint32_t vocab, uint32_t* freq) {
-  const uint64_t total = std::accumulate(counts, counts + vocab, uint64_t(0));
-  if (total == 0) return;  // an unused context keeps an all-zero row
-  std::vector<uint32_t> seen;
-  std::vector<uint64_t> rem(vocab, 0);
-  int64_t sum = 0;
-  for (uint32_t s = 0; s < vocab; ++s) {
-    if (counts[s] == 0) { freq[s] = 0; continue; }
-    const uint64_t scaled = counts[s] << kProbBits;
-    freq[s] = std::max<uint32_t>(1u, uint32_t(scaled / total));
-    rem[s] = scaled % total;
-    sum += freq[s];
-    seen.push_back(s);
-  }
-  if (sum < int64_t(kProbTotal)) {
-    std::sort(seen.begin(), seen.end(), [&](uint32_t a, uint32_t b) { return rem[a] != rem[b] ? rem[a] > rem[b] : a < b; });
-    uint32_t lack = kProbTotal - uint32_t(sum);
-    for (size_t j = 0; lack; j = (j + 1) % seen.size(), --lack) ++freq[seen[j]];
-  } else if (sum > int64_t(kProbTotal)) {
-    std::sort(seen.begin(), seen.end(), [&](uint32_t a, uint32_t b) { return rem[a] != rem[b] ? rem[a] < rem[b] : a > b; });
-    uint32_t extra = uint32_t(sum) - kProbTotal;
-    for (size_t j = 0; extra; j = (j + 1) % seen.size())
-      if (freq[seen[j]] > 1) { --freq[seen[j]]; --extra; }
-  }
-}
-
 struct StreamKind {
   uint32_t kind, vocab, nctx;
   StreamKind(uint32_t k, uint32_t nr, uint32_t nc) : kind(k), vocab(k ? 64u : 1024u), nctx(k ? 1024u : nr * nc) {}
@@ -90,36 +90,6 @@ void tally(const uint16_t* w, uint64_t n, const Geometry& g, const StreamKind& k
     else ++counts[size_t(context_of(g, c)) * k.vocab + m];
   }
   for (uint32_t cx = 0; cx < k.nctx; ++cx) quantise_counts(&counts[size_t(cx) * k.vocab], k.vocab, freq + size_t(cx) * k.vocab);
-}
-
-// Emits the stream in decode order: 4-byte little-endian state the decoder starts from, then the
-// renormalisation bytes.  Coding runs from the last symbol to the first.
-bool emit_stream(const uint16_t* w, uint64_t n, const Geometry& g, const StreamKind& k, const uint32_t* freq,
-                 std::vector<uint8_t>& out) {
-  std::vector<uint32_t> start(size_t(k.nctx) * k.vocab);
-  for (uint32_t cx = 0; cx < k.nctx; ++cx) {
-    uint32_t run = 0;
-    for (uint32_t s = 0; s < k.vocab; ++s) { start[size_t(cx) * k.vocab + s] = run; run += freq[size_t(cx) * k.vocab + s]; }
-  }
-  std::vector<uint8_t> tail;
-  tail.reserve(size_t(n / 2) + 16);
-  uint32_t x = kStateLow;
-  Cursor c;
-  if (n) c.seek(n - 1, g.cols);
-  for (uint64_t i = n; i-- > 0;) {
-    const uint32_t m = main_symbol(w[i]);
-    const size_t at = k.kind ? size_t(m) * k.vocab + residual_symbol(w[i]) : size_t(context_of(g, c)) * k.vocab + m;
-    const uint32_t f = freq[at];
-    if (f == 0) return false;
-    const uint64_t ceiling = (uint64_t(kStateLow >> kProbBits) << 8) * f;
-    while (x >= ceiling) { tail.push_back(uint8_t(x)); x >>= 8; }
-    x = ((x / f) << kProbBits) + (x % f) + start[at];
-    if (i) c.prev(g.cols);
-  }
-  out.resize(tail.size() + 4);
-  for (int b = 0; b < 4; ++b) out[b] = uint8_t(x >> (8 * b));
-  std::reverse_copy(tail.begin(), tail.end(), out.begin() + 4);
-  return true;
 }
 
 enum WalkStatus { kOk = 0, kBadTables = 2, kBadStream = 3, kOffsetOverflow = 4 };
@@ -211,14 +181,12 @@ int bcx_encode(const uint16_t* w, uint64_t n, uint32_t rows, uint32_t cols, cons
     const Geometry g{cols, nc, rc, cc};
     const StreamKind k(kind, nr, nc);
     tally(w, n, g, k, freq);
-    std::vector<uint8_t> bytes;
-    if (!emit_stream(w, n, g, k, freq, bytes)) return 3;
-    auto* p = static_cast<uint8_t*>(std::malloc(bytes.size()));
-    if (!p) return 2;
-    std::memcpy(p, bytes.data(), bytes.size());
-    *stream = p;
-    *stream_n = bytes.size();
+    // Emitted in decode order: 4-byte little-endian state the decoder starts from, then the renormalisation bytes; coding
+    // runs from the last symbol to the first.
+    if (!encode_stream(w, rows, cols, rc, cc, nr, nc, kind, freq, stream, stream_n)) return 3;
     return 0;
+  } catch (const std::bad_alloc&) {
+    return 2;
   } catch (...) {
     return 3;
   }

@@ -7,6 +7,7 @@
 //   residual = sign << 5 | mantissa[4:0]              6 bits, vocabulary 64
 #pragma once
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <cstring>
 #include <vector>
@@ -18,6 +19,11 @@ inline uint32_t residual_symbol(uint16_t w) { return ((uint32_t(w) >> 10) & 32u)
 inline uint16_t join_word(uint32_t main, uint32_t residual) {
   return uint16_t((main << 5) | (residual & 31u) | ((residual & 32u) << 10));
 }
+
+// bcx_host.cpp, bcx_frame.cpp
+void quantise_counts(const uint64_t* counts, uint32_t vocab, uint32_t* freq);
+bool encode_stream(const uint16_t* words, uint32_t rows, uint32_t cols, const uint8_t* rc, const uint8_t* cc, uint32_t nr, uint32_t nc, uint32_t kind,
+                   const uint32_t* freq, uint8_t** stream, size_t* size);
 
 constexpr uint32_t kBucketShift = 4;                   // 16 slots per bucket
 constexpr uint32_t kBuckets = 65536u >> kBucketShift;  // 4096 buckets per context

@@ -57,14 +57,18 @@ def index_frame(frame: bytes, stride: int = 1024, *, keep_words: bool = False):
     frame's source digest.  ``keep_words`` also returns the decoded words (key ``words``)."""
     if not isinstance(stride, int) or not 1 <= stride <= 65536:
         raise base.CodecError("invalid checkpoint stride")
-    if len(frame) < base.HEADER.size + 32 or hashlib.sha256(frame[:-32]).digest() != frame[-32:]:
+    if len(frame) < base.HEADER.size + 32:
         raise base.CodecError("invalid frame checksum/length")
-    f = base.parse(frame)
+    frame = bytes(frame)
+    seal = hashlib.sha256(memoryview(frame)[:-32])
+    if seal.digest() != frame[-32:]:
+        raise base.CodecError("invalid frame checksum/length")
+    f = base.parse_sealed(frame)
+    seal.update(frame[-32:])
     r, c = f["shape"]
     n = r * c
     out = {"shape": (r, c), "mode": f["mode"], "nr": f["nr"], "nc": f["nc"], "stride": stride,
-           "source_sha256": f["digest"].hex(), "frame_sha256": hashlib.sha256(bytes(frame)).hexdigest(),
-           "frame_bytes": len(frame)}
+           "source_sha256": f["digest"].hex(), "frame_sha256": seal.hexdigest(), "frame_bytes": len(frame)}
     if f["mode"] == 1:
         out["raw"] = f["raw"]
         if keep_words:
@@ -72,20 +76,28 @@ def index_frame(frame: bytes, stride: int = 1024, *, keep_words: bool = False):
         return out
     nr, nc = f["nr"], f["nc"]
     sf = np.frombuffer(f["main_table"], dtype="<u4").copy().reshape(nr * nc, 1024)
-    states, offsets, main = checkpoints(f["main_stream"], sf, f["rows"], f["columns"], (r, c), nr, nc, stride)
-    out.update(rows=f["rows"], columns=f["columns"], main_freq=sf,
-               main_stream=np.frombuffer(f["main_stream"], dtype=np.uint8).copy(), main_states=states,
-               main_offsets=offsets, residual_stream=np.frombuffer(f["residual_stream"], dtype=np.uint8).copy())
-    if f["mode"] == 128:
-        rf = np.frombuffer(f["residual_table"], dtype="<u4").copy().reshape(1024, 64)
-        rstates, roffsets, residual = checkpoints(f["residual_stream"], rf, f["rows"], f["columns"], (r, c), nr, nc,
-                                                  stride, main)
-        out.update(residual_freq=rf, residual_states=rstates, residual_offsets=roffsets)
-    else:
-        residual = base._unpack6(_native.lib(), f["residual_stream"], n)
-    words = base.join_words(main, residual)
-    if hashlib.sha256(words.tobytes()).digest() != f["digest"]:
-        raise base.CodecError("indexed source checksum mismatch")
+    rf = np.frombuffer(f["residual_table"], dtype="<u4").copy().reshape(1024, 64) if f["mode"] == 128 else None
+    try:
+        quick = base.frame_words(f, stride)
+    except base.CodecError as exc:
+        raise base.CodecError("indexed source checksum mismatch") from exc
+    if quick is not None:
+        words, marks = quick
+    else:   # something is wrong with a stream or its tables, or they are unusual: one stream after the other
+        marks = {}
+        marks["main_states"], marks["main_offsets"], main = checkpoints(f["main_stream"], sf, f["rows"], f["columns"], (r, c), nr, nc, stride)
+        if rf is not None:
+            marks["residual_states"], marks["residual_offsets"], residual = checkpoints(f["residual_stream"], rf, f["rows"], f["columns"], (r, c),
+                                                                                       nr, nc, stride, main)
+        else:
+            residual = base._unpack6(_native.lib(), f["residual_stream"], n)
+        words = base.join_words(main, residual)
+        if hashlib.sha256(words.tobytes()).digest() != f["digest"]:
+            raise base.CodecError("indexed source checksum mismatch")
+    out.update(rows=f["rows"], columns=f["columns"], main_freq=sf, main_stream=np.frombuffer(f["main_stream"], dtype=np.uint8).copy(),
+               residual_stream=np.frombuffer(f["residual_stream"], dtype=np.uint8).copy(), **marks)
+    if rf is not None:
+        out["residual_freq"] = rf
     if keep_words:
         out["words"] = words.reshape(r, c)
     return out

@@ -74,6 +74,28 @@ int bcx_checkpoint(const uint8_t* stream, size_t stream_bytes, uint64_t n, uint3
                    const uint16_t* resctx, const uint32_t* freq, uint32_t stride, uint32_t* states,
                    uint32_t* offsets, uint16_t* symbols);
 
+/* Whole-frame passes (csrc/bcx_frame.cpp): the arithmetic of the functions above, arranged for one pass per frame.
+ * Sums of word & 0x7FFF per row and per column, from which the classes are ranked (cr/bitexact_context_codec.py).
+ * 0 ok, 1 arguments, 3 other. */
+int grb_bctx_magnitudes(const uint16_t* words, uint32_t rows, uint32_t cols, uint64_t* row_sum, uint64_t* col_sum);
+/* The tables of both streams (bcx_frequencies of kinds 0 and 1) and a lower bound of the conditional residual stream's bytes:
+ * an encoder need not produce it when raw residuals are no larger than that.  0 ok, 1 arguments, 3 other. */
+int grb_bctx_frequencies(const uint16_t* words, uint32_t rows, uint32_t cols, const uint8_t* row_class, const uint8_t* col_class,
+                         uint32_t nr, uint32_t nc, uint32_t* main_freq, uint32_t* residual_freq, uint64_t* residual_floor);
+/* One stream under given tables (bcx_encode without the counting).  *stream is malloc'ed: release it with bcx_free. */
+int grb_bctx_encode_stream(const uint16_t* words, uint32_t rows, uint32_t cols, const uint8_t* row_class, const uint8_t* col_class,
+                           uint32_t nr, uint32_t nc, uint32_t kind, const uint32_t* freq, uint8_t** stream, size_t* stream_bytes);
+/* The words of a frame in one pass over its streams and, with stride > 0, the restart points before every stride-th word
+ * (states and offsets as bcx_checkpoint gives them).  residual_freq == NULL: raw residuals (mode 0).  progress (optional)
+ * receives the number of finished rows as they are finished, so that another thread can follow.  0 ok; 1 arguments;
+ * 2 malformed in some way, or tables this pass does not take: outputs must be discarded, bcx_decode and bcx_checkpoint say
+ * how; 3 other. */
+int grb_bctx_frame_words(const uint8_t* main_stream, size_t main_bytes, const uint8_t* residual, size_t residual_bytes, uint32_t rows,
+                         uint32_t cols, const uint8_t* row_class, const uint8_t* col_class, uint32_t nr, uint32_t nc,
+                         const uint32_t* main_freq, const uint32_t* residual_freq, uint32_t stride, uint32_t* main_states,
+                         uint32_t* main_offsets, uint32_t* residual_states, uint32_t* residual_offsets, uint16_t* words,
+                         uint64_t* progress);
+
 /* Tables for grb_bctx_decode_words: cum = u32[nctx][vocab+1] prefix sums, bucket = u16[nctx][4096] symbol
  * owning the first slot of each 16-slot bucket.  Takes the place of the cumulative tables the reference
  * builds in CudaContextTensor.__init__, cr/bitexact_context_gpu.py:120-125.  0 ok, 1 arguments, 2 tables. */
