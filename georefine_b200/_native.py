@@ -5,6 +5,8 @@ There is no fallback: if the library is missing and cannot be built, importing a
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import threading
 from pathlib import Path
@@ -13,6 +15,7 @@ from . import build as _build
 
 _LOCK = threading.Lock()
 _LIB = None
+_FASTCALL = None
 
 U8P = ctypes.POINTER(ctypes.c_uint8)
 U16P = ctypes.POINTER(ctypes.c_uint16)
@@ -153,6 +156,31 @@ def lib():
             _declare(handle)
             _LIB = handle
         return _LIB
+
+
+def fastcall():
+    """The extension module that makes the hot call without ctypes (csrc/fastcall.c)."""
+    global _FASTCALL
+    if _FASTCALL is None:
+        lib()                                 # builds both when sources are newer
+        loader = importlib.machinery.ExtensionFileLoader("_fastcall", str(_build.FASTCALL))
+        _FASTCALL = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", str(_build.FASTCALL), loader=loader))
+        loader.exec_module(_FASTCALL)
+    return _FASTCALL
+
+
+def raw_stream(device_index: int) -> int:
+    """cudaStream_t of the current stream of a device, without making a Stream object of it."""
+    import torch
+
+    return torch._C._cuda_getCurrentRawStream(device_index)
+
+
+class LinearRecord(ctypes.Structure):
+    """The constant arguments of one weight's linear (csrc/fastcall.c)."""
+
+    _fields_ = [("entry", VOIDP), ("image", VOIDP), ("header", VOIDP), ("workspace", VOIDP), ("workspace_bytes", ctypes.c_uint64),
+                ("status", VOIDP), ("next_image", VOIDP), ("next_header", VOIDP)]
 
 
 def check(status: int, what: str) -> None:

@@ -1,4 +1,5 @@
-"""Builds libgeorefine_b200.so (host coder + CUDA kernels + C ABI) in-tree for sm_100a with nvcc.
+"""Builds libgeorefine_b200.so (host coder + CUDA kernels + C ABI) in-tree for sm_100a with nvcc, and _fastcall.so, the
+binding of its hot call for this Python.
 
     python -m georefine_b200.build [--force] [--verbose]
 
@@ -10,12 +11,14 @@ from __future__ import annotations
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 OUT = PKG / "_build" / "libgeorefine_b200.so"
 SOURCES = [CSRC / "capi.cu", CSRC / "bcx_host.cpp", CSRC / "bcx_frame.cpp", CSRC / "bxr_build.cpp"]
+FASTCALL_SOURCE, FASTCALL = CSRC / "fastcall.c", PKG / "_build" / "_fastcall.so"
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
          "-Xcompiler", "-pthread", "-shared"]
 
@@ -25,9 +28,9 @@ def _inputs():
 
 
 def needs_build() -> bool:
-    if not OUT.exists():
+    if not OUT.exists() or not FASTCALL.exists():
         return True
-    stamp = OUT.stat().st_mtime
+    stamp = min(OUT.stat().st_mtime, FASTCALL.stat().st_mtime)
     return any(p.stat().st_mtime > stamp for p in _inputs())
 
 
@@ -44,6 +47,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         sys.stderr.write(run.stderr)
     if run.returncode:
         raise RuntimeError("nvcc failed:\n" + run.stderr[-4000:])
+    run = subprocess.run([shutil.which("gcc") or "cc", "-O2", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], str(FASTCALL_SOURCE), "-o",
+                          str(FASTCALL)], capture_output=True, text=True)
+    if run.returncode:
+        raise RuntimeError("the call binding failed to build:\n" + run.stderr[-4000:])
     return OUT
 
 

@@ -20,6 +20,24 @@ LAYOUTS = {"rans": 0, "raw": 1, "window": 2, "window4": 3}   # bxr_format.h: BXR
 DEFAULT_LAYOUT = "window4"                       # the fastest layout (12 bits/weight); "window" 11.3, "rans" 11.1 bits/weight
 
 
+_BF16 = None
+
+
+def _bfloat16():
+    global _BF16
+    if _BF16 is None:
+        import torch
+
+        _BF16 = torch.bfloat16
+    return _BF16
+
+
+def _current_device() -> int:
+    import torch
+
+    return torch._C._cuda_getDevice()
+
+
 def sm_count(device) -> int:
     import torch
 
@@ -108,6 +126,8 @@ class ResidentWeight:
             if hashlib.sha256(words.astype("<u2").tobytes()).digest() != bytes(h.source_sha256):
                 raise ValueError("resident image does not reproduce its source digest")
         self.device = torch.device(device)
+        if self.device.index is None:
+            self.device = torch.device(self.device.type, torch.cuda.current_device())
         self.N, self.K = int(h.rows), int(h.cols)
         self.mode = int(h.mode)
         self.image = torch.from_numpy(image).to(self.device)
@@ -115,6 +135,7 @@ class ResidentWeight:
         self.max_m = 0
         self.workspace = None
         self.next_weight = None     # see then()
+        self._bound = None          # see _bind()
         self.reserve(max_m)
 
     @classmethod
@@ -196,28 +217,27 @@ class ResidentWeight:
             raise ValueError(f"resident decode reported status {self.status.item()}")
         return out
 
-    def _run(self, entry, x, y, bias, extra=()):
-        import torch
-
-        if x.dim() != 2 or y.dim() != 2 or x.dtype != torch.bfloat16 or y.dtype != torch.bfloat16:
+    def _checked(self, x, y):
+        """The batch size of a call, its shapes and types checked."""
+        m, k = x.shape
+        rows, n = y.shape
+        if x.dtype is not _bfloat16() or y.dtype is not _BF16:
             raise ValueError("x and y must be 2-D BF16 tensors")
-        m = x.shape[0]
-        if x.shape[1] != self.K or y.shape != (m, self.N) or x.stride(1) != 1 or y.stride(1) != 1:
+        if k != self.K or rows != m or n != self.N or x.stride(1) != 1 or y.stride(1) != 1:
             raise ValueError("shape mismatch: x [M, K], y [M, N], unit inner stride")
-        if m == 0:
-            return
         if m > self.max_m and min(m, 128) > min(self.max_m, 128):
             raise ValueError(f"batch of {m} rows exceeds the reserved scratch ({self.max_m}); call reserve() first")
-        args = (self.image.data_ptr(), ctypes.byref(self.header), x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0),
-                None if bias is None else bias.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(),
-                self.status.data_ptr(), torch.cuda.current_stream(self.device).cuda_stream, *extra)
-        if torch.cuda.current_device() == self.device.index:   # the usual case: skip the device switch
-            st = entry(*args)
-        else:
-            with torch.cuda.device(self.device):
-                st = entry(*args)
-        if st:
-            _native.check(st, entry.__name__)
+        return m
+
+    def _bind(self):
+        """The call record of this weight: address, and what it was made from, so that a replaced buffer is noticed."""
+        nxt = self.next_weight
+        record = _native.LinearRecord(
+            ctypes.cast(_native.lib().grb_bxr_gemm_next, ctypes.c_void_p).value, self.image.data_ptr(), ctypes.addressof(self.header),
+            self.workspace.data_ptr(), self.workspace.numel(), self.status.data_ptr(), None if nxt is None else nxt.image.data_ptr(),
+            None if nxt is None else ctypes.addressof(nxt.header))
+        self._bound = (self.image, self.workspace, self.status, nxt, ctypes.addressof(record), _native.fastcall().gemm, record)
+        return self._bound
 
     def then(self, next_weight):
         """Tells this weight which one the stream multiplies by next (None: nobody).  A hint for the kernel: while a
@@ -228,15 +248,42 @@ class ResidentWeight:
 
     def gemm(self, x, y, bias=None):
         """tcgen05 path, any M; rows of y are bitwise independent of M."""
-        nxt = self.next_weight
-        if nxt is None:
-            self._run(_native.lib().grb_bxr_gemm, x, y, bias)
+        if x.dim() != 2 or y.dim() != 2:
+            raise ValueError("x and y must be 2-D BF16 tensors")
+        m = self._checked(x, y)
+        if not m:
+            return
+        bound = self._bound
+        if bound is None or bound[0] is not self.image or bound[1] is not self.workspace or bound[2] is not self.status or bound[3] is not self.next_weight:
+            bound = self._bind()
+        index = self.device.index
+        call = bound[5]
+        args = (bound[4], x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0), 0 if bias is None else bias.data_ptr(), _native.raw_stream(index))
+        if _current_device() == index:   # the usual case: skip the device switch
+            st = call(*args)
         else:
-            self._run(_native.lib().grb_bxr_gemm_next, x, y, bias, extra=(nxt.image.data_ptr(), ctypes.byref(nxt.header)))
+            import torch
+
+            with torch.cuda.device(self.device):
+                st = call(*args)
+        if st:
+            _native.check(st, "grb_bxr_gemm")
 
     def gemv(self, x, y, bias=None):
         """CUDA-core path, M <= 8; rows of y are bitwise independent of M within 1..8."""
-        self._run(_native.lib().grb_bxr_gemv, x, y, bias)
+        import torch
+
+        if x.dim() != 2 or y.dim() != 2:
+            raise ValueError("x and y must be 2-D BF16 tensors")
+        m = self._checked(x, y)
+        if not m:
+            return
+        with torch.cuda.device(self.device):
+            st = _native.lib().grb_bxr_gemv(self.image.data_ptr(), ctypes.byref(self.header), x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0),
+                                            None if bias is None else bias.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(),
+                                            self.status.data_ptr(), self._stream())
+        if st:
+            _native.check(st, "grb_bxr_gemv")
 
     def __call__(self, x, y):
         self.gemm(x, y)
@@ -245,7 +292,7 @@ class ResidentWeight:
         import torch
 
         lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1])
+        x2 = x if len(lead) == 1 else x.reshape(-1, x.shape[-1])
         if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
             if self.K % 8:  # the kernels want a row stride that is a multiple of 16 bytes
                 padded = torch.zeros((x2.shape[0], (self.K + 7) // 8 * 8), device=self.device, dtype=torch.bfloat16)
@@ -253,11 +300,17 @@ class ResidentWeight:
                 x2 = padded[:, :self.K]
             else:
                 x2 = x2.contiguous()
-        y = torch.empty((x2.shape[0], self.N), device=self.device, dtype=torch.bfloat16) if out is None else out.reshape(-1, self.N)
-        if x2.shape[0] > self.max_m:
-            self.reserve(x2.shape[0])
+        m = x2.shape[0]
+        if out is not None:
+            y = out.reshape(-1, self.N)
+        elif x.dtype is _bfloat16() and x.device == self.device:
+            y = x.new_empty((m, self.N))
+        else:
+            y = torch.empty((m, self.N), device=self.device, dtype=torch.bfloat16)
+        if m > self.max_m:
+            self.reserve(m)
         self.gemm(x2, y, bias)
-        return y.reshape(*lead, self.N)
+        return y if len(lead) == 1 and out is None else y.reshape(*lead, self.N)
 
     def check_status(self) -> int:
         """Host read of the device status word (synchronises); 0 means every call since the last reset was clean."""

@@ -34,8 +34,10 @@ class BctxLinear(nn.Module):
         return self.context_weight.decode()
 
     def forward(self, x):
-        self.forward_calls += 1
-        bias = None if self.bias is None else self.bias.to(torch.bfloat16)
+        self.__dict__["forward_calls"] += 1       # (past nn.Module's attribute machinery: this is a per-call path)
+        bias = self._parameters["bias"]
+        if bias is not None and bias.dtype is not torch.bfloat16:
+            bias = bias.to(torch.bfloat16)
         return self.context_weight.linear(x, bias=bias)
 
 
