@@ -158,14 +158,15 @@ def lib():
         return _LIB
 
 
-def fastcall():
-    """The extension module that makes the hot call without ctypes (csrc/fastcall.c)."""
+def gemm_next():
+    """(the call without ctypes of csrc/fastcall.c, the address of grb_bxr_gemm_next it takes first)."""
     global _FASTCALL
     if _FASTCALL is None:
-        lib()                                 # builds both when sources are newer
+        entry = ctypes.cast(lib().grb_bxr_gemm_next, VOIDP).value     # (builds both libraries when sources are newer)
         loader = importlib.machinery.ExtensionFileLoader("_fastcall", str(_build.FASTCALL))
-        _FASTCALL = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", str(_build.FASTCALL), loader=loader))
-        loader.exec_module(_FASTCALL)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", str(_build.FASTCALL), loader=loader))
+        loader.exec_module(module)
+        _FASTCALL = module.gemm_next, entry
     return _FASTCALL
 
 
@@ -174,13 +175,6 @@ def raw_stream(device_index: int) -> int:
     import torch
 
     return torch._C._cuda_getCurrentRawStream(device_index)
-
-
-class LinearRecord(ctypes.Structure):
-    """The constant arguments of one weight's linear (csrc/fastcall.c)."""
-
-    _fields_ = [("entry", VOIDP), ("image", VOIDP), ("header", VOIDP), ("workspace", VOIDP), ("workspace_bytes", ctypes.c_uint64),
-                ("status", VOIDP), ("next_image", VOIDP), ("next_header", VOIDP)]
 
 
 def check(status: int, what: str) -> None:

@@ -135,7 +135,6 @@ class ResidentWeight:
         self.max_m = 0
         self.workspace = None
         self.next_weight = None     # see then()
-        self._bound = None          # see _bind()
         self.reserve(max_m)
 
     @classmethod
@@ -229,16 +228,6 @@ class ResidentWeight:
             raise ValueError(f"batch of {m} rows exceeds the reserved scratch ({self.max_m}); call reserve() first")
         return m
 
-    def _bind(self):
-        """The call record of this weight: address, and what it was made from, so that a replaced buffer is noticed."""
-        nxt = self.next_weight
-        record = _native.LinearRecord(
-            ctypes.cast(_native.lib().grb_bxr_gemm_next, ctypes.c_void_p).value, self.image.data_ptr(), ctypes.addressof(self.header),
-            self.workspace.data_ptr(), self.workspace.numel(), self.status.data_ptr(), None if nxt is None else nxt.image.data_ptr(),
-            None if nxt is None else ctypes.addressof(nxt.header))
-        self._bound = (self.image, self.workspace, self.status, nxt, ctypes.addressof(record), _native.fastcall().gemm, record)
-        return self._bound
-
     def then(self, next_weight):
         """Tells this weight which one the stream multiplies by next (None: nobody).  A hint for the kernel: while a
         launch over this weight winds down, the L2 is asked for the first blobs of the next one.  Returns
@@ -253,12 +242,11 @@ class ResidentWeight:
         m = self._checked(x, y)
         if not m:
             return
-        bound = self._bound
-        if bound is None or bound[0] is not self.image or bound[1] is not self.workspace or bound[2] is not self.status or bound[3] is not self.next_weight:
-            bound = self._bind()
-        index = self.device.index
-        call = bound[5]
-        args = (bound[4], x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0), 0 if bias is None else bias.data_ptr(), _native.raw_stream(index))
+        nxt, index = self.next_weight, self.device.index
+        call, entry = _native.gemm_next()
+        args = (entry, self.image.data_ptr(), ctypes.addressof(self.header), x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0),
+                0 if bias is None else bias.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(), self.status.data_ptr(),
+                _native.raw_stream(index), 0 if nxt is None else nxt.image.data_ptr(), 0 if nxt is None else ctypes.addressof(nxt.header))
         if _current_device() == index:   # the usual case: skip the device switch
             st = call(*args)
         else:
