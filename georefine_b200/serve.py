@@ -284,8 +284,9 @@ class BatchDecoder:
                 self.page_table[slot, p] = page
 
     # ---- the step ----------------------------------------------------------------------------------------------
-    def _trunk(self, n: int, advance: bool) -> None:
-        """One pass of rows 0..n-1 through the stack on the current stream; no allocation, no host synchronisation."""
+    def _trunk(self, n: int, advance: bool, head: bool = True) -> None:
+        """One pass of rows 0..n-1 through the stack on the current stream; no allocation, no host synchronisation.
+        ``head=False`` stops at the residual stream: no logits, no arg-max."""
         import torch
 
         cfg, w = self.cfg, self.w
@@ -304,6 +305,8 @@ class BatchDecoder:
             self._row_parallel(layer.down, "down", self.act[:n], self.down_out[:n])
             delta = self.down_out[:n]
         ops.rmsnorm(h, w.final_norm, x, delta=delta, eps=cfg.eps)          # h now holds the final residual stream
+        if not head:
+            return
         w.lm_head(x, self.logits[:n])
         ops.argmax(self.logits[:n], self.next_token[:n])
         if advance:
@@ -346,12 +349,28 @@ class BatchDecoder:
             self.run(kind, n)
 
     def set_rows(self, slots, positions, tokens) -> None:
-        """Host -> device: which (slot, position, token) each of the first len(slots) rows carries."""
+        """Host -> device: which (slot, position, token) each of the first len(slots) rows carries.  The rows are there,
+        for every stream, when the call returns."""
+        import torch
+
+        self.queue_rows(slots, positions, tokens)
+        torch.cuda.current_stream(self.dev).synchronize()
+
+    def absorb(self, slots, positions, tokens) -> None:
+        """Queues the rows and the step that appends them to their sequences' KV pages; their logits are not wanted."""
+        self.queue_rows(slots, positions, tokens)
+        self._trunk(len(slots), False, head=False)
+
+    def queue_rows(self, slots, positions, tokens) -> None:
+        """``set_rows`` without the wait, for a caller whose step follows on the same stream.  The rows go through pinned
+        memory that the caching host allocator does not hand out again before the copies are done; copies from
+        pageable memory would each wait for everything the stream has before them."""
         import torch
 
         n = len(slots)
-        rows = torch.tensor([list(slots), list(positions), list(tokens)], dtype=torch.int32)
-        self.row_seq[:n].copy_(rows[0]); self.row_pos[:n].copy_(rows[1]); self.tokens[:n].copy_(rows[2])
+        rows = torch.tensor([list(slots), list(positions), list(tokens)], dtype=torch.int32, pin_memory=True)
+        for src, dst in zip(rows, (self.row_seq, self.row_pos, self.tokens)):
+            dst[:n].copy_(src, non_blocking=True)
 
     def streamed_bytes(self, rows_context) -> dict:
         """Bytes one step streams: the compressed weights, and the KV cache of rows whose contexts are given."""
@@ -378,6 +397,8 @@ class Batcher:
         self.d, self.buckets = decoder, tuple(b for b in buckets if b <= decoder.max_rows)
         self.active = {}            # slot -> {"pos": position of the next input token, "tokens": generated so far}
         self._order, self._dirty = [], True
+        # (a decoder need not have these two: rows set and run step by step are the same rows)
+        self._rows, self._absorb = getattr(decoder, "queue_rows", decoder.set_rows), getattr(decoder, "absorb", None)
 
     def admit(self, prompt_ids, *, sampler=None) -> int:
         """Processes a prompt and returns the sequence's slot; its first generated token is in ``active[slot]['tokens']``
@@ -389,17 +410,27 @@ class Batcher:
         self.sync_tokens()                    # the row buffers are about to be reused for the prompt
         slot = d.open_slot()
         d.ensure_pages(slot, len(ids))
-        first = None
-        for lo in range(0, len(ids), d.max_rows):
-            chunk = ids[lo:lo + d.max_rows]
-            d.set_rows([slot] * len(chunk), range(lo, lo + len(chunk)), chunk)
-            d.run("verify", len(chunk), graph=False)
-            first = int(d.next_token[len(chunk) - 1].item())
+        first = int(d.next_token[self._take_in(slot, 0, ids) - 1].item())
         if sampler is not None:
-            first = int(sampler.draw(d.logits[len(chunk) - 1][None])[0])
+            first = int(sampler.draw(d.logits[(len(ids) - 1) % d.max_rows][None])[0])
         self.active[slot] = {"pos": len(ids), "tokens": [first]}
         self._dirty = True
         return slot
+
+    def _take_in(self, slot: int, first: int, ids) -> int:
+        """Runs the tokens ``ids`` at positions ``first``.. of a sequence through the decoder in chunks of its rows; returns
+        the number of rows of the last chunk.  The chunks follow one another on the stream without the host waiting for
+        any of them, and the output head runs for the last one only: the other rows' logits have no reader."""
+        d = self.d
+        for lo in range(0, len(ids), d.max_rows):
+            chunk = ids[lo:lo + d.max_rows]
+            rows = [slot] * len(chunk), range(first + lo, first + lo + len(chunk)), chunk
+            if lo + len(chunk) < len(ids) and self._absorb is not None:
+                self._absorb(*rows)
+            else:
+                self._rows(*rows)
+                d.run("verify", len(chunk), graph=False)
+        return len(chunk)
 
     def retire(self, slot: int) -> None:
         self.sync_tokens()
@@ -441,7 +472,7 @@ class Batcher:
             self.sync_tokens()
             self._order = wanted
             pad = b - n
-            d.set_rows(self._order + [d.pad_slot] * pad, [self.active[s]["pos"] for s in self._order] + [0] * pad,
+            self._rows(self._order + [d.pad_slot] * pad, [self.active[s]["pos"] for s in self._order] + [0] * pad,
                        [self.active[s]["tokens"][-1] for s in self._order] + [0] * pad)
             self._dirty = False
         d.run("ar", b)
@@ -482,7 +513,7 @@ class Batcher:
         out, at = {}, 0
         if len(slots) > d.max_rows:
             raise ValueError("verify pass larger than the decoder's row buffers")
-        d.set_rows(slots, positions, tokens)
+        self._rows(slots, positions, tokens)
         d.run("verify", len(slots))
         argmax_rows = d.next_token[:len(slots)].tolist()
         for slot, ds in drafts.items():
@@ -611,10 +642,7 @@ class FastSession:
         seq, d = self.batcher.active[st.slot], self.d
         feed = [seq["tokens"][-1]] + ids[:-1]
         d.ensure_pages(st.slot, seq["pos"] + len(ids))
-        for lo in range(0, len(feed), d.max_rows):
-            chunk = feed[lo:lo + d.max_rows]
-            d.set_rows([st.slot] * len(chunk), range(seq["pos"] + lo, seq["pos"] + lo + len(chunk)), chunk)
-            d.run("verify", len(chunk), graph=False)
+        self.batcher._take_in(st.slot, seq["pos"], feed)
         seq["tokens"] += ids
         seq["pos"] += len(ids)
         self.batcher._dirty = True
