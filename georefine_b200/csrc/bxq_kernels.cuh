@@ -22,7 +22,7 @@ constexpr int kWideWarpMma2 = 19;      // MMA issuer of the odd chunks
 constexpr int kWideWarpXLoader = 18;   // TMA loads of activation tiles
 constexpr int kWideWarpEpilogue = 20;  // 4 warps: warp % 4 = the tensor-memory lane quarter a warp may read
 
-// Tensor memory: columns [0, 256) accumulators, FP32: an item has two, one per MMA issuer (even chunks, odd chunks;
+// Tensor memory (up to NB = 128): columns [0, 256) accumulators, FP32: an item has two, one per MMA issuer (even chunks, odd chunks;
 // the epilogue adds them), NB columns each.  Up to NB = 64 two items fit (one being multiplied, one being drained);
 // at NB = 128 there is room for one, and the issuers wait for the drain at an item boundary while the decoders fill
 // the operand stages.  Columns [256, 512): the decoded weights of four chunks, 64 columns each (two 128 x 64 atoms, two
@@ -30,8 +30,13 @@ constexpr int kWideWarpEpilogue = 20;  // 4 warps: warp % 4 = the tensor-memory 
 // NB = 16 with 7 stages, 8 activation stages and 6 requests in flight, every M = 1 launch got slower, gate|up by 4.6 us.)
 constexpr int kWideNextBlobs = 8;      // blobs per CTA of the next launch that a finishing CTA asks the L2 for
 constexpr uint32_t kWideTmemCols = 512;
+// The 192-column tile, for batches above 128 rows: its accumulators take 384 columns and leave two operand stages, enough
+// because a chunk's multiply (768 tensor-core cycles) is longer than the hand-over it has to hide.  Such a batch is bound by
+// the number of its passes over the weights: at 128 columns the tensor core is busy for 38 % of a pass, and a pass costs
+// little more at 192 (34816 x 5120: 63.3 -> 78.1 us).  768 rows, six passes -> four: 34816 x 5120 394 -> 320 us,
+// 5120 x 17408 217 -> 184 us, 5120 x 5120 94 -> 75 us.
 template <int NB>
-constexpr int kWideStages = 4;
+constexpr int kWideStages = NB <= 128 ? 4 : 2;
 template <int NB>
 constexpr uint32_t kWideOperandCol = kWideTmemCols - 64u * kWideStages<NB>;
 
@@ -47,7 +52,9 @@ struct BxqSmem {
   static constexpr uint32_t kReserve = 1024 /* alignment slack */ + 512 /* barriers, flags */;
   // the epilogue warps turn their accumulator columns around in shared memory (a lane holds one weight row, memory
   // wants consecutive rows together): 16 columns x 32 rows x 4 bytes per warp
-  static constexpr uint32_t kTurn = (MODE == kUmma) ? 2048u : 0u;
+  // (8 columns at a time where the activation ring leaves no room for 16)
+  static constexpr int kTurnCols = NB <= 128 ? 16 : 8;
+  static constexpr uint32_t kTurn = (MODE == kUmma) ? kTurnCols * 128u : 0u;
   static constexpr int kInFit = int((232448u - kReserve - kX * kXStage - 4 * kTurn) / BXQ_BLOB_MAX);
   static constexpr int kIn = kInFit > 7 ? 7 : kInFit;   // (more barriers would not fit the one-per-lane set-up)
   static constexpr uint32_t xs = 0;
@@ -56,12 +63,12 @@ struct BxqSmem {
   static constexpr uint32_t bars = in + kIn * BXQ_BLOB_MAX;
   // barrier order: in_full, in_empty [kIn each]; op_full, op_empty [kOp each]; x_full [kX]; acc_full, acc_empty
   // [2 each]; final; tile_full, tile_used [kRing each] (the closing reduction)
-  static constexpr uint32_t kRing = (NB <= 64) ? 4 : 2;  // tiles in flight in the closing reduction (kWideTileRing)
+  static constexpr uint32_t kRing = (NB <= 64) ? 4 : (NB <= 128) ? 2 : 1;  // tiles in flight in the closing reduction (kWideTileRing)
   static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + kX + 4 + 1 + 2 * kRing;
   static constexpr uint32_t misc = (bars + 8 * nbars + 15) & ~15u;  // tmem base, abort flag, decision
   static constexpr uint32_t total = misc + 48;
   static constexpr uint32_t alloc = total + 1024;
-  static_assert(MODE != kUmma || kIn >= 4, "ring too shallow");
+  static_assert(MODE != kUmma || kIn >= 3, "ring too shallow");
   // what keeps the activation loader at most one barrier phase behind the MMA issuer (see its role below)
   static_assert(MODE != kUmma || (kXLag < kX && kOp + kXLag + 1 > kX), "activation ring and lag do not fit the operand ring");
   static_assert(MODE != kUmma || 2 * NB * (NB <= 64 ? 2 : 1) <= int(kWideOperandCol<NB>), "accumulators overlap the operand columns");
@@ -130,7 +137,7 @@ __device__ __forceinline__ WideSpan wide_span(uint32_t unit, uint32_t unit_end, 
 // takes part, lies at [0, T) and was never in memory).  A thread owns the same few float4 positions of every tile and
 // keeps their running sums in registers.  `fetched` counts the tiles brought in so far by this CTA (barrier phases).
 template <int NB>
-constexpr uint32_t kWideTileRing = NB <= 64 ? 4 : 2;  // (1 + ring) x NB x 512 bytes of shared memory
+constexpr uint32_t kWideTileRing = NB <= 64 ? 4 : NB <= 128 ? 2 : 1;  // (1 + ring) x NB x 512 bytes of shared memory
 
 template <int NB>
 __device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const RoleCtx& ctx, uint32_t row_block, uint32_t first,
@@ -582,7 +589,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t taddr = tmem_base + ((e * 32) << 16) + buf * 2 * NB;   // even-chunk accumulator; the odd one NB columns on
       const bool two = item.chunk_end - item.chunk_begin > 1;                // a one-chunk item has no odd chunk
       const float b = (args.bias && row < args.rows) ? __bfloat162float(args.bias[row]) : 0.f;
-      constexpr int kStep = 16;  // accumulator columns per tensor-memory load
+      constexpr int kStep = L::kTurnCols;  // accumulator columns per tensor-memory load
       // The CTA's last item, if it is part of a split row block, keeps its tile in shared memory (all of it is free
       // by now: every blob and every activation tile has been multiplied).  If the other tiles of the row block are already in memory -
       // the usual case, they were finished long ago as some CTA's first item - this tile never goes to memory at
@@ -602,10 +609,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
                           item.row_block * BXR_ROWS + e * 32 + 32 <= args.rows;
       for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
         uint32_t v[kStep];
-        tmem_ld16(taddr + m0, v);
+        tmem_ld(taddr + m0, v);
         if (two) {
           uint32_t odd[kStep];
-          tmem_ld16(taddr + NB + m0, odd);
+          tmem_ld(taddr + NB + m0, odd);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < kStep; ++i) v[i] = __float_as_uint(__fadd_rn(__uint_as_float(v[i]), __uint_as_float(odd[i])));

@@ -25,6 +25,15 @@ int cuda_status(cudaError_t e) { return e == cudaSuccess ? GRB_OK : GRB_ERR_CUDA
 
 uint32_t batch_tile(uint32_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
 
+// Batches above 128 rows over 4-bit window images: a pass over the weights may take 192 rows, and costs little more than
+// one of 128.  Rows of the next pass when `left` are still to be multiplied: 192 unless two passes of 128 do for what is
+// left just as well (193 to 256 rows).
+constexpr uint32_t kWideTile = 192;
+uint32_t wide_pass_rows(uint32_t left) {
+  if (left <= 128) return left;
+  return left <= kWideTile ? left : left <= 256 ? 128 : kWideTile;
+}
+
 uint64_t counter_bytes(const bxr_header* h) { return (uint64_t(h->row_blocks) * 4 + 255) & ~uint64_t(255); }
 
 bool header_ok(const bxr_header* h) {
@@ -103,6 +112,17 @@ uint32_t cluster_of(const BxrArgs& a) {
   return (p >= 2 && p <= 8 && a.chunks >= p) ? p : 1;
 }
 
+// Does a batch above 128 rows need more scratch than one of 128?  (Clusters keep their partial tiles in shared memory.)
+bool wide_tile_image(const bxr_header* h) {
+  if (h->mode != BXR_MODE_WINDOW4) return false;
+  BxrArgs a{};
+  a.row_blocks = h->row_blocks;
+  a.chunks = h->chunks;
+  a.workers = h->workers;
+  a.window4 = true;
+  return cluster_of(a) == 1;
+}
+
 template <int MODE>
 constexpr int kFusedThreads = MODE == kUmma ? kThreadsUmma : kThreadsSimt;
 
@@ -175,6 +195,12 @@ int gemm_tile(BxrArgs a, const void* x, int64_t ldx, cudaStream_t stream) {
   if (st) return st;
   if (a.window4) return launch_wide<kUmma, NB>(a, map, stream);
   return a.window ? launch_window<kUmma, NB>(a, map, stream) : launch<kUmma, NB>(a, map, stream);
+}
+
+int gemm_tile_wide(const BxrArgs& a, const void* x, int64_t ldx, cudaStream_t stream) {
+  CUtensorMap map;
+  const int st = make_x_map(&map, x, ldx, a.m, a.cols, kWideTile);
+  return st ? st : launch_wide<kUmma, int(kWideTile)>(a, map, stream);
 }
 
 template <int M>
@@ -294,7 +320,7 @@ extern "C" {
 
 uint64_t grb_bxr_workspace_bytes(const bxr_header* h, uint32_t max_m) {
   if (!header_ok(h) || !max_m) return 0;
-  const uint64_t tile = batch_tile(max_m > 128 ? 128 : max_m);
+  const uint64_t tile = max_m > 128 && wide_tile_image(h) ? kWideTile : batch_tile(max_m > 128 ? 128 : max_m);
   return counter_bytes(h) + uint64_t(h->partial_slots) * tile * BXR_ROWS * 4;
 }
 
@@ -456,12 +482,15 @@ int grb_bxr_gemm_next(const void* image, const bxr_header* h, const void* x, int
     a.next_units = next_header->row_blocks * next_header->chunks;
     a.next_workers = next_header->workers;
   }
-  // Batches above one tile are processed as consecutive tiles: one pass over the weights per 128 rows.
-  for (uint32_t m0 = 0; m0 < m; m0 += 128) {
-    a.m = m - m0 < 128 ? m - m0 : 128;
+  // Batches above one tile are processed as consecutive tiles, one pass over the weights each.  The wide tile needs wider
+  // slots for its partial tiles; a caller whose scratch was sized for 128 rows gets tiles of 128.
+  const bool wide = m > 128 && a.window4 && (cluster_of(a) > 1 || ws_bytes >= counter_bytes(h) + uint64_t(h->partial_slots) * kWideTile * BXR_ROWS * 4);
+  for (uint32_t m0 = 0; m0 < m; m0 += a.m) {
+    a.m = wide ? wide_pass_rows(m - m0) : std::min(m - m0, 128u);
     const auto* xt = static_cast<const __nv_bfloat16*>(x) + size_t(m0) * ldx;
     a.y = static_cast<__nv_bfloat16*>(y) + size_t(m0) * ldy;
-    switch (batch_tile(a.m)) {
+    if (a.m > 128) st = gemm_tile_wide(a, xt, ldx, stream);
+    else switch (batch_tile(a.m)) {
       case 16: st = gemm_tile<16>(a, xt, ldx, stream); break;
       case 32: st = gemm_tile<32>(a, xt, ldx, stream); break;
       case 64: st = gemm_tile<64>(a, xt, ldx, stream); break;

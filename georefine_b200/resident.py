@@ -193,8 +193,19 @@ class ResidentWeight:
             return
         need = int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(self.header), max_m))
         need = max(need, int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(self.header), GEMV_MAX_M)))
-        self.workspace = torch.zeros(max(need, 256), device=self.device, dtype=torch.uint8)
+        if self.workspace is None or need > self.workspace.numel():
+            self.workspace = torch.zeros(max(need, 256), device=self.device, dtype=torch.uint8)
         self.max_m = max_m
+
+    def _widen(self, m: int) -> None:
+        """Scratch for the 192-row passes of a batch above 128 rows, on the first such batch.  The scratch it replaces lives
+        as long as the weight: a captured graph may have its address.  During a capture nothing is allocated and the
+        batch runs in passes of 128 rows, which the scratch has room for."""
+        import torch
+
+        if not torch.cuda.is_current_stream_capturing():
+            self._narrow_workspace = self.workspace
+            self.reserve(m)
 
     # -- device entry points -------------------------------------------------------------------------
     def _stream(self):
@@ -242,6 +253,8 @@ class ResidentWeight:
         m = self._checked(x, y)
         if not m:
             return
+        if m > 128 >= self.max_m:
+            self._widen(m)
         nxt, index = self.next_weight, self.device.index
         call, entry = _native.gemm_next()
         args = (entry, self.image.data_ptr(), ctypes.addressof(self.header), x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0),
