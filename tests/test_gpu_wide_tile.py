@@ -53,3 +53,24 @@ def test_scratch_of_128_rows_still_serves_any_batch():
     assert r.max_m == 400
     graph.replay()
     assert r.check_status() == 0 and torch.equal(y, want)
+
+
+@pytest.mark.parametrize("length", [128, 129, 256, 257, 513, 640, 1000])
+def test_prompt_in_wide_chunks_equals_chunks_of_a_step(length):
+    from georefine_b200 import serve
+
+    dev = torch.device("cuda:0")
+    cfg = serve.DecoderConfig(hidden=640, layers=2, heads=10, kv_heads=2, ffn=1792, vocab=1000)
+    weights = serve.DecoderWeights.synthetic(cfg, dev, seed=5)
+    ids = torch.randint(0, cfg.vocab, (length,), generator=torch.Generator().manual_seed(length)).tolist()
+    got = []
+    for wide in (False, True):
+        d = serve.BatchDecoder(weights, max_rows=128, max_slots=2, max_context=1024, device=dev)
+        assert d.prompt_rows == serve.PROMPT_ROWS
+        b = serve.Batcher(d)
+        if not wide:
+            b._absorb = None
+        slot = b.admit(ids)
+        tokens = list(b.active[slot]["tokens"]) + [b.step()[slot] for _ in range(3)]
+        got.append((tokens, d.kv.clone(), d.logits[:1].clone()))
+    assert got[0][0] == got[1][0] and torch.equal(got[0][1][:, :, :-1], got[1][1][:, :, :-1]) and torch.equal(got[0][2], got[1][2])
