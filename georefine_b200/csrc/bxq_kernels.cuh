@@ -33,8 +33,8 @@ constexpr uint32_t kWideTmemCols = 512;
 // The 192-column tile, for batches above 128 rows: its accumulators take 384 columns and leave two operand stages, enough
 // because a chunk's multiply (768 tensor-core cycles) is longer than the hand-over it has to hide.  Such a batch is bound by
 // the number of its passes over the weights: at 128 columns the tensor core is busy for 38 % of a pass, and a pass costs
-// little more at 192 (34816 x 5120: 63.3 -> 78.1 us).  768 rows, six passes -> four: 34816 x 5120 394 -> 320 us,
-// 5120 x 17408 217 -> 184 us, 5120 x 5120 94 -> 75 us.
+// little more at 192 (34816 x 5120: 62 -> 74.4 us).  768 rows, six passes -> four: 34816 x 5120 394 -> 306 us,
+// 5120 x 17408 217 -> 177 us, 5120 x 5120 94 -> 72 us.
 template <int NB>
 constexpr int kWideStages = NB <= 128 ? 4 : 2;
 template <int NB>
@@ -589,7 +589,9 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t taddr = tmem_base + ((e * 32) << 16) + buf * 2 * NB;   // even-chunk accumulator; the odd one NB columns on
       const bool two = item.chunk_end - item.chunk_begin > 1;                // a one-chunk item has no odd chunk
       const float b = (args.bias && row < args.rows) ? __bfloat162float(args.bias[row]) : 0.f;
-      constexpr int kStep = L::kTurnCols;  // accumulator columns per tensor-memory load
+      constexpr int kStep = 16, kCols = L::kTurnCols;  // accumulator columns per tensor-memory load, and per turn-around
+      // (a load's round trip is what a step waits for: 16 columns per load where only 8 fit the turn-around took a
+      // pass of 192 rows over 34816 x 5120 from 76.1 to 74.4 us, over 5120 x 5120 from 19.1 to 18.5 us)
       // The CTA's last item, if it is part of a split row block, keeps its tile in shared memory (all of it is free
       // by now: every blob and every activation tile has been multiplied).  If the other tiles of the row block are already in memory -
       // the usual case, they were finished long ago as some CTA's first item - this tile never goes to memory at
@@ -609,10 +611,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
                           item.row_block * BXR_ROWS + e * 32 + 32 <= args.rows;
       for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
         uint32_t v[kStep];
-        tmem_ld(taddr + m0, v);
+        tmem_ld16(taddr + m0, v);
         if (two) {
           uint32_t odd[kStep];
-          tmem_ld(taddr + NB + m0, odd);
+          tmem_ld16(taddr + NB + m0, odd);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < kStep; ++i) v[i] = __float_as_uint(__fadd_rn(__uint_as_float(v[i]), __uint_as_float(odd[i])));
@@ -626,20 +628,23 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         } else if (item.parts == 1) {
           if (y_wide) {
 #pragma unroll
-            for (int i = 0; i < kStep; ++i) {
-              const float f = __uint_as_float(v[i]);
-              const __nv_bfloat16 h = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
-              sts_u16(turn + (i * 32 + lane) * 2, uint32_t(*reinterpret_cast<const uint16_t*>(&h)));
-            }
-            __syncwarp();
+            for (int h = 0; h < kStep; h += kCols) {
 #pragma unroll
-            for (int j = 0; j < kStep / 8; ++j) {  // a store: 8 columns x 64 bytes (32 rows)
-              const uint32_t ml = j * 8 + (lane >> 2), m = m0 + ml;
-              const uint4 piece = lds128(turn + ml * 64 + (lane & 3) * 16);
-              if (m < args.m)
-                *reinterpret_cast<uint4*>(args.y + size_t(m) * args.ldy + item.row_block * BXR_ROWS + e * 32 + (lane & 3) * 8) = piece;
+              for (int i = 0; i < kCols; ++i) {
+                const float f = __uint_as_float(v[h + i]);
+                const __nv_bfloat16 o = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
+                sts_u16(turn + (i * 32 + lane) * 2, uint32_t(*reinterpret_cast<const uint16_t*>(&o)));
+              }
+              __syncwarp();
+#pragma unroll
+              for (int j = 0; j < kCols / 8; ++j) {  // a store: 8 columns x 64 bytes (32 rows)
+                const uint32_t ml = j * 8 + (lane >> 2), m = m0 + h + ml;
+                const uint4 piece = lds128(turn + ml * 64 + (lane & 3) * 16);
+                if (m < args.m)
+                  *reinterpret_cast<uint4*>(args.y + size_t(m) * args.ldy + item.row_block * BXR_ROWS + e * 32 + (lane & 3) * 8) = piece;
+              }
+              __syncwarp();
             }
-            __syncwarp();
           } else if (row < args.rows) {
 #pragma unroll
             for (int i = 0; i < kStep; ++i)
@@ -650,15 +655,18 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < kStep; ++i) sts32(turn + (i * 32 + lane) * 4, v[i]);
-          __syncwarp();
+          for (int h = 0; h < kStep; h += kCols) {
 #pragma unroll
-          for (int j = 0; j < kStep / 4; ++j) {  // a store: 4 columns x 128 bytes (32 rows)
-            const uint32_t ml = j * 4 + (lane >> 3), m = m0 + ml;
-            const uint4 piece = lds128(turn + ml * 128 + (lane & 7) * 16);
-            if (m < mcols) stg128(args.partials + (size_t(item.slot) * NB + m) * BXR_ROWS + e * 32 + (lane & 7) * 4, piece, stay);
+            for (int i = 0; i < kCols; ++i) sts32(turn + (i * 32 + lane) * 4, v[h + i]);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < kCols / 4; ++j) {  // a store: 4 columns x 128 bytes (32 rows)
+              const uint32_t ml = j * 4 + (lane >> 3), m = m0 + h + ml;
+              const uint4 piece = lds128(turn + ml * 128 + (lane & 7) * 16);
+              if (m < mcols) stg128(args.partials + (size_t(item.slot) * NB + m) * BXR_ROWS + e * 32 + (lane & 7) * 4, piece, stay);
+            }
+            __syncwarp();
           }
-          __syncwarp();
         }
       }
       tc_fence_before();
