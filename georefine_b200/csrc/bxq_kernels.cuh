@@ -548,7 +548,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         if ((i & 1) == which) {
           if (!ctx.wait(bar_op_full + 8 * so, pho)) { live = false; break; }
           tc_fence_after();
-          if (lane == 0) {
+          if (elect_one()) {
             const uint32_t a_tmem = tmem_base + kWideOperandCol<NB> + so * 64;
             const uint64_t bdesc = umma_desc_sw128(smem + L::xs + sx * L::kXStage);
             uint32_t accumulate = i >= 2 ? 1u : 0u;
@@ -566,7 +566,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         if (++so == kOpN) { so = 0; pho ^= 1; }
         if (++sx == kXN) sx = 0;
       }
-      if (live && lane == 0) umma_commit(bar_acc_full + 8 * buf);
+      if (live && elect_one()) umma_commit(bar_acc_full + 8 * buf);
       __syncwarp();
     }
   } else if (MODE == kUmma && warp >= kWideWarpEpilogue) {
