@@ -26,8 +26,8 @@ int cuda_status(cudaError_t e) { return e == cudaSuccess ? GRB_OK : GRB_ERR_CUDA
 uint32_t batch_tile(uint32_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
 
 // Batches above 128 rows over 4-bit window images: a pass over the weights may take 192 rows, and costs little more than
-// one of 128.  Rows of the next pass when `left` are still to be multiplied: 192 unless two passes of 128 do for what is
-// left just as well (193 to 256 rows).
+// one of 128 (34816 x 5120: 74 against 62 us).  Rows of the next pass when `left` are still to be multiplied: 192 (129 rows:
+// 70 us in one pass, 110 us in two), except that 193 to 256 rows take two passes either way and 128-column ones cost less.
 constexpr uint32_t kWideTile = 192;
 uint32_t wide_pass_rows(uint32_t left) {
   if (left <= 128) return left;
@@ -582,7 +582,8 @@ int grb_rmsnorm_bf16(void* h, int64_t ldh, const void* delta, int64_t ldd, const
   if ((reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(out) |
        reinterpret_cast<uintptr_t>(delta)) & 15)
     return GRB_ERR_ARGUMENT;
-  return launch_step(rmsnorm_kernel, dim3(rows), dim3(kRmsThreads), 0, static_cast<cudaStream_t>(cuda_stream),
+  const auto kernel = hidden <= 4 * 8 * kRmsThreads ? rmsnorm_kernel<4> : rmsnorm_kernel<kRmsVectors>;
+  return launch_step(kernel, dim3(rows), dim3(kRmsThreads), 0, static_cast<cudaStream_t>(cuda_stream),
                      static_cast<__nv_bfloat16*>(h), ldh, static_cast<const __nv_bfloat16*>(delta), ldd,
                      static_cast<const __nv_bfloat16*>(weight), static_cast<__nv_bfloat16*>(out), ldo, hidden, eps, unit_offset);
 }
