@@ -28,7 +28,7 @@ from .resident import ResidentWeight
 
 PAGE = ops.PAGE
 # Rows of a prompt that go through the stack together: two 192-row passes over each weight and one set of the small
-# kernels, for 60 MB of row buffers at a hidden width of 5120.  1000 tokens over four layers: 6.65 -> 5.79 ms.
+# kernels, for 60 MB of row buffers at a hidden width of 5120.  1000 tokens over four layers: 6.65 -> 5.8 ms.
 PROMPT_ROWS = 384
 
 
