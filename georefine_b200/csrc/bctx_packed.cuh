@@ -408,6 +408,9 @@ __global__ void __launch_bounds__(kPackedThreads, 1) bctx_packed_kernel(const Bc
     check(s, a.bytes, a.size, a.states, a.offsets);
     if (CODED) check(t, a.raw, uint32_t(a.raw_size), a.raw_states, a.raw_offsets);
     if (bad) packed_report(a, bad, false);
+    // The piece asked for last may still be under way, and copies keep no order among themselves: without this wait it
+    // could land on top of the next block's bytes in the same ring.
+    cp_async_wait<0>();
   }
   if (threadIdx.x == 0) mbar_wait(bar, 0);   // no copy may be under way when the CTA ends
 }

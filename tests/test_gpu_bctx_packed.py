@@ -37,3 +37,27 @@ def test_packed_decode_and_row_gather_are_exact(orc, shape, stride, classes, coa
         with pytest.raises(IndexError):
             t.gather_rows(torch.tensor([0, wrong]))
     assert np.array_equal(t.gather_rows(ids).view(torch.uint16).cpu().numpy(), words[ids.numpy()])
+
+
+# More blocks than a CTA has lanes (at most 1024): every lane walks a second block through the ring that the first one used.
+# rows that are whole blocks (decoded class by class; also one row of 1536 blocks gathered), rows of whole runs of 16, any rows
+ROUNDS = [((4100, 1024), 16), ((3, 24576), 16), ((4100, 2064), 32), ((4100, 1030), 16)]
+
+
+@pytest.mark.parametrize("shape,stride", ROUNDS)
+@pytest.mark.parametrize("coarse", [False, True])
+def test_lanes_that_walk_several_blocks(orc, shape, stride, coarse):
+    from georefine_b200 import codec
+    from georefine_b200.gpu import CudaContextTensor
+
+    words = orc.synthetic_weight_words(*shape, 11)
+    if coarse:
+        words &= 0xFFF8
+    t = CudaContextTensor(codec.encode(words), stride=stride, walk_stride=stride, device="cuda:0", fused=False)
+    assert t._packed is not None and t.mode == (128 if coarse else 0)
+    if shape[0] > 148:
+        assert -(-words.size // stride) > 148 * 1024
+    for _ in range(3):
+        assert np.array_equal(t.decode().view(torch.uint16).cpu().numpy(), words)
+    ids = torch.arange(shape[0]).flip(0)[:200]
+    assert np.array_equal(t.gather_rows(ids).view(torch.uint16).cpu().numpy(), words[ids.numpy()])
