@@ -173,6 +173,18 @@ def _packed_tables(indexed, stride):
     return packed, image, by_class
 
 
+class _Outcome:
+    """Where the kernel writes how a checked decode went: two words of pinned host memory, {status bits, an index was out of
+    range}.  One call has it to itself from the launch until it has read it."""
+
+    def __init__(self):
+        import torch
+
+        self._memory = torch.zeros(2, dtype=torch.int32).pin_memory()
+        self.at = self._memory.data_ptr()
+        self.words = (ctypes.c_uint32 * 2).from_address(self.at)
+
+
 class CudaContextTensor:
     """A BCTX frame resident on one GPU: the unchanged streams with their restart index (for ``decode`` and
     ``gather_rows``) and, for rank-2 weights, the resident image the fused linear streams.
@@ -233,10 +245,7 @@ class CudaContextTensor:
                 self._bucket_shift[kind] = shift
         self.error = torch.zeros((), device=self.device, dtype=torch.int32)
         self._error_clear = True
-        # outcome of a checked decode, written by the kernel into host memory: {status bits, an index was out of range}
-        self._flags = torch.zeros(2, dtype=torch.int32).pin_memory()
-        self._flags_at = self._flags.data_ptr()
-        self._flag_words = (ctypes.c_uint32 * 2).from_address(self._flags_at)
+        self._outcomes = [_Outcome()]       # those no call is using; a thread that finds none makes its own
         self.resident = None
         if fused and words is not None:
             self.resident = ResidentWeight.from_words(words, device=self.device, source_sha256=bytes.fromhex(self.source_sha256),
@@ -281,13 +290,17 @@ class CudaContextTensor:
         if not self._error_clear:
             self.error.zero_()
         wait = check or ids is not None
-        flags = self._flag_words
-        if wait:
-            flags[0] = flags[1] = 0
         self._error_clear = wait        # unknown until somebody waits for the launch
+        outcome = None
+        if wait:
+            try:
+                outcome = self._outcomes.pop()
+            except IndexError:
+                outcome = _Outcome()
+            outcome.words[0] = outcome.words[1] = 0
         stream = torch.cuda.current_stream(self.device)
         args = (*self._packed_args, None if ids is None else ids.data_ptr(), count, result.data_ptr(), self.error.data_ptr(),
-                self._flags_at if wait else None, stream.cuda_stream)
+                outcome.at if wait else None, stream.cuda_stream)
         if torch.cuda.current_device() == self.device.index:
             status = _native.lib().grb_bctx_decode_packed(*args)
         else:
@@ -297,9 +310,11 @@ class CudaContextTensor:
             _native.check(status, "grb_bctx_decode_packed")
         if wait:
             stream.synchronize()
-            if flags[0] or flags[1]:
+            failed, outside = outcome.words
+            self._outcomes.append(outcome)
+            if failed or outside:
                 self._error_clear = False
-                if flags[1]:
+                if outside:
                     raise IndexError("embedding row outside tensor")
                 if check:
                     raise base.CodecError("CUDA decoder checkpoint mismatch")

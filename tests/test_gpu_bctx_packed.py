@@ -61,3 +61,37 @@ def test_lanes_that_walk_several_blocks(orc, shape, stride, coarse):
         assert np.array_equal(t.decode().view(torch.uint16).cpu().numpy(), words)
     ids = torch.arange(shape[0]).flip(0)[:200]
     assert np.array_equal(t.gather_rows(ids).view(torch.uint16).cpu().numpy(), words[ids.numpy()])
+
+
+def test_threads_that_share_a_tensor_see_their_own_outcome(orc):
+    """One thread asks for rows that exist, the other for one that does not: neither's verdict reaches the other."""
+    import threading
+
+    from georefine_b200 import codec
+    from georefine_b200.gpu import CudaContextTensor
+
+    words = orc.synthetic_weight_words(64, 4096, 5)
+    t = CudaContextTensor(codec.encode(words), device="cuda:0", fused=False)
+    wrong, rounds = [], 300
+
+    def ask(ids, bad):
+        stream, ids = torch.cuda.Stream(), ids.cuda()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            for _ in range(rounds):
+                try:
+                    rows = t.gather_rows(ids)
+                    if bad or not torch.equal(rows.view(torch.int16), want):
+                        wrong.append("no error for a row outside" if bad else "wrong words")
+                except IndexError:
+                    if not bad:
+                        wrong.append("the other thread's error")
+
+    good = torch.arange(64).flip(0)
+    want = torch.from_numpy(words[good.numpy()].view(np.int16)).cuda()
+    threads = [threading.Thread(target=ask, args=a) for a in ((good, False), (torch.tensor([0, 64]), True)) for _ in range(2)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not wrong, (len(wrong), wrong[:3])
