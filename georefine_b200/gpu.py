@@ -244,7 +244,7 @@ class CudaContextTensor:
                 self.buffers[kind + "_bucket"] = torch.from_numpy(bucket).to(self.device)
                 self._bucket_shift[kind] = shift
         self.error = torch.zeros((), device=self.device, dtype=torch.int32)
-        self._error_clear = True
+        self._error_clear, self._captured = True, False     # is the word known to be zero; may a graph's replay write it
         self._outcomes = [_Outcome()]       # those no call is using; a thread that finds none makes its own
         self.resident = None
         if fused and words is not None:
@@ -287,10 +287,14 @@ class CudaContextTensor:
         else:
             count = ids.numel()
             result = torch.empty((*ids.shape, self.shape[1]), device=self.device, dtype=torch.bfloat16)
-        if not self._error_clear:
-            self.error.zero_()
         wait = check or ids is not None
-        self._error_clear = wait        # unknown until somebody waits for the launch
+        # A call that waits for its launch leaves the word as it found it, at zero, and need not clear it for the next one
+        # that waits.  All others clear it on the stream, where a captured graph does so on every replay.
+        if not (wait and self._error_clear):
+            self.error.zero_()
+        if not wait and torch.cuda.is_current_stream_capturing():
+            self._captured = True
+        self._error_clear = wait and not self._captured
         outcome = None
         if wait:
             try:

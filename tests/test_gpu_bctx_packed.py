@@ -95,3 +95,22 @@ def test_threads_that_share_a_tensor_see_their_own_outcome(orc):
     for th in threads:
         th.join()
     assert not wrong, (len(wrong), wrong[:3])
+
+
+def test_a_replay_clears_the_error_word_of_the_one_before(orc):
+    from georefine_b200 import codec
+    from georefine_b200.gpu import CudaContextTensor
+
+    words = orc.synthetic_weight_words(64, 512, 5)
+    t = CudaContextTensor(codec.encode(words), device="cuda:0", fused=False)
+    assert np.array_equal(t.decode().view(torch.uint16).cpu().numpy(), words)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = t.decode(check=False)
+    for eager in (lambda: t.decode(check=False), t.decode):
+        t.error.fill_(4)                                     # as a replay over broken streams leaves it
+        graph.replay()
+        assert int(t.error.item()) == 0 and np.array_equal(out.view(torch.uint16).cpu().numpy(), words)
+        t.error.fill_(4)
+        eager()
+        assert int(t.error.item()) == 0
