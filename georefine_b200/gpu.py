@@ -236,9 +236,14 @@ class CudaContextTensor:
                 self.buffers["part_of"] = torch.from_numpy(parts.view(np.int32)).to(self.device)
                 self._packed.parts, self._packed.share = len(parts), int((parts[:, 3] - parts[:, 2]).max())
                 self._packed.rows_by_class, self._packed.part_of = self.buffers["rows_by_class"].data_ptr(), self.buffers["part_of"].data_ptr()
+        if self._packed is not None:
+            self._gather_limit = self._packed_gather_limit(by_class)
+        # bctx_decode_kernel's tables: for frames without packed ones, and for gathers that it does better and that are not yet
+        # a whole decode
+        looked_up = self._packed is None or (by_class and self._gather_limit < self.shape[0])
         for kind in ("main", "residual"):
             table = indexed.get(kind + "_freq")
-            if table is not None and self._packed is None:
+            if table is not None and looked_up:
                 cum, bucket, shift = _lookup_tables(table)
                 self.buffers[kind + "_cum"] = torch.from_numpy(cum).to(self.device)
                 self.buffers[kind + "_bucket"] = torch.from_numpy(bucket).to(self.device)
@@ -257,6 +262,24 @@ class CudaContextTensor:
         if self._packed is not None:
             self._packed_args = ctypes.byref(self._descriptor), ctypes.byref(self._packed)
 
+    def _packed_gather_limit(self, by_class) -> int:
+        """How many rows ``gather_rows`` takes through the packed kernel at most.
+
+        By class a CTA brings in its class's tables for every single row, 23 to 35 us per wave of CTAs, while
+        ``bctx_decode_kernel`` takes any number of rows at once in 200 to 400 us; they meet between 10 waves (9504 x 5120 words
+        with coded residuals, 2048 rows: 485 against 390 us) and 30 (2048 x 5120, raw residuals).  As many rows as the tensor
+        has are one decode and an index (32768 rows of a 9504 x 5120 table: 430 us; by class 7100 us).  With the tables of all classes in
+        every CTA a row costs what its words cost, and the tensor is decoded and indexed when that saves more words than
+        the extra pass and the check of the row numbers cost (60 us, 24 M words; 32768 rows of 2048 x 5000: 499 -> 234 us)."""
+        rows, cols = self.shape
+        if not by_class:
+            return rows + (24 << 20) // cols
+        coded, shape, per_row = self.mode == 128, self._packed.shape, cols // self.walk_stride
+        lanes = min(1024, -(-per_row // 32) * 32)
+        memory = 128 + self.nc * shape[1] + shape[4] - shape[3] + cols + cols // 8 + 32 + lanes * (128 if coded else 64)
+        per_sm = max(1, min((228 << 10) // (memory + 1024), 1024 // lanes))      # (64 registers a thread)
+        return 10 * per_sm * sm_count(self.device)
+
     def _make_descriptor(self):
         b = self.buffers
         t = _native.BctxTensor()
@@ -265,13 +288,13 @@ class CudaContextTensor:
         t.row_class, t.col_class = b["rows"].data_ptr(), b["columns"].data_ptr()
         t.main_stream, t.main_bytes = b["main_stream"].data_ptr(), b["main_stream"].numel()
         t.main_states, t.main_offsets = b["main_states"].data_ptr(), b["main_offsets"].data_ptr()
-        if self._packed is None:
+        if "main_cum" in b:
             t.main_cum, t.main_bucket = b["main_cum"].data_ptr(), b["main_bucket"].data_ptr()
             t.main_bucket_shift = self._bucket_shift["main"]
         t.residual_stream, t.residual_bytes = b["residual_stream"].data_ptr(), b["residual_stream"].numel()
         if self.mode == 128:
             t.residual_states, t.residual_offsets = b["residual_states"].data_ptr(), b["residual_offsets"].data_ptr()
-            if self._packed is None:
+            if "residual_cum" in b:
                 t.residual_cum, t.residual_bucket = b["residual_cum"].data_ptr(), b["residual_bucket"].data_ptr()
                 t.residual_bucket_shift = self._bucket_shift["residual"]
         return t
@@ -358,20 +381,20 @@ class CudaContextTensor:
     def gather_rows(self, ids, *, check=True):
         """Rows ``ids`` (any shape) as BF16 [..., cols].  Only the blocks of the requested rows are decoded when the frame has
         packed tables or a row is a whole number of restart blocks; otherwise (raw frames, strides that do not divide the
-        row) the tensor is decoded once and indexed."""
+        row), and when more rows are asked for than that is worth, the tensor is decoded once and indexed."""
         import torch
 
         rows, cols = self.shape
         ids = ids.to(device=self.device, dtype=torch.int64)
         if ids.numel() == 0:
             return torch.empty((*ids.shape, cols), device=self.device, dtype=torch.bfloat16)
-        if self._packed is not None:
+        if self._packed is not None and ids.numel() <= self._gather_limit:
             return self._decode_packed(ids.contiguous(), check=check)
         lowest, highest = torch.aminmax(ids)
         if int(lowest) < 0 or int(highest) >= rows:
             raise IndexError("embedding row outside tensor")
         blocks_per_row, ragged = divmod(cols, self.walk_stride)
-        if self.mode == 1 or ragged:
+        if self.mode == 1 or ragged or (self._packed is not None and ids.numel() >= rows):
             return self.decode(check=check)[ids]
         first_block = ids.reshape(-1, 1) * blocks_per_row
         wanted = (first_block + torch.arange(blocks_per_row, device=self.device)).reshape(-1)

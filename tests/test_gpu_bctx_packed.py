@@ -114,3 +114,32 @@ def test_a_replay_clears_the_error_word_of_the_one_before(orc):
         t.error.fill_(4)
         eager()
         assert int(t.error.item()) == 0
+
+
+@pytest.mark.parametrize("shape,classes", [((6000, 128), (16, 4)), ((6000, 130), (16, 4)), ((2600, 256), (64, 16)), ((40, 512), (16, 4))])
+@pytest.mark.parametrize("coarse", [False, True])
+def test_gathers_on_both_sides_of_the_packed_limit(orc, shape, classes, coarse):
+    """Rows by the packed kernel, by the general one and out of a whole decode are the same bits, and refuse the same."""
+    from georefine_b200 import codec
+    from georefine_b200.gpu import CudaContextTensor
+
+    words = orc.synthetic_weight_words(*shape, 9)
+    if coarse:
+        words &= 0xFFF8
+    t = CudaContextTensor(codec.encode(words, row_classes=classes[0], col_classes=classes[1]), device="cuda:0", fused=False)
+    limits = {t._gather_limit} if shape[1] % t.walk_stride else {t._gather_limit, 100, shape[0] + 100}
+    if shape[0] <= t._gather_limit:
+        limits -= {100}                                      # no tables for the general kernel: it would not be taken
+    for limit in sorted(limits):
+        t._gather_limit = limit
+        for count in (limit, limit + 1, shape[0], shape[0] + 1):
+            if not 0 < count * shape[1] < 40_000_000:
+                continue
+            ids = torch.randint(0, shape[0], (count,), generator=torch.Generator().manual_seed(count))
+            ids[0], ids[-1] = shape[0] - 1, 0
+            rows = t.gather_rows(ids.reshape(1, -1))
+            assert rows.shape == (1, count, shape[1]) and np.array_equal(rows[0].view(torch.uint16).cpu().numpy(), words[ids.numpy()])
+            for wrong in (-1, shape[0]):
+                ids[count // 2] = wrong
+                with pytest.raises(IndexError):
+                    t.gather_rows(ids)
