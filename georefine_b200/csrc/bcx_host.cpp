@@ -298,7 +298,7 @@ int grb_bctx_build_lookup(const uint32_t* freq, uint32_t nctx, uint32_t vocab, u
 // The models packed for shared memory (PackedShape in bcx_model.h): shape = {log2 slots per main bucket, bytes per main
 // context, log2 slots per residual bucket, offset of the residual contexts, bytes}.  residual_freq == NULL: raw residuals.
 // With image == NULL only the shape is computed.  Returns 0, 1 on bad arguments, 2 for invalid tables, 4 when `resident` main
-// contexts and the residual contexts do not fit `limit` bytes.
+// contexts and the residual contexts do not fit `limit` bytes, or a main symbol with a frequency has no residual model.
 int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t resident, uint32_t limit,
                          uint32_t shape[5], uint8_t* image) {
   try {

@@ -115,19 +115,22 @@ class PackedTables {
     }
     resid_live_.assign(1024, 0);
     resid_entries_ = resid_contexts_ = 0;
+    unpaired_ = false;
     for (uint32_t s = 0; resid_ && s < 1024; ++s) {
       if (!count(resid_ + size_t(s) * 64, 64, resid_live_[s])) return false;
       if (!occurs_[s]) continue;
-      if (!resid_live_[s]) return false;      // a main symbol that occurs has a residual
+      unpaired_ |= !resid_live_[s];
       ++resid_contexts_;
       resid_entries_ += resid_live_[s];
     }
     return true;
   }
-  // The bucket widths with the fewest scan steps (rare symbols, which share buckets, are mostly main symbols) whose tables, `resident` main contexts of them, fit `limit` bytes; false
-  // when none do.
+  // The bucket widths with the fewest scan steps (rare symbols, which share buckets, are mostly main symbols) whose tables,
+  // `resident` main contexts of them, fit `limit` bytes; false when none do, or the packed form cannot hold the models.
   bool shape(uint32_t resident, uint32_t limit, PackedShape& out) const {
-    if (ranks_ > 255) return false;
+    // (a main symbol that has a frequency but no residual model: valid as long as the streams never code it, and left
+    // to the kernel whose scan is bounded by the vocabulary)
+    if (ranks_ > 255 || unpaired_) return false;
     uint64_t best = ~uint64_t(0);
     for (uint32_t ms = 3; ms <= 8; ++ms)
       for (uint32_t rs = resid_ ? 4 : 8; rs <= 8; ++rs) {
@@ -189,6 +192,7 @@ class PackedTables {
 
   const uint32_t *main_ = nullptr, *resid_ = nullptr;
   uint32_t nctx_ = 0, ranks_ = 0, resid_entries_ = 0, resid_contexts_ = 0;
+  bool unpaired_ = false;
   std::vector<uint8_t> occurs_;
   std::vector<uint32_t> resid_live_;
 };

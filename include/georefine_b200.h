@@ -151,8 +151,8 @@ int grb_bctx_decode_words(const grb_bctx_tensor* tensor, const int64_t* block_id
 /* A frame's models packed for the shared memory of one SM (csrc/bcx_model.h, PackedShape): shape = {log2 slots per main
  * bucket, bytes per main context, log2 slots per residual bucket, offset of the residual contexts, bytes}.  residual_freq:
  * the tables of a mode 128 frame, NULL for raw residuals.  image == NULL computes the shape only.  0 ok, 1 arguments,
- * 2 invalid tables, 4 `resident` main contexts and the residual contexts do not fit `limit` bytes: use
- * grb_bctx_decode_words.  The kernel keeps them in the 227 KB of an SM's shared memory next to 64 bytes per lane and stream
+ * 2 invalid tables, 4 `resident` main contexts and the residual contexts do not fit `limit` bytes, or a main symbol that has a
+ * frequency in some context has no residual model: use grb_bctx_decode_words.  The kernel keeps them in the 227 KB of an SM's shared memory next to 64 bytes per lane and stream
  * and 9/8 bytes per column. */
 int grb_bctx_pack_tables(const uint32_t* main_freq, uint32_t nctx, const uint32_t* residual_freq, uint32_t resident, uint32_t limit,
                          uint32_t shape[5], uint8_t* image);
