@@ -15,6 +15,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <thread>
 #include <vector>
@@ -34,12 +35,30 @@ namespace {
 constexpr uint32_t kTotal = 1u << 16;
 constexpr uint32_t kLow = 1u << 23;
 
+// fn(0) .. fn(threads - 1), each on a thread of its own where one can be started, else on this one.  What a share throws is
+// thrown here, once all of them are over.
 template <class Fn>
 void on_threads(uint32_t threads, const Fn& fn) {
+  std::vector<std::exception_ptr> failed(threads);
+  const auto share = [&](uint32_t t) noexcept {
+    try {
+      fn(t);
+    } catch (...) {
+      failed[t] = std::current_exception();
+    }
+  };
   std::vector<std::thread> pool;
-  for (uint32_t t = 1; t < threads; ++t) pool.emplace_back([&fn, t] { fn(t); });
-  fn(0);
+  pool.reserve(threads);
+  uint32_t t = 1;
+  try {
+    for (; t < threads; ++t) pool.emplace_back(share, t);
+  } catch (...) {   // no thread to be had, or no memory for it
+  }
+  share(0);
+  for (; t < threads; ++t) share(t);
   for (auto& th : pool) th.join();
+  for (const auto& e : failed)
+    if (e) std::rethrow_exception(e);
 }
 // Threads worth starting for n words: one per 128 K words, at most 8.
 uint32_t threads_for(uint64_t n) {
