@@ -263,6 +263,7 @@ def _frequencies_kind(lib, a, rc, cc, nr, nc, kind):
 
 
 def _decoder_choice():
+    """Which of the library's two stream decoders the environment names; None: neither, the whole-frame pass is taken."""
     choice = os.environ.get("GEOREFINE_CONTEXT_COMPACT_RANS")
     if choice not in (None, "0", "1"):
         raise CodecError("GEOREFINE_CONTEXT_COMPACT_RANS must be 0 or 1")
@@ -453,11 +454,12 @@ def _decode_sealed(frame):
     rows, cols = f["shape"]
     if f["mode"] == MODE_WORDS:
         return f["raw"].reshape(rows, cols)
-    _decoder_choice()
-    quick = frame_words(f)
-    if quick is not None:
-        return quick[0]
-    # something is wrong with a stream or its tables, or they are unusual: one stream after the other, with its own verdict
+    if _decoder_choice() is None:
+        quick = frame_words(f)
+        if quick is not None:
+            return quick[0]
+    # a decoder was asked for by name, something is wrong with a stream or its tables, or they are unusual: one stream
+    # after the other, with its own verdict
     lib = _lib()
     common = (f["rows"], f["columns"], rows, cols, f["nr"], f["nc"])
     main = _decode_kind(lib, f["main_stream"], f["main_table"], *common, 0)

@@ -46,3 +46,28 @@ def test_residual_floor_is_below_the_stream_and_close(orc, seed, mask):
     stream = codec._encode_under(lib, a, rc, cc, 16, 4, 1, residual)
     # the bound gives away 0.0114 bits per word and what bytes before rare symbols cost
     assert floor <= len(stream) <= floor + 0.0114 / 8 * a.size + 64 + 0.02 * len(stream)
+
+
+@pytest.mark.parametrize("choice,decoder", [(None, None), ("0", "bcx_decode"), ("1", "bcx_decode_compact")])
+@pytest.mark.parametrize("mask", [0xFFFF, 0xFFF8])
+def test_the_environment_chooses_the_stream_decoder(orc, monkeypatch, choice, decoder, mask):
+    words = orc.synthetic_weight_words(300, 999, 3) & np.uint16(mask)
+    frame = codec.encode(words)
+    lib, called = codec._lib(), []
+
+    class Watched:
+        def __getattr__(self, name):
+            called.append(name)
+            return getattr(lib, name)
+
+    monkeypatch.setattr(codec, "_lib", Watched)
+    if choice is None:
+        monkeypatch.delenv("GEOREFINE_CONTEXT_COMPACT_RANS", raising=False)
+    else:
+        monkeypatch.setenv("GEOREFINE_CONTEXT_COMPACT_RANS", choice)
+    assert np.array_equal(codec.decode(frame), words)
+    streams = 2 if mask != 0xFFFF else 1
+    assert [name for name in called if name.startswith("bcx_decode")] == ([decoder] * streams if decoder else [])
+    monkeypatch.setenv("GEOREFINE_CONTEXT_COMPACT_RANS", "2")
+    with pytest.raises(codec.CodecError, match="must be 0 or 1"):
+        codec.decode(frame)
