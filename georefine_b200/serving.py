@@ -35,7 +35,8 @@ class BctxLinear(nn.Module):
 
     def forward(self, x):
         self.__dict__["forward_calls"] += 1       # (past nn.Module's attribute machinery: this is a per-call path)
-        bias = self._parameters["bias"]
+        # (a parametrized bias, or a plain tensor put in its place, is not among the parameters)
+        bias = self._parameters["bias"] if "bias" in self._parameters else self.bias
         if bias is not None and bias.dtype is not torch.bfloat16:
             bias = bias.to(torch.bfloat16)
         return self.context_weight.linear(x, bias=bias)
