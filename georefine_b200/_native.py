@@ -159,14 +159,21 @@ def lib():
 
 
 def gemm_next():
-    """(the call without ctypes of csrc/fastcall.c, the address of grb_bxr_gemm_next it takes first)."""
+    """(a function of the address of grb_bxr_gemm_next and its arguments as integers, that address): the call without ctypes of
+    csrc/fastcall.c, or ctypes where that could not be built for this interpreter."""
     global _FASTCALL
     if _FASTCALL is None:
-        entry = ctypes.cast(lib().grb_bxr_gemm_next, VOIDP).value     # (builds both libraries when sources are newer)
-        loader = importlib.machinery.ExtensionFileLoader("_fastcall", str(_build.FASTCALL))
-        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", str(_build.FASTCALL), loader=loader))
-        loader.exec_module(module)
-        _FASTCALL = module.gemm_next, entry
+        entry = ctypes.cast(lib().grb_bxr_gemm_next, VOIDP).value     # (builds the library when sources are newer)
+        if _build.build_fastcall():
+            loader = importlib.machinery.ExtensionFileLoader("_fastcall", str(_build.FASTCALL))
+            module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", str(_build.FASTCALL), loader=loader))
+            loader.exec_module(module)
+            call = module.gemm_next
+        else:
+            i64, u32, u64 = ctypes.c_int64, ctypes.c_uint32, ctypes.c_uint64
+            by_address = ctypes.CFUNCTYPE(ctypes.c_int, VOIDP, VOIDP, VOIDP, i64, u32, VOIDP, i64, VOIDP, VOIDP, u64, VOIDP, VOIDP, VOIDP, VOIDP)(entry)
+            call = lambda _, *args: by_address(*args)
+        _FASTCALL = call, entry
     return _FASTCALL
 
 
