@@ -540,13 +540,13 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const WideSpan item = wide_span(u, unit_end, args.chunks);
       u += item.chunk_end - item.chunk_begin;
       const uint32_t buf = n_item % kAccBufs, use = n_item / kAccBufs;
-      if (ctx.aborted() || !ctx.wait(bar_acc_empty + 8 * buf, (use & 1) ^ 1)) { live = false; break; }
+      if (!__all_sync(0xFFFFFFFFu, !ctx.aborted() && ctx.wait(bar_acc_empty + 8 * buf, (use & 1) ^ 1))) { live = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + (buf * 2 + which) * NB;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
         const uint32_t i = c - item.chunk_begin;
         if ((i & 1) == which) {
-          if (!ctx.wait(bar_op_full + 8 * so, pho)) { live = false; break; }
+          if (!ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
           tc_fence_after();
           if (elect_one()) {
             const uint32_t a_tmem = tmem_base + kWideOperandCol<NB> + so * 64;

@@ -127,6 +127,11 @@ struct RoleCtx {
       atomicOr(status, ((((bar - bars) >> 3) + 1u) & 0xFFu) << 8 | (blockIdx.x & 0xFFu) << 16);
     return false;
   }
+  // The same with one verdict for all lanes of a warp that goes on to elect one of them.  Every lane times its own wait:
+  // where the barrier completes as the limit runs out, some lanes would go on, and wait for good for the others.
+  __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity) const {
+    return __all_sync(0xFFFFFFFFu, wait(bar, parity));
+  }
 };
 
 // The two rANS streams of a lane (the forward and the backward reader of one segment), advanced together
