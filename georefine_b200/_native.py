@@ -27,7 +27,7 @@ EXPORTS = (
     "bcx_encode", "bcx_frequencies", "bcx_decode", "bcx_decode_compact", "bcx_free", "bcx_pack6", "bcx_unpack6",
     "bcx_checkpoint", "grb_bctx_build_lookup", "grb_bctx_decode_words", "grb_bctx_magnitudes", "grb_bctx_frequencies", "grb_bctx_encode_stream",
     "grb_bctx_frame_words", "grb_bctx_pack_tables", "grb_bctx_decode_packed", "bxr_build", "bxr_free", "bxr_decode_host",
-    "bxr_validate", "bxr_layout_version", "grb_bxr_workspace_bytes", "grb_bxr_decode", "grb_bxr_gemm", "grb_bxr_gemv", "grb_bxr_gemm_next", "grb_kernel_attributes",
+    "bxr_validate", "bxr_layout_version", "grb_bxr_workspace_bytes", "grb_bxr_decode", "grb_bxr_gemm", "grb_bxr_gemv", "grb_bxr_gemm_next", "grb_bxr_gemm_partials", "grb_kernel_attributes",
     "grb_static_scratch_bytes", "grb_bxr_gemv_static", "grb_dense_gemv_bf16", "grb_peer_control_bytes", "grb_peer_enable", "grb_peer_allreduce_bf16",
     "grb_peer_alloc", "grb_peer_free", "grb_peer_open", "grb_peer_close",
     "grb_rmsnorm_bf16", "grb_silu_mul_bf16", "grb_argmax_bf16", "grb_attn_decode_bf16",
@@ -108,6 +108,7 @@ def _declare(lib):
     lib.grb_bxr_gemm.argtypes = linear
     lib.grb_bxr_gemv.argtypes = linear
     lib.grb_bxr_gemm_next.argtypes = linear + [VOIDP, ctypes.POINTER(BxrHeader)]
+    lib.grb_bxr_gemm_partials.argtypes = linear[:10] + [VOIDP, u64] + linear[10:] + [VOIDP, ctypes.POINTER(BxrHeader)]
     lib.grb_kernel_attributes.argtypes = [ci, ctypes.POINTER(ci * 5)]
     lib.grb_static_scratch_bytes.argtypes = []
     lib.grb_static_scratch_bytes.restype = u64
@@ -158,20 +159,21 @@ def lib():
         return _LIB
 
 
-def gemm_next():
-    """(a function of the address of grb_bxr_gemm_next and its arguments as integers, that address): the call without ctypes of
+def gemm_partials():
+    """(a function of the address of grb_bxr_gemm_partials and its arguments as integers, that address): the call without ctypes of
     csrc/fastcall.c, or ctypes where that could not be built for this interpreter."""
     global _FASTCALL
     if _FASTCALL is None:
-        entry = ctypes.cast(lib().grb_bxr_gemm_next, VOIDP).value     # (builds the library when sources are newer)
+        entry = ctypes.cast(lib().grb_bxr_gemm_partials, VOIDP).value     # (builds the library when sources are newer)
         if _build.build_fastcall():
             loader = importlib.machinery.ExtensionFileLoader("_fastcall", str(_build.FASTCALL))
             module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_fastcall", str(_build.FASTCALL), loader=loader))
             loader.exec_module(module)
-            call = module.gemm_next
+            call = module.gemm_partials
         else:
             i64, u32, u64 = ctypes.c_int64, ctypes.c_uint32, ctypes.c_uint64
-            by_address = ctypes.CFUNCTYPE(ctypes.c_int, VOIDP, VOIDP, VOIDP, i64, u32, VOIDP, i64, VOIDP, VOIDP, u64, VOIDP, VOIDP, VOIDP, VOIDP)(entry)
+            by_address = ctypes.CFUNCTYPE(ctypes.c_int, VOIDP, VOIDP, VOIDP, i64, u32, VOIDP, i64, VOIDP, VOIDP, u64, VOIDP, u64,
+                                          VOIDP, VOIDP, VOIDP, VOIDP)(entry)
             call = lambda _, *args: by_address(*args)
         _FASTCALL = call, entry
     return _FASTCALL

@@ -464,6 +464,12 @@ int grb_bxr_gemm(const void* image, const bxr_header* h, const void* x, int64_t 
 int grb_bxr_gemm_next(const void* image, const bxr_header* h, const void* x, int64_t ldx, uint32_t m, void* y, int64_t ldy,
                       const void* bias, void* ws, uint64_t ws_bytes, uint32_t* status, void* cuda_stream, const void* next_image,
                       const bxr_header* next_header) {
+  return grb_bxr_gemm_partials(image, h, x, ldx, m, y, ldy, bias, ws, ws_bytes, nullptr, 0, status, cuda_stream, next_image, next_header);
+}
+
+int grb_bxr_gemm_partials(const void* image, const bxr_header* h, const void* x, int64_t ldx, uint32_t m, void* y, int64_t ldy,
+                          const void* bias, void* ws, uint64_t ws_bytes, void* partials, uint64_t partials_bytes, uint32_t* status,
+                          void* cuda_stream, const void* next_image, const bxr_header* next_header) {
   const uint32_t tile = batch_tile(m > 128 ? 128 : m);
   int st = check_linear(image, h, x, ldx, m, y, ldy, ws, ws_bytes, status, tile);
   if (st) return st;
@@ -483,8 +489,12 @@ int grb_bxr_gemm_next(const void* image, const bxr_header* h, const void* x, int
     a.next_workers = next_header->workers;
   }
   // Batches above one tile are processed as consecutive tiles, one pass over the weights each.  The wide tile needs wider
-  // slots for its partial tiles; a caller whose scratch was sized for 128 rows gets tiles of 128.
-  const bool wide = m > 128 && a.window4 && (cluster_of(a) > 1 || ws_bytes >= counter_bytes(h) + uint64_t(h->partial_slots) * kWideTile * BXR_ROWS * 4);
+  // slots for its partial tiles: lent ones, or scratch that was sized for them; a caller who has neither gets tiles of 128.
+  const uint64_t wide_slots = uint64_t(h->partial_slots) * kWideTile * BXR_ROWS * 4;
+  if (partials && (reinterpret_cast<uintptr_t>(partials) & 15)) return GRB_ERR_WORKSPACE;
+  const bool lent = m > 128 && partials && partials_bytes >= wide_slots;
+  if (lent) a.partials = static_cast<float*>(partials);
+  const bool wide = m > 128 && a.window4 && (cluster_of(a) > 1 || lent || ws_bytes >= counter_bytes(h) + wide_slots);
   for (uint32_t m0 = 0; m0 < m; m0 += a.m) {
     a.m = wide ? wide_pass_rows(m - m0) : std::min(m - m0, 128u);
     const auto* xt = static_cast<const __nv_bfloat16*>(x) + size_t(m0) * ldx;

@@ -44,6 +44,14 @@ def sm_count(device) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count
 
 
+def _of_a_graph(block) -> bool:
+    """Did the allocator take the block from the private pool of a capture?"""
+    import torch
+
+    at = block.data_ptr()
+    return any(s["address"] <= at < s["address"] + s["total_size"] and tuple(s["segment_pool_id"]) != (0, 0) for s in torch.cuda.memory_snapshot())
+
+
 def default_workers(rows: int, cols: int, sms: int) -> int:
     """How many persistent CTAs an image is built for when the caller does not say: one per SM, except for small
     weights with fewer 128-row blocks than SMs, where a multiple of the row-block count is better when it costs few
@@ -133,7 +141,11 @@ class ResidentWeight:
         self.image = torch.from_numpy(image).to(self.device)
         self.status = torch.zeros(1, device=self.device, dtype=torch.int32)
         self.max_m = 0
-        self.workspace = None
+        self.workspace, self._outgrown = None, []
+        sizes = [int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(h), m)) for m in (128, 129)]
+        counters = (int(h.row_blocks) * 4 + 255) & ~255
+        # partial tiles of the 192-row passes of a batch above 128 rows, where they are larger than those of 128 rows
+        self.wide_scratch_bytes = sizes[1] - counters if sizes[1] > sizes[0] else 0
         self.next_weight = None     # see then()
         self.reserve(max_m)
 
@@ -160,7 +172,7 @@ class ResidentWeight:
         other = copy.copy(self)
         other.image = self.image.clone()
         other.status = self.status.clone()
-        other.workspace = self.workspace.clone()
+        other.workspace, other._outgrown = self.workspace.clone(), []
         other.next_weight = None
         return other
 
@@ -176,36 +188,52 @@ class ResidentWeight:
 
     @property
     def resident_bytes(self) -> int:
-        ws = 0 if self.workspace is None else self.workspace.numel()
-        return self.bytes + ws + 4
+        return self.bytes + sum(ws.numel() for ws in (self.workspace, *self._outgrown)) + 4
 
     def backend_identity(self):
         h = self.header
         return {"format": "BXR1", "mode": self.mode, "workers": int(h.workers), "items": int(h.items),
                 "partial_slots": int(h.partial_slots), "library": str(_native.library_path().name)}
 
+    def _scratch_bytes(self, m: int) -> int:
+        size = _native.lib().grb_bxr_workspace_bytes
+        return max(256, *(int(size(ctypes.byref(self.header), rows)) for rows in (min(m, 128), GEMV_MAX_M)))
+
     def reserve(self, max_m: int) -> None:
-        """Scratch for batches up to max_m rows (FP32 partial tiles + counters); zero-filled once."""
+        """Scratch for batches up to max_m rows (FP32 partial tiles + counters); zero-filled once.  Batches above 128 rows need
+        no more of it.  Scratch that it replaces lives as long as the weight: a captured graph may have its address."""
         import torch
 
         max_m = max(int(max_m), GEMV_MAX_M)
         if max_m <= self.max_m:
             return
-        need = int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(self.header), max_m))
-        need = max(need, int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(self.header), GEMV_MAX_M)))
+        need = self._scratch_bytes(max_m)
         if self.workspace is None or need > self.workspace.numel():
-            self.workspace = torch.zeros(max(need, 256), device=self.device, dtype=torch.uint8)
+            if self.workspace is not None:
+                self._outgrown.append(self.workspace)
+            self.workspace = torch.zeros(need, device=self.device, dtype=torch.uint8)
         self.max_m = max_m
 
-    def _widen(self, m: int) -> None:
-        """Scratch for the 192-row passes of a batch above 128 rows, on the first such batch.  The scratch it replaces lives
-        as long as the weight: a captured graph may have its address.  During a capture nothing is allocated and the
-        batch runs in passes of 128 rows, which the scratch has room for."""
+    def _capturing(self) -> bool:
         import torch
 
-        if not torch.cuda.is_current_stream_capturing():
-            self._narrow_workspace = self.workspace
-            self.reserve(m)
+        with torch.cuda.device(self.device):
+            return torch.cuda.is_current_stream_capturing()
+
+    def _lent_scratch(self, capturing: bool):
+        """Partial tiles for one batch above 128 rows, from the stream's allocator and back to it after the call: all weights of
+        a stack share one block, and one graph's share a block of the graph's own pool.  None - the batch then runs in
+        passes of 128 rows - when there is no memory, or a capture that the allocator does not know of is under way, whose
+        graph could not keep the block."""
+        import torch
+
+        if not self.wide_scratch_bytes:
+            return None
+        try:
+            block = torch.empty(self.wide_scratch_bytes, device=self.device, dtype=torch.uint8)
+            return block if not capturing or _of_a_graph(block) else None
+        except torch.cuda.OutOfMemoryError:
+            return None
 
     # -- device entry points -------------------------------------------------------------------------
     def _stream(self):
@@ -235,9 +263,11 @@ class ResidentWeight:
             raise ValueError("x and y must be 2-D BF16 tensors")
         if k != self.K or rows != m or n != self.N or x.stride(1) != 1 or y.stride(1) != 1:
             raise ValueError("shape mismatch: x [M, K], y [M, N], unit inner stride")
+        return m
+
+    def _within_reserve(self, m):
         if m > self.max_m and min(m, 128) > min(self.max_m, 128):
             raise ValueError(f"batch of {m} rows exceeds the reserved scratch ({self.max_m}); call reserve() first")
-        return m
 
     def then(self, next_weight):
         """Tells this weight which one the stream multiplies by next (None: nobody).  A hint for the kernel: while a
@@ -246,20 +276,31 @@ class ResidentWeight:
         self.next_weight = next_weight
         return next_weight
 
-    def gemm(self, x, y, bias=None):
-        """tcgen05 path, any M; rows of y are bitwise independent of M."""
+    def gemm(self, x, y, bias=None, *, scratch=None):
+        """tcgen05 path, any M; rows of y are bitwise independent of M.
+
+        A batch above 128 rows may take 192 rows per pass over the weights.  For their partial tiles it borrows ``scratch``
+        (uint8, ``wide_scratch_bytes`` of it, not used by anything else until the call's work is done), or asks the allocator."""
         if x.dim() != 2 or y.dim() != 2:
             raise ValueError("x and y must be 2-D BF16 tensors")
         m = self._checked(x, y)
         if not m:
             return
-        if m > 128 >= self.max_m:
-            self._widen(m)
+        self._within_reserve(m)
+        self._multiply(x, y, bias, m, self.workspace, scratch)
+
+    def _multiply(self, x, y, bias, m, workspace, scratch):
+        if m > 128 and scratch is None:
+            capturing = self._capturing()
+            if not capturing:
+                self.max_m = max(self.max_m, m)
+            scratch = self._lent_scratch(capturing)
         nxt, index = self.next_weight, self.device.index
-        call, entry = _native.gemm_next()
+        call, entry = _native.gemm_partials()
         args = (entry, self.image.data_ptr(), ctypes.addressof(self.header), x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0),
-                0 if bias is None else bias.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(), self.status.data_ptr(),
-                _native.raw_stream(index), 0 if nxt is None else nxt.image.data_ptr(), 0 if nxt is None else ctypes.addressof(nxt.header))
+                0 if bias is None else bias.data_ptr(), workspace.data_ptr(), workspace.numel(), 0 if scratch is None else scratch.data_ptr(),
+                0 if scratch is None else scratch.numel(), self.status.data_ptr(), _native.raw_stream(index),
+                0 if nxt is None else nxt.image.data_ptr(), 0 if nxt is None else ctypes.addressof(nxt.header))
         if _current_device() == index:   # the usual case: skip the device switch
             st = call(*args)
         else:
@@ -279,6 +320,7 @@ class ResidentWeight:
         m = self._checked(x, y)
         if not m:
             return
+        self._within_reserve(m)
         with torch.cuda.device(self.device):
             st = _native.lib().grb_bxr_gemv(self.image.data_ptr(), ctypes.byref(self.header), x.data_ptr(), x.stride(0), m, y.data_ptr(), y.stride(0),
                                             None if bias is None else bias.data_ptr(), self.workspace.data_ptr(), self.workspace.numel(),
@@ -308,8 +350,14 @@ class ResidentWeight:
             y = x.new_empty((m, self.N))
         else:
             y = torch.empty((m, self.N), device=self.device, dtype=torch.bfloat16)
-        if m > self.max_m:
-            self.reserve(m)
+        if m > self.max_m and min(m, 128) > min(self.max_m, 128):
+            if self._capturing():
+                # Scratch of the graph's own pool, for this call only: its zero fill is the graph's, and nothing outside the
+                # graph may count on it.
+                if self._checked(x2, y):
+                    self._multiply(x2, y, bias, m, torch.zeros(self._scratch_bytes(m), device=self.device, dtype=torch.uint8), None)
+                return y if len(lead) == 1 and out is None else y.reshape(*lead, self.N)
+            self.reserve(min(m, 128))
         self.gemm(x2, y, bias)
         return y if len(lead) == 1 and out is None else y.reshape(*lead, self.N)
 

@@ -28,7 +28,8 @@ from .resident import ResidentWeight
 
 PAGE = ops.PAGE
 # Rows of a prompt that go through the stack together: two 192-row passes over each weight and one set of the small
-# kernels, for 60 MB of row buffers at a hidden width of 5120.  1000 tokens over four layers: 6.65 -> 5.8 ms.
+# kernels, for 60 MB of row buffers and 28 MB of partial tiles at the benchmark's shapes, whatever the number of layers.
+# 1000 tokens over four layers: 6.65 -> 5.8 ms.
 PROMPT_ROWS = 384
 
 
@@ -262,6 +263,10 @@ class BatchDecoder:
         for w in weights.linears():
             if hasattr(w, "reserve"):
                 w.reserve(min(self.max_rows, 128))
+        # Batches above 128 rows leave partial tiles behind inside a linear: one block for all of them, taken here, before
+        # anybody sizes anything else by the memory that is left (28 MB at the benchmark's shapes).
+        wide_bytes = max((w.wide_scratch_bytes for w in weights.linears() if type(w) is ResidentWeight), default=0)
+        self._partials = torch.empty(wide_bytes, device=self.dev, dtype=torch.uint8) if self.prompt_rows > 128 and wide_bytes else None
         self.graphs = {}
 
     # ---- sequence slots and pages (host bookkeeping; the device sees only the page table) ---------------------
@@ -302,32 +307,38 @@ class BatchDecoder:
         delta = None
         for i, layer in enumerate(w.layers):
             ops.rmsnorm(h, layer.norm1, x, delta=delta, eps=cfg.eps)       # (the previous layer's MLP output joins the stream here)
-            layer.qkv(x, self.qkv[:n])
+            self._linear(layer.qkv, x, self.qkv[:n])
             for lo in range(0, n, self.max_rows):       # (rows see positions up to their own: those of earlier slices are appended)
                 rows = slice(lo, min(n, lo + self.max_rows))
                 self.attn(self.qkv[rows], self.cos, self.sin, self.row_seq[rows], self.row_pos[rows], self.page_table, self.kv[i, 0],
                           self.kv[i, 1], self.ctx[rows])
             self._row_parallel(layer.o, "o", self.ctx[:n], self.o_out[:n])
             ops.rmsnorm(h, layer.norm2, x, delta=self.o_out[:n], eps=cfg.eps)
-            layer.gate_up(x, self.gate_up[:n])
+            self._linear(layer.gate_up, x, self.gate_up[:n])
             ops.silu_mul(self.gate_up[:n], self.act[:n])
             self._row_parallel(layer.down, "down", self.act[:n], self.down_out[:n])
             delta = self.down_out[:n]
         ops.rmsnorm(h, w.final_norm, x, delta=delta, eps=cfg.eps)          # h now holds the final residual stream
         if not head:
             return
-        w.lm_head(x, self.logits[:n])
+        self._linear(w.lm_head, x, self.logits[:n])
         ops.argmax(self.logits[:n], self.next_token[:n])
         if advance:
             self.tokens[:n].copy_(self.next_token[:n])
             self.row_pos[:n].add_(1)
 
+    def _linear(self, linear, x, out) -> None:
+        if self._partials is not None and x.shape[0] > 128 and type(linear) is ResidentWeight:
+            linear.gemm(x, out, scratch=self._partials)
+        else:
+            linear(x, out)
+
     def _row_parallel(self, linear, slot: str, x, out) -> None:
         """out = linear(x), summed over the ranks when the weight is split by columns."""
         if self.peer is None:
-            linear(x, out)
+            self._linear(linear, x, out)
         else:
-            linear(x, self.peer.slot(slot, out.shape[0], out.shape[1]))
+            self._linear(linear, x, self.peer.slot(slot, out.shape[0], out.shape[1]))
             self.peer.reduce(slot, out)
 
     def run(self, kind: str, n: int, *, graph: bool = True) -> None:

@@ -248,6 +248,15 @@ int grb_bxr_gemm_next(const void* device_image, const bxr_header* header, const 
                       int64_t ldy, const void* bias, void* workspace, uint64_t workspace_bytes, uint32_t* status,
                       void* cuda_stream, const void* next_device_image, const bxr_header* next_header);
 
+/* grb_bxr_gemm_next with partial tiles lent for this call: `partials` (device, 16-byte aligned, contents of no account) takes
+ * those of a batch above 128 rows, so that one block serves all weights of a stream and every workspace is sized for 128
+ * rows.  192 rows per pass need grb_bxr_workspace_bytes(h, 129) - (row_blocks * 4 rounded up to 256) bytes; less, or NULL,
+ * is as if it were not given. */
+int grb_bxr_gemm_partials(const void* device_image, const bxr_header* header, const void* x, int64_t ldx, uint32_t m, void* y,
+                          int64_t ldy, const void* bias, void* workspace, uint64_t workspace_bytes, void* partials,
+                          uint64_t partials_bytes, uint32_t* status, void* cuda_stream, const void* next_device_image,
+                          const bxr_header* next_header);
+
 /* y[m, n] = bf16( sum_k x[m, k] * W[n, k] (+ bias[n]) ) for a DENSE BF16 weight W [rows, cols] (row stride ldw), m <= 8.
  * Replaces miv_gemv_out / linear, gs/miv_gemv.py:125-191,916-959, with its numerical contract: lanes walk 16-byte
  * vectors in increasing k, eight FMAs per vector in element order, xor butterfly, K slices added in slice order, bias

@@ -26,10 +26,10 @@ def test_the_call_is_there_with_and_without_a_compiler(monkeypatch, tmp_path, br
         monkeypatch.setenv("CPATH", "")
     assert lib_build.build() == lib_build.OUT                      # the library itself needs neither
     assert lib_build.FASTCALL.exists() == (broken is None)
-    call, entry = _native.gemm_next()
-    assert call(entry, *[0] * 14) == BAD_ARGUMENT                  # reached the library: null pointers are refused there
+    call, entry = _native.gemm_partials()
+    assert call(entry, *[0] * 16) == BAD_ARGUMENT                  # reached the library: null pointers are refused there
     with pytest.raises((TypeError, ctypes.ArgumentError)):
-        call(entry, 1.5, *[0] * 13)
+        call(entry, 1.5, *[0] * 15)
 
 
 def test_a_binding_older_than_its_source_is_built_again(monkeypatch, tmp_path):

@@ -36,7 +36,7 @@ def test_rows_equal_those_of_narrow_passes(shape, workers, m):
 
 
 def test_scratch_of_128_rows_still_serves_any_batch():
-    """Inside a capture nothing is allocated: the batch runs in passes of 128 rows, with the same bits."""
+    """Inside a capture as outside: the weight's own scratch stays what 128 rows need, and the bits are the same."""
     from georefine_b200.resident import ResidentWeight
 
     g = torch.Generator().manual_seed(3)
@@ -49,7 +49,7 @@ def test_scratch_of_128_rows_still_serves_any_batch():
     with torch.cuda.graph(graph):
         r.gemm(x, y)
     assert r.max_m == 128
-    r.gemm(x, want)                                          # wide scratch from here on; the graph keeps its own
+    r.gemm(x, want)
     assert r.max_m == 400
     graph.replay()
     assert r.check_status() == 0 and torch.equal(y, want)
@@ -74,3 +74,92 @@ def test_prompt_in_wide_chunks_equals_chunks_of_a_step(length):
         tokens = list(b.active[slot]["tokens"]) + [b.step()[slot] for _ in range(3)]
         got.append((tokens, d.kv.clone(), d.logits[:1].clone()))
     assert got[0][0] == got[1][0] and torch.equal(got[0][1][:, :, :-1], got[1][1][:, :, :-1]) and torch.equal(got[0][2], got[1][2])
+
+
+def _weight(n, k, workers, max_m=128):
+    from georefine_b200.resident import ResidentWeight
+
+    w = (torch.randn(n, k, generator=torch.Generator().manual_seed(n)) * 0.02).to(torch.bfloat16)
+    r = ResidentWeight.from_words(w.view(torch.int16).numpy().view(np.uint16), torch.device("cuda:0"), layout="window4", workers=workers, max_m=max_m)
+    return r, lambda m: torch.randn(m, k, generator=torch.Generator().manual_seed(m)).to(torch.bfloat16).cuda()
+
+
+@pytest.mark.parametrize("entry", ["gemm", "linear"])
+def test_graphs_keep_their_scratch_whatever_is_multiplied_afterwards(entry):
+    """Graphs captured below and above 128 rows, on a weight whose scratch has to grow in between, replayed at the end;
+    eager calls between a capture and its first replay."""
+    r, rows = _weight(3000, 1152, 37, max_m=8)               # 37 workers: no clusters, row blocks shared by CTAs
+    assert r.wide_scratch_bytes > 0
+    sizes = (8, 100, 400) if entry == "linear" else (8, 400)
+    full, _ = _weight(3000, 1152, 37)
+    want = {m: torch.empty(m, 3000, dtype=torch.bfloat16, device="cuda") for m in (8, 100, 400)}
+    x = {m: rows(m) for m in want}
+    for m in want:
+        for lo in range(0, m, 128):
+            full.gemm(x[m][lo:lo + 128], want[m][lo:lo + 128])
+    graphs, first = {}, r.workspace
+    out = {m: torch.full_like(want[m], float("nan")) for m in want}
+    for m in sizes:
+        if entry == "gemm" and m > 8:
+            r.reserve(128)
+        graphs[m] = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graphs[m]):
+            if entry == "linear":
+                r.linear(x[m], out=out[m])
+            else:
+                r.gemm(x[m], out[m])
+    for m in (8, 100, 400, 100, 8):                          # before any replay
+        assert torch.equal(r.linear(x[m]), want[m]), m
+    assert first.data_ptr() in [ws.data_ptr() for ws in (r.workspace, *r._outgrown)]
+    for _ in range(2):
+        for m in sizes:
+            out[m].fill_(float("nan"))
+            graphs[m].replay()
+            assert torch.equal(out[m], want[m]), m
+    assert r.check_status() == 0
+
+
+def test_wide_batches_leave_no_memory_behind(monkeypatch):
+    import gc
+
+    r, rows = _weight(5000, 1152, 148)
+    x, want = rows(400), torch.empty(400, 5000, dtype=torch.bfloat16, device="cuda")
+    y = torch.empty_like(want)
+    for lo in range(0, 400, 128):
+        r.gemm(x[lo:lo + 128], want[lo:lo + 128])
+    gc.collect()
+    held, said = torch.cuda.memory_allocated(), r.resident_bytes
+    r.gemm(x, y)
+    assert torch.equal(y, want)
+    assert torch.cuda.memory_allocated() == held and r.resident_bytes == said == r.bytes + r.workspace.numel() + 4
+    lent = torch.empty(r.wide_scratch_bytes, dtype=torch.uint8, device="cuda").fill_(255)     # contents of no account
+    r.gemm(x, y.fill_(float("nan")), scratch=lent)
+    assert torch.equal(y, want)
+    r.gemm(x, y.fill_(float("nan")), scratch=lent[:-256])    # too little: passes of 128 rows
+    assert torch.equal(y, want)
+
+    empty = torch.empty
+
+    def none_left(*size, **kw):
+        if kw.get("dtype") is torch.uint8:
+            raise torch.cuda.OutOfMemoryError("no memory left")
+        return empty(*size, **kw)
+
+    monkeypatch.setattr(torch, "empty", none_left)
+    r.gemm(x, y.fill_(float("nan")))
+    assert torch.equal(y, want) and r.check_status() == 0
+
+
+def test_a_long_prompt_leaves_no_memory_behind():
+    from georefine_b200 import serve
+
+    dev = torch.device("cuda:0")
+    cfg = serve.DecoderConfig(hidden=640, layers=2, heads=10, kv_heads=2, ffn=1792, vocab=1000)
+    weights = serve.DecoderWeights.synthetic(cfg, dev, seed=5)
+    d = serve.BatchDecoder(weights, max_rows=128, max_slots=2, max_context=1024, device=dev)
+    b = serve.Batcher(d)
+    said = sum(w.resident_bytes for w in weights.linears())
+    b.admit([1, 2, 3])                                       # (libraries loaded)
+    held = torch.cuda.memory_allocated()
+    b.admit([i % 1000 for i in range(900)])
+    assert torch.cuda.memory_allocated() == held and sum(w.resident_bytes for w in weights.linears()) == said
