@@ -379,16 +379,21 @@ class BatchDecoder:
     def absorb(self, slots, positions, tokens) -> None:
         """Queues the rows (up to ``prompt_rows``, each sequence's in the order of their positions) and the step that appends
         them to their sequences' KV pages; their logits are not wanted."""
-        self.queue_rows(slots, positions, tokens)
+        self._queue(slots, positions, tokens, self.prompt_rows)
         self._trunk(len(slots), False, head=False)
 
     def queue_rows(self, slots, positions, tokens) -> None:
         """``set_rows`` without the wait, for a caller whose step follows on the same stream.  The rows go through pinned
         memory that the caching host allocator does not hand out again before the copies are done; copies from
         pageable memory would each wait for everything the stream has before them."""
+        self._queue(slots, positions, tokens, self.max_rows)
+
+    def _queue(self, slots, positions, tokens, most) -> None:
         import torch
 
         n = len(slots)
+        if n > most:      # (the buffers may be longer than what the caller's kind of pass takes)
+            raise ValueError(f"{n} rows in a pass of up to {most}")
         rows = torch.tensor([list(slots), list(positions), list(tokens)], dtype=torch.int32, pin_memory=True)
         for src, dst in zip(rows, (self.row_seq, self.row_pos, self.tokens)):
             dst[:n].copy_(src, non_blocking=True)

@@ -163,3 +163,18 @@ def test_a_long_prompt_leaves_no_memory_behind():
     held = torch.cuda.memory_allocated()
     b.admit([i % 1000 for i in range(900)])
     assert torch.cuda.memory_allocated() == held and sum(w.resident_bytes for w in weights.linears()) == said
+
+
+def test_more_rows_than_a_pass_takes_are_refused():
+    from georefine_b200 import serve
+
+    dev = torch.device("cuda:0")
+    cfg = serve.DecoderConfig(hidden=640, layers=1, heads=10, kv_heads=2, ffn=1792, vocab=1000)
+    d = serve.BatchDecoder(serve.DecoderWeights.synthetic(cfg, dev, seed=5), max_rows=128, max_slots=2, max_context=1024, device=dev)
+    before = d.tokens.clone(), d.row_seq.clone(), d.row_pos.clone()
+    for put, n in ((d.set_rows, 129), (d.queue_rows, d.prompt_rows), (d.absorb, d.prompt_rows + 1)):
+        with pytest.raises(ValueError):
+            put([0] * n, range(n), [1] * n)
+    assert all(torch.equal(a, b) for a, b in zip(before, (d.tokens, d.row_seq, d.row_pos)))
+    d.set_rows([0] * 128, range(128), [1] * 128)
+    assert d.row_pos[:128].tolist() == list(range(128))
