@@ -365,6 +365,8 @@ int grb_bctx_decode_packed(const grb_bctx_tensor* t, const grb_bctx_packed* p, c
     return GRB_ERR_ARGUMENT;
   const bool coded = t->mode == 128;
   if ((t->mode != 0 && !coded) || (coded && (!t->residual_states || !t->residual_offsets))) return GRB_ERR_ARGUMENT;
+  // (the kernel reads the raw residuals of whole runs without looking at their end)
+  if (!coded && t->residual_bytes < t->n / 4 * 3 + (t->n % 4 * 6 + 7) / 8) return GRB_ERR_ARGUMENT;
   const uint32_t contexts = t->nr * t->nc, shift = p->shape[0], ctx_bytes = p->shape[1], bytes = p->shape[4];
   if (shift < 3 || shift > 8 || !contexts || (ctx_bytes & 15) || (bytes & 15) || ctx_bytes < (131072u >> shift) + 8 ||
       p->shape[3] != uint64_t(contexts) * ctx_bytes || p->shape[3] > bytes || p->shape[2] < 4 || p->shape[2] > 8)
