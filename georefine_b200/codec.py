@@ -128,14 +128,19 @@ _BESIDE_WORDS = 1 << 16      # smaller tensors are done before another thread ha
 
 class _Beside:
     """``fn()`` on another thread while this one goes on (hashing, compression and the library's calls release the
-    interpreter lock); at once when ``worth`` is false.  ``result()`` waits and returns or raises."""
+    interpreter lock); at once when ``worth`` is false or there is no thread to be had.  ``result()`` waits and returns or raises."""
 
     def __init__(self, fn, worth=True):
         self._value, self._error, self._thread = None, None, None
         if worth:
-            self._thread = threading.Thread(target=self._run, args=(fn,), daemon=True)
-            self._thread.start()
-        else:
+            try:
+                thread = threading.Thread(target=self._run, args=(fn,), daemon=True)
+                thread.start()
+            except RuntimeError:      # no thread to be had: a limit is reached, or the interpreter is shutting down
+                worth = False
+            else:
+                self._thread = thread
+        if not worth:
             self._run(fn)
 
     def _run(self, fn):

@@ -33,3 +33,30 @@ def test_workers_that_get_no_memory_report_it(spare):
     assert [line.split()[0] for line in run.stdout.splitlines()] == ["frequencies", "labels"]
     if spare == 1500:
         assert run.stdout.split() == ["frequencies", "done", "labels", "done"]
+
+
+@pytest.mark.parametrize("mask", [0xFFFF, 0xFFF8])
+def test_frames_are_made_and_read_without_a_second_thread(orc, monkeypatch, mask):
+    import threading
+
+    import numpy as np
+
+    from georefine_b200 import codec
+    from georefine_b200.gpu import index_frame
+
+    words = orc.synthetic_weight_words(300, 999, 3) & np.uint16(mask)
+    assert words.size >= codec._BESIDE_WORDS
+    want = codec.encode(words)
+
+    def refused(self):
+        raise RuntimeError("can't start new thread")
+
+    monkeypatch.setattr(threading.Thread, "start", refused)
+    frame = codec.encode(words)
+    assert frame == want and np.array_equal(codec.decode(frame), words)
+    assert np.array_equal(index_frame(frame, 128, keep_words=True)["words"], words)
+    for at in (codec.HEADER.size + 5, len(frame) // 2, len(frame) - 1):
+        broken = bytearray(frame)
+        broken[at] ^= 1
+        with pytest.raises(codec.CodecError, match="frame checksum mismatch"):
+            codec.decode(bytes(broken))
