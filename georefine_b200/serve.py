@@ -31,6 +31,7 @@ PAGE = ops.PAGE
 # kernels, for 60 MB of row buffers and 28 MB of partial tiles at the benchmark's shapes, whatever the number of layers.
 # 1000 tokens over four layers: 6.65 -> 5.8 ms.
 PROMPT_ROWS = 384
+STAGING = 4     # passes whose rows may be on their way to the device at a time
 
 
 @dataclass(frozen=True)
@@ -267,6 +268,7 @@ class BatchDecoder:
         # anybody sizes anything else by the memory that is left (28 MB at the benchmark's shapes).
         wide_bytes = max((w.wide_scratch_bytes for w in weights.linears() if type(w) is ResidentWeight), default=0)
         self._partials = torch.empty(wide_bytes, device=self.dev, dtype=torch.uint8) if self.prompt_rows > 128 and wide_bytes else None
+        self._staging, self._staged = [(torch.zeros(3, R, dtype=i32).pin_memory(), torch.cuda.Event()) for _ in range(STAGING)], 0
         self.graphs = {}
 
     # ---- sequence slots and pages (host bookkeeping; the device sees only the page table) ---------------------
@@ -383,9 +385,9 @@ class BatchDecoder:
         self._trunk(len(slots), False, head=False)
 
     def queue_rows(self, slots, positions, tokens) -> None:
-        """``set_rows`` without the wait, for a caller whose step follows on the same stream.  The rows go through pinned
-        memory that the caching host allocator does not hand out again before the copies are done; copies from
-        pageable memory would each wait for everything the stream has before them."""
+        """``set_rows`` without the wait, for a caller whose step follows on the same stream.  The rows go through the decoder's
+        own pinned memory: copies from pageable memory would each wait for everything the stream has before them, and a
+        pinned allocation in the middle of serving costs milliseconds."""
         self._queue(slots, positions, tokens, self.max_rows)
 
     def _queue(self, slots, positions, tokens, most) -> None:
@@ -394,9 +396,14 @@ class BatchDecoder:
         n = len(slots)
         if n > most:      # (the buffers may be longer than what the caller's kind of pass takes)
             raise ValueError(f"{n} rows in a pass of up to {most}")
-        rows = torch.tensor([list(slots), list(positions), list(tokens)], dtype=torch.int32, pin_memory=True)
-        for src, dst in zip(rows, (self.row_seq, self.row_pos, self.tokens)):
-            dst[:n].copy_(src, non_blocking=True)
+        rows = torch.tensor([list(slots), list(positions), list(tokens)], dtype=torch.int32)
+        staging, copied = self._staging[self._staged % STAGING]
+        self._staged += 1
+        copied.synchronize()             # the pass that used this place before has taken its rows
+        staging[:, :n].copy_(rows)
+        for src, dst in zip(staging, (self.row_seq, self.row_pos, self.tokens)):
+            dst[:n].copy_(src[:n], non_blocking=True)
+        copied.record(torch.cuda.current_stream(self.dev))
 
     def streamed_bytes(self, rows_context) -> dict:
         """Bytes one step streams: the compressed weights, and the KV cache of rows whose contexts are given."""

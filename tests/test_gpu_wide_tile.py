@@ -178,3 +178,26 @@ def test_more_rows_than_a_pass_takes_are_refused():
     assert all(torch.equal(a, b) for a, b in zip(before, (d.tokens, d.row_seq, d.row_pos)))
     d.set_rows([0] * 128, range(128), [1] * 128)
     assert d.row_pos[:128].tolist() == list(range(128))
+
+
+def test_rows_reach_the_device_in_order_without_allocating():
+    """Passes queued far ahead of the device, of sizes never seen before: every one finds its own rows."""
+    from georefine_b200 import serve
+
+    dev = torch.device("cuda:0")
+    cfg = serve.DecoderConfig(hidden=640, layers=1, heads=10, kv_heads=2, ffn=1792, vocab=1000)
+    d = serve.BatchDecoder(serve.DecoderWeights.synthetic(cfg, dev, seed=5), max_rows=128, max_slots=2, max_context=1024, device=dev)
+    pinned = torch.cuda.host_memory_stats()["num_host_alloc"]
+    sizes, seen = [1, 2, 3, 7, 128, 64, 5, 33, 127, 1, 100, 17], []
+    torch.cuda._sleep(20_000_000)                            # some 10 ms of work before them
+    for i, n in enumerate(sizes):
+        d.queue_rows([i % 2] * n, range(i, i + n), [100 * i + j for j in range(n)])
+        seen.append((d.row_seq[:n].clone(), d.row_pos[:n].clone(), d.tokens[:n].clone()))
+    for i, (n, (seq, pos, tok)) in enumerate(zip(sizes, seen)):
+        assert seq.tolist() == [i % 2] * n and pos.tolist() == list(range(i, i + n)) and tok.tolist() == [100 * i + j for j in range(n)]
+    d.set_rows([1] * 50, range(50), [9] * 50)
+    d.run("ar", 50)
+    for _ in range(3):
+        d.set_rows([1] * 51, range(51), [9] * 51)
+        d.run("ar", 51)
+    assert torch.cuda.host_memory_stats()["num_host_alloc"] == pinned
