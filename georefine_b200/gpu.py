@@ -175,14 +175,26 @@ def _packed_tables(indexed, stride):
 
 class _Outcome:
     """Where the kernel writes how a checked decode went: two words of pinned host memory, {status bits, an index was out of
-    range}.  One call has it to itself from the launch until it has read it."""
+    range}.  One call has it to itself from the launch until it has read it.  The places of all tensors come from one
+    block (a pinned allocation costs milliseconds): as many as calls are under way at a time, 512 per block."""
 
-    def __init__(self):
-        import torch
+    free = []
 
-        self._memory = torch.zeros(2, dtype=torch.int32).pin_memory()
-        self.at = self._memory.data_ptr()
-        self.words = (ctypes.c_uint32 * 2).from_address(self.at)
+    def __init__(self, block, at):
+        self._block, self.at = block, at
+        self.words = (ctypes.c_uint32 * 2).from_address(at)
+
+    @classmethod
+    def take(cls):
+        try:
+            return cls.free.pop()
+        except IndexError:
+            import torch
+
+            block = torch.zeros(512, 2, dtype=torch.int32).pin_memory()
+            first, *others = (cls(block, block.data_ptr() + 8 * i) for i in range(512))
+            cls.free.extend(others)
+            return first
 
 
 class CudaContextTensor:
@@ -250,7 +262,7 @@ class CudaContextTensor:
                 self._bucket_shift[kind] = shift
         self.error = torch.zeros((), device=self.device, dtype=torch.int32)
         self._error_clear, self._captured = True, False     # is the word known to be zero; may a graph's replay write it
-        self._outcomes = [_Outcome()]       # those no call is using; a thread that finds none makes its own
+        _Outcome.free.append(_Outcome.take())      # (the first block is allocated here and not by the first call)
         self.resident = None
         if fused and words is not None:
             self.resident = ResidentWeight.from_words(words, device=self.device, source_sha256=bytes.fromhex(self.source_sha256),
@@ -320,10 +332,7 @@ class CudaContextTensor:
         self._error_clear = wait and not self._captured
         outcome = None
         if wait:
-            try:
-                outcome = self._outcomes.pop()
-            except IndexError:
-                outcome = _Outcome()
+            outcome = _Outcome.take()
             outcome.words[0] = outcome.words[1] = 0
         stream = torch.cuda.current_stream(self.device)
         args = (*self._packed_args, None if ids is None else ids.data_ptr(), count, result.data_ptr(), self.error.data_ptr(),
@@ -338,7 +347,7 @@ class CudaContextTensor:
         if wait:
             stream.synchronize()
             failed, outside = outcome.words
-            self._outcomes.append(outcome)
+            _Outcome.free.append(outcome)
             if failed or outside:
                 self._error_clear = False
                 if outside:

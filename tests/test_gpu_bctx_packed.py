@@ -143,3 +143,21 @@ def test_gathers_on_both_sides_of_the_packed_limit(orc, shape, classes, coarse):
                 ids[count // 2] = wrong
                 with pytest.raises(IndexError):
                     t.gather_rows(ids)
+
+
+def test_tensors_share_one_pinned_block(orc):
+    """Outcomes of checked decodes need no pinned allocation per tensor, and every place comes back, also after an error."""
+    from georefine_b200 import codec, gpu
+
+    words = orc.synthetic_weight_words(32, 256, 5)
+    frame = codec.encode(words)
+    gpu.CudaContextTensor(frame, device="cuda:0", fused=False).decode()
+    pinned = torch.cuda.host_memory_stats()["num_host_alloc"]
+    tensors = [gpu.CudaContextTensor(frame, device="cuda:0", fused=False) for _ in range(5)]
+    places = len(gpu._Outcome.free)
+    for t in tensors:
+        assert np.array_equal(t.decode().view(torch.uint16).cpu().numpy(), words)
+        with pytest.raises(IndexError):
+            t.gather_rows(torch.tensor([32]))
+        assert len(t.gather_rows(torch.tensor([31]))) == 1
+    assert len(gpu._Outcome.free) == places and torch.cuda.host_memory_stats()["num_host_alloc"] == pinned
