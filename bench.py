@@ -622,7 +622,8 @@ def indexed_decode_times(device):
         t = CudaContextTensor(frame, stride=1024, walk_stride=walk, device=device, fused=False)
         ok = bool(np.array_equal(t.decode().view(torch.int16).cpu().numpy().view(np.uint16), words))
         us = timed_us(lambda: t.decode(check=False))
-        out[f"bctx_decode_kernel_stride{walk}"] = {"us": round(us, 1), "dense_GBps": round(2 * words.size / us / 1e3, 1), "bit_exact": ok,
+        kernel = "bctx_decode_kernel" if t._packed is None else "bctx_packed_kernel"
+        out[f"{kernel}_stride{walk}"] = {"us": round(us, 1), "dense_GBps": round(2 * words.size / us / 1e3, 1), "bit_exact": ok,
                                                    "index_bytes": int(sum(v.numel() * v.element_size() for k, v in t.buffers.items()
                                                                           if k.endswith(("_states", "_offsets"))))}
         if walk == 1024:

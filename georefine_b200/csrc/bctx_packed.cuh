@@ -10,8 +10,8 @@
 // bucket, its 8-byte entry (first slot, frequency, symbol), every second symbol a word of the stream.  The window moves by
 // selects, not by a branch; a bucket tells its two symbols apart, so that the forward scan is left to rare symbols (with one
 // rank per bucket some lane of a warp scanned at nearly every symbol).  A main symbol and the residual of the one before it
-// are looked up together: their chains are independent.  What is left is 100 instructions per warp and pair of symbols at
-// 68 % of the issue slots, the integer pipe 71 % and shared memory 70 % busy.
+// are looked up together: their chains are independent.  What is left is 100 instructions per warp and word at 63 % of
+// the issue slots, with the integer pipe 66 % and the shared-memory data pipe 73 % busy.
 // 4096 x 4096 words with coded residuals, 128 per lane: 305 us before (tables in global memory, one CTA of 64 lanes after
 // another), 118 us with the tables of all 64 contexts in shared memory (room for 14 warps), 86 us with one row class per CTA
 // (28 warps).  128 rows of 5120 words with raw residuals: 160 us before, 25 us.

@@ -8,7 +8,7 @@
 // branched on, and the tables of the four contexts a row can meet (32 KB) stay in the first-level cache.  The residual
 // chain (mode 128), the raw residuals and the joining of the words fit beside the main chain.  Encoding replaces the division
 // by a multiplication with a precomputed reciprocal and writes its bytes unconditionally.
-// 1024 x 2048 words: encode() 47 -> 13 ms, decode() 38 -> 15 ms (with hashing and compression on other threads).
+// 1024 x 2048 words: encode() 47 -> 13 ms, decode() 38 -> 16 ms (with hashing and compression on other threads).
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -230,6 +230,8 @@ GRB_CLONES bool frame_words_raw(const FrameJob& j, Stream s, Stream t) { return 
 GRB_CLONES bool frame_words_coded(const FrameJob& j, Stream s, Stream t) { return frame_words<true>(j, s, t); }
 
 // ---- encoding -------------------------------------------------------------------------------------------------
+// The division-free form of the update is the one of F. Giesen's public-domain byte-wise rANS coder (ryg_rans: bound, reciprocal,
+// bias and complemented frequency per symbol), here with a 64-bit reciprocal, which needs no shift.
 // What coding one symbol needs: a renormalisation bound, the reciprocal ceil(2^64 / f) (exact for 32-bit states), and the
 // state's new value as q * scale + x + bias with q = floor(x / f).  f == 1 has no such reciprocal: with 2^64 - 1 the quotient
 // comes out as x - 1, which its bias makes good.

@@ -3,8 +3,8 @@
 ``ResidentWeight`` follows the descriptor protocol of the reference's serving engines
 (``glc_serve/fastdec.py:172-188`` ``Lin``, ``glc_serve/tbe_desc.py:127-157`` ``TBELin``,
 ``glc_serve/bigemm.py:468-507`` ``BILin``): attributes ``kind``, ``N``, ``K``, ``bytes``, ``coded_bytes`` and
-``__call__(x[M,K], y[M,N])`` writing into a preallocated ``y`` with no allocation and no host
-synchronisation, so a call can be captured in a CUDA graph.
+``__call__(x[M,K], y[M,N])`` writing into a preallocated ``y`` with no allocation (but the scratch that batches above
+128 rows borrow, see ``gemm``) and no host synchronisation, so a call can be captured in a CUDA graph.
 """
 from __future__ import annotations
 
