@@ -346,7 +346,7 @@ class CudaContextTensor:
             _native.check(status, "grb_bctx_decode_packed")
         if wait:
             stream.synchronize()
-            failed, outside = outcome.words
+            failed, outside = outcome.words[0], outcome.words[1]
             _Outcome.free.append(outcome)
             if failed or outside:
                 self._error_clear = False

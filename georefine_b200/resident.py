@@ -266,7 +266,7 @@ class ResidentWeight:
         return m
 
     def _within_reserve(self, m):
-        if m > self.max_m and min(m, 128) > min(self.max_m, 128):
+        if min(m, 128) > min(self.max_m, 128):
             raise ValueError(f"batch of {m} rows exceeds the reserved scratch ({self.max_m}); call reserve() first")
 
     def then(self, next_weight):
@@ -286,7 +286,8 @@ class ResidentWeight:
         m = self._checked(x, y)
         if not m:
             return
-        self._within_reserve(m)
+        if m > self.max_m:
+            self._within_reserve(m)
         self._multiply(x, y, bias, m, self.workspace, scratch)
 
     def _multiply(self, x, y, bias, m, workspace, scratch):
