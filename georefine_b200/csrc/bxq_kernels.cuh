@@ -4,9 +4,9 @@
 //   * kUmma  : a lane holds the 32 weights of its row and phase in 16 registers and writes them with one tcgen05.st
 //              into tensor memory, where tcgen05.mma takes them as its A operand (M = 128 weight rows; the batch is
 //              N, read from shared memory).  Shared memory carries only what comes from outside the SM: chunk blobs
-//              and activation tiles.  Two threads issue the MMAs, chunk about, each into an accumulator of its own.  (In the 3-bit window kernel the operand tile lives in shared memory, and its
-//              stores plus the tensor core's reads of it are more than 40 % of all shared-memory traffic, which sets
-//              that kernel's pace; its per-chunk exception patching is what keeps it from using tensor memory: done
+//              and activation tiles.  One elected lane issues all MMAs of an item into one accumulator.  (In the 3-bit
+//              window kernel the operand tile lives in shared memory, and its stores plus the tensor core's reads of it
+//              are more than 40 % of all shared-memory traffic, which sets that kernel's pace; its per-chunk exception patching is what keeps it from using tensor memory: done
 //              in registers it costs more instructions than the decode itself.)
 //   * kDense : decode twin (parity tests, ResidentWeight.decode).
 // Same persistent, warp-specialised pipeline and work partition as the other fused kernels; any batch size, the
@@ -17,35 +17,34 @@
 namespace grb {
 
 constexpr int kWideWarpLoader = 16;    // bulk copies of chunk blobs
-constexpr int kWideWarpMma = 17;       // TMEM owner and MMA issuer of the even chunks of an item
-constexpr int kWideWarpMma2 = 19;      // MMA issuer of the odd chunks
-constexpr int kWideWarpXLoader = 18;   // TMA loads of activation tiles
+constexpr int kWideWarpMma = 17;       // TMEM owner and MMA issuer
+constexpr int kWideWarpXLoader = 18;   // TMA loads of activation tiles (warp 19 has no role)
 constexpr int kWideWarpEpilogue = 20;  // 4 warps: warp % 4 = the tensor-memory lane quarter a warp may read
 
-// Tensor memory (up to NB = 128): columns [0, 256) accumulators, FP32: an item has two, one per MMA issuer (even chunks, odd chunks;
-// the epilogue adds them), NB columns each.  Up to NB = 64 two items fit (one being multiplied, one being drained);
-// at NB = 128 there is room for one, and the issuers wait for the drain at an item boundary while the decoders fill
-// the operand stages.  Columns [256, 512): the decoded weights of four chunks, 64 columns each (two 128 x 64 atoms, two
-// BF16 per column).  (The narrow tiles would leave room for six or seven stages and a deeper activation ring; measured at
-// NB = 16 with 7 stages, 8 activation stages and 6 requests in flight, every M = 1 launch got slower, gate|up by 4.6 us.)
+// Tensor memory: columns [0, 256) accumulators, FP32, one of NB columns per item.  Up to NB = 128 two items fit, one being
+// multiplied while the other is drained.  (Two issuing threads with an accumulator each, chunk about, which the epilogue
+// added, left room for one item at NB = 128, whose drain the issuers then waited for; since the issuing lane is an elected
+// one it keeps up alone.  34816 x 5120 at 128 rows 61.6 -> 59.7 us, 5120 x 17408 35.7 -> 35.2 us, 5120 x 5120 at 192 rows
+// 17.8 -> 17.2 us; one row unchanged.)  Columns [256, 512): the decoded weights of four chunks, 64 columns each (two 128 x 64
+// atoms, two BF16 per column).  (The narrow tiles would leave room for six or seven stages and a deeper activation ring;
+// measured at NB = 16 with 7 stages, 8 activation stages and 6 requests in flight, every M = 1 launch got slower, gate|up by
+// 4.6 us.)
 constexpr int kWideNextBlobs = 8;      // blobs per CTA of the next launch that a finishing CTA asks the L2 for
 constexpr uint32_t kWideTmemCols = 512;
-// The 192-column tile, for batches above 128 rows: its accumulators take 384 columns and leave two operand stages, enough
-// because a chunk's multiply (768 tensor-core cycles) is longer than the hand-over it has to hide.  Such a batch is bound by
+// The 192-column tile, for batches above 128 rows: room for one item's accumulator.  Such a batch is bound by
 // the number of its passes over the weights: at 128 columns the tensor core is busy for 38 % of a pass, and a pass costs
-// little more at 192 (34816 x 5120: 62 -> 74.4 us).  768 rows, six passes -> four: 34816 x 5120 394 -> 306 us,
-// 5120 x 17408 217 -> 177 us, 5120 x 5120 94 -> 72 us.
+// little more at 192 (34816 x 5120: 60 -> 72.5 us).
 template <int NB>
-constexpr int kWideStages = NB <= 128 ? 4 : 2;
-template <int NB>
-constexpr uint32_t kWideOperandCol = kWideTmemCols - 64u * kWideStages<NB>;
+constexpr int kWideAccBufs = NB <= 128 ? 2 : 1;  // items whose accumulators fit tensor memory at once
+constexpr int kWideStages = 4;
+constexpr uint32_t kWideOperandCol = kWideTmemCols - 64u * kWideStages;
 
 // Shared-memory plan: a ring of chunk blobs and a ring of activation tiles (two NB x 64 atoms per chunk), the
 // latter requested kXLag chunks ahead of the weights they will meet (they come from L2 with a latency of about a
 // microsecond).
 template <int MODE, int NB>
 struct BxqSmem {
-  static constexpr int kOp = (MODE == kUmma) ? kWideStages<NB> : 0;
+  static constexpr int kOp = (MODE == kUmma) ? kWideStages : 0;
   static constexpr int kX = (MODE == kUmma) ? (NB <= 64 ? 4 : 3) : 0;
   static constexpr int kXLag = 2;
   static constexpr uint32_t kXStage = 2 * NB * 128;
@@ -71,7 +70,7 @@ struct BxqSmem {
   static_assert(MODE != kUmma || kIn >= 3, "ring too shallow");
   // what keeps the activation loader at most one barrier phase behind the MMA issuer (see its role below)
   static_assert(MODE != kUmma || (kXLag < kX && kOp + kXLag + 1 > kX), "activation ring and lag do not fit the operand ring");
-  static_assert(MODE != kUmma || 2 * NB * (NB <= 64 ? 2 : 1) <= int(kWideOperandCol<NB>), "accumulators overlap the operand columns");
+  static_assert(MODE != kUmma || NB * kWideAccBufs<NB> <= int(kWideOperandCol), "accumulators overlap the operand columns");
   static_assert(8 * nbars + 64 <= 512, "barrier area");
   static_assert(MODE != kUmma || (1 + kRing) * NB * 512u <= bars, "the closing reduction's tiles would overwrite the barriers");
   static_assert(alloc <= 232448, "exceeds the 227 KB of shared memory a CTA may opt into");
@@ -297,7 +296,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   constexpr uint32_t kTmemCols = kWideTmemCols;
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;
   constexpr uint32_t kXN = L::kX ? L::kX : 1;
-  constexpr uint32_t kAccBufs = NB <= 64 ? 2 : 1;  // items whose accumulators fit tensor memory at once
+  constexpr uint32_t kAccBufs = kWideAccBufs<NB>;
 
   // The blob loader's own barriers first of all (blobs of one size: it needs nothing else to start its copies): their
   // fences complete while the CTA's share of the work is being computed.
@@ -354,7 +353,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps + 1;  // op_full: + the loader's go-ahead
       else if (n >= 2u * L::kIn + 2 * L::kOp + L::kX) {
         const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + L::kX);  // acc_full x2, acc_empty x2, final, tile_full x2, tile_used x2
-        count = j < 2 ? 2u : j < 5 ? 4u : j < 5 + L::kRing ? 1u : uint32_t(kDecoderWarps + 4);  // acc_full: both MMA issuers commit
+        count = j < 2 ? 1u : j < 5 ? 4u : j < 5 + L::kRing ? 1u : uint32_t(kDecoderWarps + 4);
       }
       mbar_init(ctx.bars + 8 * n, count);
     }
@@ -388,7 +387,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     const uint32_t raw_at = BXQ_RAW_AT + ((2 * q) * BXR_ROWS + r) * 16;
     const uint32_t code_at = BXQ_CODES_AT + 4 * (q * BXR_ROWS + r);
     // this lane's 16 operand columns: lane = row, columns = its 32 weights inside the chunk's atom
-    const uint32_t operand_at = ((rg * 32u) << 16) + kWideOperandCol<NB> + (q >> 1) * 32 + (q & 1) * 16;
+    const uint32_t operand_at = ((rg * 32u) << 16) + kWideOperandCol + (q >> 1) * 32 + (q & 1) * 16;
     bool live = true;
     uint32_t next_base = first_base;
     for (uint32_t u = unit_begin; u < unit_end && live;) {
@@ -527,13 +526,9 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         }
       }
     }
-  } else if (MODE == kUmma && (warp == kWideWarpMma || warp == kWideWarpMma2)) {
+  } else if (MODE == kUmma && warp == kWideWarpMma) {
     // ------------------------------------------------------------------ MMA issue: one wait, eight MMAs, one commit
-    // Issuing takes a thread about a hundred cycles per MMA, more than the tensor core needs for it: two threads
-    // take turns chunk by chunk.  The order of additions has to be a fixed one, so each has an accumulator of its own:
-    // chunk i of an item (counted from the item's first) goes to accumulator i mod 2, whatever the batch size.
     constexpr uint32_t idesc = umma_idesc_bf16(NB);
-    const uint32_t which = warp == kWideWarpMma2 ? 1u : 0u;
     uint32_t n_item = 0, so = 0, pho = 0, sx = 0;
     bool live = true;
     for (uint32_t u = unit_begin; u < unit_end && live; ++n_item) {
@@ -542,27 +537,24 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t buf = n_item % kAccBufs, use = n_item / kAccBufs;
       if (!__all_sync(0xFFFFFFFFu, !ctx.aborted() && ctx.wait(bar_acc_empty + 8 * buf, (use & 1) ^ 1))) { live = false; break; }
       tc_fence_after();
-      const uint32_t d_tmem = tmem_base + (buf * 2 + which) * NB;
+      const uint32_t d_tmem = tmem_base + buf * NB;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
-        const uint32_t i = c - item.chunk_begin;
-        if ((i & 1) == which) {
-          if (!ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
-          tc_fence_after();
-          if (elect_one()) {
-            const uint32_t a_tmem = tmem_base + kWideOperandCol<NB> + so * 64;
-            const uint64_t bdesc = umma_desc_sw128(smem + L::xs + sx * L::kXStage);
-            uint32_t accumulate = i >= 2 ? 1u : 0u;
+        if (!ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t a_tmem = tmem_base + kWideOperandCol + so * 64;
+          const uint64_t bdesc = umma_desc_sw128(smem + L::xs + sx * L::kXStage);
+          uint32_t accumulate = c != item.chunk_begin ? 1u : 0u;
 #pragma unroll
-            for (uint32_t a = 0; a < 2; ++a)
+          for (uint32_t a = 0; a < 2; ++a)
 #pragma unroll
-              for (uint32_t k = 0; k < 4; ++k) {
-                umma_bf16_ts(d_tmem, a_tmem + a * 32 + k * 8, bdesc + a * (NB * 128 >> 4) + 2 * k, idesc, accumulate);
-                accumulate = 1;
-              }
-            umma_commit(bar_op_empty + 8 * so);
-          }
-          __syncwarp();
+            for (uint32_t k = 0; k < 4; ++k) {
+              umma_bf16_ts(d_tmem, a_tmem + a * 32 + k * 8, bdesc + a * (NB * 128 >> 4) + 2 * k, idesc, accumulate);
+              accumulate = 1;
+            }
+          umma_commit(bar_op_empty + 8 * so);
         }
+        __syncwarp();
         if (++so == kOpN) { so = 0; pho ^= 1; }
         if (++sx == kXN) sx = 0;
       }
@@ -586,8 +578,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * buf, use & 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t row = item.row_block * BXR_ROWS + r;
-      const uint32_t taddr = tmem_base + ((e * 32) << 16) + buf * 2 * NB;   // even-chunk accumulator; the odd one NB columns on
-      const bool two = item.chunk_end - item.chunk_begin > 1;                // a one-chunk item has no odd chunk
+      const uint32_t taddr = tmem_base + ((e * 32) << 16) + buf * NB;
       const float b = (args.bias && row < args.rows) ? __bfloat162float(args.bias[row]) : 0.f;
       constexpr int kStep = 16, kCols = L::kTurnCols;  // accumulator columns per tensor-memory load, and per turn-around
       // (a load's round trip is what a step waits for: 16 columns per load where only 8 fit the turn-around took a
@@ -612,15 +603,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
         uint32_t v[kStep];
         tmem_ld16(taddr + m0, v);
-        if (two) {
-          uint32_t odd[kStep];
-          tmem_ld16(taddr + NB + m0, odd);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < kStep; ++i) v[i] = __float_as_uint(__fadd_rn(__uint_as_float(v[i]), __uint_as_float(odd[i])));
-        } else {
-          tmem_ld_wait();
-        }
+        tmem_ld_wait();
         if (keep) {
 #pragma unroll
           for (int i = 0; i < kStep; ++i)
