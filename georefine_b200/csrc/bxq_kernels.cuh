@@ -39,14 +39,13 @@ constexpr int kWideAccBufs = NB <= 128 ? 2 : 1;  // items whose accumulators fit
 constexpr int kWideStages = 4;
 constexpr uint32_t kWideOperandCol = kWideTmemCols - 64u * kWideStages;
 
-// Shared-memory plan: a ring of chunk blobs and a ring of activation tiles (two NB x 64 atoms per chunk), the
-// latter requested kXLag chunks ahead of the weights they will meet (they come from L2 with a latency of about a
-// microsecond).
+// Shared-memory plan: a ring of chunk blobs and a ring of activation tiles (two NB x 64 atoms per chunk; they come from L2
+// with a latency of about a microsecond, so a stage is asked for again the moment its multiply is through).
 template <int MODE, int NB>
 struct BxqSmem {
   static constexpr int kOp = (MODE == kUmma) ? kWideStages : 0;
   static constexpr int kX = (MODE == kUmma) ? (NB <= 64 ? 4 : 3) : 0;
-  static constexpr int kXLag = 2;
+  static constexpr bool kXOwn = kX != kOp;   // activation stages are handed back on barriers of their own
   static constexpr uint32_t kXStage = 2 * NB * 128;
   static constexpr uint32_t kReserve = 1024 /* alignment slack */ + 512 /* barriers, flags */;
   // the epilogue warps turn their accumulator columns around in shared memory (a lane holds one weight row, memory
@@ -60,16 +59,14 @@ struct BxqSmem {
   static constexpr uint32_t turn = xs + kX * kXStage;
   static constexpr uint32_t in = turn + 4 * kTurn;
   static constexpr uint32_t bars = in + kIn * BXQ_BLOB_MAX;
-  // barrier order: in_full, in_empty [kIn each]; op_full, op_empty [kOp each]; x_full [kX]; acc_full, acc_empty
-  // [2 each]; final; tile_full, tile_used [kRing each] (the closing reduction)
+  // barrier order: in_full, in_empty [kIn each]; op_full, op_empty [kOp each]; x_full [kX]; x_empty [kX, if kXOwn];
+  // acc_full, acc_empty [2 each]; final; tile_full, tile_used [kRing each] (the closing reduction)
   static constexpr uint32_t kRing = (NB <= 64) ? 4 : (NB <= 128) ? 2 : 1;  // tiles in flight in the closing reduction (kWideTileRing)
-  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + kX + 4 + 1 + 2 * kRing;
+  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + (kXOwn ? 2 : 1) * kX + 4 + 1 + 2 * kRing;
   static constexpr uint32_t misc = (bars + 8 * nbars + 15) & ~15u;  // tmem base, abort flag, decision
   static constexpr uint32_t total = misc + 48;
   static constexpr uint32_t alloc = total + 1024;
   static_assert(MODE != kUmma || kIn >= 3, "ring too shallow");
-  // what keeps the activation loader at most one barrier phase behind the MMA issuer (see its role below)
-  static_assert(MODE != kUmma || (kXLag < kX && kOp + kXLag + 1 > kX), "activation ring and lag do not fit the operand ring");
   static_assert(MODE != kUmma || NB * kWideAccBufs<NB> <= int(kWideOperandCol), "accumulators overlap the operand columns");
   static_assert(8 * nbars + 64 <= 512, "barrier area");
   static_assert(MODE != kUmma || (1 + kRing) * NB * 512u <= bars, "the closing reduction's tiles would overwrite the barriers");
@@ -291,7 +288,8 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   const uint32_t bar_in_full = ctx.bars, bar_in_empty = bar_in_full + 8 * L::kIn;
   const uint32_t bar_op_full = bar_in_empty + 8 * L::kIn, bar_op_empty = bar_op_full + 8 * L::kOp;
   const uint32_t bar_x_full = bar_op_empty + 8 * L::kOp;
-  const uint32_t bar_acc_full = bar_x_full + 8 * L::kX, bar_acc_empty = bar_acc_full + 16, bar_final = bar_acc_empty + 16;
+  const uint32_t bar_x_empty = L::kXOwn ? bar_x_full + 8 * L::kX : bar_op_empty;   // (rings of one length: stage i of both is free together)
+  const uint32_t bar_acc_full = bar_x_full + 8 * L::kX * (L::kXOwn ? 2 : 1), bar_acc_empty = bar_acc_full + 16, bar_final = bar_acc_empty + 16;
   const uint32_t bar_tile_full = bar_final + 8, bar_tile_used = bar_tile_full + 8 * L::kRing;
   constexpr uint32_t kTmemCols = kWideTmemCols;
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;
@@ -348,11 +346,11 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
 #pragma unroll
     for (uint32_t n = i; n < L::nbars; n += 32) {
       if (n < uint32_t(L::kIn) && args.blob_stride16) continue;                    // in_full: the loader's own (above)
-      uint32_t count = 1;                                                          // in_full, op_empty, x_full
+      uint32_t count = 1;                                                          // in_full, op_empty, x_full, x_empty
       if (n >= uint32_t(L::kIn) && n < 2u * L::kIn) count = kDecoderWarps;          // in_empty
-      else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps + 1;  // op_full: + the loader's go-ahead
-      else if (n >= 2u * L::kIn + 2 * L::kOp + L::kX) {
-        const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + L::kX);  // acc_full x2, acc_empty x2, final, tile_full x2, tile_used x2
+      else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps;  // op_full
+      else if (n >= 2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX) {
+        const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX);  // acc_full x2, acc_empty x2, final, tile_full, tile_used
         count = j < 2 ? 1u : j < 5 ? 4u : j < 5 + L::kRing ? 1u : uint32_t(kDecoderWarps + 4);
       }
       mbar_init(ctx.bars + 8 * n, count);
@@ -494,42 +492,28 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     if (ctx.aborted() && lane == 0)
       for (uint32_t u = (issued > uint32_t(L::kIn) ? issued - L::kIn : 0); u < issued; ++u) mbar_wait(bar_in_full + 8 * (u % L::kIn), (u / L::kIn) & 1);
   } else if (MODE == kUmma && warp == kWideWarpXLoader) {
-    // ------------------------------------------------------------------ activation tiles by TMA, and the go-ahead
-    // One thread.  Chunk v of this CTA (in the order the items list them) uses activation stage v % kX and operand
-    // stage v % kOp (tensor memory).  The tiles of chunk v are requested once chunk v - kX has been multiplied (its stage is free);
-    // kXLag chunks later the thread waits for them and gives the MMA warp the go-ahead by arriving on the operand
-    // stage's `full` barrier, which the decoder warps complete.  "Chunk c has been multiplied" is the phase of
-    // op_empty[c % kOp] that the MMA warp's commit completes; this thread is never more than one phase behind it,
-    // because the multiply of chunk c + kOp needs its own go-ahead.
+    // ------------------------------------------------------------------ activation tiles by TMA
+    // One thread.  Chunk v of this CTA (in the order the items list them) uses activation stage v % kX, which is free once
+    // chunk v - kX has been multiplied.  (A tile that has arrived is the issuer's at once.  When this thread passed tiles on,
+    // two chunks behind its requests, the pass stood behind waits for older multiplies: the four linears of a layer at one
+    // row 98.5 -> 93 us, a step of one sequence 505 -> 479 us without it.)
     if (lane == 0) {
       grid_dependency_wait();
       const uint64_t stay = l2_policy_evict_last();  // every CTA reads the same activation tiles
-      bool live = true;
       uint32_t c_v = unit_begin % args.chunks;  // the chunk (column block) to request next: wraps at the end of a row block
-      auto multiplied = [&](uint32_t c) { return ctx.wait(bar_op_empty + 8 * (c % kOpN), (c / kOpN) & 1); };
-      for (uint32_t v = 0; v < unit_count + L::kXLag && live; ++v) {
-        if (ctx.aborted()) break;
-        // the go-ahead first: the request below waits for a multiply that may need it
-        if (v >= uint32_t(L::kXLag)) {
-          const uint32_t w = v - L::kXLag;
-          if (!ctx.wait(bar_x_full + 8 * (w % kXN), (w / kXN) & 1)) { live = false; break; }
-          if (w >= kOpN && !multiplied(w - kOpN)) { live = false; break; }
-          mbar_arrive(bar_op_full + 8 * (w % kOpN));
-        }
-        if (v < unit_count) {
-          if (v >= kXN && !multiplied(v - kXN)) { live = false; break; }
-          const uint32_t sx = v % kXN, stage = smem + L::xs + sx * L::kXStage;
-          mbar_arrive_expect_tx(bar_x_full + 8 * sx, L::kXStage);
-          tma_load_2d(stage, &tmap_x, int(c_v * BXR_COLS), 0, bar_x_full + 8 * sx, stay);
-          tma_load_2d(stage + NB * 128, &tmap_x, int(c_v * BXR_COLS + 64), 0, bar_x_full + 8 * sx, stay);
-          if (++c_v == args.chunks) c_v = 0;
-        }
+      for (uint32_t v = 0; v < unit_count; ++v) {
+        const uint32_t sx = v % kXN, stage = smem + L::xs + sx * L::kXStage;
+        if (ctx.aborted() || !ctx.wait(bar_x_empty + 8 * sx, ((v / kXN) & 1) ^ 1)) break;
+        mbar_arrive_expect_tx(bar_x_full + 8 * sx, L::kXStage);
+        tma_load_2d(stage, &tmap_x, int(c_v * BXR_COLS), 0, bar_x_full + 8 * sx, stay);
+        tma_load_2d(stage + NB * 128, &tmap_x, int(c_v * BXR_COLS + 64), 0, bar_x_full + 8 * sx, stay);
+        if (++c_v == args.chunks) c_v = 0;
       }
     }
   } else if (MODE == kUmma && warp == kWideWarpMma) {
-    // ------------------------------------------------------------------ MMA issue: one wait, eight MMAs, one commit
+    // ------------------------------------------------------------------ MMA issue: eight per chunk, then its stages go back
     constexpr uint32_t idesc = umma_idesc_bf16(NB);
-    uint32_t n_item = 0, so = 0, pho = 0, sx = 0;
+    uint32_t n_item = 0, so = 0, pho = 0, sx = 0, phx = 0;
     bool live = true;
     for (uint32_t u = unit_begin; u < unit_end && live; ++n_item) {
       const WideSpan item = wide_span(u, unit_end, args.chunks);
@@ -539,7 +523,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + buf * NB;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
-        if (!ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
+        if (!ctx.wait_warp(bar_x_full + 8 * sx, phx) || !ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
         tc_fence_after();
         if (elect_one()) {
           const uint32_t a_tmem = tmem_base + kWideOperandCol + so * 64;
@@ -553,10 +537,11 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
               accumulate = 1;
             }
           umma_commit(bar_op_empty + 8 * so);
+          if (L::kXOwn) umma_commit(bar_x_empty + 8 * sx);
         }
         __syncwarp();
         if (++so == kOpN) { so = 0; pho ^= 1; }
-        if (++sx == kXN) sx = 0;
+        if (++sx == kXN) { sx = 0; phx ^= 1; }
       }
       if (live && elect_one()) umma_commit(bar_acc_full + 8 * buf);
       __syncwarp();
