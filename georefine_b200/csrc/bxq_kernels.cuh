@@ -34,19 +34,35 @@ constexpr uint32_t kWideTmemCols = 512;
 // The 192-column tile, for batches above 128 rows: room for one item's accumulator.  Such a batch is bound by
 // the number of its passes over the weights: at 128 columns the tensor core is busy for 38 % of a pass, and a pass costs
 // little more at 192 (34816 x 5120: 60 -> 72.5 us).
-template <int NB>
-constexpr int kWideAccBufs = NB <= 128 ? 2 : 1;  // items whose accumulators fit tensor memory at once
-constexpr int kWideStages = 4;
-constexpr uint32_t kWideOperandCol = kWideTmemCols - 64u * kWideStages;
+//
+// Pairs of CTAs (PAIR, cta_group::2), for batches above 128 rows.  Such a batch is bound by the power cap (a pass of 192 rows
+// by single CTAs settles at 1.25 GHz), that is by what a multiply costs in energy besides the multiply: decoding and
+// streaming a chunk, and bringing its activations in through L2.  Two CTAs of a cluster walk the same chunks of two row blocks side by
+// side; the one of even rank issues MMAs of M = 256 for both, each CTA's tensor memory holding the decoded weights and the
+// accumulators of its own row block and each CTA's shared memory half of the activation rows.  With that and two
+// accumulator tiles (T = 2) a pass takes 384 rows, so that a chunk is streamed, decoded and written to tensor memory once for
+// twice the rows and meets half the activation bytes per row.  At 384 rows, two passes before and one now: 34816 x 5120 147 ->
+// 109 us, 5120 x 17408 86 -> 75 us, 7168 x 5120 42 -> 33 us, 5120 x 5120 36 -> 27 us.  (Barriers that a peer arrives on with
+// release and acquire at cluster scope cost 1.4 us a chunk; the plain forms order what matters here, the completed tensor
+// memory stores and bulk copies.  At 128 rows pairs gain nothing: 34816 x 5120 58.4 against 59.4 us, 7168 x 5120 18.4 against
+// 17.0 us.)
+template <int NB, int T>
+constexpr int kWideAccBufs = T == 1 && NB <= 128 ? 2 : 1;  // items whose accumulators fit tensor memory at once
+template <int NB, int T>
+constexpr int kWideStages = T * NB <= 256 ? 4 : 2;         // (two are enough at 384 columns: a chunk's multiply takes 1536 tensor-core cycles)
+template <int NB, int T>
+constexpr uint32_t kWideOperandCol = kWideTmemCols - 64u * kWideStages<NB, T>;
 
-// Shared-memory plan: a ring of chunk blobs and a ring of activation tiles (two NB x 64 atoms per chunk; they come from L2
-// with a latency of about a microsecond, so a stage is asked for again the moment its multiply is through).
-template <int MODE, int NB>
+// Shared-memory plan: a ring of chunk blobs and a ring of activation tiles (T x two atoms of 64 columns per chunk, each of the
+// rows this CTA brings in).
+template <int MODE, int NB, int T, bool PAIR>
 struct BxqSmem {
-  static constexpr int kOp = (MODE == kUmma) ? kWideStages : 0;
-  static constexpr int kX = (MODE == kUmma) ? (NB <= 64 ? 4 : 3) : 0;
-  static constexpr bool kXOwn = kX != kOp;   // activation stages are handed back on barriers of their own
-  static constexpr uint32_t kXStage = 2 * NB * 128;
+  static constexpr int kOp = (MODE == kUmma) ? kWideStages<NB, T> : 0;
+  static constexpr uint32_t kXRows = NB / (PAIR ? 2 : 1);     // activation rows of one tile that this CTA holds
+  static constexpr uint32_t kXAtom = kXRows * 128;
+  static constexpr uint32_t kXStage = T * 2 * kXAtom;
+  static constexpr int kX = (MODE != kUmma) ? 0 : kXStage <= 16384 ? (PAIR ? 5 : 4) : kXStage <= 24576 ? 4 : 3;
+  static constexpr bool kXOwn = kX != kOp;                    // activation stages are handed back on barriers of their own
   static constexpr uint32_t kReserve = 1024 /* alignment slack */ + 512 /* barriers, flags */;
   // the epilogue warps turn their accumulator columns around in shared memory (a lane holds one weight row, memory
   // wants consecutive rows together): 16 columns x 32 rows x 4 bytes per warp
@@ -67,7 +83,7 @@ struct BxqSmem {
   static constexpr uint32_t total = misc + 48;
   static constexpr uint32_t alloc = total + 1024;
   static_assert(MODE != kUmma || kIn >= 3, "ring too shallow");
-  static_assert(MODE != kUmma || NB * kWideAccBufs<NB> <= int(kWideOperandCol), "accumulators overlap the operand columns");
+  static_assert(MODE != kUmma || T * NB * kWideAccBufs<NB, T> <= int(kWideOperandCol<NB, T>), "accumulators overlap the operand columns");
   static_assert(8 * nbars + 64 <= 512, "barrier area");
   static_assert(MODE != kUmma || (1 + kRing) * NB * 512u <= bars, "the closing reduction's tiles would overwrite the barriers");
   static_assert(alloc <= 232448, "exceeds the 227 KB of shared memory a CTA may opt into");
@@ -118,6 +134,9 @@ __device__ __forceinline__ void bxq_patch(uint32_t (&out)[16], uint32_t column, 
 // arithmetic: no load stands between the start of a CTA and its first blob, window base and multiply.  (The item
 // list in the image holds the same geometry plus the partial-tile bookkeeping - part, parts, slot - which the
 // epilogue reads with plenty of time to spare; bxr_validate checks that the two agree.)
+//
+// Paired images: workers 2p and 2p + 1 have the same share, share p of the (pair of row blocks, chunk) sequence; worker 2p + r
+// takes row block 2g + r of pair g.  `row_block` below counts pairs then.
 struct WideSpan {
   uint32_t row_block, chunk_begin, chunk_end;
 };
@@ -135,14 +154,18 @@ __device__ __forceinline__ WideSpan wide_span(uint32_t unit, uint32_t unit_end, 
 template <int NB>
 constexpr uint32_t kWideTileRing = NB <= 64 ? 4 : NB <= 128 ? 2 : 1;  // (1 + ring) x NB x 512 bytes of shared memory
 
-template <int NB>
+// `tile` = which of the pass's T tiles of NB batch rows.
+__device__ __forceinline__ uint32_t wide_tile_cols(uint32_t m, uint32_t tile, uint32_t nb) {  // its batch rows, in whole eights
+  return (min(m - min(m, tile * nb), nb) + 7) & ~7u;
+}
+template <int NB, int T>
 __device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const RoleCtx& ctx, uint32_t row_block, uint32_t first,
                                                      uint32_t parts, uint32_t own, uint32_t smem, uint32_t bar_full, uint32_t bar_used,
-                                                     uint32_t t, uint32_t& fetched) {
+                                                     uint32_t t, uint32_t tile, uint32_t& fetched) {
   constexpr uint32_t kThreads = (kDecoderWarps + 4) * 32;
   constexpr int kMine = (NB * 32 + kThreads - 1) / kThreads;  // float4 positions per thread
   constexpr uint32_t kTile = NB * BXR_ROWS * 4;
-  const uint32_t mcols = (args.m + 7) & ~7u, total = mcols * 32, bytes = mcols * BXR_ROWS * 4;
+  const uint32_t mcols = wide_tile_cols(args.m, tile, NB), total = mcols * 32, bytes = mcols * BXR_ROWS * 4;
   const uint32_t remote = parts - (own < parts ? 1u : 0u);
   const uint32_t lane = t & 31;
   uint32_t asked = 0;  // remote tiles requested in this call
@@ -152,7 +175,7 @@ __device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const 
     const uint32_t n = fetched + j, b = n % kRing, p = j + ((own < parts && own <= j) ? 1u : 0u);
     if (!ctx.wait(bar_used + 8 * b, ((n / kRing) & 1) ^ 1)) { live = false; return; }
     mbar_arrive_expect_tx(bar_full + 8 * b, bytes);
-    bulk_g2s(smem + kTile * (1 + b), args.partials + size_t(first + p) * NB * BXR_ROWS, bytes, bar_full + 8 * b, l2_policy_evict_first());
+    bulk_g2s(smem + kTile * (1 + b), args.partials + (size_t(first + p) * T + tile) * NB * BXR_ROWS, bytes, bar_full + 8 * b, l2_policy_evict_first());
     asked = j + 1;
   };
   if (t == 0)
@@ -195,7 +218,7 @@ __device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const 
   if (!live) return;
 #pragma unroll
   for (int k = 0; k < kMine; ++k) {
-    const uint32_t at = t + k * kThreads, m = at >> 5, row4 = row_block * BXR_ROWS + (at & 31) * 4;
+    const uint32_t at = t + k * kThreads, m = tile * NB + (at >> 5), row4 = row_block * BXR_ROWS + (at & 31) * 4;
     if (at >= total || m >= args.m || row4 >= args.rows) continue;
     float f[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
     if (args.bias)
@@ -224,21 +247,23 @@ __device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const 
 // left its FP32 tile at the start of its shared memory; after the cluster barrier each CTA adds the P tiles of ITS share
 // of the batch columns (m = rank, rank + P, ...) in rank order - its own from local shared memory, the others over
 // distributed shared memory - and writes y.  No partial tile goes to global memory, no counter, no fence, and the work
-// of the reduction is spread over the P SMs.  t = index of the calling thread among the (kDecoderWarps + 4) x 32.
-template <int NB>
-__device__ __forceinline__ void bxq_reduce_in_cluster(const BxrArgs& args, uint32_t row_block, uint32_t smem, uint32_t t) {
+// of the reduction is spread over the P SMs.  t = index of the calling thread among the (kDecoderWarps + 4) x 32; `tile` = which
+// of the pass's tiles of NB batch rows.  In a cluster of pairs (two row blocks side by side) part p of this CTA's row
+// block belongs to rank 2p + (own rank mod 2).
+template <int NB, bool PAIR>
+__device__ __forceinline__ void bxq_reduce_in_cluster(const BxrArgs& args, uint32_t row_block, uint32_t smem, uint32_t t, uint32_t tile) {
   constexpr uint32_t kThreads = (kDecoderWarps + 4) * 32;
-  const uint32_t parts = args.cluster, rank = cluster_rank();
-  const uint32_t mcols = (args.m + 7) & ~7u;
+  const uint32_t parts = args.cluster, in_cluster = cluster_rank(), rank = PAIR ? in_cluster >> 1 : in_cluster;
+  const uint32_t mcols = wide_tile_cols(args.m, tile, NB);
   const uint32_t mine = rank < mcols ? (mcols - rank + parts - 1) / parts : 0;  // batch columns rank, rank + P, ... below mcols
   for (uint32_t i = t; i < mine * 32; i += kThreads) {
     const uint32_t m = rank + (i >> 5) * parts, at = (m << 5) | (i & 31);
     const uint32_t row4 = row_block * BXR_ROWS + (i & 31) * 4;
-    if (m >= args.m || row4 >= args.rows) continue;
+    if (tile * NB + m >= args.m || row4 >= args.rows) continue;
     uint4 u[8];  // every part's piece first (independent loads in flight), then the sum in K order
 #pragma unroll
     for (uint32_t p = 0; p < 8; ++p)
-      if (p < parts) u[p] = p == rank ? lds128(smem + at * 16) : lds128_cluster(cluster_map(smem + at * 16, p));
+      if (p < parts) u[p] = p == rank ? lds128(smem + at * 16) : lds128_cluster(cluster_map(smem + at * 16, PAIR ? 2 * p + (in_cluster & 1u) : p));
     // part 0 is taken as it is: adding it to zero would lose the sign of a -0
     float f[4] = {__uint_as_float(u[0].x), __uint_as_float(u[0].y), __uint_as_float(u[0].z), __uint_as_float(u[0].w)};
 #pragma unroll
@@ -252,7 +277,7 @@ __device__ __forceinline__ void bxq_reduce_in_cluster(const BxrArgs& args, uint3
     if (args.bias)
       for (int k = 0; k < 4; ++k)
         if (row4 + k < args.rows) f[k] = __fadd_rn(f[k], __bfloat162float(args.bias[row4 + k]));
-    __nv_bfloat16* dst = args.y + size_t(m) * args.ldy + row4;
+    __nv_bfloat16* dst = args.y + size_t(tile * NB + m) * args.ldy + row4;
     if (row4 + 3 < args.rows && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
       __nv_bfloat162 lo, hi;
       lo.x = __float2bfloat16_rn(f[0]);
@@ -270,14 +295,22 @@ __device__ __forceinline__ void bxq_reduce_in_cluster(const BxrArgs& args, uint3
   }
 }
 
-template <int MODE, int NB>
+template <int MODE, int NB, int T = 1, bool PAIR = false>
 __global__ void __launch_bounds__(MODE == kUmma ? kThreadsUmma : kThreadsSimt, 1)
 bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
-  using L = BxqSmem<MODE, NB>;
+  using L = BxqSmem<MODE, NB, T, PAIR>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t worker = blockIdx.x;
+  // A row block cut into P = args.cluster parts belongs to P workers in a row.  Pairs: a cluster of 2P CTAs has two row blocks,
+  // part and row block alternating by rank.
+  uint32_t worker = blockIdx.x;
+  if (PAIR && args.cluster > 1) {
+    const uint32_t n = blockIdx.x / (2 * args.cluster), in_cluster = blockIdx.x - n * 2 * args.cluster;
+    worker = (2 * n + (in_cluster & 1u)) * args.cluster + (in_cluster >> 1);
+  }
+  const uint32_t my_rank = PAIR ? cluster_rank() : 0u;
+  const bool leader = (my_rank & 1u) == 0;                 // issues the MMAs of its pair
 
   RoleCtx ctx;
   ctx.smem = smem;
@@ -294,7 +327,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   constexpr uint32_t kTmemCols = kWideTmemCols;
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;
   constexpr uint32_t kXN = L::kX ? L::kX : 1;
-  constexpr uint32_t kAccBufs = kWideAccBufs<NB>;
+  constexpr uint32_t kAccBufs = kWideAccBufs<NB, T>, kOperandCol = kWideOperandCol<NB, T>;
+  // accumulator `tile` of the CTA's n-th item: its place in tensor memory (T = 2: one per tile) and which use of the place it is
+  auto acc_slot = [](uint32_t n_item, uint32_t tile) { return T == 1 ? n_item % kAccBufs : tile; };
+  auto acc_use = [](uint32_t n_item) { return T == 1 ? n_item / kAccBufs : n_item; };
 
   // The blob loader's own barriers first of all (blobs of one size: it needs nothing else to start its copies): their
   // fences complete while the CTA's share of the work is being computed.
@@ -305,9 +341,12 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   }
   // Work of this CTA, known from the arguments alone; the blob loader asks for its first offsets before anything
   // else so that the first copy can leave as soon as the barriers exist.
-  const uint64_t units = uint64_t(args.row_blocks) * args.chunks;
-  const uint32_t unit_begin = uint32_t(units * worker / args.workers);
-  const uint32_t unit_count = uint32_t(units * (worker + 1) / args.workers) - unit_begin;
+  const uint32_t group = args.paired ? 2u : 1u, in_group = args.paired ? worker & 1u : 0u;   // row block = (unit / chunks) * group + in_group
+  const uint64_t units = uint64_t(args.row_blocks / group) * args.chunks;
+  const uint32_t share = worker / group, shares = args.workers / group;
+  const uint32_t unit_begin = uint32_t(units * share / shares);
+  const uint32_t unit_count = uint32_t(units * (share + 1) / shares) - unit_begin;
+  auto blob_of = [&](uint32_t unit) { const uint32_t g = unit / args.chunks; return (g * group + in_group) * args.chunks + (unit - g * args.chunks); };
   uint32_t first_i0 = 0, first_i1 = 0;
   if (warp == kWideWarpLoader && unit_count && !args.blob_stride16) {
     const uint32_t mine = unit_begin + min(uint32_t(lane), unit_count - 1);
@@ -317,7 +356,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   const uint32_t unit_end = unit_begin + unit_count;
   // Decoders: the window base of this thread's row in the CTA's first item, asked for before anything else.
   uint32_t first_base = 0;
-  if (warp < kDecoderWarps && unit_count) first_base = args.base[(unit_begin / args.chunks) * BXR_ROWS + (warp & 3) * 32 + lane];
+  if (warp < kDecoderWarps && unit_count) first_base = args.base[((unit_begin / args.chunks) * group + in_group) * BXR_ROWS + (warp & 3) * 32 + lane];
   // Epilogue: where the CTA's items are in the image's list (their partial-tile bookkeeping); needed much later.
   uint32_t item_begin = 0, item_end = 0;
   if (MODE == kUmma && warp >= kWideWarpEpilogue) {
@@ -335,7 +374,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint64_t once = l2_policy_evict_first();
       for (uint32_t u = 0; u < early; ++u) {
         mbar_arrive_expect_tx(bar_in_full + 8 * u, bytes);
-        bulk_g2s(smem + L::in + u * BXQ_BLOB_MAX, args.blobs + size_t(unit_begin + u) * bytes, bytes, bar_in_full + 8 * u, once);
+        bulk_g2s(smem + L::in + u * BXQ_BLOB_MAX, args.blobs + size_t(blob_of(unit_begin + u)) * bytes, bytes, bar_in_full + 8 * u, once);
       }
     }
     __syncwarp();
@@ -346,12 +385,13 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
 #pragma unroll
     for (uint32_t n = i; n < L::nbars; n += 32) {
       if (n < uint32_t(L::kIn) && args.blob_stride16) continue;                    // in_full: the loader's own (above)
+      constexpr uint32_t kCtas = PAIR ? 2 : 1;   // CTAs whose warps arrive on a leader's barriers
       uint32_t count = 1;                                                          // in_full, op_empty, x_full, x_empty
       if (n >= uint32_t(L::kIn) && n < 2u * L::kIn) count = kDecoderWarps;          // in_empty
-      else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps;  // op_full
+      else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps * kCtas;  // op_full
       else if (n >= 2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX) {
         const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX);  // acc_full x2, acc_empty x2, final, tile_full, tile_used
-        count = j < 2 ? 1u : j < 5 ? 4u : j < 5 + L::kRing ? 1u : uint32_t(kDecoderWarps + 4);
+        count = j < 2 ? 1u : j < 4 ? 4u * kCtas : j < 5 ? 4u : j < 5 + L::kRing ? 1u : uint32_t(kDecoderWarps + 4);
       }
       mbar_init(ctx.bars + 8 * n, count);
     }
@@ -363,11 +403,12 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     mbar_fence_init();
   }
   if (MODE == kUmma && warp == kWideWarpMma) {
-    tmem_alloc(smem + L::misc, kTmemCols);
-    tmem_relinquish();
+    tmem_alloc<PAIR>(smem + L::misc, kTmemCols);
+    tmem_relinquish<PAIR>();
   }
   tc_fence_before();
-  __syncthreads();
+  if (PAIR) cluster_sync();   // the peer arrives on this CTA's barriers
+  else __syncthreads();
   tc_fence_after();
   // The image is never written by a kernel: everything up to the first access to x, bias, y or the workspace may
   // overlap the tail of the previous kernel in the stream.
@@ -377,6 +418,21 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   if (MODE == kUmma) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(smem + L::misc));
 
 
+  // Epilogue warps: tile t of the CTA's n_item-th item, from tensor memory to the start of shared memory, all of which is free
+  // by the time an item is kept.
+  auto drain_to_smem = [&](uint32_t n_item, uint32_t t, uint32_t e, uint32_t r) {
+    const uint32_t taddr = tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB, mcols = wide_tile_cols(args.m, t, NB);
+#pragma unroll 1
+    for (uint32_t m0 = 0; m0 < mcols; m0 += 16) {
+      uint32_t v[16];
+      tmem_ld16(taddr + m0, v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (m0 + i < mcols) sts32(smem + ((m0 + i) * BXR_ROWS + r) * 4, v[i]);
+    }
+  };
+
   if (warp < kDecoderWarps) {
     // ------------------------------------------------------------------ decoders: 32 weights per lane and chunk
     const uint32_t q = warp >> 2, rg = warp & 3, r = rg * 32 + lane;
@@ -385,15 +441,16 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     const uint32_t raw_at = BXQ_RAW_AT + ((2 * q) * BXR_ROWS + r) * 16;
     const uint32_t code_at = BXQ_CODES_AT + 4 * (q * BXR_ROWS + r);
     // this lane's 16 operand columns: lane = row, columns = its 32 weights inside the chunk's atom
-    const uint32_t operand_at = ((rg * 32u) << 16) + kWideOperandCol + (q >> 1) * 32 + (q & 1) * 16;
+    const uint32_t operand_at = ((rg * 32u) << 16) + kOperandCol + (q >> 1) * 32 + (q & 1) * 16;
+    const uint32_t op_full_at = PAIR ? cluster_map(bar_op_full, my_rank & ~1u) : bar_op_full;   // the issuer's
     bool live = true;
     uint32_t next_base = first_base;
     for (uint32_t u = unit_begin; u < unit_end && live;) {
       const WideSpan item = wide_span(u, unit_end, args.chunks);
       u += item.chunk_end - item.chunk_begin;
-      const uint32_t row = item.row_block * BXR_ROWS + r;
+      const uint32_t row = (item.row_block * group + in_group) * BXR_ROWS + r;
       const uint32_t base2 = next_base * 0x00800080u;
-      if (u < unit_end) next_base = args.base[row + BXR_ROWS];  // the next item's base: on its way while this item is decoded
+      if (u < unit_end) next_base = args.base[row + group * BXR_ROWS];  // the next item's base: on its way while this item is decoded
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
         if (!ctx.wait(bar_in_full + 8 * s, ph)) { live = false; break; }
         const uint32_t blob = smem + L::in + s * BXQ_BLOB_MAX;
@@ -421,7 +478,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar_op_full + 8 * so);
+          if (lane == 0) {
+            if (leader) mbar_arrive(bar_op_full + 8 * so);
+            else mbar_arrive_cluster(op_full_at + 8 * so);
+          }
           if (++so == kOpN) { so = 0; pho ^= 1; }
         } else if (row < args.rows) {
 #pragma unroll
@@ -446,7 +506,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     for (uint32_t u0 = 0; u0 < unit_count; u0 += 32) {
       uint32_t i0 = first_i0, i1 = first_i1;
       if (args.blob_stride16) {  // blobs of one size: no offsets to look up
-        i0 = (unit_begin + min(u0 + lane, unit_count - 1)) * args.blob_stride16;
+        i0 = blob_of(unit_begin + min(u0 + lane, unit_count - 1)) * args.blob_stride16;
         i1 = i0 + args.blob_stride16;
       } else if (u0) {
         const uint32_t mine = unit_begin + min(u0 + lane, unit_count - 1);
@@ -481,11 +541,14 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     // of the stream will want first - the leading blobs of its CTAs w, w + workers, ... (consecutive in memory) - so
     // that they arrive during this launch's tail and the next launch's set-up.
     if (MODE == kUmma && args.next_blobs && lane == 0 && !ctx.aborted()) {
+      const uint32_t next_group = args.next_paired ? 2u : 1u, next_shares = args.next_workers / next_group;
+      const uint64_t next_units = uint64_t(args.next_row_blocks / next_group) * args.next_chunks;
       for (uint32_t w2 = worker; w2 < args.next_workers; w2 += args.workers) {
-        const uint32_t b0 = uint32_t(uint64_t(args.next_units) * w2 / args.next_workers);
-        const uint32_t b1 = uint32_t(uint64_t(args.next_units) * (w2 + 1) / args.next_workers);
-        const uint32_t n = min(b1 - b0, uint32_t(kWideNextBlobs));
-        for (uint32_t b = 0; b < n; ++b) bulk_prefetch_l2(args.next_blobs + size_t(b0 + b) * args.next_blob_bytes, args.next_blob_bytes);
+        const uint32_t b0 = uint32_t(next_units * (w2 / next_group) / next_shares), b1 = uint32_t(next_units * (w2 / next_group + 1) / next_shares);
+        const uint32_t g = b0 / args.next_chunks, c = b0 - g * args.next_chunks;
+        const uint32_t first = (g * next_group + (args.next_paired ? w2 & 1u : 0u)) * args.next_chunks + c;
+        const uint32_t n = min(min(b1 - b0, uint32_t(kWideNextBlobs)), args.next_chunks - c);
+        for (uint32_t b = 0; b < n; ++b) bulk_prefetch_l2(args.next_blobs + size_t(first + b) * args.next_blob_bytes, args.next_blob_bytes);
       }
     }
     // after an abort: give copies still in flight a bounded time to land before the CTA exits
@@ -494,63 +557,82 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   } else if (MODE == kUmma && warp == kWideWarpXLoader) {
     // ------------------------------------------------------------------ activation tiles by TMA
     // One thread.  Chunk v of this CTA (in the order the items list them) uses activation stage v % kX, which is free once
-    // chunk v - kX has been multiplied.  (A tile that has arrived is the issuer's at once.  When this thread passed tiles on,
-    // two chunks behind its requests, the pass stood behind waits for older multiplies: the four linears of a layer at one
-    // row 98.5 -> 93 us, a step of one sequence 505 -> 479 us without it.)
+    // chunk v - kX has been multiplied.  Of a pair, each CTA brings in half of every tile's rows; both halves complete on the
+    // issuer's barrier.
     if (lane == 0) {
       grid_dependency_wait();
       const uint64_t stay = l2_policy_evict_last();  // every CTA reads the same activation tiles
+      const uint32_t x_full_at = PAIR ? cluster_map(bar_x_full, my_rank & ~1u) : bar_x_full;
       uint32_t c_v = unit_begin % args.chunks;  // the chunk (column block) to request next: wraps at the end of a row block
       for (uint32_t v = 0; v < unit_count; ++v) {
         const uint32_t sx = v % kXN, stage = smem + L::xs + sx * L::kXStage;
         if (ctx.aborted() || !ctx.wait(bar_x_empty + 8 * sx, ((v / kXN) & 1) ^ 1)) break;
-        mbar_arrive_expect_tx(bar_x_full + 8 * sx, L::kXStage);
-        tma_load_2d(stage, &tmap_x, int(c_v * BXR_COLS), 0, bar_x_full + 8 * sx, stay);
-        tma_load_2d(stage + NB * 128, &tmap_x, int(c_v * BXR_COLS + 64), 0, bar_x_full + 8 * sx, stay);
+        if (leader) mbar_arrive_expect_tx(bar_x_full + 8 * sx, L::kXStage * (PAIR ? 2 : 1));
+#pragma unroll
+        for (uint32_t t = 0; t < uint32_t(T); ++t)
+#pragma unroll
+          for (uint32_t a = 0; a < 2; ++a) {
+            const uint32_t dst = stage + (2 * t + a) * L::kXAtom;
+            const int col = int(c_v * BXR_COLS + 64 * a), row = int(t * NB + (PAIR ? (my_rank & 1u) * L::kXRows : 0u));
+            if (PAIR) tma_load_2d_pair(dst, &tmap_x, col, row, x_full_at + 8 * sx, stay);
+            else tma_load_2d(dst, &tmap_x, col, row, bar_x_full + 8 * sx, stay);
+          }
         if (++c_v == args.chunks) c_v = 0;
       }
     }
   } else if (MODE == kUmma && warp == kWideWarpMma) {
-    // ------------------------------------------------------------------ MMA issue: eight per chunk, then its stages go back
-    constexpr uint32_t idesc = umma_idesc_bf16(NB);
+    // ------------------------------------------------------------------ MMA issue: eight per chunk and tile, then the stages go back
+    constexpr uint32_t idesc = umma_idesc_bf16(NB, PAIR ? 256 : 128);
+    const uint16_t both = uint16_t(3u << (my_rank & ~1u));
+    auto commit = [&](uint32_t bar) {
+      if (PAIR) umma_commit_pair(bar, both);
+      else umma_commit(bar);
+    };
     uint32_t n_item = 0, so = 0, pho = 0, sx = 0, phx = 0;
-    bool live = true;
+    bool live = leader;
     for (uint32_t u = unit_begin; u < unit_end && live; ++n_item) {
       const WideSpan item = wide_span(u, unit_end, args.chunks);
       u += item.chunk_end - item.chunk_begin;
-      const uint32_t buf = n_item % kAccBufs, use = n_item / kAccBufs;
-      if (!__all_sync(0xFFFFFFFFu, !ctx.aborted() && ctx.wait(bar_acc_empty + 8 * buf, (use & 1) ^ 1))) { live = false; break; }
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + buf * NB;
-      for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
+      const uint32_t drained = (acc_use(n_item) & 1) ^ 1;
+      for (uint32_t c = item.chunk_begin; c < item.chunk_end && live; ++c) {
+        const bool first = c == item.chunk_begin, last = c + 1 == item.chunk_end;
+        if (first && !__all_sync(0xFFFFFFFFu, !ctx.aborted() && ctx.wait(bar_acc_empty + 8 * acc_slot(n_item, 0), drained))) { live = false; break; }
         if (!ctx.wait_warp(bar_x_full + 8 * sx, phx) || !ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t a_tmem = tmem_base + kWideOperandCol + so * 64;
-          const uint64_t bdesc = umma_desc_sw128(smem + L::xs + sx * L::kXStage);
-          uint32_t accumulate = c != item.chunk_begin ? 1u : 0u;
+        const uint32_t a_tmem = tmem_base + kOperandCol + so * 64;
 #pragma unroll
-          for (uint32_t a = 0; a < 2; ++a)
+        for (uint32_t t = 0; t < uint32_t(T); ++t) {
+          const uint32_t slot = acc_slot(n_item, t);
+          if (t && first && !ctx.wait_warp(bar_acc_empty + 8 * slot, drained)) { live = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t bdesc = umma_desc_sw128(smem + L::xs + sx * L::kXStage + 2 * t * L::kXAtom);
+            uint32_t accumulate = first ? 0u : 1u;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {
-              umma_bf16_ts(d_tmem, a_tmem + a * 32 + k * 8, bdesc + a * (NB * 128 >> 4) + 2 * k, idesc, accumulate);
-              accumulate = 1;
+            for (uint32_t a = 0; a < 2; ++a)
+#pragma unroll
+              for (uint32_t k = 0; k < 4; ++k) {
+                const uint64_t b = bdesc + a * (L::kXAtom >> 4) + 2 * k;
+                if (PAIR) umma_bf16_ts_pair(tmem_base + slot * NB, a_tmem + a * 32 + k * 8, b, idesc, accumulate);
+                else umma_bf16_ts(tmem_base + slot * NB, a_tmem + a * 32 + k * 8, b, idesc, accumulate);
+                accumulate = 1;
+              }
+            if (t + 1 == uint32_t(T)) {
+              commit(bar_op_empty + 8 * so);
+              if (L::kXOwn) commit(bar_x_empty + 8 * sx);
             }
-          umma_commit(bar_op_empty + 8 * so);
-          if (L::kXOwn) umma_commit(bar_x_empty + 8 * sx);
+            if (last) commit(bar_acc_full + 8 * slot);
+          }
+          __syncwarp();
         }
-        __syncwarp();
         if (++so == kOpN) { so = 0; pho ^= 1; }
         if (++sx == kXN) { sx = 0; phx ^= 1; }
       }
-      if (live && elect_one()) umma_commit(bar_acc_full + 8 * buf);
-      __syncwarp();
     }
   } else if (MODE == kUmma && warp >= kWideWarpEpilogue) {
     // ------------------------------------------------------------------ TMEM -> y, or -> FP32 partial tile
     const uint32_t e = warp - kWideWarpEpilogue;  // == warp % 4: the TMEM lane quarter this warp may read
     const uint32_t r = e * 32 + lane;
-    const uint32_t mcols = (args.m + 7) & ~7u;
+    const uint32_t acc_empty_at = PAIR ? cluster_map(bar_acc_empty, my_rank & ~1u) : bar_acc_empty;   // the issuer's
     uint32_t n_item = 0;
     bool live = true, early_taken = false;
     const uint64_t stay = l2_policy_evict_last();  // partial tiles are read back within the launch
@@ -559,11 +641,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     if (item_begin < item_end) item = args.items[item_begin];
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       if (it != item_begin) item = args.items[it];
-      const uint32_t buf = n_item % kAccBufs, use = n_item / kAccBufs;
-      if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * buf, use & 1)) { live = false; break; }
-      tc_fence_after();
       const uint32_t row = item.row_block * BXR_ROWS + r;
-      const uint32_t taddr = tmem_base + ((e * 32) << 16) + buf * NB;
       const float b = (args.bias && row < args.rows) ? __bfloat162float(args.bias[row]) : 0.f;
       constexpr int kStep = 16, kCols = L::kTurnCols;  // accumulator columns per tensor-memory load, and per turn-around
       // (a load's round trip is what a step waits for: 16 columns per load where only 8 fit the turn-around took a
@@ -574,9 +652,13 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       // all: no store, no fence, no counter update on the tail of the kernel.
       const bool final_item = it + 1 == item_end;
       const bool in_cluster = args.cluster > 1;  // the CTA's one item is a part of its cluster's row block
-      const bool keep = item.parts > 1 && (final_item || in_cluster);
-      const uint32_t tile = smem;           // [batch row][128 weight rows] FP32, like a partial tile in memory
+      const bool keep = item.parts > 1 && (final_item || in_cluster);   // (T = 2: the second tile waits in tensor memory for its turn)
+      const uint32_t kept = smem;           // [batch row][128 weight rows] FP32, like a partial tile in memory
       uint32_t arrived = 0;
+      if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * acc_slot(n_item, 0), acc_use(n_item) & 1)) { live = false; break; }
+      // (the second tile's last multiply may still be reading the activations in whose place a kept tile goes)
+      if (T == 2 && keep && !ctx.wait(bar_acc_full + 8, acc_use(n_item) & 1)) { live = false; break; }
+      tc_fence_after();
       if (keep && !in_cluster && e == 0 && lane == 0) arrived = ld_relaxed_gpu(args.counters + item.row_block);  // answer used after the drain; fenced there
       // A lane holds one weight row and kStep batch columns; y and the partial tiles keep the rows of one batch
       // column together.  Stored from the registers that is one narrow store instruction per column, and the
@@ -585,74 +667,97 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t turn = smem + L::turn + e * L::kTurn;
       const bool y_wide = (reinterpret_cast<uintptr_t>(args.y) & 15u) == 0 && (args.ldy & 7u) == 0 &&
                           item.row_block * BXR_ROWS + e * 32 + 32 <= args.rows;
-      for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
-        uint32_t v[kStep];
-        tmem_ld16(taddr + m0, v);
-        tmem_ld_wait();
-        if (keep) {
+      if (keep) {
+        drain_to_smem(n_item, 0, e, r);
+      } else {
+#pragma unroll 1
+        for (uint32_t t = 0; t < uint32_t(T); ++t) {
+          if (t && !ctx.wait(bar_acc_full + 8 * acc_slot(n_item, t), acc_use(n_item) & 1)) { live = false; break; }
+          if (t) tc_fence_after();
+          const uint32_t taddr = tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB, m_at = t * NB, mcols = wide_tile_cols(args.m, t, NB);
+          for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
+            uint32_t v[kStep];
+            tmem_ld16(taddr + m0, v);
+            tmem_ld_wait();
+            if (item.parts == 1) {
+              if (y_wide) {
 #pragma unroll
-          for (int i = 0; i < kStep; ++i)
-            if (m0 + i < mcols) sts32(tile + ((m0 + i) * BXR_ROWS + r) * 4, v[i]);
-        } else if (item.parts == 1) {
-          if (y_wide) {
+                for (int h = 0; h < kStep; h += kCols) {
 #pragma unroll
-            for (int h = 0; h < kStep; h += kCols) {
+                  for (int i = 0; i < kCols; ++i) {
+                    const float f = __uint_as_float(v[h + i]);
+                    const __nv_bfloat16 o = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
+                    sts_u16(turn + (i * 32 + lane) * 2, uint32_t(*reinterpret_cast<const uint16_t*>(&o)));
+                  }
+                  __syncwarp();
 #pragma unroll
-              for (int i = 0; i < kCols; ++i) {
-                const float f = __uint_as_float(v[h + i]);
-                const __nv_bfloat16 o = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
-                sts_u16(turn + (i * 32 + lane) * 2, uint32_t(*reinterpret_cast<const uint16_t*>(&o)));
+                  for (int j = 0; j < kCols / 8; ++j) {  // a store: 8 columns x 64 bytes (32 rows)
+                    const uint32_t ml = j * 8 + (lane >> 2), m = m_at + m0 + h + ml;
+                    const uint4 piece = lds128(turn + ml * 64 + (lane & 3) * 16);
+                    if (m < args.m)
+                      *reinterpret_cast<uint4*>(args.y + size_t(m) * args.ldy + item.row_block * BXR_ROWS + e * 32 + (lane & 3) * 8) = piece;
+                  }
+                  __syncwarp();
+                }
+              } else if (row < args.rows) {
+#pragma unroll
+                for (int i = 0; i < kStep; ++i)
+                  if (m_at + m0 + i < args.m) {
+                    const float f = __uint_as_float(v[i]);
+                    args.y[size_t(m_at + m0 + i) * args.ldy + row] = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
+                  }
               }
-              __syncwarp();
+            } else {
 #pragma unroll
-              for (int j = 0; j < kCols / 8; ++j) {  // a store: 8 columns x 64 bytes (32 rows)
-                const uint32_t ml = j * 8 + (lane >> 2), m = m0 + h + ml;
-                const uint4 piece = lds128(turn + ml * 64 + (lane & 3) * 16);
-                if (m < args.m)
-                  *reinterpret_cast<uint4*>(args.y + size_t(m) * args.ldy + item.row_block * BXR_ROWS + e * 32 + (lane & 3) * 8) = piece;
+              for (int h = 0; h < kStep; h += kCols) {
+#pragma unroll
+                for (int i = 0; i < kCols; ++i) sts32(turn + (i * 32 + lane) * 4, v[h + i]);
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < kCols / 4; ++j) {  // a store: 4 columns x 128 bytes (32 rows)
+                  const uint32_t ml = j * 4 + (lane >> 3), m = m0 + h + ml;
+                  const uint4 piece = lds128(turn + ml * 128 + (lane & 7) * 16);
+                  if (m < mcols) stg128(args.partials + ((size_t(item.slot) * T + t) * NB + m) * BXR_ROWS + e * 32 + (lane & 7) * 4, piece, stay);
+                }
+                __syncwarp();
               }
-              __syncwarp();
             }
-          } else if (row < args.rows) {
-#pragma unroll
-            for (int i = 0; i < kStep; ++i)
-              if (m0 + i < args.m) {
-                const float f = __uint_as_float(v[i]);
-                args.y[size_t(m0 + i) * args.ldy + row] = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
-              }
           }
-        } else {
-#pragma unroll
-          for (int h = 0; h < kStep; h += kCols) {
-#pragma unroll
-            for (int i = 0; i < kCols; ++i) sts32(turn + (i * 32 + lane) * 4, v[h + i]);
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < kCols / 4; ++j) {  // a store: 4 columns x 128 bytes (32 rows)
-              const uint32_t ml = j * 4 + (lane >> 3), m = m0 + h + ml;
-              const uint4 piece = lds128(turn + ml * 128 + (lane & 7) * 16);
-              if (m < mcols) stg128(args.partials + (size_t(item.slot) * NB + m) * BXR_ROWS + e * 32 + (lane & 7) * 4, piece, stay);
-            }
-            __syncwarp();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (leader) mbar_arrive(bar_acc_empty + 8 * acc_slot(n_item, t));
+            else mbar_arrive_cluster(acc_empty_at + 8 * acc_slot(n_item, t));
           }
         }
+        if (!live) break;
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
       if (item.parts > 1 && !in_cluster) {
         // `prev` = how many tiles of the row block were in memory before this one; the CTA that completes the set
         // reduces it.  Flag words: misc + 8 and misc + 12.
         uint32_t prev;
+        bool published = false;   // of a kept item: its tiles have left for memory
         if (keep) {
           fence_proxy_async_smem();  // the tile may leave through a bulk copy
           if (e == 0 && lane == 0) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(arrived) : "memory");
           named_barrier(1, 128);
           asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 8));
           if (prev != item.parts - 1) {  // someone else is still missing: publish the tile like any other
+            published = true;
+#pragma unroll
+            for (uint32_t t = 0; t < uint32_t(T); ++t) {
+              if (t) {   // the second tile takes the place of the first, which has left
+                named_barrier(1, 128);
+                drain_to_smem(n_item, t, e, r);
+                fence_proxy_async_smem();
+                named_barrier(1, 128);
+              }
+              if (e == 0 && lane == 0) {
+                bulk_s2g(args.partials + (size_t(item.slot) * T + t) * NB * BXR_ROWS, kept, wide_tile_cols(args.m, t, NB) * BXR_ROWS * 4);
+                bulk_commit_and_wait();
+              }
+            }
             if (e == 0 && lane == 0) {
-              bulk_s2g(args.partials + size_t(item.slot) * NB * BXR_ROWS, tile, mcols * BXR_ROWS * 4);
-              bulk_commit_and_wait();
               fence_proxy_async_all();
               __threadfence();
               const uint32_t before = atomicAdd(args.counters + item.row_block, 1u);
@@ -679,10 +784,11 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           if (final_item || !early_taken) {
             if (e == 0 && lane == 0)  // {1 | (index + 1 of the tile kept in shared memory) << 8, row block, first slot, parts}
               asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(smem + L::misc + (final_item ? 16 : 32)),
-                           "r"(1u | (keep ? (item.part + 1u) << 8 : 0u)), "r"(item.row_block), "r"(first), "r"(item.parts) : "memory");
+                           // (of two published tiles only the second is still here: both come back from memory)
+                           "r"(1u | (keep && !(T == 2 && published) ? (item.part + 1u) << 8 : 0u)), "r"(item.row_block), "r"(first), "r"(item.parts) : "memory");
             early_taken = early_taken || !final_item;
           } else {
-            reduce_row_block<NB>(args, item.row_block, first, item.parts, e, 4, lane);
+            reduce_row_block<T * NB>(args, item.row_block, first, item.parts, e, 4, lane);
           }
           if (e == 0 && lane == 0) args.counters[item.row_block] = 0;
         }
@@ -693,40 +799,61 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     if (lane == 0) mbar_arrive(bar_final);
   }
 
+  const uint32_t closing_thread = (warp < kDecoderWarps ? warp : warp - 4) * 32 + lane;
   if (MODE == kUmma && args.cluster > 1) {
-    // One cluster per row block: every CTA's tile is in its shared memory once its epilogue is through; the cluster
+    // A row block's CTAs in one cluster: every CTA's tile is in its shared memory once its epilogue is through; the cluster
     // barrier makes the tiles visible to the peers, the second one keeps every CTA's shared memory alive until the
     // peers have read it.  Every thread of every CTA gets here on every path (all other waits are bounded).
     const bool worker_thread = warp < kDecoderWarps || warp >= kWideWarpEpilogue;
     const bool drained = worker_thread ? ctx.wait(bar_final, 0) : true;
-    __syncwarp();
-    cluster_sync();
-    if (worker_thread && drained && unit_count)
-      bxq_reduce_in_cluster<NB>(args, unit_begin / args.chunks, smem, (warp < kDecoderWarps ? warp : warp - 4) * 32 + lane);
-    __syncwarp();
-    cluster_sync();
+#pragma unroll
+    for (uint32_t t = 0; t < uint32_t(T); ++t) {
+      if (t && warp >= kWideWarpEpilogue && unit_count && __all_sync(0xFFFFFFFFu, drained)) {
+        drain_to_smem(0, t, warp - kWideWarpEpilogue, (warp - kWideWarpEpilogue) * 32 + lane);
+        tc_fence_before();
+      }
+      __syncwarp();
+      cluster_sync();
+      if (worker_thread && drained && unit_count)
+        bxq_reduce_in_cluster<NB, PAIR>(args, (unit_begin / args.chunks) * group + in_group, smem, closing_thread, t);
+      __syncwarp();
+      cluster_sync();
+    }
   }
 
   // Row blocks whose last partial tile came from this CTA are reduced by the 16 decoder warps and the 4 epilogue
   // warps together, once the epilogue has drained the CTA's last item.
   if (MODE == kUmma && args.cluster <= 1 && (warp < kDecoderWarps || warp >= kWideWarpEpilogue)) {
-    if (ctx.wait(bar_final, 0)) {
-      uint32_t fetched = 0;  // tiles brought in so far: position in the two-buffer ring
+    constexpr uint32_t kClosing = (kDecoderWarps + 4) * 32;
+    bool drained = ctx.wait(bar_final, 0);
+    if (T == 2) drained = named_barrier_and(2, kClosing, drained);   // (barriers below: all or none)
+    if (drained) {
+      uint32_t fetched = 0;  // tiles brought in so far: position in the ring
 #pragma unroll 1
       for (uint32_t at = 32; at >= 16; at -= 16) {
         const uint4 decision = lds128(smem + L::misc + at);  // {reduce? | own tile << 8, row block, first slot, parts}
-        if (decision.x)
-          bxq_reduce_row_block<NB>(args, ctx, decision.y, decision.z, decision.w, (decision.x >> 8) - 1u, smem, bar_tile_full, bar_tile_used,
-                                   (warp < kDecoderWarps ? warp : warp - 4) * 32 + lane, fetched);
+        if (!decision.x) continue;
+        const uint32_t own = (decision.x >> 8) - 1u;
+#pragma unroll 1
+        for (uint32_t t = 0; t < uint32_t(T); ++t) {
+          if (T == 2 && t && own < decision.w) {   // the second tile takes the place of the first once that has been added
+            named_barrier(2, kClosing);
+            if (warp >= kWideWarpEpilogue) drain_to_smem(0, t, warp - kWideWarpEpilogue, (warp - kWideWarpEpilogue) * 32 + lane);
+            named_barrier(2, kClosing);
+          }
+          bxq_reduce_row_block<NB, T>(args, ctx, decision.y, decision.z, decision.w, own, smem, bar_tile_full, bar_tile_used, closing_thread, t, fetched);
+        }
       }
     }
   }
 
   tc_fence_before();
-  __syncthreads();
+  __syncwarp();
+  if (PAIR) cluster_sync();   // what the peer has in flight ends at this CTA's barriers, shared memory and tensor memory
+  else __syncthreads();
   if (MODE == kUmma && warp == kWideWarpMma) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc<PAIR>(tmem_base, kTmemCols);
   }
 }
 

@@ -32,23 +32,25 @@ struct Plan {
   uint32_t partial_slots = 0;
 };
 
-// Equal shares of the (row block, chunk) sequence; a share is cut at row-block boundaries into items.
-Plan make_plan(uint32_t rows, uint32_t cols, uint32_t workers) {
+// Equal shares of the (row block, chunk) sequence; a share is cut at row-block boundaries into items.  `paired`: two workers
+// take the same share of the (pair of row blocks, chunk) sequence, one row block of each pair each.
+Plan make_plan(uint32_t rows, uint32_t cols, uint32_t workers, bool paired = false) {
   Plan p;
   p.rows = rows;
   p.cols = cols;
   p.row_blocks = (rows + BXR_ROWS - 1) / BXR_ROWS;
   p.chunks = (cols + BXR_COLS - 1) / BXR_COLS;
   p.workers = workers;
-  const uint64_t units = uint64_t(p.row_blocks) * p.chunks;
+  const uint32_t group = paired ? 2 : 1, shares = workers / group;
+  const uint64_t units = uint64_t(p.row_blocks / group) * p.chunks;
   p.worker_items.assign(workers + 1, 0);
   std::vector<uint32_t> parts(p.row_blocks, 0);
   for (uint32_t w = 0; w < workers; ++w) {
-    uint64_t u = units * w / workers;
-    const uint64_t end = units * (w + 1) / workers;
+    uint64_t u = units * (w / group) / shares;
+    const uint64_t end = units * (w / group + 1) / shares;
     p.worker_items[w] = uint32_t(p.items.size());
     while (u < end) {
-      const uint32_t rb = uint32_t(u / p.chunks), c0 = uint32_t(u % p.chunks);
+      const uint32_t rb = uint32_t(u / p.chunks) * group + w % group, c0 = uint32_t(u % p.chunks);
       const uint32_t c1 = uint32_t(std::min<uint64_t>(p.chunks, c0 + (end - u)));
       bxr_item it{};
       it.row_block = rb;
@@ -491,7 +493,9 @@ bool image_is_well_formed(const uint8_t* img, uint64_t bytes) {
   for (int i = 0; i < 6; ++i)
     if (begin[i] > begin[i + 1] || size[i] > begin[i + 1] - begin[i]) return false;
   // the work partition
-  const Plan plan = make_plan(h.rows, h.cols, h.workers);
+  const bool paired = h.paired == 1;
+  if (paired && (h.mode != BXR_MODE_WINDOW4 || !h.blob_stride16 || (h.row_blocks & 1) || (h.workers & 1))) return false;
+  const Plan plan = make_plan(h.rows, h.cols, h.workers, paired);
   if (plan.items.size() != h.items || plan.partial_slots != h.partial_slots) return false;
   if (std::memcmp(img + h.items_at, plan.items.data(), sizeof(bxr_item) * plan.items.size()) != 0) return false;
   if (std::memcmp(img + h.worker_items_at, plan.worker_items.data(), 4ull * (h.workers + 1ull)) != 0) return false;
@@ -554,7 +558,7 @@ int bxr_build(const uint16_t* words, uint32_t rows, uint32_t cols, uint32_t work
     Plan plan = make_plan(rows, cols, workers);
     const uint32_t rows_pad = plan.row_blocks * BXR_ROWS, cols_pad = plan.chunks * BXR_COLS;
     const uint32_t nblobs = plan.row_blocks * plan.chunks;
-    const uint32_t nitems = uint32_t(plan.items.size());
+    uint32_t nitems = uint32_t(plan.items.size());
 
     std::vector<uint8_t> base(rows_pad, 0);
     std::vector<uint32_t> lut(BXR_PROB_TOTAL, 0);
@@ -686,27 +690,6 @@ int bxr_build(const uint16_t* words, uint32_t rows, uint32_t cols, uint32_t work
       });
     }
 
-    bxr_header h{};
-    h.magic = BXR_MAGIC;
-    h.mode = raw_mode ? BXR_MODE_RAW : window4_mode ? BXR_MODE_WINDOW4 : window_mode ? BXR_MODE_WINDOW : BXR_MODE_CODED;
-    const bool coded = !raw_mode && !window_mode && !window4_mode;
-    h.rows = rows;
-    h.cols = cols;
-    h.row_blocks = plan.row_blocks;
-    h.chunks = plan.chunks;
-    h.workers = workers;
-    h.items = nitems;
-    h.partial_slots = plan.partial_slots;
-    uint64_t at = align16(sizeof(bxr_header));
-    at = (at + 255) & ~uint64_t(255);
-    h.lut_at = at;            at += coded ? sizeof(uint32_t) * BXR_PROB_TOTAL : 0;
-    h.base_at = at;           at = align16(at + rows_pad);
-    h.items_at = at;          at = align16(at + sizeof(bxr_item) * nitems);
-    h.worker_items_at = at;   at = align16(at + 4ull * (workers + 1));
-    h.states_at = at;         at = align16(at + (coded ? 4ull * states.size() : 0));
-    h.blob_index_at = at;     at = align16(at + 4ull * (nblobs + 1));
-    at = (at + 255) & ~uint64_t(255);
-    h.blobs_at = at;
     // Wide-window blobs differ only by their (rare) exception entries: pad them to one size, so that a kernel can
     // address blob b without looking its offset up (the index is written all the same).
     uint32_t blob_stride16 = 0;
@@ -718,6 +701,33 @@ int bxr_build(const uint16_t* words, uint32_t rows, uint32_t cols, uint32_t work
         blob_stride16 = uint32_t(hi >> 4);
       }
     }
+    const bool paired = blob_stride16 && bxr_paired(plan.row_blocks, plan.chunks, workers);
+    if (paired) {
+      plan = make_plan(rows, cols, workers, true);
+      nitems = uint32_t(plan.items.size());
+    }
+    bxr_header h{};
+    h.magic = BXR_MAGIC;
+    h.mode = raw_mode ? BXR_MODE_RAW : window4_mode ? BXR_MODE_WINDOW4 : window_mode ? BXR_MODE_WINDOW : BXR_MODE_CODED;
+    const bool coded = !raw_mode && !window_mode && !window4_mode;
+    h.rows = rows;
+    h.cols = cols;
+    h.row_blocks = plan.row_blocks;
+    h.chunks = plan.chunks;
+    h.workers = workers;
+    h.items = nitems;
+    h.partial_slots = plan.partial_slots;
+    h.paired = paired ? 1 : 0;
+    uint64_t at = align16(sizeof(bxr_header));
+    at = (at + 255) & ~uint64_t(255);
+    h.lut_at = at;            at += coded ? sizeof(uint32_t) * BXR_PROB_TOTAL : 0;
+    h.base_at = at;           at = align16(at + rows_pad);
+    h.items_at = at;          at = align16(at + sizeof(bxr_item) * nitems);
+    h.worker_items_at = at;   at = align16(at + 4ull * (workers + 1));
+    h.states_at = at;         at = align16(at + (coded ? 4ull * states.size() : 0));
+    h.blob_index_at = at;     at = align16(at + 4ull * (nblobs + 1));
+    at = (at + 255) & ~uint64_t(255);
+    h.blobs_at = at;
     h.blob_stride16 = blob_stride16;
     h.layout_version = BXR_LAYOUT_VERSION;
     std::vector<uint32_t> index(nblobs + 1);

@@ -135,6 +135,17 @@
 #define BXQ_PAIR_MASK 0x000F000Fu
 #define BXQ_BASE_MAX 240
 
+/* Work partition of pairs.  Workers 2p and 2p + 1 walk the same chunks of two neighbouring row blocks side by side: share p of
+ * workers / 2 equal shares of the (pair of row blocks, chunk) sequence, worker 2p + r taking row block 2g + r of pair g.  CTAs
+ * that do so can multiply as one tcgen05 pair (bxq_kernels.cuh).  Row blocks that whole workers share among themselves (workers
+ * = row blocks x P, 2 <= P <= 8) can be walked like that as they are and keep the plain partition, and so do images of
+ * fewer than eight chunks a worker, where a launch is all ramp and tail. */
+static inline int bxr_paired(uint32_t row_blocks, uint32_t chunks, uint32_t workers) {
+  if ((row_blocks & 1u) || (workers & 1u) || !row_blocks || !workers) return 0;
+  if (workers % row_blocks == 0 && workers / row_blocks >= 2 && workers / row_blocks <= 8) return 0;
+  return (uint64_t)row_blocks * chunks >= 8ull * workers;
+}
+
 /* Slot record of the pair table, 32 bits: n0[0,4) | bias[4,16) | n1[16,20) | freq[20,32).  freq <= 4095.
  * (record & 0x000F000F) * 128 is the pair of relative exponents in packed-BF16 position (an exception nibble is
  * stored as 0), freq is the top field, bias = (record >> 4) & 0xFFF. */
@@ -162,7 +173,7 @@ typedef struct bxr_header {
   uint32_t partial_slots;         /* FP32 partial tiles the workspace must hold */
   uint32_t blob_stride16;         /* nonzero: every blob has this size (16-byte units) and blob b starts at b * size */
   uint32_t layout_version;        /* BXR_LAYOUT_VERSION of the builder */
-  uint32_t reserved0;
+  uint32_t paired;                /* 1: the work partition is that of pairs of workers (wide-window images; see bxr_paired) */
   uint64_t lut_at;                /* u32[4096] slot records (absent in raw mode) */
   uint64_t base_at;               /* u8[row_blocks*128] exponent base per row */
   uint64_t items_at;              /* bxr_item[items] */

@@ -73,12 +73,13 @@ struct BxrArgs {
   uint32_t* counters;          // [row_blocks], zero between calls
   uint16_t* dense;             // kDense: rows x cols words
   uint32_t* status;
-  uint32_t cluster;            // bxq_kernel: > 1 = launched as clusters of this many CTAs, one cluster per row block
+  uint32_t cluster;            // bxq_kernel: > 1 = a row block is cut into this many parts, whose CTAs belong to one thread-block cluster
+  uint32_t paired;             // bxq_kernel: the image's shares are those of pairs of workers (bxr_format.h)
   // bxq_kernel, optional: the image the NEXT launch in the stream will read (blobs of one size).  A CTA whose own
   // loads have all been issued asks the L2 for the first blobs of the next launch's CTAs, so that HBM keeps working
   // through this launch's tail and the next launch's prologue.
   const uint8_t* next_blobs;
-  uint32_t next_blob_bytes, next_units, next_workers;
+  uint32_t next_blob_bytes, next_row_blocks, next_chunks, next_workers, next_paired;
 };
 
 template <int MODE, int NB>

@@ -25,20 +25,22 @@ int cuda_status(cudaError_t e) { return e == cudaSuccess ? GRB_OK : GRB_ERR_CUDA
 
 uint32_t batch_tile(uint32_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
 
-// Batches above 128 rows over 4-bit window images: a pass over the weights may take 192 rows, and costs little more than
-// one of 128 (34816 x 5120: 74 against 62 us).  Rows of the next pass when `left` are still to be multiplied: 192 (129 rows:
-// 70 us in one pass, 110 us in two), except that 193 to 256 rows take two passes either way and 128-column ones cost less.
-constexpr uint32_t kWideTile = 192;
-uint32_t wide_pass_rows(uint32_t left) {
-  if (left <= 128) return left;
-  return left <= kWideTile ? left : left <= 256 ? 128 : kWideTile;
+// Batches above 128 rows over 4-bit window images: a pass over the weights may take up to 192 rows, up to 384 by pairs of CTAs,
+// and costs little more than one of 128 (34816 x 5120: 58 us at 128 rows, 67 at 192, 80 at 256, 109 at 384).  Rows of the next pass when `left` are still to be multiplied and a pass may take `most`
+// (128, 192, 256 or 384).
+constexpr uint32_t kWideTile = 192, kPairTile = 384;
+uint32_t wide_pass_rows(uint32_t left, uint32_t most) {
+  if (left <= most) return left;
+  // 193 to 256 rows take two passes of single CTAs either way and 128-column ones cost less
+  return most == kWideTile && left <= 256 ? 128 : most;
 }
 
 uint64_t counter_bytes(const bxr_header* h) { return (uint64_t(h->row_blocks) * 4 + 255) & ~uint64_t(255); }
 
 bool header_ok(const bxr_header* h) {
   return h && h->magic == BXR_MAGIC && h->layout_version == BXR_LAYOUT_VERSION && h->rows && h->cols && h->workers && h->mode <= BXR_MODE_WINDOW4 &&
-         h->row_blocks == (h->rows + BXR_ROWS - 1) / BXR_ROWS && h->chunks == (h->cols + BXR_COLS - 1) / BXR_COLS;
+         h->row_blocks == (h->rows + BXR_ROWS - 1) / BXR_ROWS && h->chunks == (h->cols + BXR_COLS - 1) / BXR_COLS &&
+         (h->paired != 1 || (h->mode == BXR_MODE_WINDOW4 && h->blob_stride16 && !(h->row_blocks & 1) && !(h->workers & 1)));
 }
 
 BxrArgs view_of(const void* image, const bxr_header* h) {
@@ -62,6 +64,7 @@ BxrArgs view_of(const void* image, const bxr_header* h) {
   a.raw = h->mode == BXR_MODE_RAW;
   a.window = h->mode == BXR_MODE_WINDOW;
   a.window4 = h->mode == BXR_MODE_WINDOW4;
+  a.paired = h->paired == 1;
   return a;
 }
 
@@ -107,21 +110,18 @@ int launch_fused(const BxrArgs& a, const CUtensorMap& tmap, cudaStream_t stream,
 // Aligned partitions - workers = row blocks x P with 2 <= P <= 8 - run the 4-bit window kernel as one thread-block
 // cluster of P CTAs per row block: the K parts of a row block are then added over distributed shared memory.
 uint32_t cluster_of(const BxrArgs& a) {
-  if (!a.window4 || a.workers % a.row_blocks) return 1;
+  if (!a.window4 || a.paired || a.workers % a.row_blocks) return 1;
   const uint32_t p = a.workers / a.row_blocks;
   return (p >= 2 && p <= 8 && a.chunks >= p) ? p : 1;
 }
 
-// Does a batch above 128 rows need more scratch than one of 128?  (Clusters keep their partial tiles in shared memory.)
-bool wide_tile_image(const bxr_header* h) {
-  if (h->mode != BXR_MODE_WINDOW4) return false;
-  BxrArgs a{};
-  a.row_blocks = h->row_blocks;
-  a.chunks = h->chunks;
-  a.workers = h->workers;
-  a.window4 = true;
-  return cluster_of(a) == 1;
+// Can neighbouring row blocks be multiplied by a pair of CTAs?  Images with the partition of pairs, and clusters whose row
+// blocks come in twos (a cluster of pairs has 2P CTAs, of which eight are portable).
+bool pairs(const BxrArgs& a) {
+  if (!a.window4 || !a.blob_stride16 || (a.row_blocks & 1)) return false;
+  return a.paired || (cluster_of(a) > 1 && cluster_of(a) <= 4);
 }
+uint32_t widest_pass(const BxrArgs& a) { return !a.window4 ? 128 : pairs(a) ? kPairTile : kWideTile; }
 
 template <int MODE>
 constexpr int kFusedThreads = MODE == kUmma ? kThreadsUmma : kThreadsSimt;
@@ -134,10 +134,10 @@ template <int MODE, int NB>
 int launch_window(const BxrArgs& a, const CUtensorMap& tmap, cudaStream_t stream) {  // 3-bit window images
   return launch_fused<bxw_kernel<MODE, NB>, BxwSmem<MODE, NB>::alloc, kFusedThreads<MODE>>(a, tmap, stream);
 }
-template <int MODE, int NB>
+template <int MODE, int NB, int T = 1, bool PAIR = false>
 int launch_wide(BxrArgs a, const CUtensorMap& tmap, cudaStream_t stream) {  // 4-bit window images
   a.cluster = MODE == kUmma ? cluster_of(a) : 1;
-  return launch_fused<bxq_kernel<MODE, NB>, BxqSmem<MODE, NB>::alloc, kFusedThreads<MODE>>(a, tmap, stream, a.cluster);
+  return launch_fused<bxq_kernel<MODE, NB, T, PAIR>, BxqSmem<MODE, NB, T, PAIR>::alloc, kFusedThreads<MODE>>(a, tmap, stream, a.cluster * (PAIR ? 2 : 1));
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -197,10 +197,32 @@ int gemm_tile(BxrArgs a, const void* x, int64_t ldx, cudaStream_t stream) {
   return a.window ? launch_window<kUmma, NB>(a, map, stream) : launch<kUmma, NB>(a, map, stream);
 }
 
-int gemm_tile_wide(const BxrArgs& a, const void* x, int64_t ldx, cudaStream_t stream) {
+template <int NB, int T>
+int gemm_tile_pair(const BxrArgs& a, const void* x, int64_t ldx, cudaStream_t stream) {
   CUtensorMap map;
-  const int st = make_x_map(&map, x, ldx, a.m, a.cols, kWideTile);
-  return st ? st : launch_wide<kUmma, int(kWideTile)>(a, map, stream);
+  const int st = make_x_map(&map, x, ldx, a.m, a.cols, NB / 2);   // a CTA brings in half of a tile's rows
+  return st ? st : launch_wide<kUmma, NB, T, true>(a, map, stream);
+}
+
+// One pass over the weights: a.m rows of x.
+int gemm_pass(const BxrArgs& a, const void* x, int64_t ldx, cudaStream_t stream) {
+  if (a.m > 128 && pairs(a)) {
+    if (a.m <= 128) return gemm_tile_pair<128, 1>(a, x, ldx, stream);
+    if (a.m <= 192) return gemm_tile_pair<192, 1>(a, x, ldx, stream);
+    if (a.m <= 256) return gemm_tile_pair<128, 2>(a, x, ldx, stream);
+    return gemm_tile_pair<192, 2>(a, x, ldx, stream);
+  }
+  if (a.m > 128) {
+    CUtensorMap map;
+    const int st = make_x_map(&map, x, ldx, a.m, a.cols, kWideTile);
+    return st ? st : launch_wide<kUmma, int(kWideTile)>(a, map, stream);
+  }
+  switch (batch_tile(a.m)) {
+    case 16: return gemm_tile<16>(a, x, ldx, stream);
+    case 32: return gemm_tile<32>(a, x, ldx, stream);
+    case 64: return gemm_tile<64>(a, x, ldx, stream);
+    default: return gemm_tile<128>(a, x, ldx, stream);
+  }
 }
 
 template <int M>
@@ -320,7 +342,9 @@ extern "C" {
 
 uint64_t grb_bxr_workspace_bytes(const bxr_header* h, uint32_t max_m) {
   if (!header_ok(h) || !max_m) return 0;
-  const uint64_t tile = max_m > 128 && wide_tile_image(h) ? kWideTile : batch_tile(max_m > 128 ? 128 : max_m);
+  const BxrArgs a = view_of(nullptr, h);
+  // (clusters keep their partial tiles in shared memory)
+  const uint64_t tile = max_m > 128 && cluster_of(a) == 1 ? widest_pass(a) : batch_tile(max_m > 128 ? 128 : max_m);
   return counter_bytes(h) + uint64_t(h->partial_slots) * tile * BXR_ROWS * 4;
 }
 
@@ -487,27 +511,35 @@ int grb_bxr_gemm_partials(const void* image, const bxr_header* h, const void* x,
   if (next_image && header_ok(next_header) && a.window4 && next_header->mode == BXR_MODE_WINDOW4 && next_header->blob_stride16) {
     a.next_blobs = static_cast<const uint8_t*>(next_image) + next_header->blobs_at;
     a.next_blob_bytes = next_header->blob_stride16 << 4;
-    a.next_units = next_header->row_blocks * next_header->chunks;
+    a.next_row_blocks = next_header->row_blocks;
+    a.next_chunks = next_header->chunks;
     a.next_workers = next_header->workers;
+    a.next_paired = next_header->paired == 1;
   }
-  // Batches above one tile are processed as consecutive tiles, one pass over the weights each.  The wide tile needs wider
-  // slots for its partial tiles: lent ones, or scratch that was sized for them; a caller who has neither gets tiles of 128.
-  const uint64_t wide_slots = uint64_t(h->partial_slots) * kWideTile * BXR_ROWS * 4;
+  // Batches above one tile are processed as consecutive tiles, one pass over the weights each.  The wide tiles need wider
+  // slots for their partial tiles: lent ones, or scratch that was sized for them; a caller who has neither gets tiles of 128.
   if (partials && (reinterpret_cast<uintptr_t>(partials) & 15)) return GRB_ERR_WORKSPACE;
-  const bool lent = m > 128 && partials && partials_bytes >= wide_slots;
-  if (lent) a.partials = static_cast<float*>(partials);
-  const bool wide = m > 128 && a.window4 && (cluster_of(a) > 1 || lent || ws_bytes >= counter_bytes(h) + wide_slots);
-  for (uint32_t m0 = 0; m0 < m; m0 += a.m) {
-    a.m = wide ? wide_pass_rows(m - m0) : std::min(m - m0, 128u);
-    const auto* xt = static_cast<const __nv_bfloat16*>(x) + size_t(m0) * ldx;
-    a.y = static_cast<__nv_bfloat16*>(y) + size_t(m0) * ldy;
-    if (a.m > 128) st = gemm_tile_wide(a, xt, ldx, stream);
-    else switch (batch_tile(a.m)) {
-      case 16: st = gemm_tile<16>(a, xt, ldx, stream); break;
-      case 32: st = gemm_tile<32>(a, xt, ldx, stream); break;
-      case 64: st = gemm_tile<64>(a, xt, ldx, stream); break;
-      default: st = gemm_tile<128>(a, xt, ldx, stream); break;
+  uint32_t most = 128;
+  if (m > 128 && a.window4) {
+    const uint32_t widest = widest_pass(a);
+    const uint64_t row = uint64_t(h->partial_slots) * BXR_ROWS * 4;     // one batch row of every slot
+    auto fits = [&](uint64_t bytes) {
+      for (uint32_t rows : {384u, 256u, 192u})
+        if (rows <= widest && (rows != 256 || widest == kPairTile) && bytes >= rows * row) return rows;
+      return 128u;
+    };
+    if (cluster_of(a) > 1) {
+      most = widest;
+    } else {
+      most = partials ? fits(partials_bytes) : 128u;
+      if (most > 128) a.partials = static_cast<float*>(partials);
+      else most = fits(ws_bytes - counter_bytes(h));
     }
+  }
+  for (uint32_t m0 = 0; m0 < m; m0 += a.m) {
+    a.m = wide_pass_rows(m - m0, most);
+    a.y = static_cast<__nv_bfloat16*>(y) + size_t(m0) * ldy;
+    st = gemm_pass(a, static_cast<const __nv_bfloat16*>(x) + size_t(m0) * ldx, ldx, stream);
     if (st) return st;
   }
   return GRB_OK;

@@ -39,6 +39,10 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// An arrival on a barrier of another CTA of the cluster (`bar` from cluster_map).
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 constexpr uint32_t kSuspendHintNs = 20000;
 // One probe of the barrier.  `suspend`: let the hardware park the thread for up to kSuspendHintNs while the phase is incomplete.  That keeps
 // waiting warps out of the issue slots (it pays when the decoders are short of them: the rANS kernels) at the price
@@ -119,6 +123,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int 
       "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// The same by one CTA of a tcgen05 pair: the data lands in this CTA's shared memory, `bar` (from cluster_map) may be the
+// barrier of either CTA of the pair.  No multicast: every byte goes to one CTA.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, int x, int y, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(dst),
+      "l"(tmap), "r"(bar), "r"(x), "r"(y), "l"(policy)
+      : "memory");
+}
 // Hint: bring [src, src + bytes) into the L2 (16-byte aligned, a multiple of 16 bytes); nothing waits for it.
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
@@ -185,14 +197,21 @@ __device__ __forceinline__ void sts128(uint32_t a, uint4 v) {
 }
 
 // ---- tcgen05 ----------------------------------------------------------------------------------------
+// PAIR: by one warp in each of the two CTAs of a pair (cluster ranks 2i and 2i + 1), whose kernel uses no other group.
+template <bool PAIR = false>
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t columns) {  // whole warp
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(columns) : "memory");
+  if constexpr (PAIR) asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(columns) : "memory");
+  else asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(columns) : "memory");
 }
+template <bool PAIR = false>
 __device__ __forceinline__ void tmem_relinquish() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if constexpr (PAIR) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  else asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
+template <bool PAIR = false>
 __device__ __forceinline__ void tmem_dealloc(uint32_t addr, uint32_t columns) {  // whole warp
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(columns) : "memory");
+  if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(columns) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(columns) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -215,6 +234,17 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, u
       "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same by a pair of CTAs, issued by one thread of the one with the even cluster rank: M = 256, each CTA's tensor memory holds
+// its own 128 rows of A (at a_tmem) and of D (at d_tmem), each CTA's shared memory one half of B's N rows (same address in
+// both).
+__device__ __forceinline__ void umma_bf16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // True in one lane of a converged warp, always the same one.  Issuing from the lane this names, not from lane 0 of a
 // divergent branch, tells the compiler that the operands are uniform: 5120 x 17408 at 128 rows 36.3 -> 35.7 us, 5120 x
 // 5120 at one row 12.85 -> 12.6 us.
@@ -226,6 +256,10 @@ __device__ __forceinline__ bool elect_one() {
 // The barrier gets one arrival when every MMA issued so far by this thread has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// The same for MMAs of a pair: one arrival on the barrier at this address in every CTA of `mask` (bit = cluster rank).
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t mask) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(mask) : "memory");
 }
 // 32 lanes x 8 consecutive 32-bit columns: thread t of the warp receives lane (base lane + t).
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
@@ -270,9 +304,9 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   return uint64_t((smem_addr >> 4) & 0x3FFFu) | (uint64_t(1) << 16) | (uint64_t(1024 >> 4) << 32) | (uint64_t(1) << 46) |
          (uint64_t(2) << 61);
 }
-// BF16 x BF16 -> FP32, both operands K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(uint32_t n) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+// BF16 x BF16 -> FP32, both operands K-major, M = 128 (256 for a pair of CTAs), N = n.
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(uint32_t n, uint32_t m = 128) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
 // Programmatic dependent launch.  grid_dependents_may_launch() lets the next kernel in the stream start its
@@ -305,6 +339,19 @@ __device__ __forceinline__ uint4 lds128_cluster(uint32_t a) {
   return v;
 }
 
+// Barrier over `threads` threads that tells each whether `ok` held for all of them.
+__device__ __forceinline__ bool named_barrier_and(uint32_t id, uint32_t threads, bool ok) {
+  uint32_t all;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %3, 0;\n\t"
+      "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(all)
+      : "r"(id), "r"(threads), "r"(uint32_t(ok))
+      : "memory");
+  return all != 0;
+}
 __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }

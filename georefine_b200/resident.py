@@ -144,7 +144,7 @@ class ResidentWeight:
         self.workspace, self._outgrown = None, []
         sizes = [int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(h), m)) for m in (128, 129)]
         counters = (int(h.row_blocks) * 4 + 255) & ~255
-        # partial tiles of the 192-row passes of a batch above 128 rows, where they are larger than those of 128 rows
+        # partial tiles of the widest passes of a batch above 128 rows, where they are larger than those of 128 rows
         self.wide_scratch_bytes = sizes[1] - counters if sizes[1] > sizes[0] else 0
         self.next_weight = None     # see then()
         self.reserve(max_m)
@@ -279,7 +279,7 @@ class ResidentWeight:
     def gemm(self, x, y, bias=None, *, scratch=None):
         """tcgen05 path, any M; rows of y are bitwise independent of M.
 
-        A batch above 128 rows may take 192 rows per pass over the weights.  For their partial tiles it borrows ``scratch``
+        A batch above 128 rows may take 192 or 384 rows per pass over the weights.  For their partial tiles it borrows ``scratch``
         (uint8, ``wide_scratch_bytes`` of it, not used by anything else until the call's work is done), or asks the allocator."""
         if x.dim() != 2 or y.dim() != 2:
             raise ValueError("x and y must be 2-D BF16 tensors")

@@ -27,9 +27,9 @@ from . import ops
 from .resident import ResidentWeight
 
 PAGE = ops.PAGE
-# Rows of a prompt that go through the stack together: two 192-row passes over each weight and one set of the small
-# kernels, for 60 MB of row buffers and 28 MB of partial tiles at the benchmark's shapes, whatever the number of layers.
-# 1000 tokens over four layers: 6.65 -> 5.8 ms.
+# Rows of a prompt that go through the stack together: one pass over each weight and one set of the small
+# kernels, for 60 MB of row buffers and 57 MB of partial tiles at the benchmark's shapes, whatever the number of layers.
+# 1000 tokens over four layers: 5.5 -> 4.8 ms with one pass for them instead of two.
 PROMPT_ROWS = 384
 STAGING = 4     # passes whose rows may be on their way to the device at a time
 
@@ -265,7 +265,7 @@ class BatchDecoder:
             if hasattr(w, "reserve"):
                 w.reserve(min(self.max_rows, 128))
         # Batches above 128 rows leave partial tiles behind inside a linear: one block for all of them, taken here, before
-        # anybody sizes anything else by the memory that is left (28 MB at the benchmark's shapes).
+        # anybody sizes anything else by the memory that is left (57 MB at the benchmark's shapes).
         wide_bytes = max((w.wide_scratch_bytes for w in weights.linears() if type(w) is ResidentWeight), default=0)
         self._partials = torch.empty(wide_bytes, device=self.dev, dtype=torch.uint8) if self.prompt_rows > 128 and wide_bytes else None
         self._staging, self._staged = [(torch.zeros(3, R, dtype=i32).pin_memory(), torch.cuda.Event()) for _ in range(STAGING)], 0

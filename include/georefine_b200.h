@@ -215,7 +215,7 @@ int bxr_decode_host(const uint8_t* image, uint64_t image_bytes, uint16_t* words)
  * FP32 partial tiles of row blocks shared by several CTAs, preceded by one counter per row block.
  * The scratch must be zero-filled once after allocation; the kernels leave the counters at zero.
  * Scratch for max_m = 128 serves every larger batch, in passes of 128 rows over the weights; with scratch for max_m > 128
- * a 4-bit window image takes up to 192 rows per pass. */
+ * a 4-bit window image takes up to 192 rows per pass, or up to 384 where its row blocks are multiplied in pairs. */
 uint64_t grb_bxr_workspace_bytes(const bxr_header* header, uint32_t max_m);
 
 /* Decode twin: writes rows*cols BF16 words.  Replaces CudaContextTensor.decode() for a resident image,
@@ -250,7 +250,7 @@ int grb_bxr_gemm_next(const void* device_image, const bxr_header* header, const 
 
 /* grb_bxr_gemm_next with partial tiles lent for this call: `partials` (device, 16-byte aligned, contents of no account) takes
  * those of a batch above 128 rows, so that one block serves all weights of a stream and every workspace is sized for 128
- * rows.  192 rows per pass need grb_bxr_workspace_bytes(h, 129) - (row_blocks * 4 rounded up to 256) bytes; less, or NULL,
+ * rows.  The widest passes need grb_bxr_workspace_bytes(h, 129) - (row_blocks * 4 rounded up to 256) bytes; less, or NULL,
  * is as if it were not given. */
 int grb_bxr_gemm_partials(const void* device_image, const bxr_header* header, const void* x, int64_t ldx, uint32_t m, void* y,
                           int64_t ldy, const void* bias, void* workspace, uint64_t workspace_bytes, void* partials,
