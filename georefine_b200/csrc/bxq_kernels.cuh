@@ -18,7 +18,8 @@ namespace grb {
 
 constexpr int kWideWarpLoader = 16;    // bulk copies of chunk blobs
 constexpr int kWideWarpMma = 17;       // TMEM owner and MMA issuer
-constexpr int kWideWarpXLoader = 18;   // TMA loads of activation tiles (warp 19 has no role)
+constexpr int kWideWarpXLoader = 18;   // TMA loads of activation tiles
+constexpr int kWideWarpSlices = 19;    // partial tiles of the closing reduction
 constexpr int kWideWarpEpilogue = 20;  // 4 warps: warp % 4 = the tensor-memory lane quarter a warp may read
 
 // Tensor memory: columns [0, 256) accumulators, FP32, one of NB columns per item.  Up to NB = 128 two items fit, one being
@@ -42,7 +43,7 @@ constexpr uint32_t kWideTmemCols = 512;
 // accumulators of its own row block and each CTA's shared memory half of the activation rows.  With that and two
 // accumulator tiles (T = 2) a pass takes 384 rows, so that a chunk is streamed, decoded and written to tensor memory once for
 // twice the rows and meets half the activation bytes per row.  At 384 rows, two passes before and one now: 34816 x 5120 147 ->
-// 109 us, 5120 x 17408 86 -> 75 us, 7168 x 5120 42 -> 33 us, 5120 x 5120 36 -> 27 us.  (Barriers that a peer arrives on with
+// 106 us, 5120 x 17408 86 -> 64 us, 7168 x 5120 42 -> 30 us, 5120 x 5120 36 -> 25 us.  (Barriers that a peer arrives on with
 // release and acquire at cluster scope cost 1.4 us a chunk; the plain forms order what matters here, the completed tensor
 // memory stores and bulk copies.  At 128 rows pairs gain nothing: 34816 x 5120 58.4 against 59.4 us, 7168 x 5120 18.4 against
 // 17.0 us.)
@@ -65,10 +66,8 @@ struct BxqSmem {
   static constexpr bool kXOwn = kX != kOp;                    // activation stages are handed back on barriers of their own
   static constexpr uint32_t kReserve = 1024 /* alignment slack */ + 512 /* barriers, flags */;
   // the epilogue warps turn their accumulator columns around in shared memory (a lane holds one weight row, memory
-  // wants consecutive rows together): 16 columns x 32 rows x 4 bytes per warp
-  // (8 columns at a time where the activation ring leaves no room for 16)
-  static constexpr int kTurnCols = NB <= 128 ? 16 : 8;
-  static constexpr uint32_t kTurn = (MODE == kUmma) ? kTurnCols * 128u : 0u;
+  // wants consecutive rows together): so many columns x 32 rows x 2 bytes per warp
+  static constexpr uint32_t kTurnCols = NB >= 32 && kXStage <= 32768 ? 32 : 16, kTurn = (MODE == kUmma) ? kTurnCols * 64 : 0;
   static constexpr int kInFit = int((232448u - kReserve - kX * kXStage - 4 * kTurn) / BXQ_BLOB_MAX);
   static constexpr int kIn = kInFit > 7 ? 7 : kInFit;   // (more barriers would not fit the one-per-lane set-up)
   static constexpr uint32_t xs = 0;
@@ -76,16 +75,18 @@ struct BxqSmem {
   static constexpr uint32_t in = turn + 4 * kTurn;
   static constexpr uint32_t bars = in + kIn * BXQ_BLOB_MAX;
   // barrier order: in_full, in_empty [kIn each]; op_full, op_empty [kOp each]; x_full [kX]; x_empty [kX, if kXOwn];
-  // acc_full, acc_empty [2 each]; final; tile_full, tile_used [kRing each] (the closing reduction)
-  static constexpr uint32_t kRing = (NB <= 64) ? 4 : (NB <= 128) ? 2 : 1;  // tiles in flight in the closing reduction (kWideTileRing)
-  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + (kXOwn ? 2 : 1) * kX + 4 + 1 + 2 * kRing;
+  // acc_full, acc_empty [2 each]; final; slice_full, slice_used [kSlices each], swap_used, swap_full (the closing reduction)
+  // the closing reduction: the CTA's own tile of NB batch rows, and slices of kSliceRows batch rows of the others' on their way
+  static constexpr uint32_t kSliceRows = T * NB <= 128 ? NB : 64, kSlice = kSliceRows * BXR_ROWS * 4;
+  static constexpr uint32_t kSlicesFit = MODE == kUmma ? (bars - NB * 512u) / kSlice : 0, kSlices = kSlicesFit > 8 ? 8 : kSlicesFit;
+  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + (kXOwn ? 2 : 1) * kX + 4 + 1 + 2 * kSlices + 2;
   static constexpr uint32_t misc = (bars + 8 * nbars + 15) & ~15u;  // tmem base, abort flag, decision
   static constexpr uint32_t total = misc + 48;
   static constexpr uint32_t alloc = total + 1024;
   static_assert(MODE != kUmma || kIn >= 3, "ring too shallow");
   static_assert(MODE != kUmma || T * NB * kWideAccBufs<NB, T> <= int(kWideOperandCol<NB, T>), "accumulators overlap the operand columns");
   static_assert(8 * nbars + 64 <= 512, "barrier area");
-  static_assert(MODE != kUmma || (1 + kRing) * NB * 512u <= bars, "the closing reduction's tiles would overwrite the barriers");
+  static_assert(MODE != kUmma || (T * NB * 512u <= bars && kSlices >= 2), "kept tiles and slices would overwrite the barriers");
   static_assert(alloc <= 232448, "exceeds the 227 KB of shared memory a CTA may opt into");
 };
 
@@ -145,55 +146,102 @@ __device__ __forceinline__ WideSpan wide_span(uint32_t unit, uint32_t unit_end, 
   return {rb, c0, min(chunks, c0 + (unit_end - unit))};
 }
 
-// The closing reduction of a split row block, by the (kDecoderWarps + 4) x 32 threads that have nothing else left
-// to do: y[m, row] = bf16(sum of the row block's FP32 tiles in K order (+ bias)).  A reducing SM has to pull
-// (parts - 1) x NB x 512 bytes through its one L2 port, so the tiles come by bulk copy, kWideTileRing<NB> in flight,
-// into the shared memory the pipeline no longer needs (from byte T on, T = NB x 512; the CTA's own last tile, if it
-// takes part, lies at [0, T) and was never in memory).  A thread owns the same few float4 positions of every tile and
-// keeps their running sums in registers.  `fetched` counts the tiles brought in so far by this CTA (barrier phases).
-template <int NB>
-constexpr uint32_t kWideTileRing = NB <= 64 ? 4 : NB <= 128 ? 2 : 1;  // (1 + ring) x NB x 512 bytes of shared memory
-
-// `tile` = which of the pass's T tiles of NB batch rows.
-__device__ __forceinline__ uint32_t wide_tile_cols(uint32_t m, uint32_t tile, uint32_t nb) {  // its batch rows, in whole eights
-  return (min(m - min(m, tile * nb), nb) + 7) & ~7u;
+__device__ __forceinline__ uint32_t wide_pack(float lo, float hi) {
+  const __nv_bfloat162 pair = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&pair);
 }
-template <int NB, int T>
-__device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const RoleCtx& ctx, uint32_t row_block, uint32_t first,
-                                                     uint32_t parts, uint32_t own, uint32_t smem, uint32_t bar_full, uint32_t bar_used,
-                                                     uint32_t t, uint32_t tile, uint32_t& fetched) {
+
+// The closing reduction of a row block whose parts belong to the CTAs of one thread-block cluster (the partition is
+// "aligned": workers = row blocks x P, CTA rank r of cluster b owns part r of row block b, in K order).  Every CTA has
+// left its FP32 tile at the start of its shared memory; after the cluster barrier each CTA adds the P tiles of ITS share
+// of the batch columns (m = rank, rank + P, ...) in rank order - its own from local shared memory, the others over
+// distributed shared memory - and writes y.  No partial tile goes to global memory, no counter, no fence, and the work
+// of the reduction is spread over the P SMs.  t = index of the calling thread among the (kDecoderWarps + 4) x 32.  In a cluster
+// of pairs (two row blocks side by side) part p of this CTA's row block belongs to rank 2p + (own rank mod 2).
+// A peer's shared memory answers after some 1.5 us with all SMs asking, so what a thread needs is loads in flight: U positions
+// of up to MAXP parts at once, so that 128 batch rows are one round (5120 x 5120 in clusters of three at 384 rows: 27.2 -> 25.1
+// us, 7168 x 5120 in clusters of two 32.6 -> 30.4).
+template <bool PAIR, int MAXP, int U>
+__device__ __forceinline__ void bxq_reduce_in_cluster(const BxrArgs& args, uint32_t row_block, uint32_t smem, uint32_t t) {
   constexpr uint32_t kThreads = (kDecoderWarps + 4) * 32;
-  constexpr int kMine = (NB * 32 + kThreads - 1) / kThreads;  // float4 positions per thread
-  constexpr uint32_t kTile = NB * BXR_ROWS * 4;
-  const uint32_t mcols = wide_tile_cols(args.m, tile, NB), total = mcols * 32, bytes = mcols * BXR_ROWS * 4;
-  const uint32_t remote = parts - (own < parts ? 1u : 0u);
-  const uint32_t lane = t & 31;
-  uint32_t asked = 0;  // remote tiles requested in this call
-  bool live = true;
-  constexpr uint32_t kRing = kWideTileRing<NB>;
-  auto ask = [&](uint32_t j) {  // thread 0: the j-th remote tile into buffer (fetched + j) % kRing, once its last readers are done
-    const uint32_t n = fetched + j, b = n % kRing, p = j + ((own < parts && own <= j) ? 1u : 0u);
-    if (!ctx.wait(bar_used + 8 * b, ((n / kRing) & 1) ^ 1)) { live = false; return; }
-    mbar_arrive_expect_tx(bar_full + 8 * b, bytes);
-    bulk_g2s(smem + kTile * (1 + b), args.partials + (size_t(first + p) * T + tile) * NB * BXR_ROWS, bytes, bar_full + 8 * b, l2_policy_evict_first());
-    asked = j + 1;
-  };
-  if (t == 0)
-    for (uint32_t j = 0; j < kRing && j < remote && live; ++j) ask(j);
-  float4 sum[kMine];
-  uint32_t j = 0;  // remote tiles consumed
-  for (uint32_t p = 0; p < parts && live; ++p) {
-    uint32_t src = smem, b = 0;
-    if (p != own) {
-      const uint32_t n = fetched + j;
-      b = n % kRing;
-      if (!ctx.wait(bar_full + 8 * b, (n / kRing) & 1)) { live = false; break; }
-      src = smem + kTile * (1 + b);
+  const uint32_t parts = args.cluster, in_cluster = cluster_rank(), rank = PAIR ? in_cluster >> 1 : in_cluster;
+  const uint32_t mine = rank < args.m ? (args.m - rank + parts - 1) / parts : 0;  // batch columns rank, rank + P, ... below m
+  const uint32_t row4 = row_block * BXR_ROWS + (t & 31) * 4;    // (kThreads is a multiple of 32: the same for all of a thread's positions)
+  if (row4 >= args.rows) return;
+  float bias4[4] = {0.f, 0.f, 0.f, 0.f};
+  if (args.bias)
+    for (int k = 0; k < 4; ++k)
+      if (row4 + k < args.rows) bias4[k] = __bfloat162float(args.bias[row4 + k]);
+  uint32_t tile[MAXP];
+#pragma unroll
+  for (uint32_t p = 0; p < MAXP; ++p)
+    if (p < parts) tile[p] = cluster_map(smem, PAIR ? 2 * p + (in_cluster & 1u) : p);
+  for (uint32_t i0 = t; i0 < mine * 32; i0 += U * kThreads) {
+    uint4 u[U][MAXP];
+#pragma unroll
+    for (uint32_t j = 0; j < U; ++j) {
+      const uint32_t i = i0 + j * kThreads, m = rank + (i >> 5) * parts;
+#pragma unroll
+      for (uint32_t p = 0; p < MAXP; ++p)
+        if (i < mine * 32 && p < parts) u[j][p] = p == rank ? lds128(smem + ((m << 5) | (i & 31)) * 16) : lds128_cluster(tile[p] + ((m << 5) | (i & 31)) * 16);
     }
 #pragma unroll
-    for (int k = 0; k < kMine; ++k) {
-      const uint32_t at = t + k * kThreads;
-      if (at < total) {
+    for (uint32_t j = 0; j < U; ++j) {
+      const uint32_t i = i0 + j * kThreads, m = rank + (i >> 5) * parts;
+      if (i >= mine * 32) break;
+      // part 0 is taken as it is: adding it to zero would lose the sign of a -0
+      float f[4] = {__uint_as_float(u[j][0].x), __uint_as_float(u[j][0].y), __uint_as_float(u[j][0].z), __uint_as_float(u[j][0].w)};
+#pragma unroll
+      for (uint32_t p = 1; p < MAXP; ++p)
+        if (p < parts) {
+          f[0] = __fadd_rn(f[0], __uint_as_float(u[j][p].x));
+          f[1] = __fadd_rn(f[1], __uint_as_float(u[j][p].y));
+          f[2] = __fadd_rn(f[2], __uint_as_float(u[j][p].z));
+          f[3] = __fadd_rn(f[3], __uint_as_float(u[j][p].w));
+        }
+      if (args.bias)
+        for (int k = 0; k < 4; ++k) f[k] = __fadd_rn(f[k], bias4[k]);
+      __nv_bfloat16* dst = args.y + size_t(m) * args.ldy + row4;
+      if (row4 + 3 < args.rows && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(wide_pack(f[0], f[1]), wide_pack(f[2], f[3]));
+      } else {
+        for (int k = 0; k < 4; ++k)
+          if (row4 + k < args.rows) dst[k] = __float2bfloat16_rn(f[k]);
+      }
+    }
+  }
+}
+// The closing reduction of a split row block by the 16 decoder warps: y[m, row] = bf16(sum of the row block's FP32 tiles in K
+// order (+ bias)), for the batch rows [m_at, m_end) of one accumulator tile.  The others' tiles come from L2, a round trip of
+// 1.4 us with all SMs asking and up to 4 x 196 KB of them, so they are brought in by bulk copies slice by slice (BxqSmem), in the
+// order they are added, as many ahead as shared memory holds; warp kWideWarpSlices asks for them.  The CTA's own tile (part
+// `own`, none if >= parts) lies at the start of shared memory.  A thread owns the same few positions of four weight rows in every
+// slice.  Slices are whole tiles up to 128 columns (5120 x 17408 at 128 rows: 34.0 us, 35.6 with 32 rows a slice) and 64 batch
+// rows above (at 384 rows: whole 192-row tiles, one at a time, 75 us; 64 rows 64 us; 32 rows 67 us).
+// `n` counts slices through the launch (ring position and barrier phase).
+template <class L>
+__device__ __forceinline__ void bxq_add_tiles(const BxrArgs& args, const RoleCtx& ctx, uint32_t row_block, uint32_t parts, uint32_t own,
+                                              uint32_t smem, uint32_t ring, uint32_t bar_full, uint32_t bar_used, uint32_t t, uint32_t m_at, uint32_t m_end,
+                                              uint32_t& n) {
+  constexpr uint32_t kThreads = kDecoderWarps * 32, kMine = (L::kSliceRows * 32 + kThreads - 1) / kThreads;
+  const uint32_t row4 = row_block * BXR_ROWS + (t & 31) * 4;
+  float bias4[4] = {0.f, 0.f, 0.f, 0.f};
+  if (args.bias)
+    for (int i = 0; i < 4; ++i)
+      if (row4 + i < args.rows) bias4[i] = __bfloat162float(args.bias[row4 + i]);
+  for (uint32_t m0 = m_at; m0 < m_end; m0 += L::kSliceRows) {
+    float4 sum[kMine];
+    for (uint32_t p = 0; p < parts; ++p) {
+      uint32_t src = smem + (m0 - m_at) * BXR_ROWS * 4;
+      const uint32_t b = n % L::kSlices;
+      if (p != own) {
+        if (!ctx.wait(bar_full + 8 * b, (n / L::kSlices) & 1)) return;
+        src = ring + b * L::kSlice;
+      }
+#pragma unroll
+      for (uint32_t k = 0; k < kMine; ++k) {
+        const uint32_t at = t + k * kThreads;
+        if (m0 + (at >> 5) >= m_end || at >= L::kSliceRows * 32) continue;
         const uint4 u = lds128(src + at * 16);
         if (p == 0) {  // taken as it is: adding it to zero would lose the sign of a -0
           sum[k] = make_float4(__uint_as_float(u.x), __uint_as_float(u.y), __uint_as_float(u.z), __uint_as_float(u.w));
@@ -204,96 +252,31 @@ __device__ __forceinline__ void bxq_reduce_row_block(const BxrArgs& args, const 
           sum[k].w = __fadd_rn(sum[k].w, __uint_as_float(u.w));
         }
       }
-    }
-    if (p != own) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_used + 8 * b);
-      if (t == 0 && j + kRing < remote) ask(j + kRing);
-      ++j;
-    }
-  }
-  if (t == 0 && !live)  // unwinding: copies still in flight must land before the CTA may exit
-    for (uint32_t k = j; k < asked; ++k) mbar_wait(bar_full + 8 * ((fetched + k) % kRing), ((fetched + k) / kRing) & 1);
-  fetched += remote;
-  if (!live) return;
-#pragma unroll
-  for (int k = 0; k < kMine; ++k) {
-    const uint32_t at = t + k * kThreads, m = tile * NB + (at >> 5), row4 = row_block * BXR_ROWS + (at & 31) * 4;
-    if (at >= total || m >= args.m || row4 >= args.rows) continue;
-    float f[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
-    if (args.bias)
-      for (int i = 0; i < 4; ++i)
-        if (row4 + i < args.rows) f[i] = __fadd_rn(f[i], __bfloat162float(args.bias[row4 + i]));
-    __nv_bfloat16* dst = args.y + size_t(m) * args.ldy + row4;
-    if (row4 + 3 < args.rows && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
-      __nv_bfloat162 lo, hi;
-      lo.x = __float2bfloat16_rn(f[0]);
-      lo.y = __float2bfloat16_rn(f[1]);
-      hi.x = __float2bfloat16_rn(f[2]);
-      hi.y = __float2bfloat16_rn(f[3]);
-      uint2 packed;
-      packed.x = *reinterpret_cast<uint32_t*>(&lo);
-      packed.y = *reinterpret_cast<uint32_t*>(&hi);
-      *reinterpret_cast<uint2*>(dst) = packed;
-    } else {
-      for (int i = 0; i < 4; ++i)
-        if (row4 + i < args.rows) dst[i] = __float2bfloat16_rn(f[i]);
-    }
-  }
-}
-
-// The closing reduction of a row block whose parts belong to the CTAs of one thread-block cluster (the partition is
-// "aligned": workers = row blocks x P, CTA rank r of cluster b owns part r of row block b, in K order).  Every CTA has
-// left its FP32 tile at the start of its shared memory; after the cluster barrier each CTA adds the P tiles of ITS share
-// of the batch columns (m = rank, rank + P, ...) in rank order - its own from local shared memory, the others over
-// distributed shared memory - and writes y.  No partial tile goes to global memory, no counter, no fence, and the work
-// of the reduction is spread over the P SMs.  t = index of the calling thread among the (kDecoderWarps + 4) x 32; `tile` = which
-// of the pass's tiles of NB batch rows.  In a cluster of pairs (two row blocks side by side) part p of this CTA's row
-// block belongs to rank 2p + (own rank mod 2).
-template <int NB, bool PAIR>
-__device__ __forceinline__ void bxq_reduce_in_cluster(const BxrArgs& args, uint32_t row_block, uint32_t smem, uint32_t t, uint32_t tile) {
-  constexpr uint32_t kThreads = (kDecoderWarps + 4) * 32;
-  const uint32_t parts = args.cluster, in_cluster = cluster_rank(), rank = PAIR ? in_cluster >> 1 : in_cluster;
-  const uint32_t mcols = wide_tile_cols(args.m, tile, NB);
-  const uint32_t mine = rank < mcols ? (mcols - rank + parts - 1) / parts : 0;  // batch columns rank, rank + P, ... below mcols
-  for (uint32_t i = t; i < mine * 32; i += kThreads) {
-    const uint32_t m = rank + (i >> 5) * parts, at = (m << 5) | (i & 31);
-    const uint32_t row4 = row_block * BXR_ROWS + (i & 31) * 4;
-    if (tile * NB + m >= args.m || row4 >= args.rows) continue;
-    uint4 u[8];  // every part's piece first (independent loads in flight), then the sum in K order
-#pragma unroll
-    for (uint32_t p = 0; p < 8; ++p)
-      if (p < parts) u[p] = p == rank ? lds128(smem + at * 16) : lds128_cluster(cluster_map(smem + at * 16, PAIR ? 2 * p + (in_cluster & 1u) : p));
-    // part 0 is taken as it is: adding it to zero would lose the sign of a -0
-    float f[4] = {__uint_as_float(u[0].x), __uint_as_float(u[0].y), __uint_as_float(u[0].z), __uint_as_float(u[0].w)};
-#pragma unroll
-    for (uint32_t p = 1; p < 8; ++p)
-      if (p < parts) {
-        f[0] = __fadd_rn(f[0], __uint_as_float(u[p].x));
-        f[1] = __fadd_rn(f[1], __uint_as_float(u[p].y));
-        f[2] = __fadd_rn(f[2], __uint_as_float(u[p].z));
-        f[3] = __fadd_rn(f[3], __uint_as_float(u[p].w));
+      if (p != own) {
+        __syncwarp();
+        if ((t & 31) == 0) mbar_arrive(bar_used + 8 * b);
+        ++n;
       }
-    if (args.bias)
-      for (int k = 0; k < 4; ++k)
-        if (row4 + k < args.rows) f[k] = __fadd_rn(f[k], __bfloat162float(args.bias[row4 + k]));
-    __nv_bfloat16* dst = args.y + size_t(tile * NB + m) * args.ldy + row4;
-    if (row4 + 3 < args.rows && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
-      __nv_bfloat162 lo, hi;
-      lo.x = __float2bfloat16_rn(f[0]);
-      lo.y = __float2bfloat16_rn(f[1]);
-      hi.x = __float2bfloat16_rn(f[2]);
-      hi.y = __float2bfloat16_rn(f[3]);
-      uint2 packed;
-      packed.x = *reinterpret_cast<uint32_t*>(&lo);
-      packed.y = *reinterpret_cast<uint32_t*>(&hi);
-      *reinterpret_cast<uint2*>(dst) = packed;
-    } else {
-      for (int k = 0; k < 4; ++k)
-        if (row4 + k < args.rows) dst[k] = __float2bfloat16_rn(f[k]);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kMine; ++k) {
+      const uint32_t at = t + k * kThreads, m = m0 + (at >> 5);
+      if (m >= m_end || at >= L::kSliceRows * 32 || m >= args.m || row4 >= args.rows) continue;
+      float f[4] = {sum[k].x, sum[k].y, sum[k].z, sum[k].w};
+      if (args.bias)
+        for (int i = 0; i < 4; ++i) f[i] = __fadd_rn(f[i], bias4[i]);
+      __nv_bfloat16* dst = args.y + size_t(m) * args.ldy + row4;
+      if (row4 + 3 < args.rows && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(wide_pack(f[0], f[1]), wide_pack(f[2], f[3]));
+      } else {
+        for (int i = 0; i < 4; ++i)
+          if (row4 + i < args.rows) dst[i] = __float2bfloat16_rn(f[i]);
+      }
     }
   }
 }
+// (batch rows of one accumulator tile that there are, in whole eights)
+__device__ __forceinline__ uint32_t wide_tile_cols(uint32_t m, uint32_t tile, uint32_t nb) { return (min(m - min(m, tile * nb), nb) + 7) & ~7u; }
 
 template <int MODE, int NB, int T = 1, bool PAIR = false>
 __global__ void __launch_bounds__(MODE == kUmma ? kThreadsUmma : kThreadsSimt, 1)
@@ -323,7 +306,8 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   const uint32_t bar_x_full = bar_op_empty + 8 * L::kOp;
   const uint32_t bar_x_empty = L::kXOwn ? bar_x_full + 8 * L::kX : bar_op_empty;   // (rings of one length: stage i of both is free together)
   const uint32_t bar_acc_full = bar_x_full + 8 * L::kX * (L::kXOwn ? 2 : 1), bar_acc_empty = bar_acc_full + 16, bar_final = bar_acc_empty + 16;
-  const uint32_t bar_tile_full = bar_final + 8, bar_tile_used = bar_tile_full + 8 * L::kRing;
+  const uint32_t bar_slice_full = bar_final + 8, bar_slice_used = bar_slice_full + 8 * L::kSlices;
+  const uint32_t bar_swap_used = bar_slice_used + 8 * L::kSlices, bar_swap_full = bar_swap_used + 8;
   constexpr uint32_t kTmemCols = kWideTmemCols;
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;
   constexpr uint32_t kXN = L::kX ? L::kX : 1;
@@ -390,8 +374,8 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       if (n >= uint32_t(L::kIn) && n < 2u * L::kIn) count = kDecoderWarps;          // in_empty
       else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps * kCtas;  // op_full
       else if (n >= 2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX) {
-        const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX);  // acc_full x2, acc_empty x2, final, tile_full, tile_used
-        count = j < 2 ? 1u : j < 4 ? 4u * kCtas : j < 5 ? 4u : j < 5 + L::kRing ? 1u : uint32_t(kDecoderWarps + 4);
+        const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX);  // acc_full x2, acc_empty x2, final, slice_full, slice_used, swap_used, swap_full
+        count = j < 2 ? 1u : j < 4 ? 4u * kCtas : j < 5 ? 4u : j < 5 + L::kSlices ? 1u : j < 6 + 2 * L::kSlices ? uint32_t(kDecoderWarps) : 4u;
       }
       mbar_init(ctx.bars + 8 * n, count);
     }
@@ -418,18 +402,18 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   if (MODE == kUmma) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(smem + L::misc));
 
 
-  // Epilogue warps: tile t of the CTA's n_item-th item, from tensor memory to the start of shared memory, all of which is free
-  // by the time an item is kept.
-  auto drain_to_smem = [&](uint32_t n_item, uint32_t t, uint32_t e, uint32_t r) {
-    const uint32_t taddr = tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB, mcols = wide_tile_cols(args.m, t, NB);
+  // Epilogue warps: accumulator tile `t` of the CTA's n-th item, as [batch row][128 weight rows] FP32 (as in memory), to `dst`.
+  auto drain_to_smem = [&](uint32_t n_item, uint32_t t, uint32_t dst) {
+    constexpr int kStep = NB >= 32 ? 32 : 16;
+    const uint32_t e = warp - kWideWarpEpilogue;
 #pragma unroll 1
-    for (uint32_t m0 = 0; m0 < mcols; m0 += 16) {
-      uint32_t v[16];
-      tmem_ld16(taddr + m0, v);
+    for (uint32_t m0 = 0; m0 < wide_tile_cols(args.m, t, NB); m0 += kStep) {
+      uint32_t v[kStep];
+      if constexpr (kStep == 32) tmem_ld32(tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB + m0, v);
+      else tmem_ld16(tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB + m0, v);
       tmem_ld_wait();
 #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        if (m0 + i < mcols) sts32(smem + ((m0 + i) * BXR_ROWS + r) * 4, v[i]);
+      for (int i = 0; i < kStep; ++i) sts32(dst + ((m0 + i) * BXR_ROWS + e * 32 + lane) * 4, v[i]);
     }
   };
 
@@ -634,214 +618,259 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     const uint32_t r = e * 32 + lane;
     const uint32_t acc_empty_at = PAIR ? cluster_map(bar_acc_empty, my_rank & ~1u) : bar_acc_empty;   // the issuer's
     uint32_t n_item = 0;
-    bool live = true, early_taken = false;
+    bool live = true;
+    // Split row blocks that this CTA is the last to declare, and so adds up: that of its last item (misc + 16) and that of its
+    // first (misc + 32), as {1 | (index + 1 of the tile kept in shared memory) << 8, row block, first slot, parts}.
+    auto decide = [&](uint32_t at, uint32_t own, const bxr_item& i) {
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(smem + L::misc + at), "r"(1u | own << 8), "r"(i.row_block), "r"(i.slot - i.part), "r"(i.parts) : "memory");
+    };
     const uint64_t stay = l2_policy_evict_last();  // partial tiles are read back within the launch
     grid_dependency_wait();  // bias, y, partial tiles and counters may belong to the previous kernel
     bxr_item item = {};
     if (item_begin < item_end) item = args.items[item_begin];
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       if (it != item_begin) item = args.items[it];
-      const uint32_t row = item.row_block * BXR_ROWS + r;
-      const float b = (args.bias && row < args.rows) ? __bfloat162float(args.bias[row]) : 0.f;
-      constexpr int kStep = 16, kCols = L::kTurnCols;  // accumulator columns per tensor-memory load, and per turn-around
-      // (a load's round trip is what a step waits for: 16 columns per load where only 8 fit the turn-around took a
-      // pass of 192 rows over 34816 x 5120 from 76.1 to 74.4 us, over 5120 x 5120 from 19.1 to 18.5 us)
+      const uint32_t row = item.row_block * BXR_ROWS + r, row0 = item.row_block * BXR_ROWS + e * 32;
       // The CTA's last item, if it is part of a split row block, keeps its tile in shared memory (all of it is free
-      // by now: every blob and every activation tile has been multiplied).  If the other tiles of the row block are already in memory -
-      // the usual case, they were finished long ago as some CTA's first item - this tile never goes to memory at
-      // all: no store, no fence, no counter update on the tail of the kernel.
-      const bool final_item = it + 1 == item_end;
+      // by now: every blob and every activation tile has been multiplied).  If the other parts of the row block have been
+      // declared by then, this CTA adds them up and its own tile never goes to memory.  Only the first and the last item of a
+      // CTA can be part of a split row block.
       const bool in_cluster = args.cluster > 1;  // the CTA's one item is a part of its cluster's row block
-      const bool keep = item.parts > 1 && (final_item || in_cluster);   // (T = 2: the second tile waits in tensor memory for its turn)
-      const uint32_t kept = smem;           // [batch row][128 weight rows] FP32, like a partial tile in memory
-      uint32_t arrived = 0;
+      const bool keep = item.parts > 1 && (it + 1 == item_end || in_cluster);
       if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * acc_slot(n_item, 0), acc_use(n_item) & 1)) { live = false; break; }
-      // (the second tile's last multiply may still be reading the activations in whose place a kept tile goes)
-      if (T == 2 && keep && !ctx.wait(bar_acc_full + 8, acc_use(n_item) & 1)) { live = false; break; }
-      tc_fence_after();
-      if (keep && !in_cluster && e == 0 && lane == 0) arrived = ld_relaxed_gpu(args.counters + item.row_block);  // answer used after the drain; fenced there
-      // A lane holds one weight row and kStep batch columns; y and the partial tiles keep the rows of one batch
-      // column together.  Stored from the registers that is one narrow store instruction per column, and the
-      // store queue, not the memory, sets the pace (a 128-column drain took 4 400 to 10 000 cycles).  So the
-      // columns are turned around in shared memory and leave as 16-byte stores: 8 (y) or 4 (tiles) columns each.
-      const uint32_t turn = smem + L::turn + e * L::kTurn;
-      const bool y_wide = (reinterpret_cast<uintptr_t>(args.y) & 15u) == 0 && (args.ldy & 7u) == 0 &&
-                          item.row_block * BXR_ROWS + e * 32 + 32 <= args.rows;
       if (keep) {
-        drain_to_smem(n_item, 0, e, r);
-      } else {
+        // (the second tile's last multiply may still be reading the activations in whose place the first one goes)
+        if (T == 2 && !ctx.wait(bar_acc_full + 8, acc_use(n_item) & 1)) { live = false; break; }
+        tc_fence_after();
+        // A row block's counter: parts declared in the low half, parts in memory in the high half.
+        uint32_t declared = 0;
+        if (!in_cluster && e == 0 && lane == 0) declared = atomicAdd(args.counters + item.row_block, 1u) & 0xFFFFu;   // (answer used after the drain)
+        if (in_cluster) {
 #pragma unroll 1
-        for (uint32_t t = 0; t < uint32_t(T); ++t) {
-          if (t && !ctx.wait(bar_acc_full + 8 * acc_slot(n_item, t), acc_use(n_item) & 1)) { live = false; break; }
-          if (t) tc_fence_after();
-          const uint32_t taddr = tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB, m_at = t * NB, mcols = wide_tile_cols(args.m, t, NB);
-          for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
-            uint32_t v[kStep];
-            tmem_ld16(taddr + m0, v);
-            tmem_ld_wait();
-            if (item.parts == 1) {
-              if (y_wide) {
-#pragma unroll
-                for (int h = 0; h < kStep; h += kCols) {
-#pragma unroll
-                  for (int i = 0; i < kCols; ++i) {
-                    const float f = __uint_as_float(v[h + i]);
-                    const __nv_bfloat16 o = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
-                    sts_u16(turn + (i * 32 + lane) * 2, uint32_t(*reinterpret_cast<const uint16_t*>(&o)));
-                  }
-                  __syncwarp();
-#pragma unroll
-                  for (int j = 0; j < kCols / 8; ++j) {  // a store: 8 columns x 64 bytes (32 rows)
-                    const uint32_t ml = j * 8 + (lane >> 2), m = m_at + m0 + h + ml;
-                    const uint4 piece = lds128(turn + ml * 64 + (lane & 3) * 16);
-                    if (m < args.m)
-                      *reinterpret_cast<uint4*>(args.y + size_t(m) * args.ldy + item.row_block * BXR_ROWS + e * 32 + (lane & 3) * 8) = piece;
-                  }
-                  __syncwarp();
-                }
-              } else if (row < args.rows) {
-#pragma unroll
-                for (int i = 0; i < kStep; ++i)
-                  if (m_at + m0 + i < args.m) {
-                    const float f = __uint_as_float(v[i]);
-                    args.y[size_t(m_at + m0 + i) * args.ldy + row] = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
-                  }
-              }
-            } else {
-#pragma unroll
-              for (int h = 0; h < kStep; h += kCols) {
-#pragma unroll
-                for (int i = 0; i < kCols; ++i) sts32(turn + (i * 32 + lane) * 4, v[h + i]);
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < kCols / 4; ++j) {  // a store: 4 columns x 128 bytes (32 rows)
-                  const uint32_t ml = j * 4 + (lane >> 3), m = m0 + h + ml;
-                  const uint4 piece = lds128(turn + ml * 128 + (lane & 7) * 16);
-                  if (m < mcols) stg128(args.partials + ((size_t(item.slot) * T + t) * NB + m) * BXR_ROWS + e * 32 + (lane & 7) * 4, piece, stay);
-                }
-                __syncwarp();
-              }
-            }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if (leader) mbar_arrive(bar_acc_empty + 8 * acc_slot(n_item, t));
-            else mbar_arrive_cluster(acc_empty_at + 8 * acc_slot(n_item, t));
-          }
-        }
-        if (!live) break;
-      }
-      if (item.parts > 1 && !in_cluster) {
-        // `prev` = how many tiles of the row block were in memory before this one; the CTA that completes the set
-        // reduces it.  Flag words: misc + 8 and misc + 12.
-        uint32_t prev;
-        bool published = false;   // of a kept item: its tiles have left for memory
-        if (keep) {
+          for (uint32_t t = 0; t < uint32_t(T); ++t) drain_to_smem(n_item, t, smem + t * NB * BXR_ROWS * 4);
+        } else {
+          drain_to_smem(n_item, 0, smem);
+          if (e == 0 && lane == 0) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(declared) : "memory");
           fence_proxy_async_smem();  // the tile may leave through a bulk copy
-          if (e == 0 && lane == 0) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(arrived) : "memory");
           named_barrier(1, 128);
-          asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 8));
-          if (prev != item.parts - 1) {  // someone else is still missing: publish the tile like any other
-            published = true;
-#pragma unroll
-            for (uint32_t t = 0; t < uint32_t(T); ++t) {
-              if (t) {   // the second tile takes the place of the first, which has left
-                named_barrier(1, 128);
-                drain_to_smem(n_item, t, e, r);
-                fence_proxy_async_smem();
-                named_barrier(1, 128);
-              }
-              if (e == 0 && lane == 0) {
-                bulk_s2g(args.partials + (size_t(item.slot) * T + t) * NB * BXR_ROWS, kept, wide_tile_cols(args.m, t, NB) * BXR_ROWS * 4);
-                bulk_commit_and_wait();
-              }
+          asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(declared) : "r"(smem + L::misc + 8));
+          if (declared == item.parts - 1) {   // (T = 2: the second tile waits in tensor memory until the first has been added)
+            if (e == 0 && lane == 0) decide(16, item.part + 1u, item);
+          } else {   // another CTA will be the last: publish the tiles like any other
+            if (T == 2) {
+              drain_to_smem(n_item, 1, smem + NB * BXR_ROWS * 4);
+              fence_proxy_async_smem();
+              named_barrier(1, 128);
             }
             if (e == 0 && lane == 0) {
+              bulk_s2g(args.partials + size_t(item.slot) * T * NB * BXR_ROWS, smem, ((args.m + 7) & ~7u) * BXR_ROWS * 4);
+              bulk_commit_and_wait();
               fence_proxy_async_all();
               __threadfence();
-              const uint32_t before = atomicAdd(args.counters + item.row_block, 1u);
-              asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 12), "r"(before) : "memory");
+              atomicAdd(args.counters + item.row_block, 1u << 16);
             }
-            named_barrier(1, 128);
-            asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 12));
+          }
+        }
+        continue;   // (the CTA's last item: nobody waits for the accumulator)
+      }
+      tc_fence_after();
+      // A lane holds one weight row and 16 batch columns; y keeps the rows of one batch column together, so its columns are
+      // turned around by stmatrix and leave as 16-byte stores.  Partial tiles do so as they are: a store per column is one
+      // whole 128-byte line.  A drain is a chain of trips to tensor memory, beside the multiplies of the next item up to 128
+      // columns and in front of them above: so many columns a trip as the registers hold.  34816 x 5120, an item of 128
+      // columns 3.0-3.6 -> 1.9-2.2 us, of 384 7-9 -> 5 us.
+      const uint32_t turn = smem + L::turn + e * L::kTurn;
+      const bool y_wide = (reinterpret_cast<uintptr_t>(args.y) & 15u) == 0 && (args.ldy & 7u) == 0 && row0 + 32 <= args.rows;
+#pragma unroll 1
+      for (uint32_t t = 0; t < uint32_t(T); ++t) {
+        if (t) {
+          if (!ctx.wait(bar_acc_full + 8 * acc_slot(n_item, t), acc_use(n_item) & 1)) { live = false; break; }
+          tc_fence_after();
+        }
+        const uint32_t taddr = tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB, m_at = t * NB, mcols = wide_tile_cols(args.m, t, NB);
+        if (item.parts > 1) {
+          constexpr int kStep = NB >= 32 ? 32 : 16;
+          float* dst = args.partials + (size_t(item.slot) * T + t) * NB * BXR_ROWS + r;
+#pragma unroll 1
+          for (uint32_t m0 = 0; m0 < mcols; m0 += kStep, dst += kStep * BXR_ROWS) {
+            uint32_t v[kStep];
+            if constexpr (kStep == 32) tmem_ld32(taddr + m0, v);
+            else tmem_ld16(taddr + m0, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int h = 0; h < kStep; h += 8)
+              if (m0 + h < mcols) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) stg32(dst + (h + i) * BXR_ROWS, v[h + i], stay);
+              }
+          }
+        } else if (y_wide) {
+          // this lane's weight rows in the accumulator layout, and where its column of a matrix goes: unit j of a batch row's
+          // 64 bytes, the units permuted by the batch row (stores and loads free of bank conflicts)
+          float b[4];
+          if (args.bias)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) b[k] = __bfloat162float(args.bias[row0 + 8 * k + (lane >> 2)]);
+          const uint32_t put_at = turn + (lane & 7) * 64 + (((lane >> 3) ^ ((lane >> 1) & 3)) << 4);
+          const uint32_t ml = lane >> 2, get_at = turn + ml * 64 + (((lane & 3) ^ ((ml >> 1) & 3)) << 4);
+          __nv_bfloat16* dst = args.y + size_t(m_at + ml) * args.ldy + row0 + (lane & 3) * 8;
+          constexpr int kStep = L::kTurnCols, kPieces = kStep / 16;
+          uint32_t v[kPieces][16];   // 16 columns: [weight rows 0-15, 16-31][columns 0-7, 8-15][4]
+          auto load = [&](uint32_t m0) {
+#pragma unroll
+            for (int k = 0; k < kPieces; ++k) {
+              tmem_ld_16x16(taddr + m0 + 16 * k, v[k]);
+              tmem_ld_16x16(taddr + m0 + 16 * k + (16u << 16), v[k] + 8);
+            }
+          };
+          load(0);
+#pragma unroll 1
+          for (uint32_t m0 = 0; m0 < mcols; m0 += kStep) {
+            tmem_ld_wait();
+            uint32_t w[kPieces][8];
+#pragma unroll
+            for (int k = 0; k < kPieces; ++k) {
+              if (args.bias)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[k][i] = __float_as_uint(__fadd_rn(__uint_as_float(v[k][i]), b[(i >> 3) * 2 + ((i >> 1) & 1)]));
+#pragma unroll
+              for (int i = 0; i < 8; ++i) w[k][i] = wide_pack(__uint_as_float(v[k][2 * i]), __uint_as_float(v[k][2 * i + 1]));
+            }
+            if (m0 + kStep < mcols) load(m0 + kStep);   // the next columns are on their way while these are stored
+#pragma unroll
+            for (int k = 0; k < kPieces; ++k) {
+              stsm_x4_trans(put_at + 1024 * k, w[k][0], w[k][1], w[k][4], w[k][5]);           // columns 0-7: rows 0-7, 8-15, 16-23, 24-31
+              stsm_x4_trans(put_at + 1024 * k + 512, w[k][2], w[k][3], w[k][6], w[k][7]);     // columns 8-15
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 2 * kPieces; ++k) {
+              const uint4 piece = lds128(get_at + 512 * k);
+              if (m_at + m0 + 8 * k + ml < args.m) *reinterpret_cast<uint4*>(dst + 8 * k * args.ldy) = piece;
+            }
+            dst += kStep * args.ldy;
+            __syncwarp();
           }
         } else {
-          __threadfence();
-          named_barrier(1, 128);
-          if (e == 0 && lane == 0) {
-            const uint32_t before = atomicAdd(args.counters + item.row_block, 1u);
-            asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(before) : "memory");
+          const float b = (args.bias && row < args.rows) ? __bfloat162float(args.bias[row]) : 0.f;
+#pragma unroll 1
+          for (uint32_t m0 = 0; m0 < mcols; m0 += 16) {
+            uint32_t v[16];
+            tmem_ld16(taddr + m0, v);
+            tmem_ld_wait();
+            if (row < args.rows)
+#pragma unroll
+              for (int i = 0; i < 16; ++i)
+                if (m_at + m0 + i < args.m) {
+                  const float f = __uint_as_float(v[i]);
+                  args.y[size_t(m_at + m0 + i) * args.ldy + row] = __float2bfloat16_rn(args.bias ? __fadd_rn(f, b) : f);
+                }
           }
-          named_barrier(1, 128);
-          asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 8));
         }
-        if (prev == item.parts - 1) {  // every other tile of this row block is in memory: add them in K order
-          __threadfence();
-          const uint32_t first = item.slot - item.part;
-          // Reduced at the end of the CTA by the decoder and epilogue warps together (below).  Only the first and the
-          // last item of a CTA can be part of a split row block, hence two decision slots; anything else is reduced here.
-          if (final_item || !early_taken) {
-            if (e == 0 && lane == 0)  // {1 | (index + 1 of the tile kept in shared memory) << 8, row block, first slot, parts}
-              asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(smem + L::misc + (final_item ? 16 : 32)),
-                           // (of two published tiles only the second is still here: both come back from memory)
-                           "r"(1u | (keep && !(T == 2 && published) ? (item.part + 1u) << 8 : 0u)), "r"(item.row_block), "r"(first), "r"(item.parts) : "memory");
-            early_taken = early_taken || !final_item;
-          } else {
-            reduce_row_block<T * NB>(args, item.row_block, first, item.parts, e, 4, lane);
-          }
-          if (e == 0 && lane == 0) args.counters[item.row_block] = 0;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (leader) mbar_arrive(bar_acc_empty + 8 * acc_slot(n_item, t));
+          else mbar_arrive_cluster(acc_empty_at + 8 * acc_slot(n_item, t));
         }
-        named_barrier(1, 128);  // the flag words may be rewritten
       }
+      if (!live) break;
+      if (item.parts > 1) {
+        __threadfence();
+        named_barrier(1, 128);
+        if (e == 0 && lane == 0) {
+          const uint32_t before = atomicAdd(args.counters + item.row_block, 0x10001u);
+          if ((before & 0xFFFFu) == item.parts - 1) decide(32, 0, item);
+        }
+      }
+    }
+    // The CTA that is the last to declare a part adds the row block up, once the others' tiles are in memory: they were
+    // declared by CTAs that had nothing else to wait for before they published them.
+    if (e == 0 && lane == 0) {
+#pragma unroll 1
+      for (uint32_t at = 32; at >= 16; at -= 16) {
+        const uint4 d = lds128(smem + L::misc + at);
+        if (!d.x) continue;
+        const uint32_t tiles = d.w - (d.x >> 8 ? 1u : 0u);
+        const unsigned long long t0 = global_ns();
+        bool there = false;
+        while (live && !(there = (ld_acquire_gpu(args.counters + d.y) >> 16) >= tiles) && global_ns() - t0 <= kWaitLimitNs) {}
+        if (!there) {
+          ctx.abort(kStatusTimeout);
+          sts32(smem + L::misc + at, 0);
+        }
+        args.counters[d.y] = 0;
+      }
+      __threadfence();
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_final);
   }
 
-  const uint32_t closing_thread = (warp < kDecoderWarps ? warp : warp - 4) * 32 + lane;
   if (MODE == kUmma && args.cluster > 1) {
     // A row block's CTAs in one cluster: every CTA's tile is in its shared memory once its epilogue is through; the cluster
     // barrier makes the tiles visible to the peers, the second one keeps every CTA's shared memory alive until the
     // peers have read it.  Every thread of every CTA gets here on every path (all other waits are bounded).
     const bool worker_thread = warp < kDecoderWarps || warp >= kWideWarpEpilogue;
     const bool drained = worker_thread ? ctx.wait(bar_final, 0) : true;
-#pragma unroll
-    for (uint32_t t = 0; t < uint32_t(T); ++t) {
-      if (t && warp >= kWideWarpEpilogue && unit_count && __all_sync(0xFFFFFFFFu, drained)) {
-        drain_to_smem(0, t, warp - kWideWarpEpilogue, (warp - kWideWarpEpilogue) * 32 + lane);
-        tc_fence_before();
+    __syncwarp();
+    cluster_sync();
+    if (worker_thread && drained && unit_count) {
+      const uint32_t row_block = (unit_begin / args.chunks) * group + in_group, t = (warp < kDecoderWarps ? warp : warp - 4) * 32 + lane;
+      // (narrow tiles: a position a thread at most, and a shorter way through code that is read once a launch: 5120 x 5120 at
+      // one row reads one position)
+      if (NB <= 32) bxq_reduce_in_cluster<PAIR, 8, 1>(args, row_block, smem, t);
+      else switch (args.cluster) {
+        case 2: bxq_reduce_in_cluster<PAIR, 2, 4>(args, row_block, smem, t); break;
+        case 3: bxq_reduce_in_cluster<PAIR, 3, 3>(args, row_block, smem, t); break;
+        case 4: bxq_reduce_in_cluster<PAIR, 4, 2>(args, row_block, smem, t); break;
+        default: if (!PAIR) bxq_reduce_in_cluster<PAIR, 8, 1>(args, row_block, smem, t);
       }
-      __syncwarp();
-      cluster_sync();
-      if (worker_thread && drained && unit_count)
-        bxq_reduce_in_cluster<NB, PAIR>(args, (unit_begin / args.chunks) * group + in_group, smem, closing_thread, t);
-      __syncwarp();
-      cluster_sync();
     }
+    __syncwarp();
+    cluster_sync();
   }
 
-  // Row blocks whose last partial tile came from this CTA are reduced by the 16 decoder warps and the 4 epilogue
-  // warps together, once the epilogue has drained the CTA's last item.
-  if (MODE == kUmma && args.cluster <= 1 && (warp < kDecoderWarps || warp >= kWideWarpEpilogue)) {
-    constexpr uint32_t kClosing = (kDecoderWarps + 4) * 32;
-    bool drained = ctx.wait(bar_final, 0);
-    if (T == 2) drained = named_barrier_and(2, kClosing, drained);   // (barriers below: all or none)
-    if (drained) {
-      uint32_t fetched = 0;  // tiles brought in so far: position in the ring
+  // Row blocks that fell to this CTA are added up: warp kWideWarpSlices brings the others' tiles in, the decoder warps add.
+  if (MODE == kUmma && args.cluster <= 1 && (warp < kDecoderWarps || warp >= kWideWarpSlices)) {
+    const uint32_t ring = smem + NB * BXR_ROWS * 4;
+    bool live = ctx.wait(bar_final, 0);
+    uint32_t n = 0;
 #pragma unroll 1
-      for (uint32_t at = 32; at >= 16; at -= 16) {
-        const uint4 decision = lds128(smem + L::misc + at);  // {reduce? | own tile << 8, row block, first slot, parts}
-        if (!decision.x) continue;
-        const uint32_t own = (decision.x >> 8) - 1u;
+    for (uint32_t at = 32; at >= 16; at -= 16) {
+      const uint4 decision = lds128(smem + L::misc + at);  // {reduce? | own tile << 8, row block, first slot, parts}
+      if (!decision.x) continue;
+      const uint32_t own = (decision.x >> 8) - 1u, parts = decision.w;
 #pragma unroll 1
-        for (uint32_t t = 0; t < uint32_t(T); ++t) {
-          if (T == 2 && t && own < decision.w) {   // the second tile takes the place of the first once that has been added
-            named_barrier(2, kClosing);
-            if (warp >= kWideWarpEpilogue) drain_to_smem(0, t, warp - kWideWarpEpilogue, (warp - kWideWarpEpilogue) * 32 + lane);
-            named_barrier(2, kClosing);
+      for (uint32_t t = 0; t < uint32_t(T); ++t) {
+        const uint32_t cols = wide_tile_cols(args.m, t, NB);
+        if (T == 2 && t && own < parts) {   // the second tile takes the place of the first once that has been added
+          if (warp < kDecoderWarps) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_swap_used);
+            live = live && ctx.wait(bar_swap_full, 0);
+          } else if (warp >= kWideWarpEpilogue) {
+            live = __all_sync(0xFFFFFFFFu, live && ctx.wait(bar_swap_used, 0));
+            if (live) drain_to_smem(0, t, smem);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_swap_full);
           }
-          bxq_reduce_row_block<NB, T>(args, ctx, decision.y, decision.z, decision.w, own, smem, bar_tile_full, bar_tile_used, closing_thread, t, fetched);
+        }
+        if (warp < kDecoderWarps) {
+          if (live) bxq_add_tiles<L>(args, ctx, decision.y, parts, own, smem, ring, bar_slice_full, bar_slice_used, warp * 32 + lane, t * NB, t * NB + cols, n);
+        } else if (warp == kWideWarpSlices && lane == 0 && live) {
+          for (uint32_t m0 = 0; m0 < cols && live; m0 += L::kSliceRows)
+            for (uint32_t p = 0; p < parts && live; ++p) {
+              if (p == own) continue;
+              const uint32_t b = n % L::kSlices, bytes = min(L::kSliceRows, cols - m0) * BXR_ROWS * 4;
+              if (!ctx.wait(bar_slice_used + 8 * b, ((n / L::kSlices) & 1) ^ 1)) { live = false; break; }
+              mbar_arrive_expect_tx(bar_slice_full + 8 * b, bytes);
+              bulk_g2s(ring + b * L::kSlice, args.partials + ((size_t(decision.z + p) * T + t) * NB + m0) * BXR_ROWS, bytes, bar_slice_full + 8 * b, l2_policy_evict_first());
+              ++n;
+            }
+          // copies still in flight must land before the CTA may exit
+          if (!live)
+            for (uint32_t k = n > L::kSlices ? n - L::kSlices : 0; k < n; ++k) mbar_wait(bar_slice_full + 8 * (k % L::kSlices), (k / L::kSlices) & 1);
         }
       }
     }

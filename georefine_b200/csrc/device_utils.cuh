@@ -116,6 +116,9 @@ __device__ __forceinline__ void stg128(void* dst, uint4 v, uint64_t policy) {
   asm volatile("st.global.L2::cache_hint.v4.b32 [%0], {%1, %2, %3, %4}, %5;" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy)
                : "memory");
 }
+__device__ __forceinline__ void stg32(void* dst, uint32_t v, uint64_t policy) {
+  asm volatile("st.global.L2::cache_hint.b32 [%0], %1, %2;" ::"l"(dst), "r"(v), "l"(policy) : "memory");
+}
 // 2-D tiled tensor copy global -> shared (no multicast).  x is the innermost coordinate (elements).
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int x, int y, uint32_t bar) {
   asm volatile(
@@ -145,9 +148,9 @@ __device__ __forceinline__ void bulk_commit_and_wait() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-__device__ __forceinline__ uint32_t ld_relaxed_gpu(const uint32_t* p) {
+__device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -288,6 +291,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "r"(taddr)
       : "memory");
 }
+// 16 lanes x 16 columns in the layout of the warp-level MMA's accumulators: thread t receives, of columns 8g + 2 (t mod 4) and the
+// one after it, lane t / 4 in v[4g], v[4g + 1] and lane t / 4 + 8 in v[4g + 2], v[4g + 3] (lanes counted from that of taddr).
+__device__ __forceinline__ void tmem_ld_16x16(uint32_t taddr, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr)
+               : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values to shared memory, transposed: thread t holds elements 2 (t mod 4) and the one after it of
+// row t / 4 of each; lane 8j + i gives the address where column i of matrix j goes (16 bytes).
+__device__ __forceinline__ void stsm_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 32 lanes x 16 consecutive 32-bit columns: thread t of the warp writes lane (base lane + t).  Whole warp.
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
@@ -339,19 +355,6 @@ __device__ __forceinline__ uint4 lds128_cluster(uint32_t a) {
   return v;
 }
 
-// Barrier over `threads` threads that tells each whether `ok` held for all of them.
-__device__ __forceinline__ bool named_barrier_and(uint32_t id, uint32_t threads, bool ok) {
-  uint32_t all;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %3, 0;\n\t"
-      "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(all)
-      : "r"(id), "r"(threads), "r"(uint32_t(ok))
-      : "memory");
-  return all != 0;
-}
 __device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }

@@ -250,8 +250,8 @@ int grb_bxr_gemm_next(const void* device_image, const bxr_header* header, const 
 
 /* grb_bxr_gemm_next with partial tiles lent for this call: `partials` (device, 16-byte aligned, contents of no account) takes
  * those of a batch above 128 rows, so that one block serves all weights of a stream and every workspace is sized for 128
- * rows.  The widest passes need grb_bxr_workspace_bytes(h, 129) - (row_blocks * 4 rounded up to 256) bytes; less, or NULL,
- * is as if it were not given. */
+ * rows.  The widest passes need grb_bxr_workspace_bytes(h, 129) - (row_blocks * 4 rounded up to 256) bytes; less makes
+ * narrower passes, NULL or less than 192 rows need is as if it were not given. */
 int grb_bxr_gemm_partials(const void* device_image, const bxr_header* header, const void* x, int64_t ldx, uint32_t m, void* y,
                           int64_t ldy, const void* bias, void* workspace, uint64_t workspace_bytes, void* partials,
                           uint64_t partials_bytes, uint32_t* status, void* cuda_stream, const void* next_device_image,
