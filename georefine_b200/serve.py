@@ -298,9 +298,9 @@ class BatchDecoder:
                 self.page_table[slot, p] = page
 
     # ---- the step ----------------------------------------------------------------------------------------------
-    def _trunk(self, n: int, advance: bool, head: bool = True) -> None:
+    def _trunk(self, n: int, advance: bool, head: int | None = 0) -> None:
         """One pass of rows 0..n-1 through the stack on the current stream; no allocation, no host synchronisation.
-        ``head=False`` stops at the residual stream: no logits, no arg-max."""
+        ``head``: the first row that gets logits and an arg-max (as row 0 of theirs; None: no row does)."""
         import torch
 
         cfg, w = self.cfg, self.w
@@ -321,10 +321,11 @@ class BatchDecoder:
             self._row_parallel(layer.down, "down", self.act[:n], self.down_out[:n])
             delta = self.down_out[:n]
         ops.rmsnorm(h, w.final_norm, x, delta=delta, eps=cfg.eps)          # h now holds the final residual stream
-        if not head:
+        if head is None:
             return
-        self._linear(w.lm_head, x, self.logits[:n])
-        ops.argmax(self.logits[:n], self.next_token[:n])
+        logits, token = self.logits[:n - head], self.next_token[:n - head]
+        self._linear(w.lm_head, x[head:], logits)
+        ops.argmax(logits, token)
         if advance:
             self.tokens[:n].copy_(self.next_token[:n])
             self.row_pos[:n].add_(1)
@@ -378,11 +379,15 @@ class BatchDecoder:
         self.queue_rows(slots, positions, tokens)
         torch.cuda.current_stream(self.dev).synchronize()
 
-    def absorb(self, slots, positions, tokens) -> None:
+    def absorb(self, slots, positions, tokens, head=None) -> None:
         """Queues the rows (up to ``prompt_rows``, each sequence's in the order of their positions) and the step that appends
-        them to their sequences' KV pages; their logits are not wanted."""
+        them to their sequences' KV pages.  Logits are wanted of none of them, or of those from row ``head`` on (up to
+        ``max_rows``), which land in ``logits`` and ``next_token`` from row 0 on."""
+        n = len(slots)
+        if head is not None and not 0 < n - head <= self.max_rows:
+            raise ValueError(f"logits of {n - head} rows in a decoder of {self.max_rows}")
         self._queue(slots, positions, tokens, self.prompt_rows)
-        self._trunk(len(slots), False, head=False)
+        self._trunk(n, False, head)
 
     def queue_rows(self, slots, positions, tokens) -> None:
         """``set_rows`` without the wait, for a caller whose step follows on the same stream.  The rows go through the decoder's
@@ -451,23 +456,28 @@ class Batcher:
         return slot
 
     def _take_in(self, slot: int, first: int, ids) -> int:
-        """Runs the tokens ``ids`` at positions ``first``.. of a sequence through the decoder in chunks of its rows; returns
-        the number of rows of the last chunk.  The chunks follow one another on the stream without the host waiting for
-        any of them.  Only the last one has a row whose logits are read: the output head runs for it alone, and the rows
-        before it may go through the stack in wider chunks (a row's bits do not depend on the chunk it is in)."""
+        """Runs the tokens ``ids`` at positions ``first``.. of a sequence through the decoder in chunks; returns the number of
+        rows that got logits: what a whole number of ``max_rows`` leaves of them, or ``max_rows``.  The chunks follow one another
+        on the stream without the host waiting for any of them, and may be wider than a step (a row's bits do not depend on
+        the chunk it is in); the output head runs for the rows that get logits alone."""
         d = self.d
         last = (len(ids) - 1) // d.max_rows * d.max_rows
         lo = 0
         while lo < len(ids):
-            chunk = ids[lo:lo + d.max_rows] if lo == last or self._absorb is None else ids[lo:min(last, lo + d.prompt_rows)]
-            rows = [slot] * len(chunk), range(first + lo, first + lo + len(chunk)), chunk
-            if lo < last and self._absorb is not None:
-                self._absorb(*rows)
+            if self._absorb is None:
+                hi = min(len(ids), lo + d.max_rows)
+            elif len(ids) - lo <= d.prompt_rows:
+                hi = len(ids)
+            else:
+                hi = min(last, lo + d.prompt_rows)
+            rows = [slot] * (hi - lo), range(first + lo, first + hi), ids[lo:hi]
+            if self._absorb is not None:
+                self._absorb(*rows, last - lo if hi == len(ids) else None)
             else:
                 self._rows(*rows)
-                d.run("verify", len(chunk), graph=False)
-            lo += len(chunk)
-        return len(chunk)
+                d.run("verify", hi - lo, graph=False)
+            lo = hi
+        return len(ids) - last
 
     def retire(self, slot: int) -> None:
         self.sync_tokens()
