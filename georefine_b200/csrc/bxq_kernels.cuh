@@ -800,8 +800,8 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           sts32(smem + L::misc + at, 0);
         }
         args.counters[d.y] = 0;
+        __threadfence();
       }
-      __threadfence();
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_final);
