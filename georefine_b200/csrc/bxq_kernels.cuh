@@ -776,6 +776,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       }
       if (!live) break;
       if (item.parts > 1) {
+        fence_proxy_async_all();   // the tile, written by ordinary stores, is read by bulk copies
         __threadfence();
         named_barrier(1, 128);
         if (e == 0 && lane == 0) {
@@ -835,6 +836,9 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   if (MODE == kUmma && args.cluster <= 1 && (warp < kDecoderWarps || warp >= kWideWarpSlices)) {
     const uint32_t ring = smem + NB * BXR_ROWS * 4;
     bool live = ctx.wait(bar_final, 0);
+    // Bulk copies read tiles that other CTAs stored, and write over turn-around buffers that this CTA's epilogue stored: ordinary
+    // stores of others, which the barrier and the counter order before here, and this before the copies.
+    if (warp == kWideWarpSlices) fence_proxy_async_all();
     uint32_t n = 0;
 #pragma unroll 1
     for (uint32_t at = 32; at >= 16; at -= 16) {
