@@ -75,11 +75,11 @@ struct BxqSmem {
   static constexpr uint32_t in = turn + 4 * kTurn;
   static constexpr uint32_t bars = in + kIn * BXQ_BLOB_MAX;
   // barrier order: in_full, in_empty [kIn each]; op_full, op_empty [kOp each]; x_full [kX]; x_empty [kX, if kXOwn];
-  // acc_full, acc_empty [2 each]; final; slice_full, slice_used [kSlices each], swap_used, swap_full (the closing reduction)
+  // acc_full, acc_empty [2 each]; final; slice_full, slice_used [kSlices each], swap_used, swap_full (the closing reduction); meet (the epilogue warps)
   // the closing reduction: the CTA's own tile of NB batch rows, and slices of kSliceRows batch rows of the others' on their way
   static constexpr uint32_t kSliceRows = T * NB <= 128 ? NB : 64, kSlice = kSliceRows * BXR_ROWS * 4;
   static constexpr uint32_t kSlicesFit = MODE == kUmma ? (bars - NB * 512u) / kSlice : 0, kSlices = kSlicesFit > 8 ? 8 : kSlicesFit;
-  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + (kXOwn ? 2 : 1) * kX + 4 + 1 + 2 * kSlices + 2;
+  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + (kXOwn ? 2 : 1) * kX + 4 + 1 + 2 * kSlices + 3;
   static constexpr uint32_t misc = (bars + 8 * nbars + 15) & ~15u;  // tmem base, abort flag, decision
   static constexpr uint32_t total = misc + 48;
   static constexpr uint32_t alloc = total + 1024;
@@ -235,7 +235,7 @@ __device__ __forceinline__ void bxq_add_tiles(const BxrArgs& args, const RoleCtx
       uint32_t src = smem + (m0 - m_at) * BXR_ROWS * 4;
       const uint32_t b = n % L::kSlices;
       if (p != own) {
-        if (!ctx.wait(bar_full + 8 * b, (n / L::kSlices) & 1)) return;
+        if (!ctx.wait_warp(bar_full + 8 * b, (n / L::kSlices) & 1)) return;
         src = ring + b * L::kSlice;
       }
 #pragma unroll
@@ -307,7 +307,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   const uint32_t bar_x_empty = L::kXOwn ? bar_x_full + 8 * L::kX : bar_op_empty;   // (rings of one length: stage i of both is free together)
   const uint32_t bar_acc_full = bar_x_full + 8 * L::kX * (L::kXOwn ? 2 : 1), bar_acc_empty = bar_acc_full + 16, bar_final = bar_acc_empty + 16;
   const uint32_t bar_slice_full = bar_final + 8, bar_slice_used = bar_slice_full + 8 * L::kSlices;
-  const uint32_t bar_swap_used = bar_slice_used + 8 * L::kSlices, bar_swap_full = bar_swap_used + 8;
+  const uint32_t bar_swap_used = bar_slice_used + 8 * L::kSlices, bar_swap_full = bar_swap_used + 8, bar_meet = bar_swap_full + 8;
   constexpr uint32_t kTmemCols = kWideTmemCols;
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;
   constexpr uint32_t kXN = L::kX ? L::kX : 1;
@@ -374,7 +374,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       if (n >= uint32_t(L::kIn) && n < 2u * L::kIn) count = kDecoderWarps;          // in_empty
       else if (n >= 2u * L::kIn && n < 2u * L::kIn + L::kOp) count = kDecoderWarps * kCtas;  // op_full
       else if (n >= 2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX) {
-        const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX);  // acc_full x2, acc_empty x2, final, slice_full, slice_used, swap_used, swap_full
+        const uint32_t j = n - (2u * L::kIn + 2 * L::kOp + (L::kXOwn ? 2 : 1) * L::kX);  // acc_full x2, acc_empty x2, final, slice_full, slice_used, swap_used, swap_full, meet
         count = j < 2 ? 1u : j < 4 ? 4u * kCtas : j < 5 ? 4u : j < 5 + L::kSlices ? 1u : j < 6 + 2 * L::kSlices ? uint32_t(kDecoderWarps) : 4u;
       }
       mbar_init(ctx.bars + 8 * n, count);
@@ -436,7 +436,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t base2 = next_base * 0x00800080u;
       if (u < unit_end) next_base = args.base[row + group * BXR_ROWS];  // the next item's base: on its way while this item is decoded
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
-        if (!ctx.wait(bar_in_full + 8 * s, ph)) { live = false; break; }
+        // (one verdict per warp without a vote of its own: a lane whose wait ran out goes on with what is in the slot - every
+        // read stays inside it - to where the warp comes together anyway.  The same below: a stage written too early spoils
+        // sums that nobody may use.)
+        bool ok = ctx.wait(bar_in_full + 8 * s, ph);
         const uint32_t blob = smem + L::in + s * BXQ_BLOB_MAX;
         uint32_t w[4];
 #pragma unroll
@@ -453,15 +456,17 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           const uint32_t v = lds32(blob + BXQ_LIST_AT + 4 * i);
           if (((v >> 5) & 31u) == uint32_t(lane)) bxq_patch(out, v & 31u, v >> 16);
         }
-        __syncwarp();   // every lane has what it needs from the blob: hand the slot back
+        live = __all_sync(0xFFFFFFFFu, ok);   // every lane has what it needs from the blob: hand the slot back
+        if (!live) break;
         if (lane == 0) mbar_arrive(bar_in_empty + 8 * s);
         if (MODE == kUmma) {
-          if (!ctx.wait(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
+          ok = ctx.wait(bar_op_empty + 8 * so, pho ^ 1);
           tc_fence_after();
           tmem_st16(tmem_base + operand_at + so * 64, out);
           tmem_st_wait();
           tc_fence_before();
-          __syncwarp();
+          live = __all_sync(0xFFFFFFFFu, ok);
+          if (!live) break;
           if (lane == 0) {
             if (leader) mbar_arrive(bar_op_full + 8 * so);
             else mbar_arrive_cluster(op_full_at + 8 * so);
@@ -507,7 +512,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           continue;
         }
         const uint32_t bytes = (b1 - b0) << 4;
-        if (ctx.aborted() || !ctx.wait(bar_in_empty + 8 * s, ph ^ 1)) { live = false; break; }
+        if (!ctx.go_warp(bar_in_empty + 8 * s, ph ^ 1)) { live = false; break; }
         if (b1 < b0 || bytes > BXQ_BLOB_MAX || bytes < BXQ_LIST_AT) {
           ctx.abort(kStatusBadArgument);
           live = false;
@@ -580,7 +585,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t drained = (acc_use(n_item) & 1) ^ 1;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end && live; ++c) {
         const bool first = c == item.chunk_begin, last = c + 1 == item.chunk_end;
-        if (first && !__all_sync(0xFFFFFFFFu, !ctx.aborted() && ctx.wait(bar_acc_empty + 8 * acc_slot(n_item, 0), drained))) { live = false; break; }
+        if (first && !ctx.go_warp(bar_acc_empty + 8 * acc_slot(n_item, 0), drained)) { live = false; break; }
         if (!ctx.wait_warp(bar_x_full + 8 * sx, phx) || !ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
         const uint32_t a_tmem = tmem_base + kOperandCol + so * 64;
 #pragma unroll
@@ -617,7 +622,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     const uint32_t e = warp - kWideWarpEpilogue;  // == warp % 4: the TMEM lane quarter this warp may read
     const uint32_t r = e * 32 + lane;
     const uint32_t acc_empty_at = PAIR ? cluster_map(bar_acc_empty, my_rank & ~1u) : bar_acc_empty;   // the issuer's
-    uint32_t n_item = 0;
+    uint32_t n_item = 0, met = 0;
     bool live = true;
     // Split row blocks that this CTA is the last to declare, and so adds up: that of its last item (misc + 16) and that of its
     // first (misc + 32), as {1 | (index + 1 of the tile kept in shared memory) << 8, row block, first slot, parts}.
@@ -637,10 +642,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       // CTA can be part of a split row block.
       const bool in_cluster = args.cluster > 1;  // the CTA's one item is a part of its cluster's row block
       const bool keep = item.parts > 1 && (it + 1 == item_end || in_cluster);
-      if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * acc_slot(n_item, 0), acc_use(n_item) & 1)) { live = false; break; }
+      if (!ctx.go_warp(bar_acc_full + 8 * acc_slot(n_item, 0), acc_use(n_item) & 1)) { live = false; break; }
       if (keep) {
         // (the second tile's last multiply may still be reading the activations in whose place the first one goes)
-        if (T == 2 && !ctx.wait(bar_acc_full + 8, acc_use(n_item) & 1)) { live = false; break; }
+        if (T == 2 && !ctx.wait_warp(bar_acc_full + 8, acc_use(n_item) & 1)) { live = false; break; }
         tc_fence_after();
         // A row block's counter: parts declared in the low half, parts in memory in the high half.
         uint32_t declared = 0;
@@ -652,7 +657,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           drain_to_smem(n_item, 0, smem);
           if (e == 0 && lane == 0) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(declared) : "memory");
           fence_proxy_async_smem();  // the tile may leave through a bulk copy
-          named_barrier(1, 128);
+          if (!ctx.meet(bar_meet, met)) { live = false; break; }
           asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(declared) : "r"(smem + L::misc + 8));
           if (declared == item.parts - 1) {   // (T = 2: the second tile waits in tensor memory until the first has been added)
             if (e == 0 && lane == 0) decide(16, item.part + 1u, item);
@@ -660,7 +665,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
             if (T == 2) {
               drain_to_smem(n_item, 1, smem + NB * BXR_ROWS * 4);
               fence_proxy_async_smem();
-              named_barrier(1, 128);
+              if (!ctx.meet(bar_meet, met)) { live = false; break; }
             }
             if (e == 0 && lane == 0) {
               bulk_s2g(args.partials + size_t(item.slot) * T * NB * BXR_ROWS, smem, ((args.m + 7) & ~7u) * BXR_ROWS * 4);
@@ -684,7 +689,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
 #pragma unroll 1
       for (uint32_t t = 0; t < uint32_t(T); ++t) {
         if (t) {
-          if (!ctx.wait(bar_acc_full + 8 * acc_slot(n_item, t), acc_use(n_item) & 1)) { live = false; break; }
+          if (!ctx.wait_warp(bar_acc_full + 8 * acc_slot(n_item, t), acc_use(n_item) & 1)) { live = false; break; }
           tc_fence_after();
         }
         const uint32_t taddr = tmem_base + ((e * 32) << 16) + acc_slot(n_item, t) * NB, m_at = t * NB, mcols = wide_tile_cols(args.m, t, NB);
@@ -778,7 +783,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       if (item.parts > 1) {
         fence_proxy_async_all();   // the tile, written by ordinary stores, is read by bulk copies
         __threadfence();
-        named_barrier(1, 128);
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }
         if (e == 0 && lane == 0) {
           const uint32_t before = atomicAdd(args.counters + item.row_block, 0x10001u);
           if ((before & 0xFFFFu) == item.parts - 1) decide(32, 0, item);
@@ -813,7 +818,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     // barrier makes the tiles visible to the peers, the second one keeps every CTA's shared memory alive until the
     // peers have read it.  Every thread of every CTA gets here on every path (all other waits are bounded).
     const bool worker_thread = warp < kDecoderWarps || warp >= kWideWarpEpilogue;
-    const bool drained = worker_thread ? ctx.wait(bar_final, 0) : true;
+    const bool drained = worker_thread ? ctx.wait_warp(bar_final, 0) : true;
     __syncwarp();
     cluster_sync();
     if (worker_thread && drained && unit_count) {
@@ -835,7 +840,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   // Row blocks that fell to this CTA are added up: warp kWideWarpSlices brings the others' tiles in, the decoder warps add.
   if (MODE == kUmma && args.cluster <= 1 && (warp < kDecoderWarps || warp >= kWideWarpSlices)) {
     const uint32_t ring = smem + NB * BXR_ROWS * 4;
-    bool live = ctx.wait(bar_final, 0);
+    bool live = ctx.wait_warp(bar_final, 0);
     // Bulk copies read tiles that other CTAs stored, and write over turn-around buffers that this CTA's epilogue stored: ordinary
     // stores of others, which the barrier and the counter order before here, and this before the copies.
     if (warp == kWideWarpSlices) fence_proxy_async_all();
@@ -852,9 +857,9 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           if (warp < kDecoderWarps) {
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_swap_used);
-            live = live && ctx.wait(bar_swap_full, 0);
+            live = live && ctx.wait_warp(bar_swap_full, 0);
           } else if (warp >= kWideWarpEpilogue) {
-            live = __all_sync(0xFFFFFFFFu, live && ctx.wait(bar_swap_used, 0));
+            live = live && ctx.wait_warp(bar_swap_used, 0);
             if (live) drain_to_smem(0, t, smem);
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_swap_full);

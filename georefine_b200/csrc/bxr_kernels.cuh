@@ -95,7 +95,7 @@ struct BxrSmem {
   static constexpr uint32_t xf32 = segoff + kIn * kSegOffBytes;
   static constexpr uint32_t bars = (xf32 + kIn * kXStage + 15) & ~15u;
   // barrier order: in_full, in_ready, in_empty [kIn each]; op_full, op_empty [kOp each]; acc_full, acc_empty [2 each]
-  static constexpr uint32_t nbars = 3 * kIn + 2 * kOp + 4 + 2;  // + the table's arrival barrier, + the final decision
+  static constexpr uint32_t nbars = 3 * kIn + 2 * kOp + 4 + 3;  // + the table's arrival barrier, the final decision, the meeting of four warps
   static constexpr uint32_t misc = (bars + 8 * nbars + 15) & ~15u;  // tmem base, abort flag, reduce flag, spare
   static constexpr uint32_t red = misc + 48;          // GEMV: FP32 [4 phases][128 rows][8]
   static constexpr uint32_t total = red + (MODE == kGemv ? 4 * 128 * kGemvMaxM * 4 : 0);
@@ -132,6 +132,17 @@ struct RoleCtx {
   // where the barrier completes as the limit runs out, some lanes would go on, and wait for good for the others.
   __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity) const {
     return __all_sync(0xFFFFFFFFu, wait(bar, parity));
+  }
+  // A meeting of warps at `bar` (one arrival each; `met`: how often they have met there).  Unlike a named barrier it has a limit:
+  // a warp that gave up elsewhere does not hold the others for good.  False, in all lanes alike: unwind.
+  __device__ __forceinline__ bool meet(uint32_t bar, uint32_t& met) const {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+    return wait_warp(bar, met++ & 1);
+  }
+  // The go-ahead of a warp that first looks whether its CTA has given up.
+  __device__ __forceinline__ bool go_warp(uint32_t bar, uint32_t parity) const {
+    return __all_sync(0xFFFFFFFFu, !aborted() && wait(bar, parity));
   }
 };
 
@@ -296,7 +307,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   ctx.status = args.status;
   const uint32_t bar_in_full = ctx.bars, bar_in_ready = bar_in_full + 8 * L::kIn, bar_in_empty = bar_in_ready + 8 * L::kIn;
   const uint32_t bar_op_full = bar_in_empty + 8 * L::kIn, bar_op_empty = bar_op_full + 8 * L::kOp;
-  const uint32_t bar_acc_full = bar_op_empty + 8 * L::kOp, bar_acc_empty = bar_acc_full + 16, bar_lut = bar_acc_empty + 16, bar_final = bar_lut + 8;
+  const uint32_t bar_acc_full = bar_op_empty + 8 * L::kOp, bar_acc_empty = bar_acc_full + 16, bar_lut = bar_acc_empty + 16, bar_final = bar_lut + 8, bar_meet = bar_final + 8;
   constexpr uint32_t kTmemCols = (2 * NB < 32) ? 32 : 2 * NB;
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;  // ring length of the operand stages (unused outside kUmma)
 
@@ -318,6 +329,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     }
     mbar_init(bar_lut, 1);
     mbar_init(bar_final, 4);  // one arrival per epilogue warp once its items are done
+    mbar_init(bar_meet, 4);   // the epilogue warps (GEMV: the decoder warps of phase 0) meet here
     // flags: abort at misc + 4, decisions at misc + 8 and misc + 16 (misc + 0 receives the TMEM base address from the
     // allocating warp and is left alone here)
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 4), "r"(0u) : "memory");
@@ -353,7 +365,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     LaneDecoder d;
     d.lut = smem + L::lut;
     d.k = args.k;
-    uint32_t u = 0;
+    uint32_t u = 0, met = 0;
     // ring positions advance by increments (no division in the chunk loop); per-lane offsets are fixed
     uint32_t s = 0, ph = 0;                          // input ring slot of chunk u and its phase parity
     uint32_t so = atom % kOpN, pho = 0;              // operand ring stage of half-stage 2u + atom
@@ -363,7 +375,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     uint32_t st_at[4];                               // swizzled 16-byte positions of this lane's four stores
 #pragma unroll
     for (int i = 0; i < 4; ++i) st_at[i] = r * 128 + ((((q & 1) * 4 + i) ^ (r & 7)) << 4);
-    bool live = ctx.wait(bar_lut, 0);  // the slot records arrive by a bulk copy the loader issued first
+    bool live = ctx.wait_warp(bar_lut, 0);  // the slot records arrive by a bulk copy the loader issued first
     for (uint32_t it = item_begin; it < item_end && live; ++it) {
       const bxr_item item = args.items[it];
       const uint32_t row = item.row_block * BXR_ROWS + r;
@@ -375,13 +387,13 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       for (int m = 0; m < (MODE == kGemv ? kGemvMaxM : 1); ++m) acc[m] = 0.f;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c, ++u) {
         // in_ready is posted by the scanner after it has itself observed the blob's arrival (in_full)
-        if (!ctx.wait(bar_in_ready + 8 * s, ph)) { live = false; break; }
+        if (!ctx.wait_warp(bar_in_ready + 8 * s, ph)) { live = false; break; }
         const uint32_t blob = smem + L::in + s * BXR_BLOB_MAX;
         const uint32_t bounds = lds32_unaligned_pair(seg_at + s * kSegOffBytes);
         d.start_chunk(blob + BXR_WORDS_AT + 2 * (bounds & 0xFFFFu), blob + BXR_WORDS_AT + 2 * (bounds >> 16) - 2);
         uint32_t a_tile = 0;
         if (MODE == kUmma) {
-          if (!ctx.wait(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
+          if (!ctx.wait_warp(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
           a_tile = smem + L::op + so * L::kOpStage;
         }
         const uint4 raw_f = lds128(blob + raw_at);
@@ -482,7 +494,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         // phases of a row are added in phase order, parts of a row block in part order
         const uint32_t red = smem + L::red;
         const uint32_t n_item = it - item_begin;
-        if (!ctx.wait(bar_acc_empty, (n_item & 1) ^ 1)) break;  // previous item's sums have been read
+        if (!ctx.wait_warp(bar_acc_empty, (n_item & 1) ^ 1)) break;  // previous item's sums have been read
 #pragma unroll
         for (int m = 0; m < kGemvMaxM; ++m)
           if (m < NB) asm volatile("st.shared.f32 [%0], %1;" ::"r"(red + ((q * BXR_ROWS + r) * kGemvMaxM + m) * 4), "f"(acc[m]) : "memory");
@@ -490,7 +502,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         if (lane == 0) mbar_arrive(bar_acc_full);
         bool last_part = item.parts == 1;
         if (q == 0) {
-          if (!ctx.wait(bar_acc_full, n_item & 1)) break;
+          if (!ctx.wait_warp(bar_acc_full, n_item & 1)) break;
           float tot[kGemvMaxM];
 #pragma unroll
           for (int m = 0; m < kGemvMaxM; ++m) {
@@ -515,14 +527,14 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
               if (m < NB) args.partials[(size_t(item.slot) * kGemvMaxM + m) * BXR_ROWS + r] = tot[m];
             __threadfence();
           }
-          named_barrier(3, 128);
+          if (!ctx.meet(bar_meet, met)) break;
           if (item.parts > 1) {
             uint32_t prev = 0;
             if (warp == 0 && lane == 0) prev = atomicAdd(args.counters + item.row_block, 1u);
             prev = __shfl_sync(0xFFFFFFFFu, prev, 0);
             // warps 1..3 learn the decision through shared memory
             if (warp == 0 && lane == 0) asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(prev) : "memory");
-            named_barrier(3, 128);
+            if (!ctx.meet(bar_meet, met)) break;
             asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 8));
             last_part = prev == item.parts - 1;
             if (last_part) {
@@ -581,7 +593,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         const uint32_t u = u0 + i, s = u % L::kIn, ph = (u / L::kIn) & 1;
         const uint32_t b0 = __shfl_sync(0xFFFFFFFFu, i0, i), b1 = __shfl_sync(0xFFFFFFFFu, i1, i);
         uint32_t bytes = (b1 - b0) << 4;
-        if (ctx.aborted() || !ctx.wait(bar_in_empty + 8 * s, ph ^ 1)) { live = false; break; }
+        if (!ctx.go_warp(bar_in_empty + 8 * s, ph ^ 1)) { live = false; break; }
         if (b1 < b0 || bytes > BXR_BLOB_MAX || bytes < BXR_WORDS_AT) {
           ctx.abort(kStatusBadArgument);
           live = false;
@@ -609,7 +621,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const bxr_item item = args.items[it];
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c, ++u) {
         const uint32_t s = u % L::kIn, ph = (u / L::kIn) & 1;
-        if (ctx.aborted() || !ctx.wait(bar_in_full + 8 * s, ph)) { live = false; break; }
+        if (!ctx.go_warp(bar_in_full + 8 * s, ph)) { live = false; break; }
         const uint32_t blob = smem + L::in + s * BXR_BLOB_MAX;
         const uint4 cnt = lds128(blob + 16 * lane);  // this lane's 16 segment counts
         const uint32_t cw[4] = {cnt.x, cnt.y, cnt.z, cnt.w};
@@ -687,14 +699,14 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       const bxr_item item = args.items[it];
       const uint32_t buf = n_item & 1;
-      if (ctx.aborted() || !ctx.wait(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
+      if (!ctx.go_warp(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + buf * NB;
       uint32_t first = 1;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end && live; ++c, ++u)
         for (uint32_t a = 0; a < 2; ++a) {
           const uint32_t hs = 2 * u + a, so = hs % kOpN, pho = (hs / kOpN) & 1;
-          if (ctx.aborted() || !ctx.wait(bar_op_full + 8 * so, pho)) { live = false; break; }
+          if (!ctx.go_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
           tc_fence_after();
           if (lane == 0) {
             const uint32_t stage = smem + L::op + so * L::kOpStage;
@@ -716,13 +728,13 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     const uint32_t e = warp - kWarpEpilogue;  // == warp % 4: the TMEM lane quarter this warp may read
     const uint32_t r = e * 32 + lane;
     const uint32_t mcols = (args.m + 7) & ~7u;
-    uint32_t n_item = 0;
+    uint32_t n_item = 0, met = 0;
     bool live = true;
     grid_dependency_wait();  // bias, y, partial tiles and counters may belong to the previous kernel
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       const bxr_item item = args.items[it];
       const uint32_t buf = n_item & 1;
-      if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * buf, (n_item >> 1) & 1)) { live = false; break; }
+      if (!ctx.go_warp(bar_acc_full + 8 * buf, (n_item >> 1) & 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t row = item.row_block * BXR_ROWS + r;
       const uint32_t taddr = tmem_base + ((e * 32) << 16) + buf * NB;
@@ -749,12 +761,12 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
       if (item.parts > 1) {
         __threadfence();
-        named_barrier(1, 128);
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }
         if (e == 0 && lane == 0) {
           const uint32_t prev = atomicAdd(args.counters + item.row_block, 1u);
           asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(prev) : "memory");
         }
-        named_barrier(1, 128);
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }
         uint32_t prev;
         asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 8));
         if (prev == item.parts - 1) {  // every partial tile of this row block is in memory: add them in K order
@@ -770,7 +782,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           }
           if (e == 0 && lane == 0) args.counters[item.row_block] = 0;
         }
-        named_barrier(1, 128);  // the decision word may be rewritten
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }  // the decision word may be rewritten
       }
     }
     __syncwarp();
@@ -780,7 +792,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   // A row block whose last partial tile came from this CTA's final item is reduced by the 16 decoder warps and
   // the 4 epilogue warps together (20 warps instead of 4 on the critical tail of the kernel).
   if (MODE == kUmma && !args.raw && (warp < kDecoderWarps || warp >= kWarpEpilogue)) {
-    if (ctx.wait(bar_final, 0)) {
+    if (ctx.wait_warp(bar_final, 0)) {
       const uint4 decision = lds128(smem + L::misc + 16);  // {reduce?, row block, first slot, parts}
       if (decision.x)
         reduce_row_block<NB>(args, decision.y, decision.z, decision.w, warp < kDecoderWarps ? warp : warp - 4, kDecoderWarps + 4, lane);

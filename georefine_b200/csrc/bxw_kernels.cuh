@@ -40,8 +40,8 @@ struct BxwSmem {
   static constexpr uint32_t in = xs + kX * kXStage;
   static constexpr uint32_t bars = in + kIn * BXR_BLOB_MAX;
   // barrier order: in_full, in_empty [kIn each]; op_full, op_empty [kOp each]; x_full [kX]; acc_full, acc_empty
-  // [2 each]; final
-  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + kX + 4 + 1;
+  // [2 each]; final, meet
+  static constexpr uint32_t nbars = 2 * kIn + 2 * kOp + kX + 4 + 2;
   static constexpr uint32_t misc = (bars + 8 * nbars + 15) & ~15u;  // tmem base, abort flag, decision
   static constexpr uint32_t total = misc + 48;
   static constexpr uint32_t alloc = total + 1024;
@@ -118,7 +118,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   const uint32_t bar_in_full = ctx.bars, bar_in_empty = bar_in_full + 8 * L::kIn;
   const uint32_t bar_op_full = bar_in_empty + 8 * L::kIn, bar_op_empty = bar_op_full + 8 * L::kOp;
   const uint32_t bar_x_full = bar_op_empty + 8 * L::kOp;
-  const uint32_t bar_acc_full = bar_x_full + 8 * L::kX, bar_acc_empty = bar_acc_full + 16, bar_final = bar_acc_empty + 16;
+  const uint32_t bar_acc_full = bar_x_full + 8 * L::kX, bar_acc_empty = bar_acc_full + 16, bar_final = bar_acc_empty + 16, bar_meet = bar_final + 8;
   constexpr uint32_t kTmemCols = 4 * NB;  // {even, odd chunk accumulator} x two items in flight
   constexpr uint32_t kOpN = L::kOp ? L::kOp : 1;
   constexpr uint32_t kXN = L::kX ? L::kX : 1;
@@ -141,7 +141,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     if (i >= uint32_t(L::kIn) && i < 2u * L::kIn) count = kDecoderWarps;          // in_empty
     else if (i >= 2u * L::kIn && i < 2u * L::kIn + L::kOp) count = kDecoderWarps + 1;  // op_full: + the loader's go-ahead
     else if (i >= 2u * L::kIn + 2 * L::kOp + L::kX) {
-      const uint32_t j = i - (2u * L::kIn + 2 * L::kOp + L::kX);                  // acc_full x2, acc_empty x2, final
+      const uint32_t j = i - (2u * L::kIn + 2 * L::kOp + L::kX);                  // acc_full x2, acc_empty x2, final, meet
       count = j < 2 ? 2u : 4u;                                                   // both MMA issuers / the epilogue warps
     }
     if (i < L::nbars) mbar_init(ctx.bars + 8 * i, count);
@@ -186,7 +186,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t row = item.row_block * BXR_ROWS + r;
       const uint32_t base2 = uint32_t(args.base[row]) * 0x00800080u;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
-        if (!ctx.wait(bar_in_full + 8 * s, ph)) { live = false; break; }
+        if (!ctx.wait_warp(bar_in_full + 8 * s, ph)) { live = false; break; }
         const uint32_t blob = smem + L::in + s * BXR_BLOB_MAX;
         const uint32_t wa = lds32(blob + code_at), wb = lds32(blob + code_at + 4 * BXR_SEGMENTS),
                        wc = lds32(blob + code_at + 8 * BXR_SEGMENTS);
@@ -217,7 +217,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         }
         uint32_t a_tile = 0;
         if (MODE == kUmma) {
-          if (!ctx.wait(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
+          if (!ctx.wait_warp(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
           a_tile = smem + L::op + so * L::kOpStage + atom_at;
         }
 #pragma unroll
@@ -307,7 +307,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         const uint32_t u = u0 + i, s = u % L::kIn, ph = (u / L::kIn) & 1;
         const uint32_t b0 = __shfl_sync(0xFFFFFFFFu, i0, i), b1 = __shfl_sync(0xFFFFFFFFu, i1, i);
         const uint32_t bytes = (b1 - b0) << 4;
-        if (ctx.aborted() || !ctx.wait(bar_in_empty + 8 * s, ph ^ 1)) { live = false; break; }
+        if (!ctx.go_warp(bar_in_empty + 8 * s, ph ^ 1)) { live = false; break; }
         if (b1 < b0 || bytes > BXR_BLOB_MAX || bytes < BXW_LIST_AT) {
           ctx.abort(kStatusBadArgument);
           live = false;
@@ -373,13 +373,13 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       const bxr_item item = args.items[it];
       const uint32_t buf = n_item & 1;
-      if (ctx.aborted() || !ctx.wait(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
+      if (!ctx.go_warp(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + (2 * buf + parity) * NB;
       uint32_t accumulate = 0;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
         if (so == parity) {
-          if (!ctx.wait(bar_op_full + 8 * so, pho)) { live = false; break; }
+          if (!ctx.wait_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
           tc_fence_after();
           if (lane == 0) {
             const uint64_t adesc = umma_desc_sw128(smem + L::op + so * L::kOpStage), bdesc = umma_desc_sw128(smem + L::xs + sx * L::kXStage);
@@ -410,13 +410,13 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     const uint32_t e = warp - kWinWarpEpilogue;  // == warp % 4: the TMEM lane quarter this warp may read
     const uint32_t r = e * 32 + lane;
     const uint32_t mcols = (args.m + 7) & ~7u;
-    uint32_t n_item = 0, u_seen = 0;  // u_seen: chunks of this CTA before the current item
+    uint32_t n_item = 0, met = 0, u_seen = 0;  // u_seen: chunks of this CTA before the current item
     bool live = true;
     grid_dependency_wait();  // bias, y, partial tiles and counters may belong to the previous kernel
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       const bxr_item item = args.items[it];
       const uint32_t buf = n_item & 1;
-      if (ctx.aborted() || !ctx.wait(bar_acc_full + 8 * buf, (n_item >> 1) & 1)) { live = false; break; }
+      if (!ctx.go_warp(bar_acc_full + 8 * buf, (n_item >> 1) & 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t row = item.row_block * BXR_ROWS + r;
       const uint32_t taddr = tmem_base + ((e * 32) << 16) + 2 * buf * NB;
@@ -455,12 +455,12 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       if (lane == 0) mbar_arrive(bar_acc_empty + 8 * buf);
       if (item.parts > 1) {
         __threadfence();
-        named_barrier(1, 128);
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }
         if (e == 0 && lane == 0) {
           const uint32_t prev = atomicAdd(args.counters + item.row_block, 1u);
           asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(smem + L::misc + 8), "r"(prev) : "memory");
         }
-        named_barrier(1, 128);
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }
         uint32_t prev;
         asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(prev) : "r"(smem + L::misc + 8));
         if (prev == item.parts - 1) {  // every partial tile of this row block is in memory: add them in K order
@@ -476,7 +476,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           }
           if (e == 0 && lane == 0) args.counters[item.row_block] = 0;
         }
-        named_barrier(1, 128);  // the decision word may be rewritten
+        if (!ctx.meet(bar_meet, met)) { live = false; break; }  // the decision word may be rewritten
       }
     }
     __syncwarp();
@@ -486,7 +486,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   // A row block whose last partial tile came from this CTA's final item is reduced by the 16 decoder warps and
   // the 4 epilogue warps together.
   if (MODE == kUmma && (warp < kDecoderWarps || warp >= kWinWarpEpilogue)) {
-    if (ctx.wait(bar_final, 0)) {
+    if (ctx.wait_warp(bar_final, 0)) {
       const uint4 decision = lds128(smem + L::misc + 16);  // {reduce?, row block, first slot, parts}
       if (decision.x)
         reduce_row_block<NB>(args, decision.y, decision.z, decision.w, warp < kDecoderWarps ? warp : warp - 4, kDecoderWarps + 4, lane);

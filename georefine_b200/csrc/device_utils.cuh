@@ -355,8 +355,4 @@ __device__ __forceinline__ uint4 lds128_cluster(uint32_t a) {
   return v;
 }
 
-__device__ __forceinline__ void named_barrier(uint32_t id, uint32_t threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 }  // namespace grb
