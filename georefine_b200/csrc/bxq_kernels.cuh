@@ -427,19 +427,17 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     // this lane's 16 operand columns: lane = row, columns = its 32 weights inside the chunk's atom
     const uint32_t operand_at = ((rg * 32u) << 16) + kOperandCol + (q >> 1) * 32 + (q & 1) * 16;
     const uint32_t op_full_at = PAIR ? cluster_map(bar_op_full, my_rank & ~1u) : bar_op_full;   // the issuer's
-    bool live = true;
     uint32_t next_base = first_base;
-    for (uint32_t u = unit_begin; u < unit_end && live;) {
+    for (uint32_t u = unit_begin; u < unit_end;) {
       const WideSpan item = wide_span(u, unit_end, args.chunks);
       u += item.chunk_end - item.chunk_begin;
       const uint32_t row = (item.row_block * group + in_group) * BXR_ROWS + r;
       const uint32_t base2 = next_base * 0x00800080u;
       if (u < unit_end) next_base = args.base[row + group * BXR_ROWS];  // the next item's base: on its way while this item is decoded
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
-        // (one verdict per warp without a vote of its own: a lane whose wait ran out goes on with what is in the slot - every
-        // read stays inside it - to where the warp comes together anyway.  The same below: a stage written too early spoils
-        // sums that nobody may use.)
-        bool ok = ctx.wait(bar_in_full + 8 * s, ph);
+        // (On any content of the slot every read stays inside it, and a stage written too early spoils sums that nobody may use.
+        // Votes on these two waits: 34816 x 5120 at one row 42.5 -> 44.9 us.)
+        ctx.wait_or_go_on(bar_in_full + 8 * s, ph);
         const uint32_t blob = smem + L::in + s * BXQ_BLOB_MAX;
         uint32_t w[4];
 #pragma unroll
@@ -456,17 +454,15 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           const uint32_t v = lds32(blob + BXQ_LIST_AT + 4 * i);
           if (((v >> 5) & 31u) == uint32_t(lane)) bxq_patch(out, v & 31u, v >> 16);
         }
-        live = __all_sync(0xFFFFFFFFu, ok);   // every lane has what it needs from the blob: hand the slot back
-        if (!live) break;
+        __syncwarp();   // every lane has what it needs from the blob: hand the slot back
         if (lane == 0) mbar_arrive(bar_in_empty + 8 * s);
         if (MODE == kUmma) {
-          ok = ctx.wait(bar_op_empty + 8 * so, pho ^ 1);
+          ctx.wait_or_go_on(bar_op_empty + 8 * so, pho ^ 1);
           tc_fence_after();
           tmem_st16(tmem_base + operand_at + so * 64, out);
           tmem_st_wait();
           tc_fence_before();
-          live = __all_sync(0xFFFFFFFFu, ok);
-          if (!live) break;
+          __syncwarp();
           if (lane == 0) {
             if (leader) mbar_arrive(bar_op_full + 8 * so);
             else mbar_arrive_cluster(op_full_at + 8 * so);

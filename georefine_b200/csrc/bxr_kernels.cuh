@@ -123,10 +123,30 @@ struct RoleCtx {
   // (diagnostic only).
   __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity) const {
     if (mbar_wait(bar, parity, suspend)) return true;
+    ran_out(bar);
+    return false;
+  }
+  __device__ __forceinline__ void ran_out(uint32_t bar) const {
     asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u) : "memory");
     if ((atomicOr(status, kStatusTimeout) & kStatusTimeout) == 0)
       atomicOr(status, ((((bar - bars) >> 3) + 1u) & 0xFFu) << 8 | (blockIdx.x & 0xFFu) << 16);
-    return false;
+  }
+  // A bounded wait without a verdict: it ends when the phase is complete, when the CTA has given up or when the limit runs out, and
+  // the caller goes on in all three, with what is there.  For roles that stay in bounds on any data and that a vote per wait would
+  // slow down; none of their lanes leaves the others, and what they make after an abort nobody may use.
+  __device__ __forceinline__ void wait_or_go_on(uint32_t bar, uint32_t parity) const {
+    if (mbar_try_wait(bar, parity, suspend)) return;
+    const unsigned long long t0 = global_ns();
+    for (;;) {
+#pragma unroll 1
+      for (int i = 0; i < 64; ++i)
+        if (mbar_try_wait(bar, parity, suspend)) return;
+      if (aborted()) return;
+      if (global_ns() - t0 > kWaitLimitNs) {
+        ran_out(bar);
+        return;
+      }
+    }
   }
   // The same with one verdict for all lanes of a warp that goes on to elect one of them.  Every lane times its own wait:
   // where the barrier completes as the limit runs out, some lanes would go on, and wait for good for the others.

@@ -36,16 +36,10 @@ def test_a_warp_has_one_verdict_on_a_wait(path):
     text = path.read_text()
     kernel = text[text.index("_kernel(const BxrArgs args"):]
     single = _without(kernel, r"if \([^;{}]*lane == 0[^;{}]*\) \{")      # blocks of one lane have nobody to part from
-    lines = [line.strip() for line in single.splitlines()]
-    for i, line in enumerate(lines):
-        if not re.search(r"\bctx\.wait\(", line):
-            continue
-        # the lane goes on, whatever its verdict, to a vote that decides for the warp before anything else can end the loop
-        assert re.match(r"(bool )?ok = ctx\.wait\(", line), line
-        rest = lines[i + 1:]
-        vote = next(n for n, after in enumerate(rest) if "live = __all_sync(0xFFFFFFFFu, ok)" in after)
-        assert not any(re.search(r"\b(break|return|continue)\b", after.split("//")[0]) for after in rest[:vote])
-        assert rest[vote + 1].startswith("if (!live) break;")
+    assert "ctx.wait(" not in single
+    # a wait without a verdict: nobody leaves after it, so nobody parts
+    for line in re.findall(r".*wait_or_go_on.*", single):
+        assert re.match(r" +ctx\.wait_or_go_on\(.*\);$", line)
     helpers = (CSRC / "bxr_kernels.cuh").read_text()
     assert "return __all_sync(0xFFFFFFFFu, !aborted() && wait(bar, parity));" in helpers     # go_warp
     assert "return wait_warp(bar, met++ & 1);" in helpers                                    # meet
