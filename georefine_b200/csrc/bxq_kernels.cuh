@@ -629,6 +629,14 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     grid_dependency_wait();  // bias, y, partial tiles and counters may belong to the previous kernel
     bxr_item item = {};
     if (item_begin < item_end) item = args.items[item_begin];
+    // A row block's counter: parts declared in the low half, parts in memory in the high half.  A part may be declared by any CTA
+    // that runs, since it waits for nobody before the part is in memory, and the last to declare adds.  A first item with another
+    // after it is declared right here: declared with its tile, it was now and then the last of its row block, and its CTA added
+    // up two row blocks one after the other.  8704 x 5120 at 128 rows 25.7 -> 22.5 us, 5120 x 8704 26.4 -> 23.1, 4096 x
+    // 14336 30.3 -> 26.8.
+    const bool early = args.cluster <= 1 && item_end - item_begin > 1 && item.parts > 1;
+    uint32_t first_declared = 0;
+    if (early && e == 0 && lane == 0) first_declared = atomicAdd(args.counters + item.row_block, 1u);
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       if (it != item_begin) item = args.items[it];
       const uint32_t row = item.row_block * BXR_ROWS + r, row0 = item.row_block * BXR_ROWS + e * 32;
@@ -643,7 +651,6 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         // (the second tile's last multiply may still be reading the activations in whose place the first one goes)
         if (T == 2 && !ctx.wait_warp(bar_acc_full + 8, acc_use(n_item) & 1)) { live = false; break; }
         tc_fence_after();
-        // A row block's counter: parts declared in the low half, parts in memory in the high half.
         uint32_t declared = 0;
         if (!in_cluster && e == 0 && lane == 0) declared = atomicAdd(args.counters + item.row_block, 1u) & 0xFFFFu;   // (answer used after the drain)
         if (in_cluster) {
@@ -781,8 +788,8 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         __threadfence();
         if (!ctx.meet(bar_meet, met)) { live = false; break; }
         if (e == 0 && lane == 0) {
-          const uint32_t before = atomicAdd(args.counters + item.row_block, 0x10001u);
-          if ((before & 0xFFFFu) == item.parts - 1) decide(32, 0, item);
+          atomicAdd(args.counters + item.row_block, 1u << 16);
+          if ((first_declared & 0xFFFFu) == item.parts - 1) decide(32, 0, item);
         }
       }
     }

@@ -15,7 +15,7 @@ def _in_order(text, *parts):
 
 def test_partial_tiles_are_fenced_before_they_are_counted():
     epilogue = KERNEL[KERNEL.index("warp >= kWideWarpEpilogue) {\n    // ---"):]
-    _in_order(epilogue, "stg32(dst", "fence_proxy_async_all();", "__threadfence();", "0x10001u")     # stored tile by tile
+    _in_order(epilogue, "stg32(dst", "fence_proxy_async_all();", "__threadfence();", "1u << 16")     # stored tile by tile
     _in_order(epilogue, "drain_to_smem(n_item, 0, smem);", "fence_proxy_async_smem();", "bulk_s2g(")    # sent from shared memory
 
 
