@@ -275,6 +275,19 @@ __device__ __forceinline__ void bxq_add_tiles(const BxrArgs& args, const RoleCtx
     }
   }
 }
+// Waits until `tiles` parts of a row block are in memory and clears the block's counter.  All have been declared, by CTAs that
+// wait for nobody before they publish.  False if the limit ran out: the counter is then left as it is, since parts may still
+// be counted into it, and the host has to clear the workspace before the next launch over it.
+__device__ __forceinline__ bool bxq_parts_in_memory(const BxrArgs& args, const RoleCtx& ctx, uint32_t row_block, uint32_t tiles) {
+  const unsigned long long t0 = global_ns();
+  while ((ld_acquire_gpu(args.counters + row_block) >> 16) < tiles)
+    if (global_ns() - t0 > kWaitLimitNs) {
+      ctx.abort(kStatusTimeout);
+      return false;
+    }
+  args.counters[row_block] = 0;
+  return true;
+}
 // (batch rows of one accumulator tile that there are, in whole eights)
 __device__ __forceinline__ uint32_t wide_tile_cols(uint32_t m, uint32_t tile, uint32_t nb) { return (min(m - min(m, tile * nb), nb) + 7) & ~7u; }
 
@@ -800,15 +813,7 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       for (uint32_t at = 32; at >= 16; at -= 16) {
         const uint4 d = lds128(smem + L::misc + at);
         if (!d.x) continue;
-        const uint32_t tiles = d.w - (d.x >> 8 ? 1u : 0u);
-        const unsigned long long t0 = global_ns();
-        bool there = false;
-        while (live && !(there = (ld_acquire_gpu(args.counters + d.y) >> 16) >= tiles) && global_ns() - t0 <= kWaitLimitNs) {}
-        if (!there) {
-          ctx.abort(kStatusTimeout);
-          sts32(smem + L::misc + at, 0);
-        }
-        args.counters[d.y] = 0;
+        if (!bxq_parts_in_memory(args, ctx, d.y, d.w - (d.x >> 8 ? 1u : 0u))) sts32(smem + L::misc + at, 0);
         __threadfence();
       }
     }

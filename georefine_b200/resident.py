@@ -143,7 +143,7 @@ class ResidentWeight:
         self.max_m = 0
         self.workspace, self._outgrown = None, []
         sizes = [int(_native.lib().grb_bxr_workspace_bytes(ctypes.byref(h), m)) for m in (128, 129)]
-        counters = (int(h.row_blocks) * 4 + 255) & ~255
+        self._counter_bytes = counters = (int(h.row_blocks) * 4 + 255) & ~255
         # partial tiles of the widest passes of a batch above 128 rows, where they are larger than those of 128 rows
         self.wide_scratch_bytes = sizes[1] - counters if sizes[1] > sizes[0] else 0
         self.next_weight = None     # see then()
@@ -242,17 +242,19 @@ class ResidentWeight:
         return torch.cuda.current_stream(self.device).cuda_stream
 
     def decode(self, *, check=True):
-        """Dense BF16 [N, K] decoded from the image by the decode twin of the fused kernels."""
+        """Dense BF16 [N, K] decoded from the image by the decode twin of the fused kernels.  What it reports joins what the
+        status word already holds (an earlier product's timeout among it); ``check`` looks at this call's own report."""
         import torch
 
         out = torch.empty((self.N, self.K), device=self.device, dtype=torch.bfloat16)
-        self.status.zero_()
+        status = torch.zeros_like(self.status) if check else self.status
         with torch.cuda.device(self.device):
             st = _native.lib().grb_bxr_decode(self.image.data_ptr(), ctypes.byref(self.header), out.data_ptr(),
-                                              self.status.data_ptr(), self._stream())
+                                              status.data_ptr(), self._stream())
         _native.check(st, "grb_bxr_decode")
-        if check and self.status.item() != 0:
-            raise ValueError(f"resident decode reported status {self.status.item()}")
+        if check and status.item() != 0:
+            self.status |= status
+            raise ValueError(f"resident decode reported status {status.item()}")
         return out
 
     def _checked(self, x, y):
@@ -365,3 +367,14 @@ class ResidentWeight:
     def check_status(self) -> int:
         """Host read of the device status word (synchronises); 0 means every call since the last reset was clean."""
         return int(self.status.item())
+
+    def reset(self) -> None:
+        """After a nonzero ``check_status()``: waits for the device, then clears the counters of the scratch - a launch that gave
+        up may have counted parts that nobody added, and the next one would add tiles of it - and the status word."""
+        import torch
+
+        torch.cuda.synchronize(self.device)
+        for scratch in (self.workspace, *self._outgrown):
+            scratch[:self._counter_bytes].zero_()
+        self.status.zero_()
+        torch.cuda.synchronize(self.device)

@@ -213,7 +213,8 @@ int bxr_decode_host(const uint8_t* image, uint64_t image_bytes, uint16_t* words)
 
 /* Bytes of caller-owned device scratch the fused entry points need for this image and batch tile:
  * FP32 partial tiles of row blocks shared by several CTAs, preceded by one counter per row block.
- * The scratch must be zero-filled once after allocation; the kernels leave the counters at zero.
+ * The scratch must be zero-filled once after allocation; the kernels leave the counters at zero.  After a call that set
+ * GRB_STATUS_TIMEOUT they may not be: wait for the stream and zero the scratch again before its next use.
  * Scratch for max_m = 128 serves every larger batch, in passes of 128 rows over the weights; with scratch for max_m > 128
  * a 4-bit window image takes up to 192 rows per pass, or up to 384 where its row blocks are multiplied in pairs. */
 uint64_t grb_bxr_workspace_bytes(const bxr_header* header, uint32_t max_m);

@@ -13,3 +13,11 @@ def test_a_first_item_is_declared_when_its_cta_starts():
     assert before.index("grid_dependency_wait();") < before.index("first_declared = atomicAdd(")     # (the counters may be the launch before's)
     stored = loop[loop.index("stg32(dst"):]
     assert "atomicAdd(args.counters + item.row_block, 1u << 16);" in stored and "0x10001u" not in EPILOGUE
+
+
+def test_a_counter_is_cleared_only_when_all_its_parts_are_in_memory():
+    """A part published after the wait for it ran out would stay counted, and a later launch add its tile too early."""
+    assert KERNEL.count("args.counters[") == 1
+    wait = KERNEL[KERNEL.index("bool bxq_parts_in_memory("):]
+    wait = wait[:wait.index("\n}\n")]
+    assert wait.index("while ((ld_acquire_gpu(") < wait.index("return false;") < wait.index("args.counters[row_block] = 0;")
