@@ -21,3 +21,11 @@ def test_a_counter_is_cleared_only_when_all_its_parts_are_in_memory():
     wait = KERNEL[KERNEL.index("bool bxq_parts_in_memory("):]
     wait = wait[:wait.index("\n}\n")]
     assert wait.index("while ((ld_acquire_gpu(") < wait.index("return false;") < wait.index("args.counters[row_block] = 0;")
+
+
+def test_the_warp_that_asks_for_tiles_waits_for_them():
+    """(With the wait in the epilogue, a fence and a barrier stood between a tile's arrival and its copy: short launches got slower.)"""
+    assert "bxq_parts_in_memory(" not in EPILOGUE
+    closing = KERNEL[KERNEL.index("// Row blocks that fell to this CTA are added up"):]
+    asked = closing.index("if (warp == kWideWarpSlices && lane == 0)")
+    assert asked < closing.index("bxq_parts_in_memory(") < closing.index("bulk_g2s(") and "__threadfence" not in closing

@@ -21,4 +21,4 @@ def test_partial_tiles_are_fenced_before_they_are_counted():
 
 def test_slices_are_asked_for_after_a_fence():
     closing = KERNEL[KERNEL.index("// Row blocks that fell to this CTA are added up"):]
-    _in_order(closing, "bar_final, 0)", "fence_proxy_async_all();", "bulk_g2s(")
+    _in_order(closing, "bar_final, 0)", "bxq_parts_in_memory(", "fence_proxy_async_all();", "bulk_g2s(")
