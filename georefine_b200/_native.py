@@ -27,7 +27,7 @@ EXPORTS = (
     "bcx_encode", "bcx_frequencies", "bcx_decode", "bcx_decode_compact", "bcx_free", "bcx_pack6", "bcx_unpack6",
     "bcx_checkpoint", "grb_bctx_build_lookup", "grb_bctx_decode_words", "grb_bctx_magnitudes", "grb_bctx_frequencies", "grb_bctx_encode_stream",
     "grb_bctx_frame_words", "grb_bctx_pack_tables", "grb_bctx_decode_packed", "bxr_build", "bxr_free", "bxr_decode_host",
-    "bxr_validate", "bxr_layout_version", "grb_bxr_workspace_bytes", "grb_bxr_decode", "grb_bxr_gemm", "grb_bxr_gemv", "grb_bxr_gemm_next", "grb_bxr_gemm_partials", "grb_kernel_attributes",
+    "bxr_validate", "bxr_layout_version", "bxr_partition_version", "grb_bxr_workspace_bytes", "grb_bxr_decode", "grb_bxr_gemm", "grb_bxr_gemv", "grb_bxr_gemm_next", "grb_bxr_gemm_partials", "grb_kernel_attributes",
     "grb_static_scratch_bytes", "grb_bxr_gemv_static", "grb_dense_gemv_bf16", "grb_peer_control_bytes", "grb_peer_enable", "grb_peer_allreduce_bf16",
     "grb_peer_alloc", "grb_peer_free", "grb_peer_open", "grb_peer_close",
     "grb_rmsnorm_bf16", "grb_silu_mul_bf16", "grb_argmax_bf16", "grb_attn_decode_bf16",
@@ -98,8 +98,9 @@ def _declare(lib):
     lib.bxr_free.restype = None
     lib.bxr_decode_host.argtypes = [U8P, u64, U16P]
     lib.bxr_validate.argtypes = [U8P, u64]
-    lib.bxr_layout_version.argtypes = []
-    lib.bxr_layout_version.restype = u32
+    for version in (lib.bxr_layout_version, lib.bxr_partition_version):
+        version.argtypes = []
+        version.restype = u32
     lib.grb_bxr_workspace_bytes.argtypes = [ctypes.POINTER(BxrHeader), u32]
     lib.grb_bxr_workspace_bytes.restype = u64
     lib.grb_bxr_decode.argtypes = [VOIDP, ctypes.POINTER(BxrHeader), VOIDP, VOIDP, VOIDP]
@@ -131,7 +132,7 @@ def _declare(lib):
     lib.grb_peer_allreduce_bf16.argtypes = [VOIDP, ctypes.POINTER(VOIDP), ctypes.POINTER(VOIDP), u64, u32, u32, VOIDP, u64, u64, VOIDP, VOIDP]
     for name in EXPORTS:
         if name not in ("bcx_free", "bxr_free", "grb_bxr_workspace_bytes", "grb_static_scratch_bytes", "grb_peer_control_bytes",
-                        "bxr_layout_version"):
+                        "bxr_layout_version", "bxr_partition_version"):
             getattr(lib, name).restype = ci
 
 

@@ -530,6 +530,7 @@ bool image_is_well_formed(const uint8_t* img, uint64_t bytes) {
 extern "C" {
 
 uint32_t bxr_layout_version(void) { return BXR_LAYOUT_VERSION; }
+uint32_t bxr_partition_version(void) { return BXR_PARTITION_VERSION; }
 
 // 0 when the image is structurally sound (see image_is_well_formed), 1 otherwise.  Never throws, never reads outside
 // [image, image + image_bytes).

@@ -42,10 +42,14 @@
 #include <stdint.h>
 
 #define BXR_MAGIC 0x31525842u /* "BXR1" */
-/* Bumped whenever a blob layout, the work partition or the header changes: an image of another version is refused by
+/* Bumped whenever a blob layout or the header changes, or an image can no longer be cut as it was: an image of another version is refused by
  * bxr_validate (and by the disk cache, whose key includes it) instead of being streamed by kernels that no longer
  * understand it. */
 #define BXR_LAYOUT_VERSION 2u
+/* The rule by which bxr_build cuts the work of an image among its workers; bumped when a shape gets another partition (2: that of
+ * pairs).  Images cut by an earlier rule stay valid - their header says how they are cut - but their products have other
+ * last bits and speeds, so it is part of a cache's key. */
+#define BXR_PARTITION_VERSION 2u
 #define BXR_ROWS 128
 #define BXR_COLS 128
 #define BXR_PHASES 4       /* lanes per row: phase q owns chunk columns [32q, 32q+32) */

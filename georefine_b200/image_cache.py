@@ -7,7 +7,7 @@ that changes the content, writes renamed into place last, a completion marker, p
 "full" verification, a failed entry moved aside and never fatal) and spreads first-time conversion over CPU workers
 (``glc_serve/context_parallel_startup.py``).  This module does the same for resident images.
 
-Layout under the cache root, one entry per (source digest, shape, layout, workers, layout version of the library)::
+Layout under the cache root, one entry per (source digest, shape, layout, workers, layout and partition version of the library)::
 
     <root>/<key[:2]>/<key>.bxr        the image, written to <key>.bxr.partial-<host>-<pid>-<nonce> and renamed
     <root>/<key[:2]>/<key>.json       the entry's description, written last: its presence marks the entry complete
@@ -51,17 +51,28 @@ def default_cache_root() -> Path:
 
 
 def layout_version() -> int:
-    """The resident layout version of the loaded library: part of every key, so entries written by a build with
-    another blob layout or work partition are never looked at."""
+    """The resident layout version of the loaded library: part of every key, as ``partition_version`` is, so entries written
+    by a build with another blob layout or work partition are never looked at."""
     from . import _native
 
     return int(_native.lib().bxr_layout_version())
 
 
+def partition_version() -> int:
+    """The rule by which the loaded library cuts an image's work among its workers."""
+    from . import _native
+
+    return int(_native.lib().bxr_partition_version())
+
+
+def _description(source_sha256: str, shape, layout: str, workers: int) -> dict:
+    """What an entry is an entry of."""
+    return {"schema": SCHEMA, "cache_format": CACHE_FORMAT, "layout_version": layout_version(), "partition_version": partition_version(),
+            "source_sha256": source_sha256, "shape": [int(shape[0]), int(shape[1])], "layout": layout, "workers": int(workers)}
+
+
 def cache_key(source_sha256: str, shape, layout: str, workers: int) -> str:
-    material = {"schema": SCHEMA, "cache_format": CACHE_FORMAT, "layout_version": layout_version(),
-                "source_sha256": source_sha256, "shape": [int(shape[0]), int(shape[1])], "layout": layout,
-                "workers": int(workers)}
+    material = _description(source_sha256, shape, layout, workers)
     return hashlib.sha256(json.dumps(material, sort_keys=True, separators=(",", ":")).encode()).hexdigest()
 
 
@@ -108,10 +119,7 @@ class ImageCache:
                 self.stats["misses"] += 1
                 return None
             meta = json.loads(meta_path.read_text(encoding="utf-8"))
-            want = {"schema": SCHEMA, "cache_format": CACHE_FORMAT, "layout_version": layout_version(),
-                    "source_sha256": source_sha256, "shape": [int(shape[0]), int(shape[1])], "layout": layout,
-                    "workers": int(workers)}
-            for name, value in want.items():
+            for name, value in _description(source_sha256, shape, layout, workers).items():
                 if meta.get(name) != value:
                     raise ImageCacheError(f"description field {name} differs")
             if image_path.stat().st_size != meta.get("image_bytes"):
@@ -155,9 +163,7 @@ class ImageCache:
                 f.flush()
                 os.fsync(f.fileno())
             os.replace(partial, image_path)
-            meta = {"schema": SCHEMA, "cache_format": CACHE_FORMAT, "layout_version": int(h.layout_version),
-                    "source_sha256": source, "shape": list(shape),
-                    "layout": layout, "workers": workers, "mode": int(h.mode), "image_bytes": len(data),
+            meta = {**_description(source, shape, layout, workers), "mode": int(h.mode), "image_bytes": len(data),
                     "image_sha256": hashlib.sha256(data).hexdigest(), "coded_bytes": int(h.coded_bytes)}
             tmp = meta_path.with_name(meta_path.name + f".partial-{uuid.uuid4().hex[:8]}")
             tmp.write_text(json.dumps(meta, sort_keys=True), encoding="utf-8")

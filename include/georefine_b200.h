@@ -205,6 +205,9 @@ void bxr_free(void* p);
  * (gs/transcode_cache.py) before trusting them. */
 int bxr_validate(const uint8_t* image, uint64_t image_bytes);
 uint32_t bxr_layout_version(void);
+/* The rule by which bxr_build cuts an image's work among its workers.  Images cut by an earlier one stay valid; a cache that is to
+ * serve what bxr_build would make now keeps it in its key. */
+uint32_t bxr_partition_version(void);
 
 /* Host twin of the GPU decoder, used to bind an image to its source digest before upload (the check the
  * reference makes at cr/bitexact_context_gpu.py:104-105).  Runs bxr_validate first.  0 ok, 1 malformed image,
