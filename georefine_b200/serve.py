@@ -18,6 +18,7 @@ All per-sequence state is indexed by absolute position (KV pages), so a rewind i
 """
 from __future__ import annotations
 
+import inspect
 import math
 from dataclasses import dataclass, field
 
@@ -435,8 +436,10 @@ class Batcher:
         self.d, self.buckets = decoder, tuple(b for b in buckets if b <= decoder.max_rows)
         self.active = {}            # slot -> {"pos": position of the next input token, "tokens": generated so far}
         self._order, self._dirty = [], True
-        # (a decoder need not have these two: rows set and run step by step are the same rows)
+        # (a decoder need not have these: rows set and run step by step are the same rows, and so are the last rows of a
+        # prompt where ``absorb`` gives no logits)
         self._rows, self._absorb = getattr(decoder, "queue_rows", decoder.set_rows), getattr(decoder, "absorb", None)
+        self._absorb_head = self._absorb is not None and "head" in inspect.signature(self._absorb).parameters
 
     def admit(self, prompt_ids, *, sampler=None) -> int:
         """Processes a prompt and returns the sequence's slot; its first generated token is in ``active[slot]['tokens']``
@@ -462,17 +465,19 @@ class Batcher:
         the chunk it is in); the output head runs for the rows that get logits alone."""
         d = self.d
         last = (len(ids) - 1) // d.max_rows * d.max_rows
-        lo = 0
+        lo, head = 0, self._absorb is not None and self._absorb_head
         while lo < len(ids):
-            if self._absorb is None:
+            if self._absorb is None or (lo == last and not head):
                 hi = min(len(ids), lo + d.max_rows)
-            elif len(ids) - lo <= d.prompt_rows:
+            elif head and len(ids) - lo <= d.prompt_rows:
                 hi = len(ids)
             else:
                 hi = min(last, lo + d.prompt_rows)
             rows = [slot] * (hi - lo), range(first + lo, first + hi), ids[lo:hi]
-            if self._absorb is not None:
-                self._absorb(*rows, last - lo if hi == len(ids) else None)
+            if self._absorb is not None and hi < len(ids):
+                self._absorb(*rows)
+            elif head:
+                self._absorb(*rows, head=last - lo)
             else:
                 self._rows(*rows)
                 d.run("verify", hi - lo, graph=False)
