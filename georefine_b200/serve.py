@@ -385,7 +385,9 @@ class BatchDecoder:
         them to their sequences' KV pages.  Logits are wanted of none of them, or of those from row ``head`` on (up to
         ``max_rows``), which land in ``logits`` and ``next_token`` from row 0 on."""
         n = len(slots)
-        if head is not None and not 0 < n - head <= self.max_rows:
+        if head is not None and not 0 <= head < n:
+            raise ValueError(f"logits from row {head} on of {n} rows")
+        if head is not None and n - head > self.max_rows:
             raise ValueError(f"logits of {n - head} rows in a decoder of {self.max_rows}")
         self._queue(slots, positions, tokens, self.prompt_rows)
         self._trunk(n, False, head)

@@ -1,4 +1,6 @@
 """How a prompt's rows reach a decoder: whole ones of this package, and a user's own with fewer entry points (host only)."""
+import types
+
 import pytest
 
 from georefine_b200 import serve
@@ -41,3 +43,11 @@ def test_first_token_of_a_prompt(kind, length):
     if kind is ThreeArguments:      # as before: all but the last rows taken in, the last of them a step of their own
         last = (length - 1) // 8 * 8
         assert sum(d.absorbed) == last and d.runs == [("verify", length - last, False)]
+
+
+@pytest.mark.parametrize("rows,head", [(200, 0), (200, 71), (100, -5), (100, 100), (100, 101)])
+def test_absorb_refuses_rows_it_has_no_logits_for(rows, head):
+    # (200 rows fit the pass: nothing but the check of the head may refuse them)
+    d = types.SimpleNamespace(max_rows=128, prompt_rows=384)
+    with pytest.raises(ValueError, match="logits"):
+        serve.BatchDecoder.absorb(d, [0] * rows, range(rows), [1] * rows, head)
