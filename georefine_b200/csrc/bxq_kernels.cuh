@@ -539,13 +539,9 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     // of the stream will want first - the leading blobs of its CTAs w, w + workers, ... (consecutive in memory) - so
     // that they arrive during this launch's tail and the next launch's set-up.
     if (MODE == kUmma && args.next_blobs && lane == 0 && !ctx.aborted()) {
-      const uint32_t next_group = args.next_paired ? 2u : 1u, next_shares = args.next_workers / next_group;
-      const uint64_t next_units = uint64_t(args.next_row_blocks / next_group) * args.next_chunks;
       for (uint32_t w2 = worker; w2 < args.next_workers; w2 += args.workers) {
-        const uint32_t b0 = uint32_t(next_units * (w2 / next_group) / next_shares), b1 = uint32_t(next_units * (w2 / next_group + 1) / next_shares);
-        const uint32_t g = b0 / args.next_chunks, c = b0 - g * args.next_chunks;
-        const uint32_t first = (g * next_group + (args.next_paired ? w2 & 1u : 0u)) * args.next_chunks + c;
-        const uint32_t n = min(min(b1 - b0, uint32_t(kWideNextBlobs)), args.next_chunks - c);
+        uint32_t first;
+        const uint32_t n = bxr_leading_blobs(args.next_row_blocks, args.next_chunks, args.next_workers, args.next_paired, w2, kWideNextBlobs, &first);
         for (uint32_t b = 0; b < n; ++b) bulk_prefetch_l2(args.next_blobs + size_t(first + b) * args.next_blob_bytes, args.next_blob_bytes);
       }
     }

@@ -150,6 +150,28 @@ static inline int bxr_paired(uint32_t row_blocks, uint32_t chunks, uint32_t work
   return (uint64_t)row_blocks * chunks >= 8ull * workers;
 }
 
+/* The blobs that lie one after another in memory from the first of worker w's share on: *first is that one, and up to `most` of
+ * the share's are counted.  In the partition of pairs the share goes on in the row block after next, elsewhere in memory. */
+#ifdef __CUDACC__
+#define BXR_HOST_DEVICE __host__ __device__
+#else
+#define BXR_HOST_DEVICE
+#endif
+BXR_HOST_DEVICE static inline uint32_t bxr_leading_blobs(uint32_t row_blocks, uint32_t chunks, uint32_t workers, uint32_t paired, uint32_t w,
+                                                         uint32_t most, uint32_t* first) {
+  const uint32_t group = paired ? 2u : 1u, share = w / group, shares = workers / group;
+  const uint64_t units = (uint64_t)(row_blocks / group) * chunks;
+  const uint32_t begin = (uint32_t)(units * share / shares);
+  uint32_t n = (uint32_t)(units * (share + 1) / shares) - begin;
+  *first = begin;
+  if (paired) {
+    const uint32_t g = begin / chunks, c = begin - g * chunks;
+    *first = (g * 2 + (w & 1u)) * chunks + c;
+    if (n > chunks - c) n = chunks - c;
+  }
+  return n < most ? n : most;
+}
+
 /* Slot record of the pair table, 32 bits: n0[0,4) | bias[4,16) | n1[16,20) | freq[20,32).  freq <= 4095.
  * (record & 0x000F000F) * 128 is the pair of relative exponents in packed-BF16 position (an exception nibble is
  * stored as 0), freq is the top field, bias = (record >> 4) & 0xFFF. */
