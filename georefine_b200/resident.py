@@ -120,6 +120,18 @@ def decode_image_host(image) -> np.ndarray:
     return out
 
 
+def largest_block(sizes, device):
+    """Device memory of the first of the (falling) sizes that there is room for; None if there is none for any."""
+    import torch
+
+    for size in sizes:
+        try:
+            return torch.empty(size, device=device, dtype=torch.uint8)
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return None
+
+
 class ResidentWeight:
     kind = "bctx"
 
@@ -146,6 +158,9 @@ class ResidentWeight:
         self._counter_bytes = counters = (int(h.row_blocks) * 4 + 255) & ~255
         # partial tiles of the widest passes of a batch above 128 rows, where they are larger than those of 128 rows
         self.wide_scratch_bytes = sizes[1] - counters if sizes[1] > sizes[0] else 0
+        # the block sizes that make a difference: the partial tiles of passes of 384, 256 and 192 rows, as far as the image has them
+        row = int(h.partial_slots) * 512
+        self.wide_scratch_sizes = [rows * row for rows in (384, 256, 192) if 0 < rows * row <= self.wide_scratch_bytes]
         self.next_weight = None     # see then()
         self.reserve(max_m)
 
@@ -222,18 +237,11 @@ class ResidentWeight:
 
     def _lent_scratch(self, capturing: bool):
         """Partial tiles for one batch above 128 rows, from the stream's allocator and back to it after the call: all weights of
-        a stack share one block, and one graph's share a block of the graph's own pool.  None - the batch then runs in
-        passes of 128 rows - when there is no memory, or a capture that the allocator does not know of is under way, whose
-        graph could not keep the block."""
-        import torch
-
-        if not self.wide_scratch_bytes:
-            return None
-        try:
-            block = torch.empty(self.wide_scratch_bytes, device=self.device, dtype=torch.uint8)
-            return block if not capturing or _of_a_graph(block) else None
-        except torch.cuda.OutOfMemoryError:
-            return None
+        a stack share one block, and one graph's share a block of the graph's own pool.  Where the widest passes' do not fit
+        the memory, those of narrower ones are asked for.  None - the batch then runs in passes of 128 rows - when none do, or
+        a capture that the allocator does not know of is under way, whose graph could not keep the block."""
+        block = largest_block(self.wide_scratch_sizes, self.device)
+        return block if block is None or not capturing or _of_a_graph(block) else None
 
     # -- device entry points -------------------------------------------------------------------------
     def _stream(self):

@@ -25,7 +25,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import ops
-from .resident import ResidentWeight
+from .resident import ResidentWeight, largest_block
 
 PAGE = ops.PAGE
 # Rows of a prompt that go through the stack together: one pass over each weight and one set of the small
@@ -266,9 +266,11 @@ class BatchDecoder:
             if hasattr(w, "reserve"):
                 w.reserve(min(self.max_rows, 128))
         # Batches above 128 rows leave partial tiles behind inside a linear: one block for all of them, taken here, before
-        # anybody sizes anything else by the memory that is left (57 MB at the benchmark's shapes).
-        wide_bytes = max((w.wide_scratch_bytes for w in weights.linears() if type(w) is ResidentWeight), default=0)
-        self._partials = torch.empty(wide_bytes, device=self.dev, dtype=torch.uint8) if self.prompt_rows > 128 and wide_bytes else None
+        # anybody sizes anything else by the memory that is left (57 MB at the benchmark's shapes; where there is less, what
+        # narrower passes need).
+        sizes = [w.wide_scratch_sizes for w in weights.linears() if type(w) is ResidentWeight and w.wide_scratch_sizes]
+        sizes = sorted({max(s[min(i, len(s) - 1)] for s in sizes) for i in range(3) if sizes}, reverse=True)
+        self._partials = largest_block(sizes, self.dev) if self.prompt_rows > 128 else None
         self._staging, self._staged = [(torch.zeros(3, R, dtype=i32).pin_memory(), torch.cuda.Event()) for _ in range(STAGING)], 0
         self.graphs = {}
 
