@@ -818,12 +818,12 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint32_t row_block = (unit_begin / args.chunks) * group + in_group, t = (warp < kDecoderWarps ? warp : warp - 4) * 32 + lane;
       // (narrow tiles: a position a thread at most, and a shorter way through code that is read once a launch: 5120 x 5120 at
       // one row reads one position)
-      if (NB <= 32) bxq_reduce_in_cluster<PAIR, 8, 1>(args, row_block, smem, t);
-      else switch (args.cluster) {
-        case 2: bxq_reduce_in_cluster<PAIR, 2, 4>(args, row_block, smem, t); break;
-        case 3: bxq_reduce_in_cluster<PAIR, 3, 3>(args, row_block, smem, t); break;
-        case 4: bxq_reduce_in_cluster<PAIR, 4, 2>(args, row_block, smem, t); break;
-        default: if (!PAIR) bxq_reduce_in_cluster<PAIR, 8, 1>(args, row_block, smem, t);
+      if constexpr (NB <= 32) bxq_reduce_in_cluster<PAIR, 8, 1>(args, row_block, smem, t);
+      else if (args.cluster == 2) bxq_reduce_in_cluster<PAIR, 2, 4>(args, row_block, smem, t);
+      else if (PAIR || args.cluster == 3) bxq_reduce_in_cluster<PAIR, 3, 3>(args, row_block, smem, t);   // (pairs: clusters of two or three parts)
+      else if constexpr (!PAIR) {
+        if (args.cluster == 4) bxq_reduce_in_cluster<PAIR, 4, 2>(args, row_block, smem, t);
+        else bxq_reduce_in_cluster<PAIR, 8, 1>(args, row_block, smem, t);
       }
     }
     __syncwarp();

@@ -26,8 +26,9 @@ int cuda_status(cudaError_t e) { return e == cudaSuccess ? GRB_OK : GRB_ERR_CUDA
 uint32_t batch_tile(uint32_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128; }
 
 // Batches above 128 rows over 4-bit window images: a pass over the weights may take up to 192 rows, up to 384 by pairs of CTAs,
-// and costs little more than one of 128 (34816 x 5120: 58 us at 128 rows, 66 at 192, 77 at 256, 106 at 384).  Rows of the next pass when `left` are still to be multiplied and a pass may take `most`
-// (128, 192, 256 or 384).
+// and costs little more than one of 128 (34816 x 5120: 58 us at 128 rows; 72 at 192 by single CTAs; 66 at 192, 77 at 256 and
+// 106 at 384 by pairs).  Rows of the next pass when `left` are still to be multiplied and a pass may take `most` (128, 192,
+// 256 or 384).
 constexpr uint32_t kWideTile = 192, kPairTile = 384;
 uint32_t wide_pass_rows(uint32_t left, uint32_t most) {
   if (left <= most) return left;
@@ -208,7 +209,6 @@ int gemm_tile_pair(const BxrArgs& a, const void* x, int64_t ldx, cudaStream_t st
 // One pass over the weights: a.m rows of x.
 int gemm_pass(const BxrArgs& a, const void* x, int64_t ldx, cudaStream_t stream) {
   if (a.m > 128 && pairs(a)) {
-    if (a.m <= 128) return gemm_tile_pair<128, 1>(a, x, ldx, stream);
     if (a.m <= 192) return gemm_tile_pair<192, 1>(a, x, ldx, stream);
     if (a.m <= 256) return gemm_tile_pair<128, 2>(a, x, ldx, stream);
     return gemm_tile_pair<192, 2>(a, x, ldx, stream);
