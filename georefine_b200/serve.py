@@ -30,7 +30,8 @@ from .resident import ResidentWeight, largest_block
 PAGE = ops.PAGE
 # Rows of a prompt that go through the stack together: one pass over each weight and one set of the small
 # kernels, for 60 MB of row buffers and 57 MB of partial tiles at the benchmark's shapes, whatever the number of layers.
-# 1000 tokens over four layers: 5.5 -> 4.8 ms with one pass for them instead of two.
+# 1000 tokens over four layers: 5.5 -> 4.8 ms with one pass for them instead of two, 4.3 ms since the rows after the last
+# full chunk go along.
 PROMPT_ROWS = 384
 STAGING = 4     # passes whose rows may be on their way to the device at a time
 
