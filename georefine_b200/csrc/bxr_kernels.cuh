@@ -103,6 +103,30 @@ struct BxrSmem {
   static_assert(alloc <= 232448, "exceeds the 227 KB of shared memory a CTA may opt into");
 };
 
+// The first wait of a launch to give up records where: bits 8..15 of the status word receive 1 + the barrier's index in the
+// kernel's barrier area, bits 16..23 the CTA (diagnostic only).  The CTA is marked aborted.
+__device__ __forceinline__ void wait_ran_out(uint32_t bar, uint32_t bars, uint32_t abort_addr, uint32_t* status) {
+  asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u) : "memory");
+  if ((atomicOr(status, kStatusTimeout) & kStatusTimeout) == 0)
+    atomicOr(status, ((((bar - bars) >> 3) + 1u) & 0xFFu) << 8 | (blockIdx.x & 0xFFu) << 16);
+}
+// A wait whose first probe has found the phase incomplete: until it is complete, the CTA has given up or the limit has run out.
+// Not inlined: copies of it in the decoders' loops cost more in instruction fetches than the call (34816 x 5120 at one row
+// 42.0 -> 40.9 us in the 4-bit layout, 59.3 -> 56.3 in the 3-bit one).
+__device__ __noinline__ void wait_or_abort(uint32_t bar, uint32_t parity, bool suspend, uint32_t abort_addr, uint32_t bars, uint32_t* status) {
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (mbar_try_wait(bar, parity, suspend)) return;
+    uint32_t aborted;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(aborted) : "r"(abort_addr));
+    if (aborted) return;
+    if (global_ns() - t0 > kWaitLimitNs) break;
+  }
+  wait_ran_out(bar, bars, abort_addr, status);
+}
+
 struct RoleCtx {
   uint32_t smem;       // aligned base (shared address)
   uint32_t bars;
@@ -118,35 +142,17 @@ struct RoleCtx {
     asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u) : "memory");
     atomicOr(status, bits);
   }
-  // Bounded wait; on expiry marks the CTA aborted.  The first wait of the launch to give up also records where:
-  // bits 8..15 of the status word receive 1 + the barrier's index in the kernel's barrier area, bits 16..23 the CTA
-  // (diagnostic only).
+  // Bounded wait; on expiry marks the CTA aborted.
   __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity) const {
     if (mbar_wait(bar, parity, suspend)) return true;
-    ran_out(bar);
+    wait_ran_out(bar, bars, abort_addr, status);
     return false;
-  }
-  __device__ __forceinline__ void ran_out(uint32_t bar) const {
-    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u) : "memory");
-    if ((atomicOr(status, kStatusTimeout) & kStatusTimeout) == 0)
-      atomicOr(status, ((((bar - bars) >> 3) + 1u) & 0xFFu) << 8 | (blockIdx.x & 0xFFu) << 16);
   }
   // A bounded wait without a verdict: it ends when the phase is complete, when the CTA has given up or when the limit runs out, and
   // the caller goes on in all three, with what is there.  For roles that stay in bounds on any data and that a vote per wait would
   // slow down; none of their lanes leaves the others, and what they make after an abort nobody may use.
   __device__ __forceinline__ void wait_or_go_on(uint32_t bar, uint32_t parity) const {
-    if (mbar_try_wait(bar, parity, suspend)) return;
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-#pragma unroll 1
-      for (int i = 0; i < 64; ++i)
-        if (mbar_try_wait(bar, parity, suspend)) return;
-      if (aborted()) return;
-      if (global_ns() - t0 > kWaitLimitNs) {
-        ran_out(bar);
-        return;
-      }
-    }
+    if (!mbar_try_wait(bar, parity, suspend)) wait_or_abort(bar, parity, suspend, abort_addr, bars, status);
   }
   // The same with one verdict for all lanes of a warp that goes on to elect one of them.  Every lane times its own wait:
   // where the barrier completes as the limit runs out, some lanes would go on, and wait for good for the others.
@@ -357,6 +363,9 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     for (int i = 1; i < 3; ++i) asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(smem + L::misc + 16 * i), "r"(0u) : "memory");
     mbar_fence_init();
   }
+  // A decoder that goes on after a wait ran out may meet offsets the scanner has not written yet.
+  if (warp != 0)
+    for (uint32_t i = threadIdx.x - 32; i < uint32_t(L::kIn) * kSegOffBytes / 16; i += blockDim.x - 32) sts128(smem + L::segoff + 16 * i, make_uint4(0, 0, 0, 0));
   if (MODE == kUmma && warp == kWarpMma) {
     tmem_alloc(smem + L::misc, kTmemCols);
     tmem_relinquish();
@@ -407,13 +416,14 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       for (int m = 0; m < (MODE == kGemv ? kGemvMaxM : 1); ++m) acc[m] = 0.f;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c, ++u) {
         // in_ready is posted by the scanner after it has itself observed the blob's arrival (in_full)
-        if (!ctx.wait_warp(bar_in_ready + 8 * s, ph)) { live = false; break; }
+        // (the slot's offsets are zero or the scanner's from some chunk: reads stay inside the shared memory whatever is in the slot)
+        ctx.wait_or_go_on(bar_in_ready + 8 * s, ph);
         const uint32_t blob = smem + L::in + s * BXR_BLOB_MAX;
         const uint32_t bounds = lds32_unaligned_pair(seg_at + s * kSegOffBytes);
         d.start_chunk(blob + BXR_WORDS_AT + 2 * (bounds & 0xFFFFu), blob + BXR_WORDS_AT + 2 * (bounds >> 16) - 2);
         uint32_t a_tile = 0;
         if (MODE == kUmma) {
-          if (!ctx.wait_warp(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
+          ctx.wait_or_go_on(bar_op_empty + 8 * so, pho ^ 1);
           a_tile = smem + L::op + so * L::kOpStage;
         }
         const uint4 raw_f = lds128(blob + raw_at);
@@ -507,8 +517,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         if (lane == 0) mbar_arrive(bar_in_empty + 8 * s);
         if (++s == L::kIn) { s = 0; ph ^= 1; }
       }
-      if (!live) break;
-      if (d.xf != BXR_STATE_LOW || d.xb != BXR_STATE_LOW) atomicOr(args.status, kStatusCheckpoint);
+      if ((d.xf != BXR_STATE_LOW || d.xb != BXR_STATE_LOW) && !ctx.aborted()) atomicOr(args.status, kStatusCheckpoint);
       if (MODE == kGemv) {
         if (it == item_begin) grid_dependency_wait();  // y, partial sums and counters
         // phases of a row are added in phase order, parts of a row block in part order
@@ -641,7 +650,7 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const bxr_item item = args.items[it];
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c, ++u) {
         const uint32_t s = u % L::kIn, ph = (u / L::kIn) & 1;
-        if (!ctx.go_warp(bar_in_full + 8 * s, ph)) { live = false; break; }
+        ctx.wait_or_go_on(bar_in_full + 8 * s, ph);
         const uint32_t blob = smem + L::in + s * BXR_BLOB_MAX;
         const uint4 cnt = lds128(blob + 16 * lane);  // this lane's 16 segment counts
         const uint32_t cw[4] = {cnt.x, cnt.y, cnt.z, cnt.w};
@@ -714,21 +723,22 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
   } else if (MODE == kUmma && warp == kWarpMma) {
     // ------------------------------------------------------------------ MMA issue
     constexpr uint32_t idesc = umma_idesc_bf16(NB);
-    uint32_t u = 0, n_item = 0;
-    bool live = true;
-    for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
-      const bxr_item item = args.items[it];
-      const uint32_t buf = n_item & 1;
-      if (!ctx.go_warp(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + buf * NB;
-      uint32_t first = 1;
-      for (uint32_t c = item.chunk_begin; c < item.chunk_end && live; ++c, ++u)
-        for (uint32_t a = 0; a < 2; ++a) {
-          const uint32_t hs = 2 * u + a, so = hs % kOpN, pho = (hs / kOpN) & 1;
-          if (!ctx.go_warp(bar_op_full + 8 * so, pho)) { live = false; break; }
-          tc_fence_after();
-          if (lane == 0) {
+    // (one lane, from end to end: nobody waits for it or it for others, so its waits need no vote)
+    if (lane == 0) {
+      uint32_t u = 0, n_item = 0;
+      bool live = true;
+      for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
+        const bxr_item item = args.items[it];
+        const uint32_t buf = n_item & 1;
+        if (ctx.aborted() || !ctx.wait(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * NB;
+        uint32_t first = 1;
+        for (uint32_t c = item.chunk_begin; c < item.chunk_end && live; ++c, ++u)
+          for (uint32_t a = 0; a < 2; ++a) {
+            const uint32_t hs = 2 * u + a, so = hs % kOpN, pho = (hs / kOpN) & 1;
+            if (ctx.aborted() || !ctx.wait(bar_op_full + 8 * so, pho)) { live = false; break; }
+            tc_fence_after();
             const uint32_t stage = smem + L::op + so * L::kOpStage;
             const uint64_t adesc = umma_desc_sw128(stage), bdesc = umma_desc_sw128(stage + kAtomBytes);
 #pragma unroll
@@ -738,10 +748,8 @@ bxr_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
             }
             umma_commit(bar_op_empty + 8 * so);
           }
-          __syncwarp();
-        }
-      if (live && lane == 0) umma_commit(bar_acc_full + 8 * buf);
-      __syncwarp();
+        if (live) umma_commit(bar_acc_full + 8 * buf);
+      }
     }
   } else if (MODE == kUmma && warp >= kWarpEpilogue) {
     // ------------------------------------------------------------------ TMEM -> y, or -> FP32 partial tile

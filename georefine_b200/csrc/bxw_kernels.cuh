@@ -180,13 +180,12 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     uint32_t st_at[4];         // swizzled 16-byte positions of this lane's four stores inside its atom
 #pragma unroll
     for (int i = 0; i < 4; ++i) st_at[i] = r * 128 + ((((q & 1) * 4 + i) ^ (r & 7)) << 4);
-    bool live = true;
-    for (uint32_t it = item_begin; it < item_end && live; ++it) {
+    for (uint32_t it = item_begin; it < item_end; ++it) {
       const bxr_item item = args.items[it];
       const uint32_t row = item.row_block * BXR_ROWS + r;
       const uint32_t base2 = uint32_t(args.base[row]) * 0x00800080u;
       for (uint32_t c = item.chunk_begin; c < item.chunk_end; ++c) {
-        if (!ctx.wait_warp(bar_in_full + 8 * s, ph)) { live = false; break; }
+        ctx.wait_or_go_on(bar_in_full + 8 * s, ph);   // (every read below stays inside the slot, whatever is in it)
         const uint32_t blob = smem + L::in + s * BXR_BLOB_MAX;
         const uint32_t wa = lds32(blob + code_at), wb = lds32(blob + code_at + 4 * BXR_SEGMENTS),
                        wc = lds32(blob + code_at + 8 * BXR_SEGMENTS);
@@ -217,7 +216,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
         }
         uint32_t a_tile = 0;
         if (MODE == kUmma) {
-          if (!ctx.wait_warp(bar_op_empty + 8 * so, pho ^ 1)) { live = false; break; }
+          ctx.wait_or_go_on(bar_op_empty + 8 * so, pho ^ 1);
           a_tile = smem + L::op + so * L::kOpStage + atom_at;
         }
 #pragma unroll
@@ -373,7 +372,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       const bxr_item item = args.items[it];
       const uint32_t buf = n_item & 1;
-      if (!ctx.go_warp(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
+      if (!ctx.wait_warp(bar_acc_empty + 8 * buf, ((n_item >> 1) & 1) ^ 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + (2 * buf + parity) * NB;
       uint32_t accumulate = 0;
@@ -416,7 +415,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     for (uint32_t it = item_begin; it < item_end && live; ++it, ++n_item) {
       const bxr_item item = args.items[it];
       const uint32_t buf = n_item & 1;
-      if (!ctx.go_warp(bar_acc_full + 8 * buf, (n_item >> 1) & 1)) { live = false; break; }
+      if (!ctx.wait_warp(bar_acc_full + 8 * buf, (n_item >> 1) & 1)) { live = false; break; }
       tc_fence_after();
       const uint32_t row = item.row_block * BXR_ROWS + r;
       const uint32_t taddr = tmem_base + ((e * 32) << 16) + 2 * buf * NB;
