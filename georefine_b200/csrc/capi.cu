@@ -478,6 +478,8 @@ static int check_linear(const void* image, const bxr_header* h, const void* x, i
   if (!image || !header_ok(h) || !x || !y || !status || !m) return GRB_ERR_ARGUMENT;
   if (ldx < int64_t(h->cols) || ldy < int64_t(h->rows) || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15))
     return GRB_ERR_ARGUMENT;
+  // (the 4-bit window kernel counts the parts of a row block in sixteen bits: 8.4 million columns, cut among as many workers)
+  if (h->mode == BXR_MODE_WINDOW4 && std::min(h->workers, h->chunks) > 0xFFFFu) return GRB_ERR_UNSUPPORTED;
   const uint64_t need = counter_bytes(h) + uint64_t(h->partial_slots) * tile_m * BXR_ROWS * 4;
   if (!ws || ws_bytes < need || (reinterpret_cast<uintptr_t>(ws) & 15)) return GRB_ERR_WORKSPACE;
   return GRB_OK;
