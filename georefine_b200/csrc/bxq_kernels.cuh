@@ -561,7 +561,8 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
       const uint64_t stay = l2_policy_evict_last();  // every CTA reads the same activation tiles
       const uint32_t x_full_at = PAIR ? cluster_map(bar_x_full, my_rank & ~1u) : bar_x_full;
       uint32_t c_v = unit_begin % args.chunks;  // the chunk (column block) to request next: wraps at the end of a row block
-      for (uint32_t v = 0; v < unit_count; ++v) {
+      uint32_t v = 0;
+      for (; v < unit_count; ++v) {
         const uint32_t sx = v % kXN, stage = smem + L::xs + sx * L::kXStage;
         if (ctx.aborted() || !ctx.wait(bar_x_empty + 8 * sx, ((v / kXN) & 1) ^ 1)) break;
         if (leader) mbar_arrive_expect_tx(bar_x_full + 8 * sx, L::kXStage * (PAIR ? 2 : 1));
@@ -576,6 +577,10 @@ bxq_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           }
         if (++c_v == args.chunks) c_v = 0;
       }
+      // after an abort: tiles on their way land before the CTA exits (of a pair, the issuer's barriers know of both halves, and
+      // its peer waits for it)
+      if (ctx.aborted() && leader)
+        for (uint32_t u = v > kXN ? v - kXN : 0; u < v; ++u) mbar_wait(bar_x_full + 8 * (u % kXN), (u / kXN) & 1);
     }
   } else if (MODE == kUmma && warp == kWideWarpMma) {
     // ------------------------------------------------------------------ MMA issue: eight per chunk and tile, then the stages go back

@@ -111,18 +111,23 @@ __device__ __forceinline__ void wait_ran_out(uint32_t bar, uint32_t bars, uint32
     atomicOr(status, ((((bar - bars) >> 3) + 1u) & 0xFFu) << 8 | (blockIdx.x & 0xFFu) << 16);
 }
 // A wait whose first probe has found the phase incomplete: until it is complete, the CTA has given up or the limit has run out.
+// After an abort it still takes a millisecond: the decoders are what keeps a CTA that gives up alive until the copies and multiplies
+// it has on their way (a few microseconds) have ended in its shared and tensor memory.
 // Not inlined: copies of it in the decoders' loops cost more in instruction fetches than the call (34816 x 5120 at one row
 // 42.0 -> 40.9 us in the 4-bit layout, 59.3 -> 56.3 in the 3-bit one).
 __device__ __noinline__ void wait_or_abort(uint32_t bar, uint32_t parity, bool suspend, uint32_t abort_addr, uint32_t bars, uint32_t* status) {
   const unsigned long long t0 = global_ns();
+  unsigned long long heard = 0;   // when the CTA was last seen not to have given up
   for (;;) {
 #pragma unroll 1
     for (int i = 0; i < 64; ++i)
       if (mbar_try_wait(bar, parity, suspend)) return;
     uint32_t aborted;
     asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(aborted) : "r"(abort_addr));
-    if (aborted) return;
-    if (global_ns() - t0 > kWaitLimitNs) break;
+    const unsigned long long waited = global_ns() - t0;
+    if (aborted && waited - min(waited, heard) > kLingerNs) return;
+    if (!aborted) heard = waited;
+    if (waited > kWaitLimitNs) break;
   }
   wait_ran_out(bar, bars, abort_addr, status);
 }

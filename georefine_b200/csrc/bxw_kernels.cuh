@@ -334,6 +334,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
     if (lane == 0) {
       grid_dependency_wait();
       bool live = true;
+      uint32_t asked = 0;                   // chunks whose tiles have been requested
       uint32_t it_v = item_begin, c_v = 0;  // cursor of the chunk to request: item and chunk inside it
       bxr_item item_v = args.items[item_begin < item_end ? item_begin : 0];
       c_v = item_v.chunk_begin;
@@ -346,6 +347,7 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           mbar_arrive_expect_tx(bar_x_full + 8 * sx, L::kXStage);
           tma_load_2d(stage, &tmap_x, int(c_v * BXR_COLS), 0, bar_x_full + 8 * sx);
           tma_load_2d(stage + NB * 128, &tmap_x, int(c_v * BXR_COLS + 64), 0, bar_x_full + 8 * sx);
+          asked = v + 1;
           if (++c_v == item_v.chunk_end && it_v + 1 < item_end) {
             item_v = args.items[++it_v];
             c_v = item_v.chunk_begin;
@@ -358,6 +360,8 @@ bxw_kernel(const BxrArgs args, const __grid_constant__ CUtensorMap tmap_x) {
           mbar_arrive(bar_op_full + 8 * (w % kOpN));
         }
       }
+      if (ctx.aborted())   // tiles on their way land before the CTA exits
+        for (uint32_t u = asked > kXN ? asked - kXN : 0; u < asked; ++u) mbar_wait(bar_x_full + 8 * (u % kXN), (u / kXN) & 1);
     }
   } else if (MODE == kUmma && (warp == kWinWarpMma || warp == kWinWarpMmaOdd)) {
     // ------------------------------------------------------------------ MMA issue: one wait, eight MMAs, one commit

@@ -20,6 +20,7 @@ enum : uint32_t {
 };
 
 constexpr unsigned long long kWaitLimitNs = 2000000000ull;  // 2 s
+constexpr unsigned long long kLingerNs = 1000000ull;         // 1 ms
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ unsigned long long global_ns() {

@@ -43,3 +43,16 @@ def test_a_warp_has_one_verdict_on_a_wait(path):
     helpers = (CSRC / "bxr_kernels.cuh").read_text()
     assert "return __all_sync(0xFFFFFFFFu, !aborted() && wait(bar, parity));" in helpers     # go_warp
     assert "return wait_warp(bar, met++ & 1);" in helpers                                    # meet
+
+
+@pytest.mark.parametrize("path", KERNELS, ids=lambda p: p.name)
+def test_a_cta_that_gives_up_outlives_its_copies(path):
+    """Decoders that no longer leave at the limit must not take the CTA to its end while its copies and multiplies are under way."""
+    helpers = (CSRC / "bxr_kernels.cuh").read_text()
+    wait = helpers[helpers.index("void wait_or_abort("):]
+    wait = wait[:wait.index("\n}\n")]
+    assert re.search(r"if \(aborted && [^;]*> kLingerNs\) return;", wait) and wait.count("return;") == 2     # (the other: the phase is complete)
+    text = path.read_text()
+    # blobs, and activation tiles that have barriers of their own, are waited for (an entropy-coded image's tiles share the operand stages')
+    waited = [bar for bar in ("bar_in_full", "bar_x_full") if f"mbar_wait({bar} + 8 * (u %" in text]
+    assert waited == (["bar_in_full"] if path.name == "bxr_kernels.cuh" else ["bar_in_full", "bar_x_full"])
